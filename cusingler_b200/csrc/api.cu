@@ -11,6 +11,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cmath>
+#include <cstddef>
 #include <map>
 #include <random>
 #include <set>
@@ -180,6 +181,31 @@ struct sgr_ctx {
     DevBuf<int32_t> d_final, d_rounds;
     DevBuf<unsigned long long> d_round_sum;  // profiling: fine-tune rounds of the listed cells
     DevBuf<float> ft_scratch;
+
+    // fine-tune by rounds (ft_rounds.cu): the reference rows in groups, laid out at training
+    int ft_copies = 0;             // table copies that fit shared memory (0: the work-queue form only)
+    int max_row = 0;               // longest thre-pool row of the reference
+    DevBuf<uint4> fr_groups;
+    DevBuf<int32_t> fr_blk_voff;
+    DevBuf<uint32_t> fr_perm, fr_pair_mask;
+    bool fr_masks = false;
+    // its per-call and per-batch buffers
+    DevBuf<int32_t> fr_cells;
+    DevBuf<int64_t> fr_blk_off;
+    DevBuf<uint16_t> fr_sorted;    // genes, run starts, run ends of the cells' rows
+    DevBuf<uint8_t> fr_top;
+    DevBuf<int> fr_ints;           // ntop, used, two active lists
+    DevBuf<FtCell> fr_par;
+    DevBuf<uint32_t> fr_eq, fr_ext;
+    DevBuf<FtEntry> fr_list;
+    DevBuf<FtQuad> fr_quads;
+    DevBuf<int2> fr_q_label;
+    DevBuf<unsigned long long> fr_un;  // active cells with their sort keys
+    DevBuf<int> fr_keys;           // counts of the sort keys
+    DevBuf<unsigned long long> fr_ctl;  // counters (FtCtl)
+    DevBuf<float> fr_scores, fr_nan;
+    unsigned long long* h_ft = nullptr;  // pinned: counters read back
+    cudaEvent_t ev_ft[2] = {nullptr, nullptr};
 
     // learned proposal
     Mlp mlp;
@@ -487,6 +513,53 @@ std::vector<int32_t> position_map(const std::vector<int32_t>& colmap, const std:
     return out;
 }
 
+// The reference's thre-pool rows as value-sorted groups in 32-row blocks for the fine-tune by rounds
+// (ft_rounds.cu), inside each label the rows with the most groups first, so that a block's rows are of
+// similar length.  fptr: the compacted rows' offsets; blk_base: first block of each label.
+void build_row_groups(sgr_ctx* ctx, const std::vector<int32_t>& fptr, const std::vector<int32_t>& blk_base) {
+    cudaStream_t s = ctx->stream;
+    const Markers& mk = ctx->mk;
+    ctx->ft_copies = ctx->pack_shift ? ft_scan_copies((int)std::max<uint32_t>(ctx->Wt, 1)) : 0;
+    if (!ctx->ft_copies) return;
+    const uint32_t R = ctx->R, L = mk.n_labels;
+    DevBuf<uint16_t> sorted;
+    DevBuf<int32_t> n_groups, d_slot;
+    sorted.ensure(std::max(fptr[R], 1));
+    n_groups.ensure(R);
+    launch_row_runs(ctx->reff_data.p, ctx->reff_indices.p, ctx->reff_indptr.p, R, ctx->max_row, sorted.p, n_groups.p, s);
+    std::vector<int32_t> ng(R);
+    SGR_CUDA(cudaMemcpyAsync(ng.data(), n_groups.p, R * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+    SGR_CUDA(cudaStreamSynchronize(s));
+    const int32_t n_blocks = blk_base[L];
+    std::vector<int32_t> slot_row((size_t)n_blocks * 32, -1), voff(n_blocks + 1, 0);
+    std::vector<uint32_t> perm(R), order;
+    int64_t at = 0;
+    for (uint32_t l = 0; l < L; ++l) {
+        const uint32_t start = mk.ctidx[2 * l], len = mk.ctidx[2 * l + 1];
+        order.resize(len);
+        for (uint32_t j = 0; j < len; ++j) order[j] = j;
+        std::stable_sort(order.begin(), order.end(),
+                         [&](uint32_t x, uint32_t y) { return ng[start + x] > ng[start + y]; });
+        for (uint32_t j = 0; j < len; ++j) {
+            perm[start + j] = order[j];
+            slot_row[(size_t)blk_base[l] * 32 + j] = (int32_t)(start + order[j]);
+            if (j % 32 == 0) {  // the block's first row is its longest
+                voff[blk_base[l] + j / 32] = (int32_t)at;
+                at += 32ll * ((ng[start + order[j]] + 1) / 2);
+                if (at > INT32_MAX) fail(SGR_ERR_UNSUPPORTED, "fine-tune reference lists exceed 2^31 vectors");
+            }
+        }
+    }
+    voff[n_blocks] = (int32_t)at;
+    ctx->fr_perm.upload(perm, s);
+    ctx->fr_blk_voff.upload(voff, s);
+    d_slot.upload(slot_row, s);
+    ctx->fr_groups.ensure(std::max<int64_t>(at, 1));
+    launch_row_groups(sorted.p, ctx->reff_indptr.p, d_slot.p, ctx->fr_blk_voff.p, (uint32_t)n_blocks * 32, ctx->Wt,
+                      ctx->fr_groups.p, s);
+    SGR_CUDA(cudaStreamSynchronize(s));  // the tables above are freed on return
+}
+
 void train(sgr_ctx* ctx, const sgr_csr* ref, const int32_t* celltypes, const char* const* label_names,
            uint32_t n_labels, const char* const* ref_genes, const char* const* qry_genes, uint32_t n_qry) {
     if (!ref || ref->on_device) fail(SGR_ERR_INVALID_ARGUMENT, "reference must be a host CSR");
@@ -615,6 +688,7 @@ void train(sgr_ctx* ctx, const sgr_csr* ref, const int32_t* celltypes, const cha
     {
         int64_t max_row = 1;
         for (uint32_t r = 0; r < ctx->R; ++r) max_row = std::max<int64_t>(max_row, fptr[r + 1] - fptr[r]);
+        ctx->max_row = (int)max_row;
         int cbits = 0;
         while ((int64_t(1) << cbits) <= max_row) ++cbits;
         const int shift = 32 - cbits;
@@ -625,6 +699,7 @@ void train(sgr_ctx* ctx, const sgr_csr* ref, const int32_t* celltypes, const cha
         ctx->pack_narrow = ctx->pack_shift > 0 && 4 * max_row * max_row * wt < (int64_t(1) << 32) &&
                            max_row * max_row * max_row < (int64_t(1) << 32);
     }
+    build_row_groups(ctx, fptr, blk_base);
     ctx->d_row_perm.upload(row_perm, s);
     ctx->d_blk_base.upload(blk_base, s);
     ctx->d_ell_off.upload(ell_off, s);
@@ -644,6 +719,20 @@ void train(sgr_ctx* ctx, const sgr_csr* ref, const int32_t* celltypes, const cha
     }
     ctx->d_ft_genes.upload(mk.ft_genes.empty() ? std::vector<uint32_t>{0} : mk.ft_genes, s);
     ctx->d_ft_idx.upload(mk.ft_idx, s);
+    // each pair's whole fine-tune list as bits over the pool (unless that takes over 256 MiB)
+    const size_t nwords = (std::max<size_t>(ctx->Wt, 1) + 31) / 32, mask_words = (size_t)mk.n_labels * mk.n_labels * nwords;
+    ctx->fr_masks = ctx->ft_copies && mask_words <= ((size_t)64 << 20);
+    if (ctx->fr_masks)
+        launch_pair_masks(ctx->d_ft_genes.p, ctx->d_ft_idx.p, (int)mk.n_labels, (int)nwords,
+                          ctx->fr_pair_mask.ensure(mask_words), s);
+    {
+        std::vector<int32_t> lorder(mk.n_labels);
+        for (uint32_t l = 0; l < mk.n_labels; ++l) lorder[l] = (int32_t)l;
+        std::stable_sort(lorder.begin(), lorder.end(),
+                         [&](int32_t x, int32_t y) { return mk.ctidx[2 * x + 1] > mk.ctidx[2 * y + 1]; });
+        ctx->d_lorder.upload(lorder, s);
+        SGR_CUDA(cudaStreamSynchronize(s));
+    }
     std::vector<int32_t> gt(mk.n_labels + 1, 0);
     for (uint32_t n = 1; n <= mk.n_labels; ++n) gt[n] = marker_count(n);
     ctx->d_gene_thre.upload(gt, s);
@@ -783,11 +872,6 @@ ScorePlan score_begin(sgr_ctx* ctx, const DevCsr& q, float p, float thre, const 
             if (ctx->h_ref_n2[r] == 0) lq[l].has_nan = 1, any_nan_ref = true;
     }
     ctx->lq.upload(lq, s);
-    std::vector<int32_t> lorder(L);
-    for (uint32_t l = 0; l < L; ++l) lorder[l] = (int32_t)l;
-    std::stable_sort(lorder.begin(), lorder.end(),
-                     [&](int32_t x, int32_t y) { return ctx->mk.ctidx[2 * x + 1] > ctx->mk.ctidx[2 * y + 1]; });
-    ctx->d_lorder.upload(lorder, s);
     for (uint32_t l = 0; l < L; ++l) pl.max_len = std::max(pl.max_len, ctx->mk.ctidx[2 * l + 1]);
     if (any_nan_ref) pl.scratch = ctx->sel_scratch.ensure((size_t)select_warps_with_scratch() * pl.max_len);
     ctx->label_scores.ensure((size_t)Q * L);
@@ -1149,6 +1233,200 @@ cudaStream_t side_stream(sgr_ctx* ctx) {
     return ctx->side;
 }
 
+// Counters of the fine-tune by rounds on the device.
+struct FtCtl {
+    unsigned long long counter, cand;  // cells to fine-tune << 36 | their score blocks; their candidates
+    int32_t total, longest;            // entries of their compacted rows; the longest row
+    int32_t n_act[2];                  // cells that go on (by the parity of the round)
+    unsigned long long stats[2];       // cell rounds, reference rows scored
+    int32_t queue[2];
+    int32_t n_list[2 * 256];
+};
+
+// Fine-tune by rounds over all cells (ft_rounds.cu), in exact mode; arguments as
+// finetune_persistent.  Returns false when a query row is too long for it.  A batch's rounds are queued one ahead of the
+// host: the count of active cells after step k is read while the scan of round k runs.
+bool finetune_rounds(sgr_ctx* ctx, const DevCsr& q, const uint8_t* flags_dev, float p, float thre, int times,
+                     const int32_t* cell_list, const int* n_list, uint32_t out_row0) {
+    cudaStream_t s = ctx->stream;
+    const Markers& mk = ctx->mk;
+    const uint32_t Q = q.n_rows, L = mk.n_labels, Wt = std::max<uint32_t>(ctx->Wt, 1);
+    if (!ctx->h_ft) {
+        SGR_CUDA(cudaMallocHost(reinterpret_cast<void**>(&ctx->h_ft), 2 * offsetof(FtCtl, queue)));
+        for (auto& e : ctx->ev_ft) SGR_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    }
+    constexpr size_t kRead = offsetof(FtCtl, queue);  // the part of the counters that the host reads
+    FtCtl* d = reinterpret_cast<FtCtl*>(ctx->fr_ctl.ensure((sizeof(FtCtl) + 7) / 8));
+    auto host_ctl = [&](int i) { return reinterpret_cast<FtCtl*>(reinterpret_cast<char*>(ctx->h_ft) + i * kRead); };
+    SGR_CUDA(cudaMemsetAsync(d, 0, sizeof(FtCtl), s));
+    ctx->d_final.ensure((size_t)out_row0 + Q);
+    ctx->d_rounds.ensure((size_t)out_row0 + Q);
+    ctx->fr_cells.ensure(Q);
+    ctx->fr_blk_off.ensure(Q);
+    uint8_t* mask = ctx->ft_row_mask.ensure(Q);
+    SGR_CUDA(cudaMemsetAsync(mask, 0, Q, s));
+    launch_ft_cells((int)Q, cell_list, n_list, (int)L, flags_dev, ctx->d_ctidx.p, ctx->fr_cells.p, ctx->fr_blk_off.p,
+                    mask, ctx->d_final.p + out_row0, ctx->d_rounds.p + out_row0, &d->counter, &d->cand, s);
+    // the cells' rows, compacted to the thre pool
+    ctx->counts.ensure((size_t)Q + 1);
+    ctx->qf_indptr.ensure((size_t)Q + 1);
+    launch_filter_count(q.indptr, q.indices, Q, q.n_cols, ctx->qry_map_thre.p, ctx->counts.p, s, mask, &d->longest);
+    launch_exclusive_scan(ctx->counts.p, ctx->qf_indptr.p, Q, ctx->scan_part.ensure(2 * (((size_t)Q + 4095) / 4096) + 1),
+                          s);
+    SGR_CUDA(cudaMemcpyAsync(&d->total, ctx->qf_indptr.p + Q, sizeof(int32_t), cudaMemcpyDeviceToDevice, s));
+    SGR_CUDA(cudaMemcpyAsync(ctx->h_ft, d, kRead, cudaMemcpyDeviceToHost, s));
+    SGR_CUDA(cudaStreamSynchronize(s));
+    const FtCtl h = *host_ctl(0);
+    const int64_t n_cells = (int64_t)(h.counter >> 36), n_blocks = (int64_t)(h.counter & ((1ull << 36) - 1));
+    if (h.longest > 8192) return false;
+    ctx->prof.acc.ft_cells += (uint64_t)n_cells;
+    ctx->prof.acc.ft_candidates += h.cand;
+    ctx->prof.acc.ft_split_cells += (uint64_t)n_cells;
+    if (n_cells == 0) return true;
+    const size_t total = std::max<int32_t>(h.total, 1);
+    ctx->qf_data.ensure(total);
+    ctx->qf_indices.ensure(total);
+    launch_filter_fill(q.data, q.indptr, q.indices, Q, q.n_cols, ctx->qry_map_thre.p, ctx->qf_indptr.p, ctx->qf_data.p,
+                       ctx->qf_indices.p, s, mask);
+    uint16_t* sorted = ctx->fr_sorted.ensure(3 * total);
+    launch_ft_sort_rows(ctx->fr_cells.p, (int)n_cells, ctx->qf_data.p, ctx->qf_indices.p, ctx->qf_indptr.p, h.longest,
+                        sorted, sorted + total, sorted + 2 * total, s);
+    uint32_t max_label = 1;
+    std::vector<LabelQ> lq(L);
+    for (uint32_t l = 0; l < L; ++l) {
+        max_label = std::max(max_label, mk.ctidx[2 * l + 1]);
+        lq[l] = make_lq(0, (int)mk.ctidx[2 * l + 1], p);
+    }
+    ctx->d_lq_label.upload(lq, s);
+    // batches: score blocks (4 GiB), cells (their e-value rows 1 GiB)
+    const int eq_stride = round_up((int)Wt + 1, 4);
+    const int64_t max_blocks = std::max<int64_t>((int64_t)1 << 25, ctx->R32 / 32);
+    const int64_t max_cells = std::max<int64_t>(1, std::min<int64_t>(131072, ((int64_t)1 << 28) / eq_stride));
+    std::vector<int64_t> cuts{0}, off;
+    if (n_blocks > max_blocks || n_cells > max_cells) {
+        off.resize(n_cells);
+        SGR_CUDA(cudaMemcpyAsync(off.data(), ctx->fr_blk_off.p, n_cells * sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+        SGR_CUDA(cudaStreamSynchronize(s));
+        for (int64_t i = 1; i < n_cells; ++i) {
+            const int64_t end = i + 1 < n_cells ? off[i + 1] : n_blocks;
+            if (end - off[cuts.back()] > max_blocks || i - cuts.back() >= max_cells) cuts.push_back(i);
+        }
+    }
+    cuts.push_back(n_cells);
+    int64_t nb = 0, nblk = 0;
+    for (size_t b = 0; b + 1 < cuts.size(); ++b) {
+        nb = std::max(nb, cuts[b + 1] - cuts[b]);
+        nblk = std::max(nblk, off.empty() ? n_blocks
+                                          : (cuts[b + 1] < n_cells ? off[cuts[b + 1]] : n_blocks) - off[cuts[b]]);
+    }
+    FtRounds a{};
+    a.groups = ctx->fr_groups.p;
+    a.blk_base = ctx->d_blk_base.p;
+    a.blk_voff = ctx->fr_blk_voff.p;
+    a.perm = ctx->fr_perm.p;
+    a.ctidx = ctx->d_ctidx.p;
+    a.lorder = ctx->d_lorder.p;
+    a.ft_genes = ctx->d_ft_genes.p;
+    a.ft_idx = ctx->d_ft_idx.p;
+    a.pair_mask = ctx->fr_masks ? ctx->fr_pair_mask.p : nullptr;
+    a.gene_thre = ctx->d_gene_thre.p;
+    a.lq = ctx->d_lq_label.p;
+    a.L = (int)L;
+    a.Wt = (int)Wt;
+    a.nwords = ((int)Wt + 31) / 32;
+    a.eq_stride = eq_stride;
+    a.shift = ctx->pack_shift;
+    a.mul = make_int3(16 * ctx->ft_copies, 2, -1);
+    a.p = p;
+    a.thre = thre;
+    a.times = times;
+    a.s_gene = sorted;
+    a.s_lo = sorted + total;
+    a.s_hi = sorted + 2 * total;
+    a.row_ptr = ctx->qf_indptr.p;
+    a.kcap = h.longest;
+    a.flags = flags_dev;
+    a.top = ctx->fr_top.ensure((size_t)nb * L);
+    int* ints = ctx->fr_ints.ensure((size_t)nb * 3);
+    a.ntop = ints;
+    a.used = ints + nb;
+    a.par = ctx->fr_par.ensure(nb);
+    a.eq = ctx->fr_eq.ensure((size_t)nb * eq_stride);
+    a.ext_min = ctx->fr_ext.ensure((size_t)nb * L * 3);
+    a.ext_max = a.ext_min + (size_t)nb * L;
+    a.blk_of = a.ext_max + (size_t)nb * L;
+    a.un = ctx->fr_un.ensure(nb);
+    a.key_count = ctx->fr_keys.ensure(((size_t)2 << 20) + 1);
+    int32_t* scan_scratch = ctx->scan_part.ensure(2 * (((size_t)1 << 20) / 4096) + 1);
+    const size_t n_quads = ((size_t)nb + 3) / 4;
+    a.list = ctx->fr_list.ensure((size_t)nb * L + n_quads * L * 4);
+    a.q_entry = a.list + (size_t)nb * L;
+    a.quads = ctx->fr_quads.ensure(n_quads);
+    a.q_label = ctx->fr_q_label.ensure(n_quads * L);
+    a.act = ints + 2 * nb;
+    a.n_list = d->n_list;
+    a.queue = d->queue;
+    a.n_act = d->n_act;
+    a.stats = d->stats;
+    a.scores = ctx->fr_scores.ensure((size_t)nblk * 32);
+    const int grid = ft_step_grid((int)nb);
+    a.nan_scratch = ctx->fr_nan.ensure((size_t)grid * max_label);
+    a.max_label = (int)max_label;
+    a.final_labels = ctx->d_final.p + out_row0;
+    a.rounds = ctx->d_rounds.p + out_row0;
+    a.status = ctx->status.p;
+    // 32-bit run sums: X = sum z s <= 2 k (e-sum of the kept entries), each e below 2 Wt and all of the
+    // query's e together k_q |S|
+    const int64_t k = ctx->max_row;
+    const bool x64 = ctx->pack_scan != 2 || 2 * k * std::min<int64_t>(2 * k, h.longest) * (int64_t)Wt >= (int64_t(1) << 32);
+    ft_rounds_setup(a, ctx->ft_copies);
+    for (size_t b = 0; b + 1 < cuts.size(); ++b) {
+        a.cells = ctx->fr_cells.p + cuts[b];
+        a.blk_off = ctx->fr_blk_off.p + cuts[b];
+        a.blk_base0 = off.empty() ? 0 : off[cuts[b]];
+        a.n_cells = (int)(cuts[b + 1] - cuts[b]);
+        if (b > 0) SGR_CUDA(cudaMemsetAsync(d, 0, sizeof(FtCtl), s));
+        SGR_CUDA(cudaMemsetAsync(a.used, 0, a.n_cells * sizeof(int), s));
+        // each round drops at least one candidate, so L rounds finish every cell
+        int most = a.n_cells;  // no more cells than this are active
+        for (int r = 0;; ++r) {
+            if (r > (int)L + 2) fail(SGR_ERR_STATE, "fine-tune rounds did not converge");
+            launch_ft_step(a, r, most, scan_scratch, s);
+            SGR_CUDA(cudaMemcpyAsync(host_ctl(r & 1), d, kRead, cudaMemcpyDeviceToHost, s));
+            SGR_CUDA(cudaEventRecord(ctx->ev_ft[r & 1], s));
+            launch_ft_scan(a, r, ctx->ft_copies, x64, s);
+            if (r == 0) continue;
+            SGR_CUDA(cudaEventSynchronize(ctx->ev_ft[(r - 1) & 1]));
+            const FtCtl* c = host_ctl((r - 1) & 1);
+            most = c->n_act[r & 1];  // cells that go on after step r - 1
+            if (most != 0) continue;
+            ctx->prof.acc.ft_cell_rounds += c->stats[0];
+            ctx->prof.acc.ft_split_rows += c->stats[1];
+            ctx->prof.acc.ft_split_rounds += (uint64_t)r;
+            break;
+        }
+    }
+    return true;
+}
+
+// The fine-tune by rounds where the trained reference and the query's rows allow it, and its results on
+// the host (final_labels: null when the caller reads ctx->d_final itself).
+bool finetune_by_rounds(sgr_ctx* ctx, const DevCsr& q, const uint8_t* flags_dev, float p, float thre, int times,
+                        int32_t* final_labels, int32_t* rounds_out, const int32_t* cell_list = nullptr,
+                        const int* n_list = nullptr, uint32_t out_row0 = 0) {
+    cudaStream_t s = ctx->stream;
+    const uint32_t Q = q.n_rows;
+    if (!ctx->ft_copies || Q == 0) return false;
+    if (!finetune_rounds(ctx, q, flags_dev, p, thre, times, cell_list, n_list, out_row0)) return false;
+    if (!final_labels) return true;
+    SGR_CUDA(cudaMemcpyAsync(final_labels, ctx->d_final.p + out_row0, Q * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+    if (rounds_out)
+        SGR_CUDA(cudaMemcpyAsync(rounds_out, ctx->d_rounds.p + out_row0, Q * sizeof(int32_t), cudaMemcpyDeviceToHost,
+                                 s));
+    check_status(ctx);
+    return true;
+}
+
 // Exact-mode fine-tune: the persistent kernel over a device work queue.  `flags_dev` is the
 // Q x L candidate-flag matrix in device memory.
 // out_row0: the cells' outputs go to ctx->d_final / d_rounds from this row on (the row of q's first
@@ -1160,6 +1438,11 @@ void finetune_persistent(sgr_ctx* ctx, const DevCsr& q, const uint8_t* flags_dev
     const Markers& mk = ctx->mk;
     const uint32_t Q = q.n_rows, L = mk.n_labels, Wt = ctx->Wt;
     const int sp_ft = ctx->prof.begin(ST_FT, s);
+    if (ctx->pack_scan && finetune_by_rounds(ctx, q, flags_dev, p, thre, times, final_labels, rounds_out, cell_list,
+                                             n_list, out_row0)) {
+        ctx->prof.end(sp_ft, s);
+        return;
+    }
     const int32_t* listed = cell_list;  // the caller's cells (cell_list is replaced by the queue order)
     const int* n_listed = n_list;
     // thre-pool rows of the cells to fine-tune (all cells, or only the listed ones)
@@ -1766,6 +2049,7 @@ sgr_status sgr_destroy(sgr_ctx* ctx) {
     cudaStream_t s = ctx->own_stream, side = ctx->side;
     cudaEvent_t e1 = ctx->ev_fork, e2 = ctx->ev_join, e3 = ctx->ev_state[0], e4 = ctx->ev_state[1];
     int32_t* hs = ctx->h_state;
+    unsigned long long* hft = ctx->h_ft;
     cudaStream_t cp = ctx->copy;
     if (cp) cudaStreamSynchronize(cp);
     std::vector<cudaEvent_t> up = ctx->up_ev;
@@ -1774,6 +2058,8 @@ sgr_status sgr_destroy(sgr_ctx* ctx) {
             if (e) up.push_back(e);
     if (ctx->sq_end) up.push_back(ctx->sq_end);
     for (cudaEvent_t e : ctx->blk_ev) up.push_back(e);
+    for (cudaEvent_t e : ctx->ev_ft)
+        if (e) up.push_back(e);
     cudaStream_t fts = ctx->ft_s;
     if (fts) cudaStreamSynchronize(fts);
     delete ctx;  // DevBuf destructors free device memory
@@ -1787,6 +2073,7 @@ sgr_status sgr_destroy(sgr_ctx* ctx) {
     if (e3) cudaEventDestroy(e3);
     if (e4) cudaEventDestroy(e4);
     if (hs) cudaFreeHost(hs);
+    if (hft) cudaFreeHost(hft);
     return SGR_OK;
 }
 

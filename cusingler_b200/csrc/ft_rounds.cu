@@ -1,0 +1,1023 @@
+// Exact fine-tune by rounds over all cells: the row scan batched by (label, four cells).
+//
+// Restates the reference's per-cell fine-tune loop (src/cusingler.cu:1138-1333 of
+// STOmics/cusingler: finetune_round + cufinetune).  The identity behind the scan is the one stated in
+// finetune.cu: with e = d + k (k = stored entries of a row inside the round's gene set S), one pass
+// over a reference row's value-sorted entries gives the exact numerator and norm over S.  Here a
+// round of every active cell is three launches:
+//   ft_step_kernel  per cell: the labels' quantiles of the round before, the keep / drop rule, then
+//                   the next round's gene set and the query's e-values;
+//   ft_plan_kernel  per quad of four active cells: the labels that at least two of them need, and the
+//                   others' entries on the work list of each label;
+//   ft_scan_kernel  per quad, then per four cells of a work list: the correlations of the labels' rows.
+// The cells of a round are put in an order in which neighbours have nearly the same candidates, so that a
+// quad's cells share most labels and one table of e-values serves hundreds of row blocks.
+//
+// What bounds the scan is one shared-memory lookup per (row entry, cell) and the integer work around
+// it.  Four cells share a pass because the entry's load, its address and its run end are then paid
+// once, and one 16-byte lookup serves the four.  The table holds each gene's four packed words
+// (1 << shift) + e (0 outside S) in C = 8 copies of 16 bytes: a quarter-warp's eight lanes read eight
+// different bank groups whatever genes they look up, so no lookup conflicts (a gene pool too wide for
+// eight copies takes fewer, and its lookups conflict).  Entries are 16-bit gene ids in groups of four
+// padded at run ends (entry 0 of a group ending a run has bit 15 set), so the run's bookkeeping is
+// done once per group, with the same instructions for every lane.
+//
+// Packed sums: P is the running sum of the packed words (count in the high bits, e-sum below bit
+// `shift`; the host picks the shift so that neither field of a whole row overflows).  At a run end,
+// acc = P - (P at the run end before) holds the run's count b and e-sum s.  With z = 2 a + b (a: kept
+// entries before the run), X = sum z s is accumulated as sum z acc modulo 2^32: the count fields add
+// (sum z b) << shift = k_r^2 << shift, which is taken off at the end.
+//
+// Measured (B200, 20,000 reference cells in 30 labels, 100,000 queries of which 48,412 take 117,724 rounds,
+// 1.3e9 row correlations of 304 entries): fine-tune 319 -> 102 ms against the per-cell kernels of
+// finetune.cu, of it the scan 89 ms (68 ps a correlation; shared-memory pipe 77 % busy, issue 71 %).
+// Scanning per label instead of per quad left a third of the warps waiting at the table's barriers
+// (82 ps); 12, 24 and 32 warps per CTA were 2 % slower, no different and 9 % slower than 16.
+
+#include <algorithm>
+#include <cstdint>
+#include <type_traits>
+
+#include "kernels.cuh"
+#include "sgr_internal.h"
+#include "stl_order.h"
+#include "device_util.cuh"
+
+namespace sgr {
+namespace {
+
+constexpr int STEP_NW = 8;             // warps of a step CTA, and of one where a round has few cells
+constexpr int STEP_NW_FEW = 32;
+constexpr int STEP_CTAS = 8;           // step CTAs per SM
+constexpr int SCAN_NW = 16;            // warps of a scan CTA (one CTA per SM: the table fills it)
+constexpr uint32_t NAN_KEY = 0xffffffffu;  // ord_key of the NaN that the scan writes
+
+// ---- at training: the reference rows in groups --------------------------------------------------
+
+// One warp per reference row: its entries sorted by (value, gene) as gene | run end << 15 at the row's
+// CSR positions, and the row's groups (runs padded to multiples of four).  Rows are at most `cap` long.
+__global__ void __launch_bounds__(256) row_runs_kernel(const float* data, const int32_t* idx, const int32_t* ptr,
+                                                       uint32_t n_rows, int cap, uint16_t* sorted, int32_t* n_groups) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpb = blockDim.x >> 5;
+    uint64_t* keys = reinterpret_cast<uint64_t*>(smem) + (size_t)warp * cap;
+    for (uint32_t row = blockIdx.x * wpb + warp; row < n_rows; row += gridDim.x * wpb) {
+        const int beg = ptr[row], k = ptr[row + 1] - beg;
+        int n = 1;
+        while (n < k) n <<= 1;
+        for (int i = lane; i < n; i += 32)
+            keys[i] = i < k ? ((uint64_t)ord_key(canon_zero(data[beg + i])) << 32) | (uint32_t)idx[beg + i] : ~0ull;
+        __syncwarp();
+        if (k > 1) warp_bitonic(keys, n, lane);
+        int groups = 0;
+        for (int j = lane; j < k; j += 32) {
+            const uint64_t key = keys[j];
+            const bool last = j + 1 == k || (uint32_t)(keys[j + 1] >> 32) != (uint32_t)(key >> 32);
+            sorted[beg + j] = (uint16_t)((uint32_t)key | (last ? 0x8000u : 0u));
+            if (last) groups += (j + 1 - lower_hi(keys, k, (uint32_t)(key >> 32)) + 3) / 4;
+        }
+        groups = __reduce_add_sync(FULL, groups);
+        if (lane == 0) n_groups[row] = groups;
+        __syncwarp();
+    }
+}
+
+// One thread per row slot (a row of a 32-row block): writes the row's groups.  Vector v of the block's
+// lane t (two groups, 16 bytes) is groups[blk_voff + 32 v + t].  slot_row: the slot's reference row, or
+// -1 for a slot past the label's last row.
+__global__ void row_groups_kernel(const uint16_t* sorted, const int32_t* ptr, const int32_t* slot_row,
+                                  const int32_t* blk_voff, uint32_t n_slots, uint32_t pad, uint4* groups) {
+    const uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x;
+    if (slot >= n_slots) return;
+    const int blk = slot >> 5, lane = slot & 31, row = slot_row[slot];
+    const int nv = (blk_voff[blk + 1] - blk_voff[blk]) / 32;
+    uint16_t* out = reinterpret_cast<uint16_t*>(groups + blk_voff[blk] + lane);
+    int j = row >= 0 ? ptr[row] : 0;
+    const int end = row >= 0 ? ptr[row + 1] : 0;
+    for (int g = 0; g < 2 * nv; ++g) {
+        uint32_t e[4] = {pad, pad, pad, pad};
+        for (int u = 0; u < 4; ++u) {
+            if (j >= end) break;
+            const uint32_t s = sorted[j++];
+            e[u] = s & 0x7fffu;
+            if (s & 0x8000u) {
+                e[0] |= 0x8000u;
+                break;
+            }
+        }
+        uint16_t* o = out + (size_t)(g >> 1) * 32 * 8 + (g & 1) * 4;
+        for (int u = 0; u < 4; ++u) o[u] = (uint16_t)e[u];
+    }
+}
+
+// Bits of each ordered pair's whole fine-tune list over the gene pool.  One warp per pair.
+__global__ void pair_mask_kernel(const uint32_t* ft_genes, const uint32_t* ft_idx, int n_pairs, int nwords,
+                                 uint32_t* mask) {
+    const int lane = threadIdx.x & 31;
+    for (int p = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; p < n_pairs; p += (gridDim.x * blockDim.x) >> 5) {
+        const uint32_t pos = ft_idx[2 * p], len = ft_idx[2 * p + 1];
+        for (uint32_t i = lane; i < len; i += 32) {
+            const uint32_t g = ft_genes[pos + i];
+            atomicOr(mask + (size_t)p * nwords + (g >> 5), 1u << (g & 31));
+        }
+    }
+}
+
+// ---- per call: the cells to fine-tune ----------------------------------------------------------
+
+// Cells with fewer than two candidates are decided here; the others are appended to `cells` with the
+// first 32-row block of their scores (blk_off), and their rows marked.  counter: cells in bits 36..,
+// blocks below; cand: candidates of the appended cells, summed.
+__global__ void __launch_bounds__(256) ft_cells_kernel(int n, const int32_t* list, const int* n_dev, int L,
+                                                       const uint8_t* flags, const uint32_t* ctidx, int32_t* cells, int64_t* blk_off,
+                                                       uint8_t* row_mask, int32_t* final_labels, int32_t* rounds,
+                                                       unsigned long long* counter, unsigned long long* cand) {
+    __shared__ unsigned long long w_tot[8];
+    __shared__ unsigned long long s_base;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (n_dev) n = *n_dev;
+    int c = 0, only = 0, q = 0;
+    unsigned long long mine = 0;
+    if (i < n) {
+        q = list ? list[i] : i;
+        const uint8_t* f = flags + (int64_t)q * L;
+        unsigned long long blocks = 0;
+        for (int l = 0; l < L; ++l)
+            if (f[l]) {
+                if (c == 0) only = l;
+                ++c;
+                blocks += (ctidx[2 * l + 1] + 31) / 32;
+            }
+        if (c >= 2) mine = (1ull << 36) | blocks;
+        else {
+            final_labels[q] = c ? only : 0;
+            rounds[q] = 0;
+        }
+    }
+    unsigned long long x = mine;
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long y = __shfl_up_sync(FULL, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) w_tot[warp] = x;
+    const int csum = __reduce_add_sync(FULL, c >= 2 ? c : 0);
+    if (lane == 0 && csum) atomicAdd(cand, (unsigned long long)csum);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        unsigned long long t = 0;
+        for (int w = 0; w < 8; ++w) {
+            const unsigned long long v = w_tot[w];
+            w_tot[w] = t;
+            t += v;
+        }
+        s_base = t ? atomicAdd(counter, t) : 0ull;
+    }
+    __syncthreads();
+    if (mine) {
+        const unsigned long long at = s_base + w_tot[warp] + x - mine;
+        cells[at >> 36] = q;
+        blk_off[at >> 36] = (int64_t)(at & ((1ull << 36) - 1));
+        row_mask[q] = 1;
+    }
+}
+
+// One warp per cell: its pool entries by value, with each entry's run as positions [lo, hi).
+__global__ void __launch_bounds__(256) ft_sort_rows_kernel(const int32_t* cells, int n, const float* data,
+                                                           const int32_t* idx, const int32_t* ptr, int cap,
+                                                           uint16_t* s_gene, uint16_t* s_lo, uint16_t* s_hi) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpb = blockDim.x >> 5;
+    uint64_t* keys = reinterpret_cast<uint64_t*>(smem) + (size_t)warp * cap;
+    for (int i = blockIdx.x * wpb + warp; i < n; i += gridDim.x * wpb) {
+        const int beg = ptr[cells[i]], k = ptr[cells[i] + 1] - beg;
+        int m = 1;
+        while (m < k) m <<= 1;
+        for (int j = lane; j < m; j += 32)
+            keys[j] = j < k ? ((uint64_t)ord_key(canon_zero(data[beg + j])) << 32) | (uint32_t)idx[beg + j] : ~0ull;
+        __syncwarp();
+        if (k > 1) warp_bitonic(keys, m, lane);
+        for (int j = lane; j < k; j += 32) {
+            const uint64_t key = keys[j];
+            const uint32_t hv = (uint32_t)(key >> 32);
+            s_gene[beg + j] = (uint16_t)(uint32_t)key;
+            s_lo[beg + j] = (uint16_t)lower_hi(keys, k, hv);
+            s_hi[beg + j] = (uint16_t)upper_hi(keys, k, hv);
+        }
+        __syncwarp();
+    }
+}
+
+// ---- a round -------------------------------------------------------------------------------------
+
+// The reference's keep / drop rule (src/cusingler.cu:1270-1295) on the list order: returns the new
+// list length, the new list in top.  One thread.
+__device__ int keep_candidates(const float* lsc, int ntop, uint8_t* top, uint8_t* tmp, float thre) {
+    int mn, mx;
+    stl::minmax(lsc, ntop, &mn, &mx);
+    const float lo = lsc[mn], hi = lsc[mx];
+    const float t = __fsub_rn(hi, thre);
+    int n = 0;
+    if (!(hi != hi)) {
+        for (int i = 0; i < ntop; ++i) {
+            const float s = lsc[i];
+            if (s <= lo || s < t) continue;
+            if (s == hi) {
+                for (int j = n; j > 0; --j) tmp[j] = tmp[j - 1];
+                tmp[0] = top[i];
+            } else {
+                tmp[n] = top[i];
+            }
+            ++n;
+        }
+    }
+    if (n == 0) {
+        tmp[0] = top[0];
+        n = 1;
+    }
+    for (int i = 0; i < n; ++i) top[i] = tmp[i];
+    return n;
+}
+
+template <int NW>
+struct StepSmem {
+    int hist[NW][256];
+    float lsc[256];
+    uint32_t off[256];  // first 32-row block of each candidate's scores
+    uint8_t top[256], tmp[256];
+    uint8_t is_cand[256];
+    long long red64[NW];
+    int red[NW];
+    int ntop, kq, nan;
+};
+
+// Step k of the batch's cells.  k = 0: candidates from the flags, the first round's setup; k > 0: the
+// decisions of round k - 1, then the setup of round k.  A cell that goes on is appended to `un` with its
+// sort key; bits > 0: and counted under the key's leading bits.  dynamic shared memory: eq (eq_stride
+// words), bits (nwords), in / before (kcap / 32 + 2 words each).
+template <int NW>
+__global__ void __launch_bounds__(NW * 32, NW == STEP_NW ? 4 : 1) ft_step_kernel(FtRounds a, int k, int bits_key) {
+    extern __shared__ __align__(16) unsigned char dyn[];
+    __shared__ StepSmem<NW> sh;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    constexpr int NT = NW * 32;
+    uint32_t* eq = reinterpret_cast<uint32_t*>(dyn);
+    uint32_t* bits = eq + a.eq_stride;
+    uint32_t* in = bits + a.nwords;           // the row's entries inside the gene set, as bits
+    uint32_t* before = in + a.kcap / 32 + 2;  // those before each word
+    const int cur = k & 1, nxt = cur ^ 1;
+    const int n = k == 0 ? a.n_cells : a.n_act[cur];
+    unsigned long long my_rounds = 0, my_rows = 0;
+    for (int it = blockIdx.x; it < n; it += gridDim.x) {
+        const int c = k == 0 ? it : a.act[it];
+        const int cell = a.cells[c];
+        uint8_t* gtop = a.top + (size_t)c * a.L;
+        const uint32_t blk0 = (uint32_t)(a.blk_off[c] - a.blk_base0);
+        __syncthreads();  // the previous cell's shared memory is no longer read
+        if (k == 0) {
+            if (warp == 0) {  // the flagged labels in ascending order (src/cusingler.cu:1305-1312)
+                int m = 0;
+                for (int base = 0; base < a.L; base += 32) {
+                    const int l = base + lane;
+                    const bool f = l < a.L && a.flags[(size_t)cell * a.L + l] != 0;
+                    const unsigned b = __ballot_sync(FULL, f);
+                    if (f) sh.top[m + __popc(b & ((1u << lane) - 1u))] = (uint8_t)l;
+                    m += __popc(b);
+                }
+                if (lane == 0) sh.ntop = m;
+            }
+        } else {
+            const int ntop = a.ntop[c];
+            for (int i = tid; i < ntop; i += NT) sh.top[i] = gtop[i];
+            if (tid == 0) {
+                sh.ntop = ntop;
+                sh.nan = 0;
+            }
+            for (int i = tid; i < ntop; i += NT) sh.off[i] = a.blk_of[(size_t)c * a.L + i];
+            __syncthreads();
+            for (int i = warp; i < ntop; i += NW) {
+                const LabelQ q = a.lq[sh.top[i]];
+                const float* v = a.scores + (size_t)sh.off[i] * 32;
+                const uint32_t kmin = a.ext_min[(size_t)c * a.L + i], kmax = a.ext_max[(size_t)c * a.L + i];
+                float r = 0.f;
+                if (q.kind == 0) r = v[0];
+                else if (kmax == NAN_KEY) {
+                    if (lane == 0) sh.nan = 1;
+                } else r = quantile_warp_core(v, q, a.p, sh.hist[warp], nullptr, lane, a.status, kmin, kmax, false);
+                if (lane == 0) sh.lsc[i] = r;
+            }
+            __syncthreads();
+            if (sh.nan && warp == 0) {
+                // lists holding NaN: libstdc++'s order depends on the list's own order, which the scan's
+                // block order is mapped back to
+                float* scratch = a.nan_scratch + (size_t)blockIdx.x * a.max_label;
+                for (int i = 0; i < ntop; ++i) {
+                    const LabelQ q = a.lq[sh.top[i]];
+                    if (q.kind == 0 || a.ext_max[(size_t)c * a.L + i] != NAN_KEY) continue;
+                    const float* v = a.scores + (size_t)sh.off[i] * 32;
+                    const uint32_t* perm = a.perm + a.ctidx[2 * sh.top[i]];
+                    for (int j = lane; j < q.len; j += 32) scratch[perm[j]] = v[j];
+                    __syncwarp();
+                    if (lane == 0) {
+                        int oob = 0;
+                        stl::sort(scratch, q.len, &oob);
+                        if (oob) atomicOr(a.status, 4);
+                        sh.lsc[i] = q.kind == 1   ? scratch[0]
+                                    : q.kind == 2 ? scratch[q.len - 1]
+                                                  : interp(a.p, q.prev_index, q.step, scratch[q.k - 1], scratch[q.k]);
+                    }
+                    __syncwarp();
+                }
+            }
+            __syncthreads();
+            if (tid == 0) sh.ntop = keep_candidates(sh.lsc, ntop, sh.top, sh.tmp, a.thre);
+        }
+        __syncthreads();
+
+        // the next round's condition
+        const int ntop = sh.ntop, done = k == 0 ? 0 : a.used[c];
+        const bool go = ntop > 1 && (a.times == 0 || done < a.times);
+        if (!go) {
+            if (tid == 0) {
+                a.final_labels[cell] = ntop > 0 ? (int32_t)sh.top[0] : 0;
+                a.rounds[cell] = done;
+            }
+            continue;
+        }
+        // gene set: union over ordered candidate pairs of the first min(len, gene_thre(n)) genes of the
+        // pair's list (src/cusingler.cu:1141-1156); a list that is not cut is one precomputed mask
+        const int gthre = a.gene_thre[ntop], np = ntop * ntop, nw = a.nwords;
+        for (int w = tid; w < nw; w += NT) bits[w] = 0u;
+        __syncthreads();
+        // A warp takes up to 32 pairs at a time, few enough that every warp gets some.  Each lane fetches
+        // one pair's list range; then the warp walks the pairs together, lanes over the mask's words (or
+        // over a cut list's genes), so that the loads of several pairs are in flight at once.
+        const int ppw = min(32, (np + NW - 1) / NW);
+        for (int base = warp * ppw; base < np; base += NW * ppw) {
+            const int pr = base + lane;
+            uint32_t pi = 0, pos = 0;
+            int len = 0;
+            if (lane < ppw && pr < np) {
+                const int i = pr / ntop, j = pr - i * ntop;
+                if (i != j) {
+                    pi = (uint32_t)sh.top[i] * a.L + sh.top[j];
+                    const uint2 r = __ldg(reinterpret_cast<const uint2*>(a.ft_idx) + pi);
+                    pos = r.x;
+                    len = (int)r.y;
+                }
+            }
+            const bool whole = a.pair_mask && len <= gthre;
+            const unsigned by_mask = __ballot_sync(FULL, whole && len > 0);
+            for (int w0 = 0; by_mask && w0 < nw; w0 += 32) {
+                uint32_t m = 0;
+#pragma unroll 8
+                for (int t = 0; t < ppw; ++t) {
+                    const size_t p = __shfl_sync(FULL, pi, t);
+                    if (((by_mask >> t) & 1u) && w0 + lane < nw) m |= __ldg(a.pair_mask + p * nw + w0 + lane);
+                }
+                if (m) atomicOr(&bits[w0 + lane], m);
+            }
+            if (whole) len = 0;
+            len = min(len, gthre);
+            const int maxn = __reduce_max_sync(FULL, len);
+            for (int e0 = 0; e0 < maxn; e0 += 32) {
+#pragma unroll 8
+                for (int t = 0; t < ppw; ++t) {
+                    const uint32_t g0 = __shfl_sync(FULL, pos, t);
+                    if (e0 + lane < __shfl_sync(FULL, len, t)) {
+                        const uint32_t g = __ldg(a.ft_genes + g0 + e0 + lane);
+                        atomicOr(&bits[g >> 5], 1u << (g & 31));
+                    }
+                }
+            }
+        }
+        __syncthreads();
+        int pc = 0;
+        for (int w = tid; w < nw; w += NT) pc += __popc(bits[w]);
+        pc = __reduce_add_sync(FULL, pc);
+        if (lane == 0) sh.red[warp] = pc;
+        __syncthreads();
+        int nS = 0;
+#pragma unroll
+        for (int w = 0; w < NW; ++w) nS += sh.red[w];
+        if (tid == 0) my_rounds++;
+        if (nS < 20) {  // keep the first candidate (src/cusingler.cu:1158-1159)
+            if (tid == 0) {
+                a.final_labels[cell] = (int32_t)sh.top[0];
+                a.rounds[cell] = done + 1;
+            }
+            continue;
+        }
+        // the query's e-values over S: |S| - k + (kept entries before the run's end) + (before its start)
+        const int beg = a.row_ptr[cell], len = a.row_ptr[cell + 1] - beg;
+        const uint32_t one = 1u << a.shift;
+        const int nwd = (len + 31) / 32;
+#pragma unroll 4
+        for (int w = warp; w < nwd; w += NW) {
+            const int j = 32 * w + lane;
+            const uint32_t g = j < len ? a.s_gene[beg + j] : 0u;
+            const unsigned b = __ballot_sync(FULL, j < len && ((bits[g >> 5] >> (g & 31)) & 1u));
+            if (lane == 0) in[w] = b;
+        }
+        for (int g = tid; g < a.eq_stride; g += NT) eq[g] = g < a.Wt && ((bits[g >> 5] >> (g & 31)) & 1u) ? one : 0u;
+        for (int l = tid; l < a.L; l += NT) sh.is_cand[l] = 0;
+        __syncthreads();
+        if (warp == 0) {
+            int m = 0;
+            for (int base = 0; base < nwd; base += 32) {
+                const int w = base + lane;
+                const int p = w < nwd ? __popc(in[w]) : 0, incl = warp_incl_scan(p, lane);
+                if (w < nwd) before[w] = (uint32_t)(m + incl - p);
+                m += __shfl_sync(FULL, incl, 31);
+            }
+            if (lane == 0) {
+                in[nwd] = 0u;
+                before[nwd] = (uint32_t)m;
+                sh.kq = m;
+            }
+        }
+        for (int i = tid; i < ntop; i += NT) sh.is_cand[sh.top[i]] = 1;
+        __syncthreads();
+        const int kq = sh.kq;
+        auto kept = [&](int x) {  // kept entries before position x
+            return (int)before[x >> 5] + __popc(in[x >> 5] & ((1u << (x & 31)) - 1u));
+        };
+        long long sq = 0;
+        for (int j = tid; j < len; j += NT) {
+            if (!((in[j >> 5] >> (j & 31)) & 1u)) continue;
+            const int e = nS - kq + kept(a.s_lo[beg + j]) + kept(a.s_hi[beg + j]);
+            eq[a.s_gene[beg + j]] = one + (uint32_t)e;
+            sq += (long long)(e - kq) * (e - kq);
+        }
+        sq = warp_sum_i64(sq);
+        if (lane == 0) sh.red64[warp] = sq;
+        __syncthreads();
+        uint4* out = reinterpret_cast<uint4*>(a.eq + (size_t)c * a.eq_stride);
+        for (int g = tid; g < a.eq_stride / 4; g += NT) out[g] = reinterpret_cast<const uint4*>(eq)[g];
+        for (int i = tid; i < ntop; i += NT) gtop[i] = sh.top[i];
+        if (tid == 0) {
+            long long nq = (long long)(nS - kq) * kq * kq;
+            for (int w = 0; w < NW; ++w) nq += sh.red64[w];
+            a.par[c] = FtCell{nq > 0 ? 1.0 / sqrt((double)nq) : 0.0, (int64_t)nq, nS, kq};
+            a.ntop[c] = ntop;
+            a.used[c] = done + 1;
+        }
+        if (warp == 0) {
+            // sort key: the candidates among the 32 longest labels as a reflected Gray code, so that cells
+            // whose candidates differ little are close
+            const unsigned m = __ballot_sync(FULL, lane < a.L && sh.is_cand[a.lorder[min(lane, a.L - 1)]]);
+            const uint32_t key = __brev(__ballot_sync(FULL, __popc(m & (0xffffffffu >> (31 - lane))) & 1));
+            if (lane == 0) {
+                a.un[atomicAdd(a.n_act + nxt, 1)] = ((unsigned long long)key << 32) | (uint32_t)c;
+                if (bits_key) atomicAdd(a.key_count + (key >> (32 - bits_key)), 1);
+            }
+        }
+        if (warp == NW - 1) {  // the candidates' score blocks
+            uint32_t acc = 0;
+            for (int base = 0; base < ntop; base += 32) {
+                const int i = base + lane;
+                const int l = i < ntop ? sh.top[i] : 0;
+                const int nb = i < ntop ? (int)(a.ctidx[2 * l + 1] + 31) / 32 : 0;
+                const int incl = warp_incl_scan(nb, lane);
+                if (i < ntop) {
+                    a.ext_min[(size_t)c * a.L + i] = 0xffffffffu;
+                    a.ext_max[(size_t)c * a.L + i] = 0u;
+                    a.blk_of[(size_t)c * a.L + i] = blk0 + acc + (uint32_t)(incl - nb);
+                }
+                acc += (uint32_t)__shfl_sync(FULL, incl, 31);
+            }
+            if (lane == 0) my_rows += (unsigned long long)acc * 32;
+        }
+    }
+    if (tid == 0 && my_rounds) atomicAdd(a.stats, my_rounds);
+    if (warp == NW - 1 && lane == 0 && my_rows) atomicAdd(a.stats + 1, my_rows);
+}
+
+__device__ __forceinline__ uint4 lds128(uint32_t addr) {
+    uint4 v;
+    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
+    return v;
+}
+
+// State of one row's pass for the four cells.
+template <bool X64>
+struct RowSums {
+    using T = typename std::conditional<X64, uint64_t, uint32_t>::type;
+    uint32_t P[4], tot[4], ka[4], B3[4];
+    T X[4];
+};
+
+// One group of four entries: w0 = entries 0 | 1 << 16 (bit 15: the group ends a run), w1 = 2 | 3 << 16.
+// m = {16 C, 2, -1} as run-time values: with them the addresses, z and acc are multiply-adds, which
+// leaves the integer ALU (half rate, as the multiplier is) and the multiplier with about the same number
+// of instructions.
+template <int C, bool X64>
+__device__ __forceinline__ void scan_group(RowSums<X64>& s, uint32_t w0, uint32_t w1, uint32_t tab, int sh,
+                                           uint32_t low, int3 m) {
+    const uint4 a = lds128((w0 & 0x7fffu) * (uint32_t)m.x + tab), b = lds128((w0 >> 16) * (uint32_t)m.x + tab);
+    const uint4 c = lds128((w1 & 0xffffu) * (uint32_t)m.x + tab), d = lds128((w1 >> 16) * (uint32_t)m.x + tab);
+    const bool end = (w0 & 0x8000u) != 0;
+    const uint32_t va[4] = {a.x, a.y, a.z, a.w}, vb[4] = {b.x, b.y, b.z, b.w};
+    const uint32_t vc[4] = {c.x, c.y, c.z, c.w}, vd[4] = {d.x, d.y, d.z, d.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        s.P[i] += va[i] + vb[i];
+        s.P[i] += vc[i] + vd[i];
+        const uint32_t t = end ? s.P[i] : s.tot[i];
+        const uint32_t acc = s.tot[i] * (uint32_t)m.z + t;
+        s.tot[i] = t;
+        const uint32_t n = acc >> sh;
+        const uint32_t z = (uint32_t)m.y * s.ka[i] + n;
+        s.ka[i] += n;
+        if (X64) s.X[i] += (uint64_t)z * (acc & low);
+        else s.X[i] += z * acc;  // the count field's part is taken off at the end
+        s.B3[i] += n * n * n;
+    }
+}
+
+constexpr int PLAN_NW = 8;
+constexpr int ITEMS_PER_CTA = 16;  // scan items per CTA that a round's quads are cut into
+constexpr int FEW_QUADS = 512;     // up to this many quads the items are sized by the round's total work
+constexpr int SPLIT_QUADS = 64;    // from this many quads on, a label that one cell alone needs goes to its work list
+
+// The active cells in the order of their keys: by rank (few cells; one warp per cell counts the smaller
+// keys), or by the keys' leading bits (start: exclusive scan of their counts, advanced here).
+__global__ void __launch_bounds__(256) ft_rank_kernel(FtRounds a, int k) {
+    const int n = a.n_act[(k & 1) ^ 1], lane = threadIdx.x & 31;
+    for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += (gridDim.x * blockDim.x) >> 5) {
+        const unsigned long long mine = a.un[i];
+        int less = 0;
+#pragma unroll 4
+        for (int j = lane; j < n; j += 32) less += a.un[j] < mine;
+        less = __reduce_add_sync(FULL, less);
+        if (lane == 0) a.act[less] = (int)(uint32_t)mine;
+    }
+}
+
+__global__ void __launch_bounds__(256) ft_place_kernel(FtRounds a, int k, int bits_key, int32_t* start) {
+    const int n = a.n_act[(k & 1) ^ 1];
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const unsigned long long u = a.un[i];
+        a.act[atomicAdd(start + (uint32_t)(u >> (64 - bits_key)), 1)] = (int)(uint32_t)u;
+    }
+}
+
+// The round's quads: the active cells in order, four at a time.  One warp per quad.
+__global__ void __launch_bounds__(PLAN_NW * 32) ft_plan_kernel(FtRounds a, int k) {
+    __shared__ uint16_t pos[PLAN_NW][4][256];  // position of each label in the four candidate lists
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, cur = k & 1;
+    const int n = a.n_act[cur ^ 1];
+    const int n_quads = (n + 3) / 4, least = n_quads >= SPLIT_QUADS ? 2 : 1;
+    for (int q = blockIdx.x * PLAN_NW + warp; q < n_quads; q += gridDim.x * PLAN_NW) {
+        const int nq = min(4, n - 4 * q);
+        const int c = lane < nq ? a.act[4 * q + lane] : 0;
+        for (int i = lane; i < 4 * 256; i += 32) (&pos[warp][0][0])[i] = 0xffffu;
+        __syncwarp();
+        for (int t = 0; t < nq; ++t) {
+            const int ct = __shfl_sync(FULL, c, t), m = a.ntop[ct];
+            for (int i = lane; i < m; i += 32) pos[warp][t][a.top[(size_t)ct * a.L + i]] = (uint16_t)i;
+        }
+        __syncwarp();
+        int cell[4];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) cell[t] = __shfl_sync(FULL, c, min(t, nq - 1));
+        int n_lab = 0, units = 0;
+        for (int base = 0; base < a.L; base += 32) {
+            const int l = base + lane;
+            FtEntry e[4];
+            int need = 0, last = 0;
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                const uint32_t i = l < a.L && t < nq ? pos[warp][t][l] : 0xffffu;
+                e[t] = FtEntry{~0u, 0u};
+                if (i != 0xffffu) {
+                    const uint32_t cp = (uint32_t)cell[t] * a.L + i;
+                    e[t] = FtEntry{cp, a.blk_of[cp]};
+                    ++need;
+                    last = t;
+                }
+            }
+            const bool in = need >= least;
+            const int nb = in ? (int)(a.ctidx[2 * l + 1] + 31) / 32 : 0;
+            const unsigned m = __ballot_sync(FULL, in);
+            const int ps = warp_incl_scan(nb, lane);
+            if (in) {
+                const size_t at_q = (size_t)q * a.L + n_lab + __popc(m & ((1u << lane) - 1u));
+                a.q_label[at_q] = make_int2(l, units + ps - nb);
+#pragma unroll
+                for (int t = 0; t < 4; ++t) a.q_entry[at_q * 4 + t] = e[t];
+            } else if (need) {
+                FtEntry x = e[0];
+#pragma unroll
+                for (int t = 1; t < 4; ++t)
+                    if (last == t) x = e[t];
+                a.list[(size_t)l * a.n_cells + atomicAdd(a.n_list + cur * 256 + l, 1)] = x;
+            }
+            n_lab += __popc(m);
+            units += __shfl_sync(FULL, ps, 31);
+        }
+        if (lane == 0) a.quads[q] = FtQuad{{cell[0], cell[1], cell[2], cell[3]}, nq, n_lab, units};
+        __syncwarp();
+    }
+}
+
+// One work item of a round: four cells and a range of 32-row blocks ("units") of the labels they need.
+struct ScanItem {
+    FtCell par[4];
+    FtEntry entry[4];  // work-list item: the cells' entries of the one label
+    int cell[4];
+    int quad;          // -1: work-list item
+    int label;         // work-list item: its label
+    int n_lab;         // labels (0: no item left)
+    int u0, u1;
+};
+
+constexpr int SCAN_PF = 4;  // genes of the next table that a thread holds in registers
+
+// Work items: the quads' labels, each quad cut into parts when a round has few quads; then the labels'
+// work lists in order of length (lorder), four entries at a time, in parts of at most `bpp` blocks.
+// Items are fetched two ahead while the current one is scanned, and a warp that has finished its blocks
+// loads its share of the next table into registers before it waits for the others, so that between two
+// items only the table's stores are left.
+template <int C, bool X64>
+__global__ void __launch_bounds__(SCAN_NW * 32, 1) ft_scan_kernel(FtRounds a, int k) {
+    extern __shared__ __align__(16) unsigned char dyn[];
+    __shared__ int pre[257];      // work-list items before each label (in lorder)
+    __shared__ int2 labs[256];    // the current item's labels and the units before each
+    __shared__ int qpre[FEW_QUADS + 1];  // few quads: items before each
+    __shared__ int s_bpp, s_upp;
+    __shared__ ScanItem items[3];  // ring: current, next, the one being fetched
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int cur = k & 1, nxt = cur ^ 1;
+    constexpr int NT = SCAN_NW * 32;
+    if (blockIdx.x == 0) {  // the next round's counters
+        for (int l = tid; l < 256; l += NT) a.n_list[nxt * 256 + l] = 0;
+        if (tid == 0) {
+            a.queue[nxt] = 0;
+            a.n_act[cur] = 0;
+        }
+    }
+    const int n_quads = (a.n_act[nxt] + 3) / 4;
+    if (n_quads == 0) return;
+    // Many quads: the same number of parts for each.  Few: parts of `upp` units so that every CTA gets some.
+    // Filling a table costs about as much as scanning one unit at full rate, and four warps (one per
+    // scheduler) scan at close to full rate, so a part is not below four units; parts are 16 units (one per
+    // warp) as soon as there are enough for every CTA.
+    const int parts = max(1, ((int)gridDim.x * ITEMS_PER_CTA + n_quads - 1) / n_quads);
+    const bool few = n_quads <= FEW_QUADS;
+    // Fetches the next work item into `it`.  One warp.
+    auto fetch = [&](ScanItem& it) {
+        for (;;) {
+            int item = 0;
+            if (lane == 0) item = atomicAdd(a.queue + cur, 1);
+            item = __shfl_sync(FULL, item, 0);
+            const int n_quad_items = few ? qpre[n_quads] : n_quads * parts;
+            if (item < n_quad_items) {
+                int q, part, upp = s_upp;
+                if (few) {
+                    int lo = 0, hi = n_quads - 1;  // qpre[lo] <= item < qpre[lo + 1]
+                    while (lo < hi) {
+                        const int mid = (lo + hi + 1) >> 1;
+                        if (qpre[mid] <= item) lo = mid;
+                        else hi = mid - 1;
+                    }
+                    q = lo;
+                    part = item - qpre[lo];
+                } else {
+                    q = item / parts;
+                    part = item - q * parts;
+                }
+                const FtQuad h = a.quads[q];
+                if (!few) upp = max(SCAN_NW, (h.units + parts - 1) / parts);
+                const int u0 = part * upp;
+                if (u0 >= h.units) continue;  // a quad with fewer parts
+                if (lane < 4) {
+                    const int c = a.quads[q].cell[lane];
+                    it.cell[lane] = c;
+                    it.par[lane] = a.par[c];
+                }
+                if (lane == 0) {
+                    it.quad = q;
+                    it.n_lab = h.n_lab;
+                    it.u0 = u0;
+                    it.u1 = min(h.units, u0 + upp);
+                }
+                return;
+            }
+            item -= n_quad_items;
+            if (item >= pre[a.L]) {
+                if (lane == 0) it.n_lab = 0;
+                return;
+            }
+            int lo = 0, hi = a.L - 1;  // pre[lo] <= item < pre[lo + 1]
+            while (lo < hi) {
+                const int mid = (lo + hi + 1) >> 1;
+                if (pre[mid] <= item) lo = mid;
+                else hi = mid - 1;
+            }
+            const int l = a.lorder[lo], nblk = (int)(a.ctidx[2 * l + 1] + 31) / 32;
+            const int lparts = (nblk + s_bpp - 1) / s_bpp, at = item - pre[lo];
+            const int q0 = at / lparts * 4, nq = min(4, a.n_list[cur * 256 + l] - q0);
+            if (lane < 4) {
+                const FtEntry e = a.list[(size_t)l * a.n_cells + q0 + min(lane, nq - 1)];
+                const int c = (int)(e.cellp / a.L);
+                it.entry[lane] = lane < nq ? e : FtEntry{~0u, 0u};
+                it.cell[lane] = c;
+                it.par[lane] = a.par[c];
+            }
+            if (lane == 0) {
+                it.quad = -1;
+                it.label = l;
+                it.n_lab = 1;
+                it.u0 = at % lparts * s_bpp;
+                it.u1 = min(nblk, it.u0 + s_bpp);
+            }
+            return;
+        }
+    };
+    if (warp == 0) {
+        unsigned long long work = 0;  // (four entries, block) pairs of the work lists
+        for (int i = lane; i < a.L; i += 32) {
+            const int l = a.lorder[i];
+            work += (unsigned long long)((a.n_list[cur * 256 + l] + 3) / 4) * ((a.ctidx[2 * l + 1] + 31) / 32);
+        }
+        for (int o = 16; o > 0; o >>= 1) work += __shfl_xor_sync(FULL, work, o);
+        const int bpp = (int)min(1ull << 24, max((unsigned long long)SCAN_NW, work / gridDim.x + 1));
+        int acc = 0;
+        for (int base = 0; base < a.L; base += 32) {
+            const int i = base + lane;
+            int n = 0;
+            if (i < a.L) {
+                const int l = a.lorder[i];
+                const int nb = (int)(a.ctidx[2 * l + 1] + 31) / 32;
+                n = (a.n_list[cur * 256 + l] + 3) / 4 * ((nb + bpp - 1) / bpp);
+            }
+            const int incl = warp_incl_scan(n, lane);
+            if (i < a.L) pre[i] = acc + incl - n;
+            acc += __shfl_sync(FULL, incl, 31);
+        }
+        if (lane == 0) {
+            pre[a.L] = acc;
+            s_bpp = bpp;
+        }
+        if (few) {
+            int total = 0;
+            for (int q = lane; q < n_quads; q += 32) total += a.quads[q].units;
+            total = __reduce_add_sync(FULL, total);
+            const int grid = (int)gridDim.x;
+            const int upp = total <= grid * SCAN_NW ? max(4, (total + grid - 1) / grid)
+                                                    : max(SCAN_NW, total / (grid * ITEMS_PER_CTA));
+            int at = 0;
+            for (int base = 0; base < n_quads; base += 32) {
+                const int q = base + lane;
+                const int n = q < n_quads ? (a.quads[q].units + upp - 1) / upp : 0, incl = warp_incl_scan(n, lane);
+                if (q < n_quads) qpre[q] = at + incl - n;
+                at += __shfl_sync(FULL, incl, 31);
+            }
+            if (lane == 0) {
+                qpre[n_quads] = at;
+                s_upp = upp;
+            }
+        }
+        __syncwarp();
+        fetch(items[0]);
+        fetch(items[1]);
+    }
+    __syncthreads();
+    const uint32_t tab = (uint32_t)__cvta_generic_to_shared(dyn) + (lane & (C - 1)) * 16;
+    const uint32_t low = (1u << a.shift) - 1u;
+    const int3 mul = a.mul;
+    // the table's words of gene g for an item's four cells
+    auto load_gene = [&](const ScanItem& it, int g) {
+        uint4 v;
+        v.x = __ldg(a.eq + (size_t)it.cell[0] * a.eq_stride + g);
+        v.y = __ldg(a.eq + (size_t)it.cell[1] * a.eq_stride + g);
+        v.z = __ldg(a.eq + (size_t)it.cell[2] * a.eq_stride + g);
+        v.w = __ldg(a.eq + (size_t)it.cell[3] * a.eq_stride + g);
+        return v;
+    };
+    // C copies, written in rotated order so that a quarter-warp's stores fall into different bank groups
+    auto store_gene = [&](int g, const uint4& v) {
+        uint4* t = reinterpret_cast<uint4*>(dyn) + (size_t)g * C;
+#pragma unroll
+        for (int i = 0; i < C; ++i) t[(i + lane) & (C - 1)] = v;
+    };
+    for (int turn = 0; items[turn].n_lab != 0; turn = turn == 2 ? 0 : turn + 1) {
+        const ScanItem& it = items[turn];
+        // the item's table and labels, into registers while other warps still scan the item before
+        uint4 pf[SCAN_PF];
+#pragma unroll
+        for (int u = 0; u < SCAN_PF; ++u)
+            if (tid + u * NT <= a.Wt) pf[u] = load_gene(it, tid + u * NT);
+        const int n_lab = it.n_lab, quad = it.quad, u1 = it.u1;
+        int2 my_lab = make_int2(it.label, 0);
+        if (quad >= 0 && tid < n_lab) my_lab = __ldg(a.q_label + (size_t)quad * a.L + tid);
+        __syncthreads();  // every warp is done with the previous item
+#pragma unroll
+        for (int u = 0; u < SCAN_PF; ++u)
+            if (tid + u * NT <= a.Wt) store_gene(tid + u * NT, pf[u]);
+        for (int g = tid + SCAN_PF * NT; g <= a.Wt; g += NT) store_gene(g, load_gene(it, g));
+        if (tid < n_lab) labs[tid] = my_lab;
+        __syncthreads();
+        // the item after next, in the slot of the one before (read by nobody since the first barrier)
+        if (warp == SCAN_NW - 1) fetch(items[turn == 0 ? 2 : turn - 1]);
+        // unit u is block u - labs[j].y of label labs[j].x
+        int j = 0, blk = 0, v0 = 0, nv = 0;
+        uint4 w = make_uint4(0u, 0u, 0u, 0u), w2 = w;
+        auto open = [&](int u) {  // the unit's label, block and first row vectors
+            while (j + 1 < n_lab && labs[j + 1].y <= u) ++j;
+            const int2 lb = labs[j];
+            blk = u - lb.y;
+            const int32_t* vo = a.blk_voff + a.blk_base[lb.x] + blk;
+            v0 = vo[0];
+            nv = (vo[1] - v0) >> 5;
+            if (nv > 0) w = __ldg(a.groups + v0 + lane);
+            if (nv > 1) w2 = __ldg(a.groups + v0 + 32 + lane);
+        };
+        int u = it.u0 + warp;
+        if (u < u1) open(u);
+        while (u < u1) {
+            const int uj = j, ub = blk;
+            FtEntry my = {~0u, 0u};
+            if (lane < 4) my = quad >= 0 ? a.q_entry[((size_t)quad * a.L + uj) * 4 + lane] : it.entry[lane];
+            const uint4* p = a.groups + v0 + lane;
+            RowSums<X64> s = {};
+            for (int v = 0; v < nv; ++v) {
+                const uint4 wn = v + 2 < nv ? __ldg(p + 32 * (v + 2)) : w;  // two vectors ahead
+                scan_group<C, X64>(s, w.x, w.y, tab, a.shift, low, mul);
+                scan_group<C, X64>(s, w.z, w.w, tab, a.shift, low, mul);
+                w = w2;
+                w2 = wn;
+            }
+            u += SCAN_NW;
+            const bool valid = ub * 32 + lane < (int)a.ctidx[2 * labs[uj].x + 1];
+            if (u < u1) open(u);  // the next unit's first vectors, on their way during the last steps
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const uint32_t cellp = __shfl_sync(FULL, my.cellp, i), sblk = __shfl_sync(FULL, my.blk, i);
+                if (cellp == ~0u) continue;  // the cell does not need this label
+                const FtCell c = it.par[i];
+                // the longest row is below 1,024 entries wherever words are packed, so kr, the squares and
+                // 4 kr^3 fit 32 bits; |S| k_q does too
+                const uint32_t kr = s.ka[i], k2 = kr * kr;
+                const int nS = c.nS;
+                const int64_t X = X64 ? (int64_t)s.X[i] : (int64_t)(uint32_t)((uint32_t)s.X[i] - (k2 << a.shift));
+                const int64_t N = X + (int64_t)(nS - (int)kr) * (int)(s.tot[i] & low) - (int64_t)(nS * c.kq) * (int)kr;
+                const uint32_t Z2 = (4u * k2 * kr - s.B3[i]) / 3u;
+                const int cc = nS - 2 * (int)kr;
+                const int64_t nr = (int64_t)Z2 + (int64_t)(int)k2 * (3 * nS - 5 * (int)kr) + (int64_t)(int)kr * (cc * cc);
+                const bool nan = c.nq == 0 || nr == 0;
+                const float v = nan ? __int_as_float(0x7fffffff)
+                                    : (float)(((double)N * c.rq) * (1.0 / sqrt((double)nr)));
+                if (valid) a.scores[(size_t)(sblk + ub) * 32 + lane] = v;
+                const uint32_t key = ord_key(v);
+                const uint32_t mn = __reduce_min_sync(FULL, valid ? key : 0xffffffffu);
+                const uint32_t mx = __reduce_max_sync(FULL, valid ? key : 0u);
+                if (lane == 0) {
+                    atomicMin(a.ext_min + cellp, mn);
+                    atomicMax(a.ext_max + cellp, mx);
+                }
+            }
+        }
+    }
+}
+
+size_t step_smem(const FtRounds& a) {
+    return sizeof(uint32_t) * ((size_t)a.eq_stride + a.nwords) + sizeof(uint32_t) * 2 * ((size_t)a.kcap / 32 + 2);
+}
+
+size_t scan_smem(int Wt, int copies) { return (size_t)(Wt + 1) * 16 * copies; }
+
+constexpr size_t kScanSmem = 221 * 1024;  // with the kernel's static shared memory (6 KB), under 227 KB
+
+template <int C>
+void launch_scan_c(const FtRounds& a, int k, bool x64, cudaStream_t s) {
+    const size_t smem = scan_smem(a.Wt, C);
+    auto kern = x64 ? ft_scan_kernel<C, true> : ft_scan_kernel<C, false>;
+    kern<<<device_sm_count(), SCAN_NW * 32, smem, s>>>(a, k);
+}
+
+template <int C>
+void scan_attr(int Wt) {
+    const int smem = (int)scan_smem(Wt, C);
+    SGR_CUDA(cudaFuncSetAttribute(ft_scan_kernel<C, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    SGR_CUDA(cudaFuncSetAttribute(ft_scan_kernel<C, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+}
+
+}  // namespace
+
+int ft_scan_copies(int Wt) {
+    for (int c = 8; c >= 1; c >>= 1)
+        if (scan_smem(Wt, c) <= kScanSmem) return c;
+    return 0;
+}
+
+void launch_row_runs(const float* data, const int32_t* idx, const int32_t* ptr, uint32_t n_rows, int longest,
+                     uint16_t* sorted, int32_t* n_groups, cudaStream_t s) {
+    if (!n_rows) return;
+    int cap = 32;
+    while (cap < longest) cap <<= 1;
+    const int wpb = std::max(1, std::min(8, (int)(96 * 1024 / (cap * 8))));
+    const size_t smem = (size_t)wpb * cap * 8;
+    SGR_CUDA(cudaFuncSetAttribute(row_runs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const unsigned blocks = std::min<unsigned>((n_rows + wpb - 1) / wpb, device_sm_count() * 8);
+    row_runs_kernel<<<blocks, 32 * wpb, smem, s>>>(data, idx, ptr, n_rows, cap, sorted, n_groups);
+    SGR_LAUNCH_CHECK();
+    count_launch();
+}
+
+void launch_row_groups(const uint16_t* sorted, const int32_t* ptr, const int32_t* slot_row, const int32_t* blk_voff,
+                       uint32_t n_slots, uint32_t pad, uint4* groups, cudaStream_t s) {
+    if (!n_slots) return;
+    row_groups_kernel<<<(n_slots + 127) / 128, 128, 0, s>>>(sorted, ptr, slot_row, blk_voff, n_slots, pad, groups);
+    SGR_LAUNCH_CHECK();
+    count_launch();
+}
+
+void launch_pair_masks(const uint32_t* ft_genes, const uint32_t* ft_idx, int L, int nwords, uint32_t* mask,
+                       cudaStream_t s) {
+    SGR_CUDA(cudaMemsetAsync(mask, 0, (size_t)L * L * nwords * sizeof(uint32_t), s));
+    pair_mask_kernel<<<std::max(1, std::min((L * L + 7) / 8, device_sm_count() * 8)), 256, 0, s>>>(ft_genes, ft_idx,
+                                                                                              L * L, nwords, mask);
+    SGR_LAUNCH_CHECK();
+    count_launch();
+}
+
+void launch_ft_cells(int n, const int32_t* list, const int* n_dev, int L, const uint8_t* flags,
+                     const uint32_t* ctidx, int32_t* cells, int64_t* blk_off, uint8_t* row_mask,
+                     int32_t* final_labels, int32_t* rounds, unsigned long long* counter, unsigned long long* cand,
+                     cudaStream_t s) {
+    if (n <= 0) return;
+    ft_cells_kernel<<<(n + 255) / 256, 256, 0, s>>>(n, list, n_dev, L, flags, ctidx, cells, blk_off, row_mask, final_labels,
+                                                    rounds, counter, cand);
+    SGR_LAUNCH_CHECK();
+    count_launch();
+}
+
+void launch_ft_sort_rows(const int32_t* cells, int n, const float* data, const int32_t* idx, const int32_t* ptr,
+                         int longest, uint16_t* s_gene, uint16_t* s_lo, uint16_t* s_hi, cudaStream_t s) {
+    if (n <= 0) return;
+    int cap = 32;
+    while (cap < longest) cap <<= 1;
+    const int wpb = std::max(1, std::min(8, (int)(96 * 1024 / (cap * 8))));
+    const size_t smem = (size_t)wpb * cap * 8;
+    SGR_CUDA(cudaFuncSetAttribute(ft_sort_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const int blocks = std::min((n + wpb - 1) / wpb, device_sm_count() * 16);
+    ft_sort_rows_kernel<<<blocks, 32 * wpb, smem, s>>>(cells, n, data, idx, ptr, cap, s_gene, s_lo, s_hi);
+    SGR_LAUNCH_CHECK();
+    count_launch();
+}
+
+int ft_step_grid(int n) { return std::max(1, std::min(n, device_sm_count() * STEP_CTAS)); }
+
+void ft_rounds_setup(const FtRounds& a, int copies) {
+    SGR_CUDA(cudaFuncSetAttribute(ft_step_kernel<STEP_NW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)step_smem(a)));
+    SGR_CUDA(cudaFuncSetAttribute(ft_step_kernel<STEP_NW_FEW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)step_smem(a)));
+    if (copies == 8) scan_attr<8>(a.Wt);
+    else if (copies == 4) scan_attr<4>(a.Wt);
+    else if (copies == 2) scan_attr<2>(a.Wt);
+    else scan_attr<1>(a.Wt);
+}
+
+// Step k, the cells that go on put in order, and the quads of round k.  n: no more cells than this.
+void launch_ft_step(const FtRounds& a, int k, int n, int32_t* scan_scratch, cudaStream_t s) {
+    // Few cells are ordered by counting the smaller keys (4,096 cells: 4,096 warps of 128 steps); more by a
+    // counting sort on a few more key bits than the cells are many, at most 20.
+    int bits = 0;
+    if (n > 4096) {
+        bits = 8;
+        while (bits < 20 && (1 << bits) < 16 * n) ++bits;
+        SGR_CUDA(cudaMemsetAsync(a.key_count, 0, sizeof(int32_t) << bits, s));
+    }
+    // With a CTA per SM or fewer, a cell's own latency decides: four times the warps for its gene set and
+    // its labels' quantiles.
+    if (n <= device_sm_count())
+        ft_step_kernel<STEP_NW_FEW><<<std::max(n, 1), STEP_NW_FEW * 32, step_smem(a), s>>>(a, k, bits);
+    else
+        ft_step_kernel<STEP_NW><<<ft_step_grid(n), STEP_NW * 32, step_smem(a), s>>>(a, k, bits);
+    SGR_LAUNCH_CHECK();
+    if (bits) {
+        int32_t* start = a.key_count + ((size_t)1 << bits);
+        launch_exclusive_scan(a.key_count, start, 1u << bits, scan_scratch, s);
+        ft_place_kernel<<<std::min((n + 255) / 256, device_sm_count() * 8), 256, 0, s>>>(a, k, bits, start);
+    } else {
+        ft_rank_kernel<<<std::max(1, std::min((n + 7) / 8, device_sm_count() * 8)), 256, 0, s>>>(a, k);
+    }
+    SGR_LAUNCH_CHECK();
+    const int blocks = std::max(1, std::min((n + 4 * PLAN_NW - 1) / (4 * PLAN_NW), device_sm_count() * 4));
+    ft_plan_kernel<<<blocks, PLAN_NW * 32, 0, s>>>(a, k);
+    SGR_LAUNCH_CHECK();
+    count_launch(3);
+}
+
+void launch_ft_scan(const FtRounds& a, int k, int copies, bool x64, cudaStream_t s) {
+    if (copies == 8) launch_scan_c<8>(a, k, x64, s);
+    else if (copies == 4) launch_scan_c<4>(a, k, x64, s);
+    else if (copies == 2) launch_scan_c<2>(a, k, x64, s);
+    else launch_scan_c<1>(a, k, x64, s);
+    SGR_LAUNCH_CHECK();
+    count_launch();
+}
+
+}  // namespace sgr

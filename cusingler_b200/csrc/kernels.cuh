@@ -282,4 +282,97 @@ void launch_ref_presort(const float* data, const int32_t* idx, const int32_t* pt
                         const int32_t* ell_len, uint32_t n_rows, int cap, uint32_t pad_gene, uint32_t* out,
                         cudaStream_t s);
 
+// ---- fine-tune by rounds over all cells (ft_rounds.cu) --------------------------------------------
+
+struct FtEntry {       // one candidate label of one cell on a label's work list
+    uint32_t cellp;    // cell * L + position in the cell's candidate list
+    uint32_t blk;      // first 32-row block of its scores
+};
+
+struct FtCell {        // a cell's query side in the current round
+    double rq;         // 1 / sqrt(nq)
+    int64_t nq;        // sum of squared doubled centred ranks over the gene set
+    int32_t nS, kq;    // genes of the set, the query's stored entries among them
+};
+
+struct FtQuad {        // four active cells of a round and the labels scanned for them together
+    int cell[4];       // the last repeated where there are fewer
+    int nq, n_lab, units;  // cells, labels, 32-row blocks of the labels
+};
+
+struct FtRounds {
+    // reference
+    const uint4* groups;        // row groups (two per vector), 32-row blocks
+    const int32_t* blk_base;    // per label: its first block
+    const int32_t* blk_voff;    // per block: first vector (blocks + 1)
+    const uint32_t* perm;       // per row slot in block order: its position in the label's row order
+    const uint32_t* ctidx;      // (start, len) per label
+    const int32_t* lorder;      // labels, longest first
+    const uint32_t* ft_genes;   // fine-tune pair lists (pool ids)
+    const uint32_t* ft_idx;     // (start, len) per ordered pair
+    const uint32_t* pair_mask;  // bits of each pair's whole list (nwords each), or nullptr
+    const int32_t* gene_thre;   // marker count per candidate count
+    const LabelQ* lq;           // quantile grid per label (start 0)
+    int L, Wt, nwords, eq_stride, shift;
+    int3 mul;                   // {16 x table copies, 2, -1}: run-time factors of the scan
+    float p, thre;
+    int times;
+    // query rows of the cells, compacted to the pool and sorted by value
+    const uint16_t *s_gene, *s_lo, *s_hi;
+    const int32_t* row_ptr;
+    int kcap;                   // longest row
+    const uint8_t* flags;
+    // batch of n_cells cells
+    const int32_t* cells;
+    const int64_t* blk_off;     // first score block of each cell (blk_base0 taken off)
+    int64_t blk_base0;
+    int n_cells;
+    uint8_t* top;               // n_cells x L candidate lists
+    int *ntop, *used;           // n_cells: list lengths, rounds run
+    FtCell* par;                // n_cells
+    uint32_t* eq;               // n_cells x eq_stride packed e-values
+    uint32_t *ext_min, *ext_max;  // n_cells x L score extremes (order keys)
+    uint32_t* blk_of;           // n_cells x L: first score block of each candidate
+    FtEntry* list;              // L x n_cells work lists (labels that one cell of its quad needs)
+    FtQuad* quads;              // ceil(n_cells / 4)
+    int2* q_label;              // per quad L: label, blocks of the quad's labels before it
+    FtEntry* q_entry;           // per quad L x 4: the cells' entries (cellp = ~0: label not needed)
+    unsigned long long* un;     // n_cells: the cells that go on, unordered (sort key << 32 | cell)
+    int* key_count;             // counts of the keys' leading bits and their scan (2 << 20 ints + 1)
+    int* act;                   // n_cells: the active cells in order
+    int* n_act;                 // 2: their number
+    int* n_list;                // 2 x 256 work-list lengths
+    int* queue;                 // 2 work-item counters
+    unsigned long long* stats;  // cell rounds, reference rows scored
+    float* scores;
+    float* nan_scratch;         // step grid x max_label
+    int max_label;
+    int32_t *final_labels, *rounds;
+    int* status;
+};
+
+// Copies of the scan's lookup table that fit shared memory for a pool of Wt genes (8, 4, 2, 1; 0: none).
+int ft_scan_copies(int Wt);
+void launch_row_runs(const float* data, const int32_t* idx, const int32_t* ptr, uint32_t n_rows, int longest,
+                     uint16_t* sorted, int32_t* n_groups, cudaStream_t s);
+void launch_row_groups(const uint16_t* sorted, const int32_t* ptr, const int32_t* slot_row, const int32_t* blk_voff,
+                       uint32_t n_slots, uint32_t pad, uint4* groups, cudaStream_t s);
+void launch_pair_masks(const uint32_t* ft_genes, const uint32_t* ft_idx, int L, int nwords, uint32_t* mask,
+                       cudaStream_t s);
+// n cells (or the first *n_dev of `list`): those with fewer than two candidates get their final label,
+// the others go to `cells` / `blk_off` (counter: cells << 36 | 32-row score blocks) and row_mask.
+void launch_ft_cells(int n, const int32_t* list, const int* n_dev, int L, const uint8_t* flags,
+                     const uint32_t* ctidx, int32_t* cells, int64_t* blk_off, uint8_t* row_mask,
+                     int32_t* final_labels, int32_t* rounds, unsigned long long* counter, unsigned long long* cand,
+                     cudaStream_t s);
+void launch_ft_sort_rows(const int32_t* cells, int n, const float* data, const int32_t* idx, const int32_t* ptr,
+                         int longest, uint16_t* s_gene, uint16_t* s_lo, uint16_t* s_hi, cudaStream_t s);
+int ft_step_grid(int n);
+// Function attributes of the step and scan kernels; call before the launches of a batch.
+void ft_rounds_setup(const FtRounds& a, int copies);
+// Step k over at most n cells and the quads of round k.  scan_scratch: launch_exclusive_scan's, 2^20 values.
+void launch_ft_step(const FtRounds& a, int k, int n, int32_t* scan_scratch, cudaStream_t s);
+// x64: the run sums in 64 bits (when 32 could overflow)
+void launch_ft_scan(const FtRounds& a, int k, int copies, bool x64, cudaStream_t s);
+
 }  // namespace sgr

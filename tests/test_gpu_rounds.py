@@ -1,0 +1,85 @@
+"""The fine-tune by rounds over all cells at the sizes where its layout has edges: lookup tables of 8, 4,
+2 and 1 copies (gene pools of about 1,100 to 8,000), labels around 32-row blocks, and cell counts around
+quads.  Labels and round counts are whole numbers and equal the oracle's."""
+
+import functools
+
+import numpy as np
+import pytest
+
+from cusingler_b200 import abi, synth
+from oracle import oracle as O
+from tests import helpers as H
+
+pytestmark = pytest.mark.gpu
+
+POOLS = {  # reference rows, genes, labels, density, marker block
+    "8 copies": (1200, 9000, 14, 0.05, (150, 220, 4.0, 6.0)),
+    "4 copies": (1500, 12000, 30, 0.03, (200, 300, 5.0, 8.0)),
+    "2 copies": (2000, 16000, 45, 0.02, (250, 330, 6.0, 10.0)),
+    "1 copy": (2600, 24000, 72, 0.015, (250, 330, 6.0, 10.0)),
+}
+
+
+WIDE = 0.4  # a threshold that keeps many candidates on well separated labels
+
+
+def _solve(prob, thre=0.05):
+    orc = O.Oracle(prob)
+    orc.train()
+    flags = orc.score(mode=1, thre=thre)[2].astype(np.uint8)
+    final, rounds = orc.finetune(mode=1, thre=thre)
+    return flags, final, rounds
+
+
+def _annotator(prob):
+    a = abi.Annotator(gpuid=0)
+    return a.train(prob.ref, prob.celltypes, prob.label_names, prob.ref_genes, prob.qry_genes)
+
+
+@functools.lru_cache(maxsize=None)
+def _pool(kind):
+    n_ref, n_genes, L, density, block = POOLS[kind]
+    w, ref, qry = synth.custom_dataset(n_ref, 40, n_genes, L, density, block=block, seed=5)
+    genes = synth.names("G", n_genes)
+    prob = O.Problem(ref, qry, synth.names("CT", L), ref.labels, genes, genes)
+    return prob, _solve(prob, WIDE)
+
+
+@pytest.mark.parametrize("kind", list(POOLS))
+@pytest.mark.parametrize("scan", [1, 2])
+def test_table_copies(kind, scan):
+    """Each table width, with 64-bit (1) and 32-bit (2) run sums."""
+    prob, (flags, final, rounds) = _pool(kind)
+    a = _annotator(prob)
+    copies = {"8 copies": 8, "4 copies": 4, "2 copies": 2, "1 copy": 1}[kind]
+    bytes_of = [16 * c * (len(a.u32(1)) + 1) for c in (copies, 2 * copies)]
+    assert bytes_of[0] <= 221 * 1024 and (copies == 8 or bytes_of[1] > 222 * 1024)
+    a.set_tuning(3, scan)
+    got, got_rounds = a.finetune(prob.qry, flags, thre=WIDE)
+    assert rounds.max() >= 2
+    assert np.array_equal(got, final) and np.array_equal(got_rounds, rounds)
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 4, 5, 7, 33, 131])
+def test_cell_counts_around_quads(n):
+    """The first n cells of a query alone: each cell's result depends on its own row only."""
+    prob = H.problem("families")
+    res = H.oracle_run("families", 1)
+    a = _annotator(prob)
+    got, rounds = a.finetune(prob.qry.rows(0, n), res["flags"][:n].astype(np.uint8))
+    assert np.array_equal(got, res["final"][:n]) and np.array_equal(rounds, res["rounds"][:n])
+
+
+def test_label_sizes_around_blocks():
+    """Labels of 1, 2, 31, 32, 33, 64, 65 and 129 reference cells."""
+    sizes = [1, 2, 31, 32, 33, 64, 65, 129]
+    w, ref, qry = synth.custom_dataset(3000, 150, 3000, len(sizes), 0.08, seed=23)
+    rows = np.concatenate([np.flatnonzero(ref.labels == lab)[:n] for lab, n in enumerate(sizes)])
+    ref = ref.take(rows)
+    assert [int(x) for x in np.bincount(ref.labels)] == sizes
+    genes = synth.names("G", ref.n_cols)
+    prob = O.Problem(ref, qry, synth.names("CT", len(sizes)), ref.labels, genes, genes)
+    flags, final, rounds = _solve(prob)
+    got, got_rounds = _annotator(prob).finetune(qry, flags)
+    assert np.array_equal(got, final) and np.array_equal(got_rounds, rounds)
