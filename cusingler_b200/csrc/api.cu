@@ -204,6 +204,8 @@ struct sgr_ctx {
     DevBuf<int> fr_keys;           // counts of the sort keys
     DevBuf<unsigned long long> fr_ctl;  // counters (FtCtl)
     DevBuf<float> fr_scores, fr_nan;
+    DevBuf<uint16_t> fr_ref_runs;  // FP32 order: the reference's entries by value, with their runs
+    bool fr_ref_runs_ready = false;
     unsigned long long* h_ft = nullptr;  // pinned: counters read back
     cudaEvent_t ev_ft[2] = {nullptr, nullptr};
 
@@ -579,6 +581,8 @@ void train(sgr_ctx* ctx, const sgr_csr* ref, const int32_t* celltypes, const cha
     ctx->R = ref->n_rows;
     ctx->ref_cols = ref->n_cols;
     ctx->ref_f16_ready = false;
+    ctx->fr_ref_runs_ready = false;
+    ctx->fr_ref_runs.release();
     if (ctx->device < 0) {  // host-only context: marker training only
         ctx->G = (int)mk.common.size();
         ctx->Kp = round_up(std::max(ctx->G, 1), 128);
@@ -1243,7 +1247,17 @@ struct FtCtl {
     int32_t n_list[2 * 256];
 };
 
-// Fine-tune by rounds over all cells (ft_rounds.cu), in exact mode; arguments as
+// FP32 order: the reference rows' thre-pool entries by value, each with its run (on first use).
+void ensure_ref_runs(sgr_ctx* ctx) {
+    if (ctx->fr_ref_runs_ready) return;
+    const size_t n = std::max<size_t>(ctx->reff_indices.n, 1);
+    uint16_t* r = ctx->fr_ref_runs.ensure(3 * n);
+    launch_ft_sort_rows(nullptr, (int)ctx->R, ctx->reff_data.p, ctx->reff_indices.p, ctx->reff_indptr.p, ctx->max_row, r,
+                        r + n, r + 2 * n, ctx->stream);
+    ctx->fr_ref_runs_ready = true;
+}
+
+// Fine-tune by rounds over all cells (ft_rounds.cu), in the context's arithmetic; arguments as
 // finetune_persistent.  Returns false when a query row is too long for it.  A batch's rounds are queued one ahead of the
 // host: the count of active cells after step k is read while the scan of round k runs.
 bool finetune_rounds(sgr_ctx* ctx, const DevCsr& q, const uint8_t* flags_dev, float p, float thre, int times,
@@ -1251,6 +1265,7 @@ bool finetune_rounds(sgr_ctx* ctx, const DevCsr& q, const uint8_t* flags_dev, fl
     cudaStream_t s = ctx->stream;
     const Markers& mk = ctx->mk;
     const uint32_t Q = q.n_rows, L = mk.n_labels, Wt = std::max<uint32_t>(ctx->Wt, 1);
+    const bool fp32 = ctx->mode == SGR_MODE_FP32REF;
     if (!ctx->h_ft) {
         SGR_CUDA(cudaMallocHost(reinterpret_cast<void**>(&ctx->h_ft), 2 * offsetof(FtCtl, queue)));
         for (auto& e : ctx->ev_ft) SGR_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
@@ -1326,6 +1341,14 @@ bool finetune_rounds(sgr_ctx* ctx, const DevCsr& q, const uint8_t* flags_dev, fl
     a.perm = ctx->fr_perm.p;
     a.ctidx = ctx->d_ctidx.p;
     a.lorder = ctx->d_lorder.p;
+    if (fp32) {
+        ensure_ref_runs(ctx);
+        const size_t n = ctx->fr_ref_runs.n / 3;
+        a.ref_gene = ctx->fr_ref_runs.p;
+        a.ref_lo = a.ref_gene + n;
+        a.ref_hi = a.ref_lo + n;
+        a.ref_ptr = ctx->reff_indptr.p;
+    }
     a.ft_genes = ctx->d_ft_genes.p;
     a.ft_idx = ctx->d_ft_idx.p;
     a.pair_mask = ctx->fr_masks ? ctx->fr_pair_mask.p : nullptr;
@@ -1391,10 +1414,11 @@ bool finetune_rounds(sgr_ctx* ctx, const DevCsr& q, const uint8_t* flags_dev, fl
         int most = a.n_cells;  // no more cells than this are active
         for (int r = 0;; ++r) {
             if (r > (int)L + 2) fail(SGR_ERR_STATE, "fine-tune rounds did not converge");
-            launch_ft_step(a, r, most, scan_scratch, s);
+            launch_ft_step(a, r, most, !fp32, scan_scratch, s);
             SGR_CUDA(cudaMemcpyAsync(host_ctl(r & 1), d, kRead, cudaMemcpyDeviceToHost, s));
             SGR_CUDA(cudaEventRecord(ctx->ev_ft[r & 1], s));
-            launch_ft_scan(a, r, ctx->ft_copies, x64, s);
+            if (fp32) launch_ft_scan32(a, r, most, s);
+            else launch_ft_scan(a, r, ctx->ft_copies, x64, s);
             if (r == 0) continue;
             SGR_CUDA(cudaEventSynchronize(ctx->ev_ft[(r - 1) & 1]));
             const FtCtl* c = host_ctl((r - 1) & 1);
@@ -1417,6 +1441,7 @@ bool finetune_by_rounds(sgr_ctx* ctx, const DevCsr& q, const uint8_t* flags_dev,
     cudaStream_t s = ctx->stream;
     const uint32_t Q = q.n_rows;
     if (!ctx->ft_copies || Q == 0) return false;
+    if (ctx->mode == SGR_MODE_FP32REF && !ft_scan32_warps((int)std::max<uint32_t>(ctx->Wt, 1))) return false;
     if (!finetune_rounds(ctx, q, flags_dev, p, thre, times, cell_list, n_list, out_row0)) return false;
     if (!final_labels) return true;
     SGR_CUDA(cudaMemcpyAsync(final_labels, ctx->d_final.p + out_row0, Q * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
@@ -1850,6 +1875,11 @@ void annotate_plain(sgr_ctx* ctx, const DevCsr& q, const sgr_csr* host, float qu
     if (ctx->mode == SGR_MODE_EXACT) {
         finetune_persistent(ctx, q, ctx->flags.p, quantile, finetune_thre, finetune_times, final_labels, nullptr);
     } else {
+        const int sp = ctx->prof.begin(ST_FT, s);
+        const bool done = finetune_by_rounds(ctx, q, ctx->flags.p, quantile, finetune_thre, finetune_times, final_labels,
+                                             nullptr);
+        ctx->prof.end(sp, s);
+        if (done) return;
         std::vector<uint8_t> fl((size_t)Q * L);
         SGR_CUDA(cudaMemcpyAsync(fl.data(), ctx->flags.p, fl.size(), cudaMemcpyDeviceToHost, s));
         check_status(ctx);
@@ -2355,11 +2385,15 @@ sgr_status sgr_finetune(sgr_ctx* ctx, const sgr_csr* qry, const uint8_t* flags, 
         reset_status(ctx);
         DevCsr q = query_on_device(ctx, qry);
         if (q.n_rows == 0) return;
+        ctx->flags.upload(flags, (size_t)q.n_rows * ctx->mk.n_labels, ctx->stream);
         if (ctx->mode == SGR_MODE_EXACT) {
-            ctx->flags.upload(flags, (size_t)q.n_rows * ctx->mk.n_labels, ctx->stream);
             finetune_persistent(ctx, q, ctx->flags.p, quantile, finetune_thre, finetune_times, final_labels, rounds);
         } else {
-            finetune_device(ctx, q, flags, quantile, finetune_thre, finetune_times, final_labels, rounds);
+            const int sp = ctx->prof.begin(ST_FT, ctx->stream);
+            const bool done = finetune_by_rounds(ctx, q, ctx->flags.p, quantile, finetune_thre, finetune_times,
+                                                 final_labels, rounds);
+            ctx->prof.end(sp, ctx->stream);
+            if (!done) finetune_device(ctx, q, flags, quantile, finetune_thre, finetune_times, final_labels, rounds);
         }
     });
 }

@@ -182,6 +182,7 @@ __global__ void __launch_bounds__(256) ft_cells_kernel(int n, const int32_t* lis
 }
 
 // One warp per cell: its pool entries by value, with each entry's run as positions [lo, hi).
+// cells = nullptr: rows 0 .. n - 1.
 __global__ void __launch_bounds__(256) ft_sort_rows_kernel(const int32_t* cells, int n, const float* data,
                                                            const int32_t* idx, const int32_t* ptr, int cap,
                                                            uint16_t* s_gene, uint16_t* s_lo, uint16_t* s_hi) {
@@ -189,7 +190,7 @@ __global__ void __launch_bounds__(256) ft_sort_rows_kernel(const int32_t* cells,
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpb = blockDim.x >> 5;
     uint64_t* keys = reinterpret_cast<uint64_t*>(smem) + (size_t)warp * cap;
     for (int i = blockIdx.x * wpb + warp; i < n; i += gridDim.x * wpb) {
-        const int beg = ptr[cells[i]], k = ptr[cells[i] + 1] - beg;
+        const int row = cells ? cells[i] : i, beg = ptr[row], k = ptr[row + 1] - beg;
         int m = 1;
         while (m < k) m <<= 1;
         for (int j = lane; j < m; j += 32)
@@ -881,6 +882,185 @@ __global__ void __launch_bounds__(SCAN_NW * 32, 1) ft_scan_kernel(FtRounds a, in
     }
 }
 
+// ---- FP32-order scan ------------------------------------------------------------------------------
+
+// The reference's spearman_reduce over one row (src/cusingler.cu:803-856): 128 contiguous gene chunks of
+// `step` genes, one FP32 multiply-add chain each, then the stride-doubling pairwise tree.  Lane t holds
+// chunks 4 t .. 4 t + 3; the sum is in lane 0.
+__device__ __forceinline__ float tree128(const float (&c)[4], int lane) {
+    float v = __fadd_rn(__fadd_rn(c[0], c[1]), __fadd_rn(c[2], c[3]));
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const float w = __shfl_down_sync(FULL, v, o);
+        if ((lane & (2 * o - 1)) == 0) v = __fadd_rn(v, w);
+    }
+    return v;
+}
+
+// Correlations of a round in the reference's FP32 order.  Work item: a cell and a part of its candidate
+// rows; one warp per row.  The ranks over S come from the row's value-sorted entries, as in the exact scan
+// (an entry's z is the kept entries before its run's end plus those before its start), so no row is sorted
+// or bucketed again.  They are scattered into a dense row in shared memory laid out [gene in chunk][chunk],
+// so that a lane reads its four chunks' next genes with one conflict-free 16-byte load.
+// Bound: issue (the row's passes over its entries and chunks).  1,000 queries x 20,000 reference cells,
+// 1,215 cell rounds of 13 candidates: 1,014 ms with the host's lists of (candidate set, row) rankings, 19 ms
+// for the 13.4e6 rows here (1.4 ns a row).
+// dense_len: floats of a dense row (128 x the longest chunk).  dynamic shared memory: the query's dense
+// row, one per warp, the slot of each pool gene (halfwords).
+__global__ void __launch_bounds__(256) ft_scan32_kernel(FtRounds a, int k, int dense_len, int parts) {
+    extern __shared__ __align__(16) unsigned char dyn[];
+    __shared__ int off[257];  // candidate rows before each label of the cell's list
+    __shared__ uint8_t top[256];
+    __shared__ int s_item;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarp = blockDim.x >> 5, NT = blockDim.x;
+    const int cur = k & 1, nxt = cur ^ 1;
+    float* x = reinterpret_cast<float*>(dyn);
+    float* y = x + (size_t)(1 + warp) * dense_len;
+    uint16_t* slot = reinterpret_cast<uint16_t*>(x + (size_t)(1 + nwarp) * dense_len);
+    int* pre = reinterpret_cast<int*>(x + dense_len);  // genes of S before each word; before the rows use y
+    if (blockIdx.x == 0 && tid == 0) {  // the next round's counters
+        a.queue[nxt] = 0;
+        a.n_act[cur] = 0;
+    }
+    const int n = a.n_act[nxt];
+    const uint32_t low = (1u << a.shift) - 1u;
+    for (;;) {
+        __syncthreads();
+        if (tid == 0) s_item = atomicAdd(a.queue + cur, 1);
+        __syncthreads();
+        const int item = s_item;
+        if (item >= n * parts) return;
+        const int c = a.act[item / parts], part = item % parts, ntop = a.ntop[c];
+        for (int i = tid; i < ntop; i += NT) top[i] = a.top[(size_t)c * a.L + i];
+        __syncthreads();
+        if (warp == 0) {
+            int acc = 0;
+            for (int base = 0; base < ntop; base += 32) {
+                const int i = base + lane, len = i < ntop ? (int)a.ctidx[2 * top[i] + 1] : 0;
+                const int incl = warp_incl_scan(len, lane);
+                if (i < ntop) off[i] = acc + incl - len;
+                acc += __shfl_sync(FULL, incl, 31);
+            }
+            if (lane == 0) off[ntop] = acc;
+        }
+        __syncthreads();
+        const int rows = off[ntop], per = max(2 * nwarp, (rows + parts - 1) / parts);
+        const int r0 = part * per, r1 = min(rows, r0 + per);
+        if (r0 >= rows) continue;  // a cell with fewer parts
+        // S in ascending gene order: position i is gene i % step of chunk i / step
+        const FtCell par = a.par[c];
+        const int nS = par.nS, step = (nS + 127) / 128;
+        const uint32_t* eq = a.eq + (size_t)c * a.eq_stride;
+        for (int w = warp; w < a.nwords; w += nwarp) {
+            const int g = 32 * w + lane;
+            const unsigned m = __ballot_sync(FULL, g < a.Wt && eq[g] != 0u);
+            if (lane == 0) pre[w] = __popc(m);
+        }
+        for (int i = tid; i < step * 128; i += NT) x[i] = 0.f;
+        __syncthreads();
+        if (warp == 0) {
+            int acc = 0;
+            for (int base = 0; base < a.nwords; base += 32) {
+                const int w = base + lane, v = w < a.nwords ? pre[w] : 0, incl = warp_incl_scan(v, lane);
+                if (w < a.nwords) pre[w] = acc + incl - v;
+                acc += __shfl_sync(FULL, incl, 31);
+            }
+        }
+        __syncthreads();
+        for (int w = warp; w < a.nwords; w += nwarp) {
+            const int g = 32 * w + lane;
+            const uint32_t e = g < a.Wt ? eq[g] : 0u;
+            const unsigned m = __ballot_sync(FULL, e != 0u);
+            const int i = pre[w] + __popc(m & ((1u << lane) - 1u)), ch = i / step, at = (i - ch * step) * 128 + ch;
+            if (g < a.Wt) slot[g] = e ? (uint16_t)at : (uint16_t)0xffff;
+            if (e) x[at] = (float)((int)(e & low) - par.kq) * 0.5f;
+        }
+        __syncthreads();  // pre (the first warp's row) is free again
+        const float4* x4 = reinterpret_cast<const float4*>(x);
+        float4* y4 = reinterpret_cast<float4*>(y);
+        float qn[4] = {0.f, 0.f, 0.f, 0.f};
+        for (int o = 0; o < step; ++o) {
+            const float4 v = x4[o * 32 + lane];
+            qn[0] = fmaf(v.x, v.x, qn[0]);
+            qn[1] = fmaf(v.y, v.y, qn[1]);
+            qn[2] = fmaf(v.z, v.z, qn[2]);
+            qn[3] = fmaf(v.w, v.w, qn[3]);
+        }
+        const float qf = tree128(qn, lane);
+        for (int r = r0 + warp; r < r1; r += nwarp) {
+            int lo = 0, hi = ntop - 1;  // off[lo] <= r < off[lo + 1]
+            while (lo < hi) {
+                const int mid = (lo + hi + 1) >> 1;
+                if (off[mid] <= r) lo = mid;
+                else hi = mid - 1;
+            }
+            const uint32_t start = a.ctidx[2 * top[lo]];
+            const int j = r - off[lo];
+            const uint32_t row = start + a.perm[start + j];
+            const int beg = a.ref_ptr[row], len = a.ref_ptr[row + 1] - beg, nwd = (len + 31) / 32;
+            // the row's entries inside S as bits: lane w holds entries 32 w ..
+            uint32_t in = 0;
+            for (int w = 0; w < nwd; ++w) {
+                const int e = 32 * w + lane;
+                const bool hit = e < len && slot[a.ref_gene[beg + e]] != 0xffffu;
+                const unsigned m = __ballot_sync(FULL, hit);
+                if (lane == w) in = m;
+            }
+            const int p = __popc(in), before = warp_incl_scan(p, lane) - p;
+            const int kr = __shfl_sync(FULL, before + p, 31);
+            // every gene of S at rank d = -k_r, then the stored ones
+            const float d0 = (float)(-kr) * 0.5f;
+            for (int o = 0; o < step; ++o) {
+                const int i = 4 * lane * step + o;
+                y4[o * 32 + lane] = make_float4(i < nS ? d0 : 0.f, i + step < nS ? d0 : 0.f,
+                                                i + 2 * step < nS ? d0 : 0.f, i + 3 * step < nS ? d0 : 0.f);
+            }
+            __syncwarp();
+            for (int w = 0; w < nwd; ++w) {
+                const int e = 32 * w + lane;
+                const uint32_t bits = __shfl_sync(FULL, in, w);
+                const bool hit = (bits >> lane) & 1u;
+                const int l0 = hit ? a.ref_lo[beg + e] : 0, h0 = hit ? a.ref_hi[beg + e] : 0;
+                const int z = __shfl_sync(FULL, before, l0 >> 5) +
+                              __popc(__shfl_sync(FULL, in, l0 >> 5) & ((1u << (l0 & 31)) - 1u)) +
+                              __shfl_sync(FULL, before, h0 >> 5) +
+                              __popc(__shfl_sync(FULL, in, h0 >> 5) & ((1u << (h0 & 31)) - 1u));
+                if (hit) y[slot[a.ref_gene[beg + e]]] = (float)(nS - 2 * kr + z) * 0.5f;
+            }
+            __syncwarp();
+            float d[4] = {0.f, 0.f, 0.f, 0.f}, rn[4] = {0.f, 0.f, 0.f, 0.f};
+            for (int o = 0; o < step; ++o) {
+                const float4 u = x4[o * 32 + lane], v = y4[o * 32 + lane];
+                d[0] = fmaf(u.x, v.x, d[0]);
+                d[1] = fmaf(u.y, v.y, d[1]);
+                d[2] = fmaf(u.z, v.z, d[2]);
+                d[3] = fmaf(u.w, v.w, d[3]);
+                rn[0] = fmaf(v.x, v.x, rn[0]);
+                rn[1] = fmaf(v.y, v.y, rn[1]);
+                rn[2] = fmaf(v.z, v.z, rn[2]);
+                rn[3] = fmaf(v.w, v.w, rn[3]);
+            }
+            const float s = tree128(d, lane), rf = tree128(rn, lane);
+            if (lane == 0) {
+                const float div = sqrtf(qf * rf);
+                const float v = div != 0.f ? s / div : __int_as_float(0x7fffffff);
+                const size_t cp = (size_t)c * a.L + lo;
+                a.scores[(size_t)a.blk_of[cp] * 32 + j] = v;
+                const uint32_t key = ord_key(v);
+                atomicMin(a.ext_min + cp, key);
+                atomicMax(a.ext_max + cp, key);
+            }
+            __syncwarp();
+        }
+    }
+}
+
+int dense_len_of(int Wt) { return (Wt + 127) / 128 * 128; }
+
+size_t scan32_smem(int Wt, int nwarp) {
+    return sizeof(float) * (size_t)(1 + nwarp) * dense_len_of(Wt) + sizeof(uint16_t) * (((size_t)Wt + 7) & ~size_t(7));
+}
+
 size_t step_smem(const FtRounds& a) {
     return sizeof(uint32_t) * ((size_t)a.eq_stride + a.nwords) + sizeof(uint32_t) * 2 * ((size_t)a.kcap / 32 + 2);
 }
@@ -981,7 +1161,7 @@ void ft_rounds_setup(const FtRounds& a, int copies) {
 }
 
 // Step k, the cells that go on put in order, and the quads of round k.  n: no more cells than this.
-void launch_ft_step(const FtRounds& a, int k, int n, int32_t* scan_scratch, cudaStream_t s) {
+void launch_ft_step(const FtRounds& a, int k, int n, bool quads, int32_t* scan_scratch, cudaStream_t s) {
     // Few cells are ordered by counting the smaller keys (4,096 cells: 4,096 warps of 128 steps); more by a
     // counting sort on a few more key bits than the cells are many, at most 20.
     int bits = 0;
@@ -1005,10 +1185,32 @@ void launch_ft_step(const FtRounds& a, int k, int n, int32_t* scan_scratch, cuda
         ft_rank_kernel<<<std::max(1, std::min((n + 7) / 8, device_sm_count() * 8)), 256, 0, s>>>(a, k);
     }
     SGR_LAUNCH_CHECK();
+    count_launch(2);
+    if (!quads) return;
     const int blocks = std::max(1, std::min((n + 4 * PLAN_NW - 1) / (4 * PLAN_NW), device_sm_count() * 4));
     ft_plan_kernel<<<blocks, PLAN_NW * 32, 0, s>>>(a, k);
     SGR_LAUNCH_CHECK();
-    count_launch(3);
+    count_launch();
+}
+
+int ft_scan32_warps(int Wt) {
+    for (int w = 8; w >= 1; --w)
+        if (scan32_smem(Wt, w) <= 200 * 1024) return w;
+    return 0;
+}
+
+void launch_ft_scan32(const FtRounds& a, int k, int n, cudaStream_t s) {
+    const int warps = ft_scan32_warps(a.Wt);
+    const size_t smem = scan32_smem(a.Wt, warps);
+    SGR_CUDA(cudaFuncSetAttribute(ft_scan32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    int per_sm = 0;
+    SGR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ft_scan32_kernel, 32 * warps, smem));
+    const int grid = device_sm_count() * std::max(1, per_sm);
+    // about eight items per CTA, so that the last ones do not leave the GPU idle
+    const int parts = std::max(1, (8 * grid + n - 1) / std::max(n, 1));
+    ft_scan32_kernel<<<grid, 32 * warps, smem, s>>>(a, k, dense_len_of(a.Wt), parts);
+    SGR_LAUNCH_CHECK();
+    count_launch();
 }
 
 void launch_ft_scan(const FtRounds& a, int k, int copies, bool x64, cudaStream_t s) {

@@ -308,6 +308,8 @@ struct FtRounds {
     const uint32_t* perm;       // per row slot in block order: its position in the label's row order
     const uint32_t* ctidx;      // (start, len) per label
     const int32_t* lorder;      // labels, longest first
+    const uint16_t *ref_gene, *ref_lo, *ref_hi;  // FP32 order: entries by value, with their runs (CSR order)
+    const int32_t* ref_ptr;
     const uint32_t* ft_genes;   // fine-tune pair lists (pool ids)
     const uint32_t* ft_idx;     // (start, len) per ordered pair
     const uint32_t* pair_mask;  // bits of each pair's whole list (nwords each), or nullptr
@@ -370,8 +372,11 @@ void launch_ft_sort_rows(const int32_t* cells, int n, const float* data, const i
 int ft_step_grid(int n);
 // Function attributes of the step and scan kernels; call before the launches of a batch.
 void ft_rounds_setup(const FtRounds& a, int copies);
-// Step k over at most n cells and the quads of round k.  scan_scratch: launch_exclusive_scan's, 2^20 values.
-void launch_ft_step(const FtRounds& a, int k, int n, int32_t* scan_scratch, cudaStream_t s);
+// Step k over at most n cells and (quads) the quads of round k.  scan_scratch: launch_exclusive_scan's, 2^20 values.
+void launch_ft_step(const FtRounds& a, int k, int n, bool quads, int32_t* scan_scratch, cudaStream_t s);
+// Round k's correlations in the reference's FP32 order.  ft_scan32_warps: 0 for a pool too wide for it.
+int ft_scan32_warps(int Wt);
+void launch_ft_scan32(const FtRounds& a, int k, int n, cudaStream_t s);
 // x64: the run sums in 64 bits (when 32 could overflow)
 void launch_ft_scan(const FtRounds& a, int k, int copies, bool x64, cudaStream_t s);
 

@@ -24,16 +24,16 @@ POOLS = {  # reference rows, genes, labels, density, marker block
 WIDE = 0.4  # a threshold that keeps many candidates on well separated labels
 
 
-def _solve(prob, thre=0.05):
+def _solve(prob, thre=0.05, mode=1):
     orc = O.Oracle(prob)
     orc.train()
-    flags = orc.score(mode=1, thre=thre)[2].astype(np.uint8)
-    final, rounds = orc.finetune(mode=1, thre=thre)
+    flags = orc.score(mode=mode, thre=thre)[2].astype(np.uint8)
+    final, rounds = orc.finetune(mode=mode, thre=thre)
     return flags, final, rounds
 
 
-def _annotator(prob):
-    a = abi.Annotator(gpuid=0)
+def _annotator(prob, mode=abi.MODE_EXACT):
+    a = abi.Annotator(gpuid=0, mode=mode)
     return a.train(prob.ref, prob.celltypes, prob.label_names, prob.ref_genes, prob.qry_genes)
 
 
@@ -61,6 +61,16 @@ def test_table_copies(kind, scan):
     assert np.array_equal(got, final) and np.array_equal(got_rounds, rounds)
 
 
+@pytest.mark.parametrize("kind", ["8 copies", "4 copies", "2 copies"])
+def test_fp32_order(kind):
+    """The FP32-order scan: gene sets of several lengths of its 128 chunks, over pools of 1,100 to 5,200 genes."""
+    prob = _pool(kind)[0]
+    flags, final, rounds = _solve(prob, WIDE, mode=0)
+    got, got_rounds = _annotator(prob, abi.MODE_FP32REF).finetune(prob.qry, flags, thre=WIDE)
+    assert rounds.max() >= 2
+    assert np.array_equal(got, final) and np.array_equal(got_rounds, rounds)
+
+
 @pytest.mark.parametrize("n", [1, 2, 3, 4, 5, 7, 33, 131])
 def test_cell_counts_around_quads(n):
     """The first n cells of a query alone: each cell's result depends on its own row only."""
@@ -71,7 +81,8 @@ def test_cell_counts_around_quads(n):
     assert np.array_equal(got, res["final"][:n]) and np.array_equal(rounds, res["rounds"][:n])
 
 
-def test_label_sizes_around_blocks():
+@pytest.mark.parametrize("mode", [abi.MODE_EXACT, abi.MODE_FP32REF])
+def test_label_sizes_around_blocks(mode):
     """Labels of 1, 2, 31, 32, 33, 64, 65 and 129 reference cells."""
     sizes = [1, 2, 31, 32, 33, 64, 65, 129]
     w, ref, qry = synth.custom_dataset(3000, 150, 3000, len(sizes), 0.08, seed=23)
@@ -80,6 +91,6 @@ def test_label_sizes_around_blocks():
     assert [int(x) for x in np.bincount(ref.labels)] == sizes
     genes = synth.names("G", ref.n_cols)
     prob = O.Problem(ref, qry, synth.names("CT", len(sizes)), ref.labels, genes, genes)
-    flags, final, rounds = _solve(prob)
-    got, got_rounds = _annotator(prob).finetune(qry, flags)
+    flags, final, rounds = _solve(prob, mode=0 if mode == abi.MODE_FP32REF else 1)
+    got, got_rounds = _annotator(prob, mode).finetune(qry, flags)
     assert np.array_equal(got, final) and np.array_equal(got_rounds, rounds)
