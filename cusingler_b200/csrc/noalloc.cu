@@ -33,10 +33,95 @@ struct LabelTable {
     LabelQ q[256];
 };
 
+constexpr int ROWS_NW = 16;  // warps of a CTA of the warp-per-row kernel
+
+// One warp per score row: every list without NaN (the fixed scratch is not used, so the grid is sized to
+// the GPU: three CTAs per SM, 48 warps).  A row with a list that the reference would sort with NaN in it is
+// left to select_noalloc_kernel, marked by first = -1.  8,000 rows x 20,000 scores in 30 labels: 1.56 ms
+// with the scratch-bound grid of select_noalloc_kernel alone (65 CTAs of 8 warps), 0.42 ms so.
+__global__ void __launch_bounds__(ROWS_NW * 32, 3) select_noalloc_rows_kernel(const float* scores, int64_t ld, int nq,
+                                                                             int L, const __grid_constant__ LabelTable lt,
+                                                                             float p, float thre, float* label_scores,
+                                                                             int32_t* first, uint8_t* flags) {
+    __shared__ int hist[ROWS_NW][256];
+    __shared__ float ls_all[ROWS_NW][256];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float* ls = ls_all[warp];
+    // a label's list widened to 16-byte bounds stays inside its row when rows start on 16 bytes
+    const bool pf = (ld % 4) == 0 && (reinterpret_cast<uintptr_t>(scores) & 15) == 0;
+    for (int q = blockIdx.x * ROWS_NW + warp; q < nq; q += gridDim.x * ROWS_NW) {
+        const float* row = scores + (size_t)q * ld;
+        auto prefetch_label = [&](int l) {  // into L2, two labels ahead (as in the score step's selection)
+            if (pf && lane == 0 && l < L) {
+                const LabelQ& d = lt.q[l];
+                const uintptr_t a0 = reinterpret_cast<uintptr_t>(row + d.start) & ~uintptr_t(15);
+                const uintptr_t a1 = (reinterpret_cast<uintptr_t>(row + d.start + d.len) + 15) & ~uintptr_t(15);
+                asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a0), "r"((uint32_t)(a1 - a0))
+                             : "memory");
+            }
+        };
+        prefetch_label(0);
+        prefetch_label(1);
+        bool sort = false;
+        for (int l = 0; l < L && !sort; ++l) {
+            prefetch_label(l + 2);
+            const LabelQ d = lt.q[l];
+            const float* v = row + d.start;
+            float r = v[0] == v[0] ? v[0] : __int_as_float(0x7fffffff);
+            if (d.kind != 0) {
+                bool nan = false, num = false;
+                uint32_t kmin = 0xffffffffu, kmax = 0u;
+                int i = lane;
+                for (; i + 96 < d.len; i += 128) {  // four independent loads in flight per lane
+                    const float x0 = v[i], x1 = v[i + 32], x2 = v[i + 64], x3 = v[i + 96];
+                    nan |= (x0 != x0) | (x1 != x1) | (x2 != x2) | (x3 != x3);
+                    num |= (x0 == x0) | (x1 == x1) | (x2 == x2) | (x3 == x3);
+                    const uint32_t u0 = ord_key(x0), u1 = ord_key(x1), u2 = ord_key(x2), u3 = ord_key(x3);
+                    kmin = min(min(kmin, min(u0, u1)), min(u2, u3));
+                    kmax = max(max(kmax, max(u0, u1)), max(u2, u3));
+                }
+                for (; i < d.len; i += 32) {
+                    const float x = v[i];
+                    nan |= x != x;
+                    num |= x == x;
+                    kmin = min(kmin, ord_key(x));
+                    kmax = max(kmax, ord_key(x));
+                }
+                nan = __any_sync(FULL, nan);
+                num = __any_sync(FULL, num);
+                kmin = __reduce_min_sync(FULL, kmin);
+                kmax = __reduce_max_sync(FULL, kmax);
+                if (nan && !num) r = __int_as_float(0x7fffffff);  // a constant query row: NaN at every grid position
+                else if (nan) sort = true;
+                else r = quantile_warp_core(v, d, p, hist[warp], nullptr, lane, nullptr, kmin, kmax, false);
+            }
+            if (lane == 0) ls[l] = r;
+        }
+        __syncwarp();
+        if (sort) {
+            if (lane == 0) first[q] = -1;
+            continue;
+        }
+        int mn = 0, mx = 0;
+        if (lane == 0) {
+            stl::minmax(ls, L, &mn, &mx);
+            first[q] = mx;
+        }
+        mx = __shfl_sync(FULL, mx, 0);
+        const float t = __fsub_rn(ls[mx], thre);
+        for (int l = lane; l < L; l += 32) {
+            label_scores[(size_t)q * L + l] = ls[l];
+            if (flags) flags[(size_t)q * L + l] = ls[l] >= t ? 1 : 0;
+        }
+        __syncwarp();
+    }
+}
+
+// A CTA per row, with the fixed scratch.  marked: only the rows that select_noalloc_rows_kernel left.
 __global__ void __launch_bounds__(256) select_noalloc_kernel(const float* scores, int64_t ld, int nq, int L,
                                                              const __grid_constant__ LabelTable lt, float p,
                                                              float thre, float* label_scores, int32_t* first,
-                                                             uint8_t* flags, float* scratch, int spw) {
+                                                             uint8_t* flags, float* scratch, int spw, bool marked) {
     __shared__ float ls[256];
     __shared__ int hist[8][256];
     __shared__ int s_mx;
@@ -50,6 +135,7 @@ __global__ void __launch_bounds__(256) select_noalloc_kernel(const float* scores
     __syncthreads();
     float* my_scratch = scratch + (size_t)(blockIdx.x * 8 + warp) * spw;
     for (int q = blockIdx.x; q < nq; q += gridDim.x) {
+        if (marked && first[q] != -1) continue;  // the same for every thread: written by the launch before
         const float* row = scores + (size_t)q * ld;
         for (int l = warp; l < L; l += 8) {
             const LabelQ d = lt.q[l];
@@ -132,9 +218,21 @@ extern "C" sgr_status sgr_select_labels_noalloc(const float* d_scores, int64_t l
         float* scratch = scratch_address(dev);
         const unsigned blocks =
             (unsigned)std::min<long>({(long)n_rows, fit_blocks, (long)device_sm_count() * 2});
+        // A CTA takes its row's labels eight at a time; a warp takes a row's labels one by one, but the grid
+        // runs 48 warps per SM.  So rows go to warps from the eighth turn of the CTAs on.
+        const bool by_warp = (long)n_rows > 8L * blocks;
+        if (by_warp) {
+            const unsigned row_blocks =
+                (unsigned)std::min<long>(((long)n_rows + ROWS_NW - 1) / ROWS_NW, (long)device_sm_count() * 3);
+            select_noalloc_rows_kernel<<<row_blocks, ROWS_NW * 32, 0, (cudaStream_t)stream>>>(
+                d_scores, ld, (int)n_rows, (int)n_labels, lt, quantile, finetune_thre, d_label_scores, d_first_labels,
+                d_flags);
+            SGR_CUDA(cudaGetLastError());
+            count_launch();
+        }
         select_noalloc_kernel<<<blocks, 256, 0, (cudaStream_t)stream>>>(
             d_scores, ld, (int)n_rows, (int)n_labels, lt, quantile, finetune_thre, d_label_scores, d_first_labels,
-            d_flags, scratch, (int)max_len);
+            d_flags, scratch, (int)max_len, by_warp);
         SGR_CUDA(cudaGetLastError());
         count_launch();
     } catch (const Error& e) {

@@ -79,3 +79,40 @@ def test_noalloc_rejects_oversized_and_bad_ranges():
     assert abi.select_labels_noalloc(1, 15, 1, bad, 0.8, 0.05, 1, 1, None) == 1       # out of range
     empty = np.array([0, 0], np.uint32)
     assert abi.select_labels_noalloc(1, 15, 1, empty, 0.8, 0.05, 1, 1, None) == 5     # EMPTY_LABEL
+
+
+@pytest.mark.parametrize("n_rows,L,pad", [(2400, 5, 0), (2401, 7, 3), (4999, 1, 1)])
+def test_noalloc_many_rows_with_nan_lists(n_rows, L, pad):
+    """Enough rows for the warp-per-row launch: rows without NaN, rows that are all NaN, rows with a NaN-bearing
+    list (left to the CTA-per-row launch), one-score labels and a row stride off 16 bytes, against the
+    oracle's percentile (std::sort order with NaN, as the reference's)."""
+    import torch
+
+    rng = np.random.default_rng(n_rows)
+    lens = rng.integers(1, 90, L)
+    if L > 1:
+        lens[0] = 1
+    starts = np.concatenate([[0], np.cumsum(lens)[:-1]])
+    ld = int(lens.sum()) + pad
+    raw = np.full((n_rows, ld), -5.0, np.float32)
+    raw[:, :lens.sum()] = rng.normal(0.4, 0.1, (n_rows, lens.sum())).astype(np.float32)
+    raw[::7, starts[-1]:starts[-1] + max(1, lens[-1] // 2)] = raw[::7, [starts[-1]]]  # ties
+    raw[11::311, :] = np.nan
+    for q in range(5, n_rows, 97):
+        raw[q, starts[-1] + int(rng.integers(lens[-1]))] = np.nan
+    ranges = np.stack([starts, lens], 1).astype(np.uint32).reshape(-1)
+    dev = torch.device("cuda", 0)
+    d = torch.from_numpy(raw).to(dev)
+    ls = torch.empty((n_rows, L), device=dev)
+    first = torch.empty(n_rows, dtype=torch.int32, device=dev)
+    flags = torch.empty((n_rows, L), dtype=torch.uint8, device=dev)
+    assert abi.select_labels_noalloc(d.data_ptr(), ld, n_rows, ranges, 0.8, 0.05, ls.data_ptr(), first.data_ptr(),
+                                     flags.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
+    ls, first, flags = ls.cpu().numpy(), first.cpu().numpy(), flags.cpu().numpy()
+    for q in sorted(set(range(0, n_rows, 41)) | set(range(5, n_rows, 97)) | set(range(11, n_rows, 311))):
+        want = np.array([O.percentile(raw[q, s:s + n], 0.8) for s, n in zip(starts, lens)], np.float32)
+        assert H.ulp_diff(ls[q], want).max() == 0, q
+        top = O.minmax(want)[1]
+        assert first[q] == top
+        with np.errstate(invalid="ignore"):
+            assert np.array_equal(flags[q], (want >= np.float32(want[top] - np.float32(0.05))).astype(np.uint8)), q
