@@ -28,45 +28,84 @@ __device__ __forceinline__ float to_f(__nv_bfloat16 v) { return __bfloat162float
 
 // C[m][n] (ldc) = sum_k A(m,k) B(k,n) (+ bias[n]) with A(m,k) = A[m*am + k*ak], B(k,n) = B[k*bk + n*bn].
 // epi 0: plain store; 1: + bias; 2: + bias, store pre-activation to Z and GELU to C.
-template <class TA, class TB>
-__global__ void __launch_bounds__(256) gemm_kernel(int M, int N, int K, const TA* A, int64_t am, int64_t ak,
-                                                   const TB* B, int64_t bk, int64_t bn, float* C, int64_t ldc,
-                                                   const float* bias, float* Z, int epi) {
-    __shared__ float As[16][64 + 1];
-    __shared__ float Bs[16][64 + 1];
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const int m0 = blockIdx.y * 64, n0 = blockIdx.x * 64;
-    float acc[4][4] = {};
-    for (int k0 = 0; k0 < K; k0 += 16) {
-        for (int i = threadIdx.x; i < 16 * 64; i += 256) {
-            const int kk = i / 64, mm = i % 64;
-            const int m = m0 + mm, k = k0 + kk;
-            As[kk][mm] = (m < M && k < K) ? to_f(A[m * am + k * ak]) : 0.f;
-            const int n = n0 + mm;
-            Bs[kk][mm] = (n < N && k < K) ? to_f(B[k * bk + n * bn]) : 0.f;
+// Every output is one chain of multiply-adds over k in ascending order, whatever the tile, so the choice of
+// a tile changes no bit.  BM x BN tile, TM x TN outputs per thread, BK steps of k per stage; the next stage
+// is loaded into registers while this one is multiplied, along whichever index is contiguous.
+// The weight gradients (256 x 256 and 256 x 30 outputs, 4,096 terms each) are bound by that chain: 64 x 64
+// tiles gave 16 and 4 CTAs, 32 x 16 tiles 128 and 16 (4,096-row step of 30 -> 256 -> 256 -> 30, with
+// colsum_kernel: 2.0 -> 0.5 ms).
+template <class TA, class TB, int BM, int BN, int TM, int TN, int BK>
+__global__ void __launch_bounds__((BM / TM) * (BN / TN)) gemm_kernel(int M, int N, int K, const TA* A, int64_t am,
+                                                                     int64_t ak, const TB* B, int64_t bk, int64_t bn,
+                                                                     float* C, int64_t ldc, const float* bias, float* Z,
+                                                                     int epi) {
+    constexpr int NT = (BM / TM) * (BN / TN), NA = BM * BK / NT, NB = BN * BK / NT;
+    static_assert(BM * BK % NT == 0 && BN * BK % NT == 0, "whole elements per thread");
+    __shared__ __align__(16) float As[BK][BM + 4];
+    __shared__ __align__(16) float Bs[BK][BN + 4];
+    const int tid = threadIdx.x, tx = tid % (BN / TN), ty = tid / (BN / TN);
+    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+    float ra[NA], rb[NB];
+    auto a_at = [&](int i, int& mm, int& kk) {
+        mm = ak == 1 ? i / BK : i % BM;
+        kk = ak == 1 ? i % BK : i / BM;
+    };
+    auto b_at = [&](int i, int& nn, int& kk) {
+        nn = bk == 1 ? i / BK : i % BN;
+        kk = bk == 1 ? i % BK : i / BN;
+    };
+    auto load = [&](int k0) {
+#pragma unroll
+        for (int t = 0; t < NA; ++t) {
+            int mm, kk;
+            a_at(tid + t * NT, mm, kk);
+            ra[t] = (m0 + mm < M && k0 + kk < K) ? to_f(A[(m0 + mm) * am + (k0 + kk) * ak]) : 0.f;
+        }
+#pragma unroll
+        for (int t = 0; t < NB; ++t) {
+            int nn, kk;
+            b_at(tid + t * NT, nn, kk);
+            rb[t] = (n0 + nn < N && k0 + kk < K) ? to_f(B[(k0 + kk) * bk + (n0 + nn) * bn]) : 0.f;
+        }
+    };
+    float acc[TM][TN] = {};
+    load(0);
+    for (int k0 = 0; k0 < K; k0 += BK) {
+#pragma unroll
+        for (int t = 0; t < NA; ++t) {
+            int mm, kk;
+            a_at(tid + t * NT, mm, kk);
+            As[kk][mm] = ra[t];
+        }
+#pragma unroll
+        for (int t = 0; t < NB; ++t) {
+            int nn, kk;
+            b_at(tid + t * NT, nn, kk);
+            Bs[kk][nn] = rb[t];
         }
         __syncthreads();
+        if (k0 + BK < K) load(k0 + BK);
 #pragma unroll
-        for (int kk = 0; kk < 16; ++kk) {
-            float a[4], b[4];
+        for (int kk = 0; kk < BK; ++kk) {
+            float a[TM], b[TN];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) a[i] = As[kk][ty * 4 + i];
+            for (int i = 0; i < TM; ++i) a[i] = As[kk][ty * TM + i];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) b[j] = Bs[kk][tx * 4 + j];
+            for (int j = 0; j < TN; ++j) b[j] = Bs[kk][tx * TN + j];
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
+            for (int i = 0; i < TM; ++i)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+                for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
         }
         __syncthreads();
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int m = m0 + ty * 4 + i;
+    for (int i = 0; i < TM; ++i) {
+        const int m = m0 + ty * TM + i;
         if (m >= M) continue;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int n = n0 + tx * 4 + j;
+        for (int j = 0; j < TN; ++j) {
+            const int n = n0 + tx * TN + j;
             if (n >= N) continue;
             float v = acc[i][j];
             if (epi >= 1) v += bias[n];
@@ -211,13 +250,42 @@ __global__ void gelu_back_kernel(const float* dH, const float* Z, float* dZ, int
     }
 }
 
-// column sums: db[n] = sum_m dZ[m][n]
-__global__ void colsum_kernel(const float* dZ, int M, int N, float* db) {
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= N) return;
+// column sums: db[n] = sum_m dZ[m][n], each one chain of additions over m in ascending order.  A CTA takes
+// 32 columns: all its threads bring 128 rows at a time into shared memory (the next rows into registers
+// meanwhile), one warp adds them.
+constexpr int COLSUM_ROWS = 128;
+
+__global__ void __launch_bounds__(256) colsum_kernel(const float* dZ, int M, int N, float* db) {
+    __shared__ float rows[COLSUM_ROWS][32];
+    constexpr int PER = COLSUM_ROWS * 32 / 256;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, n = blockIdx.x * 32 + lane;
+    float r[PER];
+    auto load = [&](int m0) {
+#pragma unroll
+        for (int t = 0; t < PER; ++t) {
+            const int m = m0 + warp + 8 * t;
+            r[t] = m < M && n < N ? dZ[(int64_t)m * N + n] : 0.f;
+        }
+    };
     float s = 0.f;
-    for (int m = 0; m < M; ++m) s += dZ[(int64_t)m * N + n];
-    db[n] = s;
+    load(0);
+    for (int m0 = 0; m0 < M; m0 += COLSUM_ROWS) {
+#pragma unroll
+        for (int t = 0; t < PER; ++t) rows[warp + 8 * t][lane] = r[t];
+        __syncthreads();
+        if (m0 + COLSUM_ROWS < M) load(m0 + COLSUM_ROWS);
+        if (warp == 0) {
+            const int most = min(COLSUM_ROWS, M - m0);
+            if (most == COLSUM_ROWS) {
+#pragma unroll 16
+                for (int m = 0; m < COLSUM_ROWS; ++m) s += rows[m][lane];
+            } else {
+                for (int m = 0; m < most; ++m) s += rows[m][lane];
+            }
+        }
+        __syncthreads();
+    }
+    if (warp == 0 && n < N) db[n] = s;
 }
 
 // softmax cross-entropy over rows of logits; writes dlogits = (p - onehot) / B and per-row loss.
@@ -305,8 +373,14 @@ __global__ void gather_rows_kernel(const float* X, const int32_t* yall, const in
 template <class TA, class TB>
 void gemm(int M, int N, int K, const TA* A, int64_t am, int64_t ak, const TB* B, int64_t bk, int64_t bn, float* C,
           int64_t ldc, const float* bias, float* Z, int epi, cudaStream_t s) {
-    dim3 grid((N + 63) / 64, (M + 63) / 64);
-    gemm_kernel<TA, TB><<<grid, 256, 0, s>>>(M, N, K, A, am, ak, B, bk, bn, C, ldc, bias, Z, epi);
+    // 64 x 64 tiles where they give every SM one; else 32 x 16 ones, eight times as many
+    if ((int64_t)((N + 63) / 64) * ((M + 63) / 64) >= device_sm_count()) {
+        dim3 grid((N + 63) / 64, (M + 63) / 64);
+        gemm_kernel<TA, TB, 64, 64, 4, 4, 16><<<grid, 256, 0, s>>>(M, N, K, A, am, ak, B, bk, bn, C, ldc, bias, Z, epi);
+    } else {
+        dim3 grid((N + 15) / 16, (M + 31) / 32);
+        gemm_kernel<TA, TB, 32, 16, 2, 2, 32><<<grid, 128, 0, s>>>(M, N, K, A, am, ak, B, bk, bn, C, ldc, bias, Z, epi);
+    }
     SGR_LAUNCH_CHECK();
     count_launch();
 }
@@ -440,21 +514,21 @@ void Mlp::backward(const float* X, const int32_t* y, int B, cudaStream_t s) {
     float* G = g.p;
     // layer 3: dW3[L x H] = dlogits^T h2, db3, dh2 = dlogits W3
     gemm<float, float>(L, H, B, dlogits.p, 1, L, h2.p, H, 1, G + off_w3, H, nullptr, nullptr, 0, s);
-    colsum_kernel<<<(L + 255) / 256, 256, 0, s>>>(dlogits.p, B, L, G + off_b3);
+    colsum_kernel<<<(L + 31) / 32, 256, 0, s>>>(dlogits.p, B, L, G + off_b3);
     count_launch();
     gemm<float, __nv_bfloat16>(B, H, L, dlogits.p, L, 1, W + off_w3, H, 1, dh.p, H, nullptr, nullptr, 0, s);
     gelu_back_kernel<<<blocks_for((int64_t)B * H), 256, 0, s>>>(dh.p, z2.p, dz.p, (int64_t)B * H);
     count_launch();
     // layer 2: dW2[H x H] = dz2^T h1, db2, dh1 = dz2 W2
     gemm<float, float>(H, H, B, dz.p, 1, H, h1.p, H, 1, G + off_w2, H, nullptr, nullptr, 0, s);
-    colsum_kernel<<<(H + 255) / 256, 256, 0, s>>>(dz.p, B, H, G + off_b2);
+    colsum_kernel<<<(H + 31) / 32, 256, 0, s>>>(dz.p, B, H, G + off_b2);
     count_launch();
     gemm<float, __nv_bfloat16>(B, H, H, dz.p, H, 1, W + off_w2, H, 1, dh.p, H, nullptr, nullptr, 0, s);
     gelu_back_kernel<<<blocks_for((int64_t)B * H), 256, 0, s>>>(dh.p, z1.p, dz.p, (int64_t)B * H);
     count_launch();
     // layer 1: dW1[H x L] = dz1^T X, db1
     gemm<float, float>(H, L, B, dz.p, 1, H, X, L, 1, G + off_w1, L, nullptr, nullptr, 0, s);
-    colsum_kernel<<<(H + 255) / 256, 256, 0, s>>>(dz.p, B, H, G + off_b1);
+    colsum_kernel<<<(H + 31) / 32, 256, 0, s>>>(dz.p, B, H, G + off_b1);
     count_launch();
     SGR_LAUNCH_CHECK();
 }
