@@ -195,7 +195,8 @@ class Annotator:
         """`ref`: an object with n_rows, n_cols, data, indices, indptr (host arrays)."""
         csr, keep = host_csr(ref.n_rows, ref.n_cols, ref.data, ref.indices, ref.indptr)
         ct = np.ascontiguousarray(celltypes, np.int32)
-        ln, rg, qg = _strs(label_names), _strs(ref_genes), _strs(qry_genes)
+        ln, rg = _strs(label_names), _strs(ref_genes)
+        qg = rg if qry_genes is ref_genes else _strs(qry_genes)
         self._check(self.L.sgr_train_ref(self.h, C.byref(csr), ct.ctypes.data, C.cast(ln, C.c_void_p),
                                          len(label_names), C.cast(rg, C.c_void_p), C.cast(qg, C.c_void_p),
                                          len(qry_genes)))

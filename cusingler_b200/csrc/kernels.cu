@@ -318,6 +318,32 @@ __global__ void __launch_bounds__(256) rank_kernel(RankLaunch a, int warp_bytes)
     }
 }
 
+// ---- reference rows ----------------------------------------------------------------------------
+
+__global__ void __launch_bounds__(256) check_columns_kernel(const int32_t* indices, int64_t n, uint32_t n_cols,
+                                                            int* status) {
+    int bad = 0;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        bad |= (uint32_t)__ldcs(indices + i) >= n_cols ? 1 : 0;
+    bad = __reduce_or_sync(FULL, bad);
+    if (bad && (threadIdx.x & 31) == 0) atomicOr(status, 1);
+}
+
+// One warp per row; both sides of the copy are contiguous (HBM traffic is what it takes).
+__global__ void __launch_bounds__(256) gather_rows_kernel(const float* data, const int32_t* indices,
+                                                          const int32_t* indptr, const uint32_t* order, uint32_t n_rows,
+                                                          const int32_t* out_ptr, float* out_data, int32_t* out_indices) {
+    const int lane = threadIdx.x & 31;
+    for (uint32_t j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; j < n_rows; j += (gridDim.x * blockDim.x) >> 5) {
+        const int src = indptr[order[j]], n = indptr[order[j] + 1] - src, dst = out_ptr[j];
+#pragma unroll 4
+        for (int i = lane; i < n; i += 32) {
+            out_data[dst + i] = __ldcs(data + src + i);
+            out_indices[dst + i] = __ldcs(indices + src + i);
+        }
+    }
+}
+
 // ---- CSR compaction --------------------------------------------------------------------------
 
 // row_mask (optional): rows with mask 0 are left empty.
@@ -803,6 +829,23 @@ void launch_rank(const RankLaunch& a, cudaStream_t s) {
     big.n_items_dev = a.n_overflow;
     big.overflow = nullptr;
     launch_rank_tier(big, 0, s);  // grid sized to the device: the row count is on the device
+}
+
+void launch_check_columns(const int32_t* indices, int64_t n, uint32_t n_cols, int* status, cudaStream_t s) {
+    if (n <= 0) return;
+    const unsigned blocks = (unsigned)std::min<int64_t>((n + 1023) / 1024, sm_count() * 8);
+    check_columns_kernel<<<blocks, 256, 0, s>>>(indices, n, n_cols, status);
+    SGR_LAUNCH_CHECK();
+    count_launch();
+}
+
+void launch_gather_rows(const float* data, const int32_t* indices, const int32_t* indptr, const uint32_t* order,
+                        uint32_t n_rows, const int32_t* out_ptr, float* out_data, int32_t* out_indices, cudaStream_t s) {
+    if (!n_rows) return;
+    const unsigned blocks = std::min<unsigned>((n_rows + 7) / 8, sm_count() * 8);
+    gather_rows_kernel<<<blocks, 256, 0, s>>>(data, indices, indptr, order, n_rows, out_ptr, out_data, out_indices);
+    SGR_LAUNCH_CHECK();
+    count_launch();
 }
 
 void launch_filter_count(const int32_t* indptr, const int32_t* indices, uint32_t n_rows, uint32_t n_cols,

@@ -84,6 +84,12 @@ void column_bits(const int32_t* colmap, uint32_t n_cols, uint32_t* bits, uint16_
 
 void launch_rank(const RankLaunch& a, cudaStream_t s);
 
+// Sets status bit 0 when one of the n column ids is not below n_cols.
+void launch_check_columns(const int32_t* indices, int64_t n, uint32_t n_cols, int* status, cudaStream_t s);
+// Row j of the output CSR (out_ptr given) is row order[j] of the input.
+void launch_gather_rows(const float* data, const int32_t* indices, const int32_t* indptr, const uint32_t* order,
+                        uint32_t n_rows, const int32_t* out_ptr, float* out_data, int32_t* out_indices, cudaStream_t s);
+
 // Compact a CSR to the columns with map[c] >= 0 (new column = map[c]); two passes.  row_max (may be
 // null, not cleared here): atomic maximum of the kept entries per row.
 void launch_filter_count(const int32_t* indptr, const int32_t* indices, uint32_t n_rows, uint32_t n_cols,

@@ -6,6 +6,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cmath>
+#include <cstring>
 #include <set>
 #include <string>
 #include <thread>
@@ -39,6 +40,16 @@ void run_parallel(int cores, size_t n, F f) {
 // otherwise each side keeps its own columns whose name is shared, renumbered in its own order.
 void intersect_genes(const HostCsr& ref, const char* const* ref_genes, const char* const* qry_genes,
                      uint32_t n_qry, Markers& m) {
+    // the same names in the same order (the usual case) are equal sets: nothing to sort
+    bool same = ref.n_cols == n_qry;
+    for (uint32_t i = 0; same && i < n_qry; ++i) same = std::strcmp(ref_genes[i], qry_genes[i]) == 0;
+    if (same) {
+        m.filter_genes = false;
+        m.ref_colmap.resize(n_qry);
+        for (uint32_t i = 0; i < n_qry; ++i) m.ref_colmap[i] = (int32_t)i;
+        m.qry_colmap = m.ref_colmap;
+        return;
+    }
     std::set<std::string> a, b;
     for (uint32_t i = 0; i < ref.n_cols; ++i) a.insert(ref_genes[i]);
     for (uint32_t i = 0; i < n_qry; ++i) b.insert(qry_genes[i]);

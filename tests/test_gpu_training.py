@@ -90,3 +90,22 @@ def test_pair_lists_longer_than_shared_memory():
     labels = np.repeat([0, 1], 40)
     X = (rng.gamma(2.0, 1.0, (labels.size, 10000)) + 3.0 * (labels[:, None] == 0)).astype(np.float32)
     _check(_dense_problem(X, labels, 2))
+
+
+@pytest.mark.parametrize("at", [0, -1])
+def test_reference_column_out_of_range_keeps_the_training_before(at):
+    """The column ids are checked on the device before anything of the context changes: a first or last
+    entry out of range is refused, and the earlier training still annotates."""
+    prob = H.problem("tiny")
+    a = abi.Annotator(gpuid=0, cores=8)
+    a.train(prob.ref, prob.celltypes, prob.label_names, prob.ref_genes, prob.qry_genes)
+    want = a.annotate(prob.qry)
+    for bad in (prob.ref.n_cols, -1):
+        indices = prob.ref.indices.copy()
+        indices[at] = bad
+        ref = synth.CSR(prob.ref.n_rows, prob.ref.n_cols, prob.ref.data, indices, prob.ref.indptr, prob.ref.labels)
+        with pytest.raises(abi.SgrError) as e:
+            a.train(ref, prob.celltypes, prob.label_names, prob.ref_genes, prob.qry_genes)
+        assert e.value.status == 1
+        got = a.annotate(prob.qry)
+        assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
