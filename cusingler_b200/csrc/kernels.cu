@@ -1017,6 +1017,16 @@ void launch_select_first(const float* scores, int64_t ld, int nq, int L, const L
                          const uint32_t* ext_min, const uint32_t* ext_max, int warps) {
     if (nq <= 0) return;
     const size_t stage_bytes = (((size_t)std::max(row_len, 1) * 4 + 15) & ~size_t(15));
+    if (warps < 0) {
+        // By size.  A staging CTA takes a row's labels 16 at a time, a warp one by one, so few rows go to CTAs;
+        // with many rows the warp form has more rows in flight and no barriers.  They meet at about 40 rows per
+        // SM where two staging CTAs fit an SM (us, CTA / warp form: 261 / 291 for 5,000 x 20,000 scores, 624 / 562
+        // for 12,345 x 20,000), and at 16 where only one does (527 / 546 for 2,400 x 40,000, 1,746 / 1,288 for
+        // 8,192 x 40,000).  Up to two turns of the 64-register form's 32 warps per SM, the 48 warps of the
+        // 40-register form finish earlier (1,288 against 1,492 at the last size), beyond they do not.
+        const long per_sm = stage_bytes <= 100 * 1024 ? 40 : 16;
+        warps = nq < per_sm * sm_count() ? 16 : nq < 64L * sm_count() ? 1 : 0;
+    }
     if (lorder && (warps == 0 || warps == 1)) {  // one warp per row, 16 warps per CTA
         auto kern = warps == 1 ? select_rows_kernel<16, 3> : select_rows_kernel<16, 2>;
         int per_sm = 0;
