@@ -160,6 +160,7 @@ struct sgr_ctx {
     DevBuf<uint32_t> ext_min, ext_max;  // per (query, label) score extremes of a score block
     DevBuf<RankItem> rank_overflow;  // rows ranked by the rank kernel's large-buffer tier
     DevBuf<int> rank_n_overflow;
+    int rank_cap = 384;          // entries of the rank kernel's first tier, from the trained reference's rows
     int limb_w = 0;              // split of the exact limbs (split_limbs), chosen at training
     int limb_base128 = 0;        // tuning: train with the base-128 split
     int corr_wide = 18;          // tuning: 128 x 256 form (8 / 16 epilogue warps, 18 overlapped), 0 128 x 160
@@ -424,6 +425,7 @@ void rank_range(sgr_ctx* ctx, const DevCsr& m, const RankGroup* group, int G, in
     a.cap = sort_cap(G);
     a.status = ctx->status.p;
     a.overflow = ctx->rank_overflow.ensure(std::max<uint32_t>(n, 1));
+    a.small_cap = ctx->rank_cap;
     a.n_overflow = ctx->rank_n_overflow.ensure(1);
     a.map_bits = map_bits;
     a.map_prefix = map_prefix;
@@ -660,12 +662,18 @@ void train(sgr_ctx* ctx, const sgr_csr* ref, const int32_t* celltypes, const cha
     DevCsr rm{ctx->ref_data.p, ctx->ref_indices.p, ctx->ref_indptr.p, ctx->R, ctx->ref_cols, (int64_t)indptr[ctx->R]};
     RankGroup g{ctx->ref_map_common.p, ctx->G, ctx->Kp, ctx->ref_limbs.p, ctx->ref_n2.p, ctx->ref_rinv.p,
                 ctx->ref_f32.p, ctx->limb_w};
+    ctx->rank_cap = 384;
+    int32_t n_over = 0;
     rank_rows(ctx, rm, g, RANK_LIMBS, NORM_SEQ, ctx->ref_bits.p, ctx->ref_prefix.p);
+    // where most rows overflow the first tier, queries would pass it in vain
+    if (sort_cap(ctx->G) > 384)
+        SGR_CUDA(cudaMemcpyAsync(&n_over, ctx->rank_n_overflow.p, sizeof(int), cudaMemcpyDeviceToHost, s));
     ctx->h_ref_n2.resize(ctx->R);
     SGR_CUDA(cudaMemcpyAsync(ctx->h_ref_n2.data(), ctx->ref_n2.p, ctx->R * sizeof(int64_t), cudaMemcpyDeviceToHost, s));
     // fine-tune: reference compacted to the thre pool, each row's entries sorted by value
     filter_csr(ctx, rm, ctx->ref_map_thre.p, ctx->reff_data, ctx->reff_indices, ctx->reff_indptr);
     // 32-row blocks per label: a block is as long as its longest row, rounded up to 4 entries
+    if (2 * (int64_t)n_over > (int64_t)ctx->R) ctx->rank_cap = 1024;
     std::vector<int32_t> fptr(ctx->R + 1);
     SGR_CUDA(cudaMemcpyAsync(fptr.data(), ctx->reff_indptr.p, (ctx->R + 1) * sizeof(int32_t), cudaMemcpyDeviceToHost,
                              s));
@@ -805,6 +813,9 @@ void correlate(sgr_ctx* ctx, bool fp32, const int8_t* A, int nq, uint32_t q0, fl
         launch_corr_simt(fp32, A, ctx->ref_limbs.p, nq, (int)ctx->R, ctx->G, ctx->Kp, ctx->q_f32.p + q0,
                          ctx->ref_f32.p, ctx->q_rinv.p + q0, ctx->ref_rinv.p, ctx->q_n2.p + q0, ctx->ref_n2.p, out,
                          ld, ctx->limb_w, ctx->stream);
+    else if (corr_few_fits(nq, (int)ctx->R, ctx->Kp))
+        launch_corr_few(A, ctx->ref_limbs.p, nq, (int)ctx->R, ctx->Kp, ctx->q_rinv.p + q0, ctx->ref_rinv.p, out, ld, ext,
+                        ctx->limb_w, ctx->stream);
     else
         launch_corr_tc(A, ctx->ref_limbs.p, nq, (int)ctx->R, ctx->Kp, ctx->q_rinv.p + q0, ctx->ref_rinv.p,
                        ctx->q_n2.p + q0, ctx->ref_n2.p, out, ld, ctx->status.p, ctx->stream, false, ext,

@@ -518,6 +518,89 @@ __global__ void __launch_bounds__(256) corr_simt_kernel(const int8_t* A, const i
     }
 }
 
+// ---- score-step correlation of a few queries ------------------------------------------------------
+//
+// A tensor-core tile holds 128 query rows, and a tile's time (28 us: its 30 K blocks and the epilogue) is the
+// same for one.  Up to NQ queries are multiplied on CUDA cores instead (dp4a on the same int8 limbs, the same
+// integers): one warp per reference row, 16-byte loads, the queries' planes in shared memory.  Bound: reading
+// the reference's planes once.  N = C (k1 P1 + P3) - (C - 1) P2 as in corr_tc.cu.
+template <int NQ>
+__global__ void __launch_bounds__(256) corr_few_kernel(const int8_t* A, const int8_t* B, int nq, int R, int Kp,
+                                                       const double* ra, const double* rb, float* out, int64_t ld,
+                                                       LabelExtremes ext, int k1, int cbase) {
+    extern __shared__ __align__(16) uint4 qs[];  // [query][plane][Kp / 16]
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpb = blockDim.x >> 5;
+    const int nv = Kp / 16, row_v = 3 * nv;
+    for (int i = threadIdx.x; i < NQ * row_v; i += blockDim.x)
+        qs[i] = __ldg(reinterpret_cast<const uint4*>(A) + (size_t)min(i / row_v, nq - 1) * row_v + i % row_v);
+    __syncthreads();
+    // each warp takes consecutive rows, so that a label's extremes are written once per warp
+    const int n_warps = gridDim.x * wpb, per = (R + n_warps - 1) / n_warps;
+    const int r0 = (blockIdx.x * wpb + warp) * per, r1 = min(R, r0 + per);
+    if (r0 >= r1) return;
+    const double rq = lane < nq ? ra[lane] : 0.0;  // lane q finishes query q
+    int lab = 0, lab_end = 0;
+    float mn = __int_as_float(0x7f800000), mx = -mn;
+    if (ext.kmin) {
+        int lo = 0, hi = ext.L - 1;
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (__ldg(ext.lstart + mid) <= r0) lo = mid;
+            else hi = mid - 1;
+        }
+        lab = lo;
+        lab_end = __ldg(ext.lstart + lab + 1);
+    }
+    auto flush = [&]() {
+        if (ext.kmin && lane < nq) {
+            atomicMin(ext.kmin + (size_t)lane * ext.L + lab, ord_key(mn));
+            atomicMax(ext.kmax + (size_t)lane * ext.L + lab, ord_key(mx));
+        }
+        mn = __int_as_float(0x7f800000);
+        mx = -mn;
+    };
+    for (int r = r0; r < r1; ++r) {
+        const uint4* b = reinterpret_cast<const uint4*>(B) + (size_t)r * row_v;
+        int P[NQ][3] = {};
+        for (int v = lane; v < nv; v += 32) {
+#pragma unroll
+            for (int plane = 0; plane < 3; ++plane) {
+                const uint4 x = __ldg(b + plane * nv + v);
+#pragma unroll
+                for (int q = 0; q < NQ; ++q) {
+                    const uint4 y = qs[q * row_v + plane * nv + v];
+                    int s = P[q][plane];
+                    s = __dp4a((int)x.x, (int)y.x, s);
+                    s = __dp4a((int)x.y, (int)y.y, s);
+                    s = __dp4a((int)x.z, (int)y.z, s);
+                    P[q][plane] = __dp4a((int)x.w, (int)y.w, s);
+                }
+            }
+        }
+        int64_t N = 0;
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+            const int p1 = __reduce_add_sync(FULL, P[q][0]), p2 = __reduce_add_sync(FULL, P[q][1]),
+                      p3 = __reduce_add_sync(FULL, P[q][2]);
+            if (lane == q) N = (int64_t)cbase * ((int64_t)k1 * p1 + p3) - (int64_t)(cbase - 1) * p2;
+        }
+        if (ext.kmin && r >= lab_end) {
+            flush();
+            do {
+                ++lab;
+                lab_end = __ldg(ext.lstart + lab + 1);
+            } while (r >= lab_end);
+        }
+        if (lane < nq) {
+            const float v = (float)(((double)N * rq) * rb[r]);
+            out[(size_t)lane * ld + r] = v;
+            mn = fminf(mn, v);
+            mx = fmaxf(mx, v);
+        }
+    }
+    flush();
+}
+
 // ---- per-label quantile ------------------------------------------------------------------------
 
 // STAGE: the block first copies the query's score row (row_len floats) into shared memory with
@@ -813,7 +896,7 @@ void column_bits(const int32_t* colmap, uint32_t n_cols, uint32_t* bits, uint16_
 
 void launch_rank(const RankLaunch& a, cudaStream_t s) {
     if (a.n_items == 0) return;
-    constexpr int kSmallCap = 384;  // 3 CTAs of 8 warps per SM with a 1,152-column stage
+    const int kSmallCap = a.small_cap;
     if (!a.overflow || a.cap <= kSmallCap) {
         RankLaunch b = a;
         b.overflow = nullptr;
@@ -976,6 +1059,26 @@ void launch_corr_simt(bool fp32ref, const int8_t* A, const int8_t* B, int nq, in
         corr_simt_kernel<true><<<grid, 256, 0, s>>>(A, B, nq, R, G, Kp, fa, fb, ra, rb, na, nb, scores, ld, m);
     else
         corr_simt_kernel<false><<<grid, 256, 0, s>>>(A, B, nq, R, G, Kp, fa, fb, ra, rb, na, nb, scores, ld, m);
+    SGR_LAUNCH_CHECK();
+    count_launch();
+}
+
+// One query (18 us at 20,000 reference rows, 13 at 1,900; the tensor-core form 29 and 28), and up to eight
+// against few rows: each costs 1 us more at 1,900 rows and 4 at 20,000 (shared-memory reads).
+bool corr_few_fits(int nq, int R, int Kp) {
+    return (nq == 1 || (nq <= 8 && (int64_t)nq * R <= 40000)) && (size_t)8 * 3 * Kp <= 96 * 1024;
+}
+
+void launch_corr_few(const int8_t* A, const int8_t* B, int nq, int R, int Kp, const double* ra, const double* rb,
+                     float* scores, int64_t ld, LabelExtremes ext, int limb_w, cudaStream_t s) {
+    if (nq <= 0 || R <= 0) return;
+    const int k1 = limb_w ? 1 : 127, cbase = limb_w ? limb_w * limb_w + 1 : 128;
+    const int n = nq <= 1 ? 1 : nq <= 2 ? 2 : nq <= 4 ? 4 : 8;
+    auto kern = n == 1 ? corr_few_kernel<1> : n == 2 ? corr_few_kernel<2> : n == 4 ? corr_few_kernel<4> : corr_few_kernel<8>;
+    const size_t smem = (size_t)n * 3 * Kp;
+    SGR_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const int blocks = std::min((R + 7) / 8, sm_count() * 4);
+    kern<<<blocks, 256, smem, s>>>(A, B, nq, R, Kp, ra, rb, scores, ld, ext, k1, cbase);
     SGR_LAUNCH_CHECK();
     count_launch();
 }

@@ -65,10 +65,11 @@ struct RankLaunch {
     int max_Kp;                 // largest Kp over the groups (smem sizing)
     int cap;                    // sort capacity per warp (power of two)
     int* status;                // device flags: bit0 column out of range, bit1 NaN value
-    // Two-tier launch: when `overflow` is set, launch_rank ranks rows of at most 384 marker entries
+    // Two-tier launch: when `overflow` is set, launch_rank ranks rows of at most small_cap marker entries
     // with a small sort buffer (more warps per SM) and appends the other rows to `overflow`
     // (capacity n_items), which a second launch with `cap` ranks; `n_overflow` is one device int.
     RankItem* overflow = nullptr;
+    int small_cap = 384;  // 3 CTAs of 8 warps per SM; 1,024 where most rows hold more entries than 384
     int* n_overflow = nullptr;
     const int* n_items_dev = nullptr;  // item count read from device memory (second tier)
     // Optional compact form of the (one) column map every group shares, kept in shared memory: bit c
@@ -194,6 +195,10 @@ struct LabelExtremes {
     uint32_t* kmax = nullptr;
 };
 
+// Exact scores of at most 8 queries on CUDA cores (the same integers, bit-identical to launch_corr_tc's).
+bool corr_few_fits(int nq, int R, int Kp);
+void launch_corr_few(const int8_t* A, const int8_t* B, int nq, int R, int Kp, const double* ra, const double* rb,
+                     float* scores, int64_t ld, LabelExtremes ext, int limb_w, cudaStream_t s);
 // gm: row bands per group of the tile order (the bands of a group sweep the reference tiles together,
 // so the CTAs at work share them through L2); 1 visits band after band.
 // limb_w: the split of the exact limbs (split_limbs; 0 = base 128).  wide_warps 8 or 16 (with

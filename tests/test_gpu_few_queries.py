@@ -1,0 +1,28 @@
+"""Scores of a few queries (the CUDA-core correlation, up to 8 rows) and of one row more (the tensor cores)
+equal the oracle's exact scores bit for bit, for either limb split."""
+
+import numpy as np
+import pytest
+
+from cusingler_b200 import abi
+from tests import helpers as H
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("kind", ["tiny", "families", "small"])
+@pytest.mark.parametrize("base128", [0, 1])
+def test_few_queries(kind, base128):
+    prob = H.problem(kind)
+    res = H.oracle_run(kind, 1)
+    a = abi.Annotator(gpuid=0)
+    a.set_tuning(11, base128)
+    a.train(prob.ref, prob.celltypes, prob.label_names, prob.ref_genes, prob.qry_genes)
+    for n in (1, 2, 3, 4, 5, 8, 9):
+        for at in (0, 37):
+            q = prob.qry.rows(at, at + n)
+            assert H.ulp_diff(a.debug_scores(q), res["raw"][at:at + n]).max() == 0
+            first, scores, flags = a.score_first(q)
+            assert H.ulp_diff(scores, res["scores"][at:at + n]).max() == 0
+            assert np.array_equal(first, res["first"][at:at + n])
+            assert np.array_equal(flags, res["flags"][at:at + n].astype(np.uint8))
