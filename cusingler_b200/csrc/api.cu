@@ -1270,7 +1270,7 @@ cudaStream_t side_stream(sgr_ctx* ctx) {
 // Counters of the fine-tune by rounds on the device.
 struct FtCtl {
     unsigned long long counter, cand;  // cells to fine-tune << 36 | their score blocks; their candidates
-    int32_t total, longest;            // entries of their compacted rows; the longest row
+    int32_t longest, pad;              // longest of their compacted rows (this batch's)
     int32_t n_act[2];                  // cells that go on (by the parity of the round)
     unsigned long long stats[2];       // cell rounds, reference rows scored
     int32_t queue[2];
@@ -1282,15 +1282,15 @@ void ensure_ref_runs(sgr_ctx* ctx) {
     if (ctx->fr_ref_runs_ready) return;
     const size_t n = std::max<size_t>(ctx->reff_indices.n, 1);
     uint16_t* r = ctx->fr_ref_runs.ensure(3 * n);
-    launch_ft_sort_rows(nullptr, (int)ctx->R, ctx->reff_data.p, ctx->reff_indices.p, ctx->reff_indptr.p, ctx->max_row, r,
+    launch_ft_sort_rows((int)ctx->R, ctx->reff_data.p, ctx->reff_indices.p, ctx->reff_indptr.p, ctx->max_row, r,
                         r + n, r + 2 * n, ctx->stream);
     ctx->fr_ref_runs_ready = true;
 }
 
 // Fine-tune by rounds over all cells (ft_rounds.cu), in the context's arithmetic; arguments as
-// finetune_persistent.  Returns false when a query row is too long for it.  A batch's rounds are queued one ahead of the
+// finetune_persistent.  A batch's rounds are queued one ahead of the
 // host: the count of active cells after step k is read while the scan of round k runs.
-bool finetune_rounds(sgr_ctx* ctx, const DevCsr& q, const uint8_t* flags_dev, float p, float thre, int times,
+void finetune_rounds(sgr_ctx* ctx, const DevCsr& q, const uint8_t* flags_dev, float p, float thre, int times,
                      const int32_t* cell_list, const int* n_list, uint32_t out_row0) {
     cudaStream_t s = ctx->stream;
     const Markers& mk = ctx->mk;
@@ -1308,34 +1308,16 @@ bool finetune_rounds(sgr_ctx* ctx, const DevCsr& q, const uint8_t* flags_dev, fl
     ctx->d_rounds.ensure((size_t)out_row0 + Q);
     ctx->fr_cells.ensure(Q);
     ctx->fr_blk_off.ensure(Q);
-    uint8_t* mask = ctx->ft_row_mask.ensure(Q);
-    SGR_CUDA(cudaMemsetAsync(mask, 0, Q, s));
     launch_ft_cells((int)Q, cell_list, n_list, (int)L, flags_dev, ctx->d_ctidx.p, ctx->fr_cells.p, ctx->fr_blk_off.p,
-                    mask, ctx->d_final.p + out_row0, ctx->d_rounds.p + out_row0, &d->counter, &d->cand, s);
-    // the cells' rows, compacted to the thre pool
-    ctx->counts.ensure((size_t)Q + 1);
-    ctx->qf_indptr.ensure((size_t)Q + 1);
-    launch_filter_count(q.indptr, q.indices, Q, q.n_cols, ctx->qry_map_thre.p, ctx->counts.p, s, mask, &d->longest);
-    launch_exclusive_scan(ctx->counts.p, ctx->qf_indptr.p, Q, ctx->scan_part.ensure(2 * (((size_t)Q + 4095) / 4096) + 1),
-                          s);
-    SGR_CUDA(cudaMemcpyAsync(&d->total, ctx->qf_indptr.p + Q, sizeof(int32_t), cudaMemcpyDeviceToDevice, s));
+                    ctx->d_final.p + out_row0, ctx->d_rounds.p + out_row0, &d->counter, &d->cand, s);
     SGR_CUDA(cudaMemcpyAsync(ctx->h_ft, d, kRead, cudaMemcpyDeviceToHost, s));
     SGR_CUDA(cudaStreamSynchronize(s));
     const FtCtl h = *host_ctl(0);
     const int64_t n_cells = (int64_t)(h.counter >> 36), n_blocks = (int64_t)(h.counter & ((1ull << 36) - 1));
-    if (h.longest > 8192) return false;
     ctx->prof.acc.ft_cells += (uint64_t)n_cells;
     ctx->prof.acc.ft_candidates += h.cand;
     ctx->prof.acc.ft_split_cells += (uint64_t)n_cells;
-    if (n_cells == 0) return true;
-    const size_t total = std::max<int32_t>(h.total, 1);
-    ctx->qf_data.ensure(total);
-    ctx->qf_indices.ensure(total);
-    launch_filter_fill(q.data, q.indptr, q.indices, Q, q.n_cols, ctx->qry_map_thre.p, ctx->qf_indptr.p, ctx->qf_data.p,
-                       ctx->qf_indices.p, s, mask);
-    uint16_t* sorted = ctx->fr_sorted.ensure(3 * total);
-    launch_ft_sort_rows(ctx->fr_cells.p, (int)n_cells, ctx->qf_data.p, ctx->qf_indices.p, ctx->qf_indptr.p, h.longest,
-                        sorted, sorted + total, sorted + 2 * total, s);
+    if (n_cells == 0) return;
     uint32_t max_label = 1;
     std::vector<LabelQ> lq(L);
     for (uint32_t l = 0; l < L; ++l) {
@@ -1393,14 +1375,15 @@ bool finetune_rounds(sgr_ctx* ctx, const DevCsr& q, const uint8_t* flags_dev, fl
     a.p = p;
     a.thre = thre;
     a.times = times;
+    const int row_stride = round_up((int)Wt, 8);
+    uint16_t* sorted = ctx->fr_sorted.ensure(3 * (size_t)nb * row_stride);
     a.s_gene = sorted;
-    a.s_lo = sorted + total;
-    a.s_hi = sorted + 2 * total;
-    a.row_ptr = ctx->qf_indptr.p;
-    a.kcap = h.longest;
+    a.s_lo = sorted + (size_t)nb * row_stride;
+    a.s_hi = sorted + 2 * (size_t)nb * row_stride;
+    a.row_stride = row_stride;
     a.flags = flags_dev;
     a.top = ctx->fr_top.ensure((size_t)nb * L);
-    int* ints = ctx->fr_ints.ensure((size_t)nb * 3);
+    int* ints = ctx->fr_ints.ensure((size_t)nb * 4);
     a.ntop = ints;
     a.used = ints + nb;
     a.par = ctx->fr_par.ensure(nb);
@@ -1417,6 +1400,7 @@ bool finetune_rounds(sgr_ctx* ctx, const DevCsr& q, const uint8_t* flags_dev, fl
     a.quads = ctx->fr_quads.ensure(n_quads);
     a.q_label = ctx->fr_q_label.ensure(n_quads * L);
     a.act = ints + 2 * nb;
+    a.row_len = ints + 3 * nb;
     a.n_list = d->n_list;
     a.queue = d->queue;
     a.n_act = d->n_act;
@@ -1429,9 +1413,11 @@ bool finetune_rounds(sgr_ctx* ctx, const DevCsr& q, const uint8_t* flags_dev, fl
     a.rounds = ctx->d_rounds.p + out_row0;
     a.status = ctx->status.p;
     // 32-bit run sums: X = sum z s <= 2 k (e-sum of the kept entries), each e below 2 Wt and all of the
-    // query's e together k_q |S|
+    // query's e together k_q |S|, k_q at most the longest query row.  That row is read back only where the
+    // pool's width alone does not decide.
     const int64_t k = ctx->max_row;
-    const bool x64 = ctx->pack_scan != 2 || 2 * k * std::min<int64_t>(2 * k, h.longest) * (int64_t)Wt >= (int64_t(1) << 32);
+    auto narrow = [&](int64_t longest) { return 2 * k * std::min<int64_t>(2 * k, longest) * (int64_t)Wt < (int64_t(1) << 32); };
+    const bool ask_longest = ctx->pack_scan == 2 && !fp32 && !narrow(Wt) && narrow(1);
     ft_rounds_setup(a, ctx->ft_copies);
     for (size_t b = 0; b + 1 < cuts.size(); ++b) {
         a.cells = ctx->fr_cells.p + cuts[b];
@@ -1440,6 +1426,10 @@ bool finetune_rounds(sgr_ctx* ctx, const DevCsr& q, const uint8_t* flags_dev, fl
         a.n_cells = (int)(cuts[b + 1] - cuts[b]);
         if (b > 0) SGR_CUDA(cudaMemsetAsync(d, 0, sizeof(FtCtl), s));
         SGR_CUDA(cudaMemsetAsync(a.used, 0, a.n_cells * sizeof(int), s));
+        launch_ft_rows(a.cells, a.n_cells, q.data, q.indices, q.indptr, q.n_cols, ctx->qry_map_thre.p, (int)Wt, row_stride,
+                       sorted, sorted + (size_t)nb * row_stride, sorted + 2 * (size_t)nb * row_stride, ints + 3 * nb,
+                       &d->longest, s);
+        bool x64 = ctx->pack_scan != 2 || !narrow(Wt);
         // each round drops at least one candidate, so L rounds finish every cell
         int most = a.n_cells;  // no more cells than this are active
         for (int r = 0;; ++r) {
@@ -1447,6 +1437,10 @@ bool finetune_rounds(sgr_ctx* ctx, const DevCsr& q, const uint8_t* flags_dev, fl
             launch_ft_step(a, r, most, !fp32, scan_scratch, s);
             SGR_CUDA(cudaMemcpyAsync(host_ctl(r & 1), d, kRead, cudaMemcpyDeviceToHost, s));
             SGR_CUDA(cudaEventRecord(ctx->ev_ft[r & 1], s));
+            if (r == 0 && ask_longest) {
+                SGR_CUDA(cudaEventSynchronize(ctx->ev_ft[0]));
+                x64 = !narrow(host_ctl(0)->longest);
+            }
             if (fp32) launch_ft_scan32(a, r, most, s);
             else launch_ft_scan(a, r, ctx->ft_copies, x64, s);
             if (r == 0) continue;
@@ -1460,11 +1454,10 @@ bool finetune_rounds(sgr_ctx* ctx, const DevCsr& q, const uint8_t* flags_dev, fl
             break;
         }
     }
-    return true;
 }
 
-// The fine-tune by rounds where the trained reference and the query's rows allow it, and its results on
-// the host (final_labels: null when the caller reads ctx->d_final itself).
+// The fine-tune by rounds where the trained reference allows it, and its results on the host
+// (final_labels: null when the caller reads ctx->d_final itself).
 bool finetune_by_rounds(sgr_ctx* ctx, const DevCsr& q, const uint8_t* flags_dev, float p, float thre, int times,
                         int32_t* final_labels, int32_t* rounds_out, const int32_t* cell_list = nullptr,
                         const int* n_list = nullptr, uint32_t out_row0 = 0) {
@@ -1472,7 +1465,7 @@ bool finetune_by_rounds(sgr_ctx* ctx, const DevCsr& q, const uint8_t* flags_dev,
     const uint32_t Q = q.n_rows;
     if (!ctx->ft_copies || Q == 0) return false;
     if (ctx->mode == SGR_MODE_FP32REF && !ft_scan32_warps((int)std::max<uint32_t>(ctx->Wt, 1))) return false;
-    if (!finetune_rounds(ctx, q, flags_dev, p, thre, times, cell_list, n_list, out_row0)) return false;
+    finetune_rounds(ctx, q, flags_dev, p, thre, times, cell_list, n_list, out_row0);
     if (!final_labels) return true;
     SGR_CUDA(cudaMemcpyAsync(final_labels, ctx->d_final.p + out_row0, Q * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
     if (rounds_out)

@@ -126,11 +126,11 @@ __global__ void pair_mask_kernel(const uint32_t* ft_genes, const uint32_t* ft_id
 // ---- per call: the cells to fine-tune ----------------------------------------------------------
 
 // Cells with fewer than two candidates are decided here; the others are appended to `cells` with the
-// first 32-row block of their scores (blk_off), and their rows marked.  counter: cells in bits 36..,
+// first 32-row block of their scores (blk_off).  counter: cells in bits 36..,
 // blocks below; cand: candidates of the appended cells, summed.
 __global__ void __launch_bounds__(256) ft_cells_kernel(int n, const int32_t* list, const int* n_dev, int L,
                                                        const uint8_t* flags, const uint32_t* ctidx, int32_t* cells, int64_t* blk_off,
-                                                       uint8_t* row_mask, int32_t* final_labels, int32_t* rounds,
+                                                       int32_t* final_labels, int32_t* rounds,
                                                        unsigned long long* counter, unsigned long long* cand) {
     __shared__ unsigned long long w_tot[8];
     __shared__ unsigned long long s_base;
@@ -177,20 +177,18 @@ __global__ void __launch_bounds__(256) ft_cells_kernel(int n, const int32_t* lis
         const unsigned long long at = s_base + w_tot[warp] + x - mine;
         cells[at >> 36] = q;
         blk_off[at >> 36] = (int64_t)(at & ((1ull << 36) - 1));
-        row_mask[q] = 1;
     }
 }
 
-// One warp per cell: its pool entries by value, with each entry's run as positions [lo, hi).
-// cells = nullptr: rows 0 .. n - 1.
-__global__ void __launch_bounds__(256) ft_sort_rows_kernel(const int32_t* cells, int n, const float* data,
-                                                           const int32_t* idx, const int32_t* ptr, int cap,
-                                                           uint16_t* s_gene, uint16_t* s_lo, uint16_t* s_hi) {
+// One warp per row: its pool entries by value, with each entry's run as positions [lo, hi).
+__global__ void __launch_bounds__(256) ft_sort_rows_kernel(int n, const float* data, const int32_t* idx,
+                                                           const int32_t* ptr, int cap, uint16_t* s_gene,
+                                                           uint16_t* s_lo, uint16_t* s_hi) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpb = blockDim.x >> 5;
     uint64_t* keys = reinterpret_cast<uint64_t*>(smem) + (size_t)warp * cap;
     for (int i = blockIdx.x * wpb + warp; i < n; i += gridDim.x * wpb) {
-        const int row = cells ? cells[i] : i, beg = ptr[row], k = ptr[row + 1] - beg;
+        const int beg = ptr[i], k = ptr[i + 1] - beg;
         int m = 1;
         while (m < k) m <<= 1;
         for (int j = lane; j < m; j += 32)
@@ -208,34 +206,214 @@ __global__ void __launch_bounds__(256) ft_sort_rows_kernel(const int32_t* cells,
     }
 }
 
+// One CTA per cell: its row's entries in the gene pool, by value, with each entry's run as positions
+// [lo, hi), at c * row_stride.  Bound by latency (the row's two dependent loads) where there are few cells
+// and by issue where there are many: 48,412 cells of 1,500 entries took 1.45 ms in three kernels (count,
+// fill, a bitonic sort by one warp per row) and two host round trips for the sizes.
+// Values are counted into 256 buckets of a linear map; an entry's place in its bucket is the smaller values
+// plus the equal ones in earlier slots.  A bucket above 128 entries (few distinct values) is sorted instead.
+// dynamic shared memory: 2 x cap keys (cap: the pool's genes; a row's columns are distinct).
+constexpr int ROWS_NT = 256;
+
+__global__ void __launch_bounds__(ROWS_NT) ft_rows_kernel(const int32_t* cells, int n, const float* data,
+                                                         const int32_t* indices, const int32_t* indptr,
+                                                         uint32_t n_cols, const int32_t* map, int cap, int row_stride,
+                                                         uint16_t* s_gene, uint16_t* s_lo, uint16_t* s_hi,
+                                                         int32_t* row_len, int* longest) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ int start[257], w_tot[ROWS_NT / 32];
+    __shared__ uint32_t s_min, s_max;
+    __shared__ int s_n, s_big;
+    uint64_t* keys = reinterpret_cast<uint64_t*>(smem);
+    uint64_t* slots = keys + cap;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    for (int c = blockIdx.x; c < n; c += gridDim.x) {
+        const int beg = indptr[cells[c]], end = indptr[cells[c] + 1];
+        __syncthreads();  // the previous cell's shared memory is no longer read
+        start[tid + 1] = 0;
+        if (tid == 0) {
+            start[0] = 0;
+            s_n = 0;
+            s_min = 0xffffffffu;
+            s_max = 0u;
+            s_big = 0;
+        }
+        __syncthreads();
+        uint32_t kmin = 0xffffffffu, kmax = 0u;
+        for (int base = beg; base < end; base += 4 * ROWS_NT) {
+            int col[4], g[4];
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                const int i = base + t * ROWS_NT + tid;
+                col[t] = i < end ? __ldg(indices + i) : -1;
+            }
+#pragma unroll
+            for (int t = 0; t < 4; ++t) g[t] = (unsigned)col[t] < n_cols ? __ldg(map + col[t]) : -1;
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                const unsigned m = __ballot_sync(FULL, g[t] >= 0);
+                if (!m) continue;
+                int at = 0;
+                if (lane == 0) at = atomicAdd(&s_n, __popc(m));
+                at = __shfl_sync(FULL, at, 0) + __popc(m & ((1u << lane) - 1u));
+                if (g[t] >= 0 && at < cap) {
+                    const uint32_t u = ord_key(canon_zero(__ldg(data + base + t * ROWS_NT + tid)));
+                    keys[at] = ((uint64_t)u << 32) | (uint32_t)g[t];
+                    kmin = min(kmin, u);
+                    kmax = max(kmax, u);
+                }
+            }
+        }
+        kmin = __reduce_min_sync(FULL, kmin);
+        kmax = __reduce_max_sync(FULL, kmax);
+        if (lane == 0) {
+            atomicMin(&s_min, kmin);
+            atomicMax(&s_max, kmax);
+        }
+        __syncthreads();
+        const int k = min(s_n, cap);
+        const float fmin = key_float(s_min), span = key_float(s_max) - fmin;
+        const float scale = (span > 0.f && span < 1e30f) ? 256.0f / span : 0.f;
+        auto bucket = [&](uint64_t key) {
+            const float t = (key_float((uint32_t)(key >> 32)) - fmin) * scale;
+            return t >= 0.f ? min(255, (int)t) : 0;
+        };
+        for (int j = tid; j < k; j += ROWS_NT) atomicAdd(&start[bucket(keys[j]) + 1], 1);
+        __syncthreads();
+        const int mine = start[tid + 1];
+        if (mine > 128) s_big = 1;
+        const int incl = warp_incl_scan(mine, lane);
+        if (lane == 31) w_tot[warp] = incl;
+        __syncthreads();
+        int before = incl - mine;
+        for (int w = 0; w < warp; ++w) before += w_tot[w];
+        uint16_t* gene = s_gene + (size_t)c * row_stride;
+        uint16_t* lo_out = s_lo + (size_t)c * row_stride;
+        uint16_t* hi_out = s_hi + (size_t)c * row_stride;
+        if (!s_big) {
+            start[tid + 1] = before;  // advanced to the bucket's end as its slots are taken
+            __syncthreads();
+            for (int j = tid; j < k; j += ROWS_NT) {
+                const uint64_t key = keys[j];
+                slots[atomicAdd(&start[bucket(key) + 1], 1)] = key;
+            }
+            __syncthreads();
+            for (int j = tid; j < k; j += ROWS_NT) {
+                const uint64_t key = slots[j];
+                const uint32_t u = (uint32_t)(key >> 32);
+                const int b = bucket(key), s0 = start[b], s1 = start[b + 1];
+                int less = 0, eq = 0, eq_before = 0;
+                for (int t = s0; t < s1; ++t) {
+                    const uint32_t v = (uint32_t)(slots[t] >> 32);
+                    less += v < u;
+                    eq += v == u;
+                    eq_before += v == u && t < j;
+                }
+                const int lo = s0 + less, at = lo + eq_before;
+                gene[at] = (uint16_t)(uint32_t)key;
+                lo_out[at] = (uint16_t)lo;
+                hi_out[at] = (uint16_t)(lo + eq);
+            }
+        } else {
+            int m = 1;
+            while (m < k) m <<= 1;  // at most 2 cap
+            for (int j = k + tid; j < m; j += ROWS_NT) keys[j] = ~0ull;
+            __syncthreads();
+            for (int size = 2; size <= m; size <<= 1)
+                for (int stride = size >> 1; stride > 0; stride >>= 1) {
+                    for (int t = tid; t < (m >> 1); t += ROWS_NT) {
+                        const int i = 2 * t - (t & (stride - 1)), j = i + stride;
+                        const uint64_t x = keys[i], y = keys[j];
+                        if ((x > y) == ((i & size) == 0)) {
+                            keys[i] = y;
+                            keys[j] = x;
+                        }
+                    }
+                    __syncthreads();
+                }
+            for (int j = tid; j < k; j += ROWS_NT) {
+                const uint64_t key = keys[j];
+                const uint32_t u = (uint32_t)(key >> 32);
+                gene[j] = (uint16_t)(uint32_t)key;
+                lo_out[j] = (uint16_t)lower_hi(keys, k, u);
+                hi_out[j] = (uint16_t)upper_hi(keys, k, u);
+            }
+        }
+        if (tid == 0) {
+            row_len[c] = k;
+            atomicMax(longest, k);
+        }
+    }
+}
+
 // ---- a round -------------------------------------------------------------------------------------
 
 // The reference's keep / drop rule (src/cusingler.cu:1270-1295) on the list order: returns the new
-// list length, the new list in top.  One thread.
-__device__ int keep_candidates(const float* lsc, int ntop, uint8_t* top, uint8_t* tmp, float thre) {
-    int mn, mx;
-    stl::minmax(lsc, ntop, &mn, &mx);
-    const float lo = lsc[mn], hi = lsc[mx];
-    const float t = __fsub_rn(hi, thre);
+// list length, the new list in top.  One warp; tmp holds the new list meanwhile.
+__device__ int keep_candidates(const float* lsc, int ntop, uint8_t* top, uint8_t* tmp, float thre, int lane) {
+    float lo = __int_as_float(0x7f800000), hi = -lo;
+    bool nan = false;
+    for (int i = lane; i < ntop; i += 32) {
+        lo = fminf(lo, lsc[i]);
+        hi = fmaxf(hi, lsc[i]);
+        nan |= lsc[i] != lsc[i];
+    }
     int n = 0;
-    if (!(hi != hi)) {
-        for (int i = 0; i < ntop; ++i) {
-            const float s = lsc[i];
-            if (s <= lo || s < t) continue;
-            if (s == hi) {
-                for (int j = n; j > 0; --j) tmp[j] = tmp[j - 1];
-                tmp[0] = top[i];
-            } else {
-                tmp[n] = top[i];
+    if (__any_sync(FULL, nan)) {  // std::minmax_element's pairwise scan decides what a NaN does
+        if (lane == 0) {
+            int mn, mx;
+            stl::minmax(lsc, ntop, &mn, &mx);
+            lo = lsc[mn];
+            hi = lsc[mx];
+            const float t = __fsub_rn(hi, thre);
+            if (!(hi != hi)) {
+                for (int i = 0; i < ntop; ++i) {
+                    const float s = lsc[i];
+                    if (s <= lo || s < t) continue;
+                    if (s == hi) {
+                        for (int j = n; j > 0; --j) tmp[j] = tmp[j - 1];
+                        tmp[0] = top[i];
+                    } else {
+                        tmp[n] = top[i];
+                    }
+                    ++n;
+                }
             }
-            ++n;
         }
+        n = __shfl_sync(FULL, n, 0);
+    } else {
+        lo = key_float(__reduce_min_sync(FULL, ord_key(lo)));
+        hi = key_float(__reduce_max_sync(FULL, ord_key(hi)));
+        const float t = __fsub_rn(hi, thre);
+        // every maximum is moved to the front, so the last of them comes first; the others keep their order
+        int n_hi = 0;
+        for (int base = 0; base < ntop; base += 32) {
+            const int i = base + lane;
+            const float s = i < ntop ? lsc[i] : lo;
+            n_hi += __popc(__ballot_sync(FULL, !(s <= lo || s < t) && s == hi));
+        }
+        int hi_seen = 0, others = 0;
+        for (int base = 0; base < ntop; base += 32) {
+            const int i = base + lane;
+            const float s = i < ntop ? lsc[i] : lo;
+            const bool keep = !(s <= lo || s < t);
+            const unsigned mh = __ballot_sync(FULL, keep && s == hi), mo = __ballot_sync(FULL, keep && s != hi);
+            const unsigned lt = (1u << lane) - 1u;
+            if (keep) {
+                if (s == hi) tmp[n_hi - 1 - (hi_seen + __popc(mh & lt))] = top[i];
+                else tmp[n_hi + others + __popc(mo & lt)] = top[i];
+            }
+            hi_seen += __popc(mh);
+            others += __popc(mo);
+        }
+        n = n_hi + others;
     }
     if (n == 0) {
-        tmp[0] = top[0];
+        if (lane == 0) tmp[0] = top[0];
         n = 1;
     }
-    for (int i = 0; i < n; ++i) top[i] = tmp[i];
+    __syncwarp();
+    for (int i = lane; i < n; i += 32) top[i] = tmp[i];
     return n;
 }
 
@@ -254,7 +432,7 @@ struct StepSmem {
 // Step k of the batch's cells.  k = 0: candidates from the flags, the first round's setup; k > 0: the
 // decisions of round k - 1, then the setup of round k.  A cell that goes on is appended to `un` with its
 // sort key; bits > 0: and counted under the key's leading bits.  dynamic shared memory: eq (eq_stride
-// words), bits (nwords), in / before (kcap / 32 + 2 words each).
+// words), bits (nwords), in / before (Wt / 32 + 2 words each).
 template <int NW>
 __global__ void __launch_bounds__(NW * 32, NW == STEP_NW ? 4 : 1) ft_step_kernel(FtRounds a, int k, int bits_key) {
     extern __shared__ __align__(16) unsigned char dyn[];
@@ -264,7 +442,7 @@ __global__ void __launch_bounds__(NW * 32, NW == STEP_NW ? 4 : 1) ft_step_kernel
     uint32_t* eq = reinterpret_cast<uint32_t*>(dyn);
     uint32_t* bits = eq + a.eq_stride;
     uint32_t* in = bits + a.nwords;           // the row's entries inside the gene set, as bits
-    uint32_t* before = in + a.kcap / 32 + 2;  // those before each word
+    uint32_t* before = in + a.Wt / 32 + 2;  // those before each word
     const int cur = k & 1, nxt = cur ^ 1;
     const int n = k == 0 ? a.n_cells : a.n_act[cur];
     unsigned long long my_rounds = 0, my_rows = 0;
@@ -330,7 +508,10 @@ __global__ void __launch_bounds__(NW * 32, NW == STEP_NW ? 4 : 1) ft_step_kernel
                 }
             }
             __syncthreads();
-            if (tid == 0) sh.ntop = keep_candidates(sh.lsc, ntop, sh.top, sh.tmp, a.thre);
+            if (warp == 0) {
+                const int m = keep_candidates(sh.lsc, ntop, sh.top, sh.tmp, a.thre, lane);
+                if (lane == 0) sh.ntop = m;
+            }
         }
         __syncthreads();
 
@@ -370,7 +551,7 @@ __global__ void __launch_bounds__(NW * 32, NW == STEP_NW ? 4 : 1) ft_step_kernel
             const unsigned by_mask = __ballot_sync(FULL, whole && len > 0);
             for (int w0 = 0; by_mask && w0 < nw; w0 += 32) {
                 uint32_t m = 0;
-#pragma unroll 8
+#pragma unroll 16
                 for (int t = 0; t < ppw; ++t) {
                     const size_t p = __shfl_sync(FULL, pi, t);
                     if (((by_mask >> t) & 1u) && w0 + lane < nw) m |= __ldg(a.pair_mask + p * nw + w0 + lane);
@@ -381,7 +562,7 @@ __global__ void __launch_bounds__(NW * 32, NW == STEP_NW ? 4 : 1) ft_step_kernel
             len = min(len, gthre);
             const int maxn = __reduce_max_sync(FULL, len);
             for (int e0 = 0; e0 < maxn; e0 += 32) {
-#pragma unroll 8
+#pragma unroll 16
                 for (int t = 0; t < ppw; ++t) {
                     const uint32_t g0 = __shfl_sync(FULL, pos, t);
                     if (e0 + lane < __shfl_sync(FULL, len, t)) {
@@ -409,7 +590,8 @@ __global__ void __launch_bounds__(NW * 32, NW == STEP_NW ? 4 : 1) ft_step_kernel
             continue;
         }
         // the query's e-values over S: |S| - k + (kept entries before the run's end) + (before its start)
-        const int beg = a.row_ptr[cell], len = a.row_ptr[cell + 1] - beg;
+        const size_t beg = (size_t)c * a.row_stride;
+        const int len = a.row_len[c];
         const uint32_t one = 1u << a.shift;
         const int nwd = (len + 31) / 32;
 #pragma unroll 4
@@ -573,14 +755,22 @@ __global__ void __launch_bounds__(PLAN_NW * 32) ft_plan_kernel(FtRounds a, int k
         const int c = lane < nq ? a.act[4 * q + lane] : 0;
         for (int i = lane; i < 4 * 256; i += 32) (&pos[warp][0][0])[i] = 0xffffu;
         __syncwarp();
-        for (int t = 0; t < nq; ++t) {
-            const int ct = __shfl_sync(FULL, c, t), m = a.ntop[ct];
-            for (int i = lane; i < m; i += 32) pos[warp][t][a.top[(size_t)ct * a.L + i]] = (uint16_t)i;
+        const int m_c = lane < nq ? a.ntop[c] : 0, most = __reduce_max_sync(FULL, m_c);
+        int cell[4], m[4];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            cell[t] = __shfl_sync(FULL, c, min(t, nq - 1));
+            m[t] = __shfl_sync(FULL, m_c, t);
+        }
+        for (int i = lane; i < most; i += 32) {
+            int l[4];
+#pragma unroll
+            for (int t = 0; t < 4; ++t) l[t] = i < m[t] ? a.top[(size_t)cell[t] * a.L + i] : -1;
+#pragma unroll
+            for (int t = 0; t < 4; ++t)
+                if (l[t] >= 0) pos[warp][t][l[t]] = (uint16_t)i;
         }
         __syncwarp();
-        int cell[4];
-#pragma unroll
-        for (int t = 0; t < 4; ++t) cell[t] = __shfl_sync(FULL, c, min(t, nq - 1));
         int n_lab = 0, units = 0;
         for (int base = 0; base < a.L; base += 32) {
             const int l = base + lane;
@@ -599,10 +789,10 @@ __global__ void __launch_bounds__(PLAN_NW * 32) ft_plan_kernel(FtRounds a, int k
             }
             const bool in = need >= least;
             const int nb = in ? (int)(a.ctidx[2 * l + 1] + 31) / 32 : 0;
-            const unsigned m = __ballot_sync(FULL, in);
+            const unsigned mk = __ballot_sync(FULL, in);
             const int ps = warp_incl_scan(nb, lane);
             if (in) {
-                const size_t at_q = (size_t)q * a.L + n_lab + __popc(m & ((1u << lane) - 1u));
+                const size_t at_q = (size_t)q * a.L + n_lab + __popc(mk & ((1u << lane) - 1u));
                 a.q_label[at_q] = make_int2(l, units + ps - nb);
 #pragma unroll
                 for (int t = 0; t < 4; ++t) a.q_entry[at_q * 4 + t] = e[t];
@@ -613,7 +803,7 @@ __global__ void __launch_bounds__(PLAN_NW * 32) ft_plan_kernel(FtRounds a, int k
                     if (last == t) x = e[t];
                 a.list[(size_t)l * a.n_cells + atomicAdd(a.n_list + cur * 256 + l, 1)] = x;
             }
-            n_lab += __popc(m);
+            n_lab += __popc(mk);
             units += __shfl_sync(FULL, ps, 31);
         }
         if (lane == 0) a.quads[q] = FtQuad{{cell[0], cell[1], cell[2], cell[3]}, nq, n_lab, units};
@@ -1062,7 +1252,7 @@ size_t scan32_smem(int Wt, int nwarp) {
 }
 
 size_t step_smem(const FtRounds& a) {
-    return sizeof(uint32_t) * ((size_t)a.eq_stride + a.nwords) + sizeof(uint32_t) * 2 * ((size_t)a.kcap / 32 + 2);
+    return sizeof(uint32_t) * ((size_t)a.eq_stride + a.nwords) + sizeof(uint32_t) * 2 * ((size_t)a.Wt / 32 + 2);
 }
 
 size_t scan_smem(int Wt, int copies) { return (size_t)(Wt + 1) * 16 * copies; }
@@ -1123,18 +1313,17 @@ void launch_pair_masks(const uint32_t* ft_genes, const uint32_t* ft_idx, int L, 
 }
 
 void launch_ft_cells(int n, const int32_t* list, const int* n_dev, int L, const uint8_t* flags,
-                     const uint32_t* ctidx, int32_t* cells, int64_t* blk_off, uint8_t* row_mask,
-                     int32_t* final_labels, int32_t* rounds, unsigned long long* counter, unsigned long long* cand,
-                     cudaStream_t s) {
+                     const uint32_t* ctidx, int32_t* cells, int64_t* blk_off, int32_t* final_labels, int32_t* rounds,
+                     unsigned long long* counter, unsigned long long* cand, cudaStream_t s) {
     if (n <= 0) return;
-    ft_cells_kernel<<<(n + 255) / 256, 256, 0, s>>>(n, list, n_dev, L, flags, ctidx, cells, blk_off, row_mask, final_labels,
-                                                    rounds, counter, cand);
+    ft_cells_kernel<<<(n + 255) / 256, 256, 0, s>>>(n, list, n_dev, L, flags, ctidx, cells, blk_off, final_labels, rounds,
+                                                    counter, cand);
     SGR_LAUNCH_CHECK();
     count_launch();
 }
 
-void launch_ft_sort_rows(const int32_t* cells, int n, const float* data, const int32_t* idx, const int32_t* ptr,
-                         int longest, uint16_t* s_gene, uint16_t* s_lo, uint16_t* s_hi, cudaStream_t s) {
+void launch_ft_sort_rows(int n, const float* data, const int32_t* idx, const int32_t* ptr, int longest,
+                         uint16_t* s_gene, uint16_t* s_lo, uint16_t* s_hi, cudaStream_t s) {
     if (n <= 0) return;
     int cap = 32;
     while (cap < longest) cap <<= 1;
@@ -1142,7 +1331,19 @@ void launch_ft_sort_rows(const int32_t* cells, int n, const float* data, const i
     const size_t smem = (size_t)wpb * cap * 8;
     SGR_CUDA(cudaFuncSetAttribute(ft_sort_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const int blocks = std::min((n + wpb - 1) / wpb, device_sm_count() * 16);
-    ft_sort_rows_kernel<<<blocks, 32 * wpb, smem, s>>>(cells, n, data, idx, ptr, cap, s_gene, s_lo, s_hi);
+    ft_sort_rows_kernel<<<blocks, 32 * wpb, smem, s>>>(n, data, idx, ptr, cap, s_gene, s_lo, s_hi);
+    SGR_LAUNCH_CHECK();
+    count_launch();
+}
+
+void launch_ft_rows(const int32_t* cells, int n, const float* data, const int32_t* indices, const int32_t* indptr,
+                    uint32_t n_cols, const int32_t* map, int Wt, int row_stride, uint16_t* s_gene, uint16_t* s_lo,
+                    uint16_t* s_hi, int32_t* row_len, int* longest, cudaStream_t s) {
+    if (n <= 0) return;
+    const size_t smem = (size_t)Wt * 16;
+    SGR_CUDA(cudaFuncSetAttribute(ft_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    ft_rows_kernel<<<std::min(n, device_sm_count() * 16), ROWS_NT, smem, s>>>(
+        cells, n, data, indices, indptr, n_cols, map, Wt, row_stride, s_gene, s_lo, s_hi, row_len, longest);
     SGR_LAUNCH_CHECK();
     count_launch();
 }
@@ -1170,10 +1371,12 @@ void launch_ft_step(const FtRounds& a, int k, int n, bool quads, int32_t* scan_s
         while (bits < 20 && (1 << bits) < 16 * n) ++bits;
         SGR_CUDA(cudaMemsetAsync(a.key_count, 0, sizeof(int32_t) << bits, s));
     }
-    // With a CTA per SM or fewer, a cell's own latency decides: four times the warps for its gene set and
-    // its labels' quantiles.
-    if (n <= device_sm_count())
-        ft_step_kernel<STEP_NW_FEW><<<std::max(n, 1), STEP_NW_FEW * 32, step_smem(a), s>>>(a, k, bits);
+    // With few cells a cell's own latency decides: four times the warps for its gene set and its labels'
+    // quantiles.  With many labels a few cells hold on to most of them and take ten times as long as the
+    // others, so there the line lies higher.
+    if (n <= (a.L > 64 ? 16 : 2) * device_sm_count())
+        ft_step_kernel<STEP_NW_FEW><<<std::max(std::min(n, 2 * device_sm_count()), 1), STEP_NW_FEW * 32, step_smem(a),
+                                      s>>>(a, k, bits);
     else
         ft_step_kernel<STEP_NW><<<ft_step_grid(n), STEP_NW * 32, step_smem(a), s>>>(a, k, bits);
     SGR_LAUNCH_CHECK();

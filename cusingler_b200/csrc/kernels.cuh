@@ -332,8 +332,8 @@ struct FtRounds {
     int times;
     // query rows of the cells, compacted to the pool and sorted by value
     const uint16_t *s_gene, *s_lo, *s_hi;
-    const int32_t* row_ptr;
-    int kcap;                   // longest row
+    const int32_t* row_len;     // per cell; its entries start at cell * row_stride
+    int row_stride;
     const uint8_t* flags;
     // batch of n_cells cells
     const int32_t* cells;
@@ -373,13 +373,18 @@ void launch_row_groups(const uint16_t* sorted, const int32_t* ptr, const int32_t
 void launch_pair_masks(const uint32_t* ft_genes, const uint32_t* ft_idx, int L, int nwords, uint32_t* mask,
                        cudaStream_t s);
 // n cells (or the first *n_dev of `list`): those with fewer than two candidates get their final label,
-// the others go to `cells` / `blk_off` (counter: cells << 36 | 32-row score blocks) and row_mask.
+// the others go to `cells` / `blk_off` (counter: cells << 36 | 32-row score blocks).
 void launch_ft_cells(int n, const int32_t* list, const int* n_dev, int L, const uint8_t* flags,
-                     const uint32_t* ctidx, int32_t* cells, int64_t* blk_off, uint8_t* row_mask,
-                     int32_t* final_labels, int32_t* rounds, unsigned long long* counter, unsigned long long* cand,
-                     cudaStream_t s);
-void launch_ft_sort_rows(const int32_t* cells, int n, const float* data, const int32_t* idx, const int32_t* ptr,
-                         int longest, uint16_t* s_gene, uint16_t* s_lo, uint16_t* s_hi, cudaStream_t s);
+                     const uint32_t* ctidx, int32_t* cells, int64_t* blk_off, int32_t* final_labels, int32_t* rounds,
+                     unsigned long long* counter, unsigned long long* cand, cudaStream_t s);
+// Rows 0 .. n - 1 of a compacted CSR by value, with their runs (at the CSR's positions).
+void launch_ft_sort_rows(int n, const float* data, const int32_t* idx, const int32_t* ptr, int longest,
+                         uint16_t* s_gene, uint16_t* s_lo, uint16_t* s_hi, cudaStream_t s);
+// The cells' query rows compacted to the pool (map) and by value, with their runs, row_stride apart.
+// longest: atomic maximum of the rows' lengths.
+void launch_ft_rows(const int32_t* cells, int n, const float* data, const int32_t* indices, const int32_t* indptr,
+                    uint32_t n_cols, const int32_t* map, int Wt, int row_stride, uint16_t* s_gene, uint16_t* s_lo,
+                    uint16_t* s_hi, int32_t* row_len, int* longest, cudaStream_t s);
 int ft_step_grid(int n);
 // Function attributes of the step and scan kernels; call before the launches of a batch.
 void ft_rounds_setup(const FtRounds& a, int copies);
