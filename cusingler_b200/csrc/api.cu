@@ -93,6 +93,7 @@ struct Profiler {
 }  // namespace
 
 struct sgr_ctx {
+    DevArena arena;  // first: the buffers below return their memory to it
     int device = 0;
     int cores = 1;
     cudaStream_t stream = nullptr;      // the stream work runs on
@@ -206,6 +207,7 @@ struct sgr_ctx {
     DevBuf<unsigned long long> fr_ctl;  // counters (FtCtl)
     DevBuf<float> fr_scores, fr_nan;
     DevBuf<uint16_t> fr_ref_runs;  // FP32 order: the reference's entries by value, with their runs
+    size_t fr_ref_runs_stride = 0;
     bool fr_ref_runs_ready = false;
     unsigned long long* h_ft = nullptr;  // pinned: counters read back
     cudaEvent_t ev_ft[2] = {nullptr, nullptr};
@@ -301,10 +303,28 @@ struct PhaseClock {
     }
 };
 
+// After a failed call: nothing queued may read caller memory or a released buffer any more.
+void drain(sgr_ctx* ctx) {
+    for (cudaStream_t s : {ctx->stream, ctx->side, ctx->copy, ctx->ft_s})
+        if (s) cudaStreamSynchronize(s);
+    cudaGetLastError();
+    ctx->prof.spans.clear();
+    ctx->prof.used = 0;
+    ctx->prof.rounds_pending = false;
+}
+
 template <class F>
 sgr_status guarded(sgr_ctx* ctx, F&& f) {
     if (!ctx) return SGR_ERR_INVALID_ARGUMENT;
     ctx->err.clear();
+    struct UseArena {  // the context's last call left its streams finished: released blocks may be reused
+        DevArena* before = DevArena::current();
+        explicit UseArena(DevArena& a) {
+            a.settle();
+            DevArena::current() = &a;
+        }
+        ~UseArena() { DevArena::current() = before; }
+    } use_arena(ctx->arena);
     try {
         if (ctx->device >= 0) SGR_CUDA(cudaSetDevice(ctx->device));
         const uint64_t l0 = launch_count();
@@ -317,20 +337,15 @@ sgr_status guarded(sgr_ctx* ctx, F&& f) {
         return SGR_OK;
     } catch (const Error& e) {
         ctx->err = e.what();
-        if (ctx->stream) cudaStreamSynchronize(ctx->stream);
-        if (ctx->side) cudaStreamSynchronize(ctx->side);
-        if (ctx->copy) cudaStreamSynchronize(ctx->copy);  // no copy may read caller memory after return
-        if (ctx->ft_s) cudaStreamSynchronize(ctx->ft_s);
-        cudaGetLastError();
-        ctx->prof.spans.clear();
-        ctx->prof.used = 0;
-        ctx->prof.rounds_pending = false;
+        drain(ctx);
         return e.code;
     } catch (const std::bad_alloc&) {
         ctx->err = "host allocation failed";
+        drain(ctx);
         return SGR_ERR_OUT_OF_MEMORY;
     } catch (const std::exception& e) {
         ctx->err = e.what();
+        drain(ctx);
         return SGR_ERR_INVALID_ARGUMENT;
     }
 }
@@ -1280,7 +1295,7 @@ struct FtCtl {
 // FP32 order: the reference rows' thre-pool entries by value, each with its run (on first use).
 void ensure_ref_runs(sgr_ctx* ctx) {
     if (ctx->fr_ref_runs_ready) return;
-    const size_t n = std::max<size_t>(ctx->reff_indices.n, 1);
+    const size_t n = ctx->fr_ref_runs_stride = std::max<size_t>(ctx->reff_indices.n, 1);
     uint16_t* r = ctx->fr_ref_runs.ensure(3 * n);
     launch_ft_sort_rows((int)ctx->R, ctx->reff_data.p, ctx->reff_indices.p, ctx->reff_indptr.p, ctx->max_row, r,
                         r + n, r + 2 * n, ctx->stream);
@@ -1355,7 +1370,7 @@ void finetune_rounds(sgr_ctx* ctx, const DevCsr& q, const uint8_t* flags_dev, fl
     a.lorder = ctx->d_lorder.p;
     if (fp32) {
         ensure_ref_runs(ctx);
-        const size_t n = ctx->fr_ref_runs.n / 3;
+        const size_t n = ctx->fr_ref_runs_stride;
         a.ref_gene = ctx->fr_ref_runs.p;
         a.ref_lo = a.ref_gene + n;
         a.ref_hi = a.ref_lo + n;
@@ -1418,7 +1433,7 @@ void finetune_rounds(sgr_ctx* ctx, const DevCsr& q, const uint8_t* flags_dev, fl
     const int64_t k = ctx->max_row;
     auto narrow = [&](int64_t longest) { return 2 * k * std::min<int64_t>(2 * k, longest) * (int64_t)Wt < (int64_t(1) << 32); };
     const bool ask_longest = ctx->pack_scan == 2 && !fp32 && !narrow(Wt) && narrow(1);
-    ft_rounds_setup(a, ctx->ft_copies);
+    ft_rounds_setup(ctx->ft_copies);
     for (size_t b = 0; b + 1 < cuts.size(); ++b) {
         a.cells = ctx->fr_cells.p + cuts[b];
         a.blk_off = ctx->fr_blk_off.p + cuts[b];

@@ -810,7 +810,7 @@ void launch_ref_presort(const float* data, const int32_t* idx, const int32_t* pt
     if (!n_rows) return;
     int wpb = std::max(1, std::min(8, (200 * 1024) / (cap * 8)));
     const size_t smem = (size_t)wpb * cap * 8;
-    SGR_CUDA(cudaFuncSetAttribute(ref_presort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_smem(ref_presort_kernel, 200 * 1024);
     const unsigned blocks = std::min<unsigned>((n_rows + wpb - 1) / wpb, device_sm_count() * 8);
     ref_presort_kernel<<<blocks, 32 * wpb, smem, s>>>(data, idx, ptr, ell_base, ell_len, n_rows, cap, pad_gene, out);
     SGR_LAUNCH_CHECK();

@@ -1257,6 +1257,8 @@ size_t step_smem(const FtRounds& a) {
 
 size_t scan_smem(int Wt, int copies) { return (size_t)(Wt + 1) * 16 * copies; }
 
+constexpr size_t kStepSmem = 128 * 1024;    // the widest pool (14,143 genes) takes 60 KB
+constexpr size_t kScan32Smem = 200 * 1024;
 constexpr size_t kScanSmem = 221 * 1024;  // with the kernel's static shared memory (6 KB), under 227 KB
 
 template <int C>
@@ -1267,10 +1269,9 @@ void launch_scan_c(const FtRounds& a, int k, bool x64, cudaStream_t s) {
 }
 
 template <int C>
-void scan_attr(int Wt) {
-    const int smem = (int)scan_smem(Wt, C);
-    SGR_CUDA(cudaFuncSetAttribute(ft_scan_kernel<C, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    SGR_CUDA(cudaFuncSetAttribute(ft_scan_kernel<C, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+void scan_attr() {
+    allow_smem(ft_scan_kernel<C, true>, kScanSmem);
+    allow_smem(ft_scan_kernel<C, false>, kScanSmem);
 }
 
 }  // namespace
@@ -1288,7 +1289,7 @@ void launch_row_runs(const float* data, const int32_t* idx, const int32_t* ptr, 
     while (cap < longest) cap <<= 1;
     const int wpb = std::max(1, std::min(8, (int)(96 * 1024 / (cap * 8))));
     const size_t smem = (size_t)wpb * cap * 8;
-    SGR_CUDA(cudaFuncSetAttribute(row_runs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_smem(row_runs_kernel, 96 * 1024);
     const unsigned blocks = std::min<unsigned>((n_rows + wpb - 1) / wpb, device_sm_count() * 8);
     row_runs_kernel<<<blocks, 32 * wpb, smem, s>>>(data, idx, ptr, n_rows, cap, sorted, n_groups);
     SGR_LAUNCH_CHECK();
@@ -1329,7 +1330,7 @@ void launch_ft_sort_rows(int n, const float* data, const int32_t* idx, const int
     while (cap < longest) cap <<= 1;
     const int wpb = std::max(1, std::min(8, (int)(96 * 1024 / (cap * 8))));
     const size_t smem = (size_t)wpb * cap * 8;
-    SGR_CUDA(cudaFuncSetAttribute(ft_sort_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_smem(ft_sort_rows_kernel, 96 * 1024);
     const int blocks = std::min((n + wpb - 1) / wpb, device_sm_count() * 16);
     ft_sort_rows_kernel<<<blocks, 32 * wpb, smem, s>>>(n, data, idx, ptr, cap, s_gene, s_lo, s_hi);
     SGR_LAUNCH_CHECK();
@@ -1341,7 +1342,7 @@ void launch_ft_rows(const int32_t* cells, int n, const float* data, const int32_
                     uint16_t* s_hi, int32_t* row_len, int* longest, cudaStream_t s) {
     if (n <= 0) return;
     const size_t smem = (size_t)Wt * 16;
-    SGR_CUDA(cudaFuncSetAttribute(ft_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_smem(ft_rows_kernel, kScanSmem);
     ft_rows_kernel<<<std::min(n, device_sm_count() * 16), ROWS_NT, smem, s>>>(
         cells, n, data, indices, indptr, n_cols, map, Wt, row_stride, s_gene, s_lo, s_hi, row_len, longest);
     SGR_LAUNCH_CHECK();
@@ -1350,15 +1351,13 @@ void launch_ft_rows(const int32_t* cells, int n, const float* data, const int32_
 
 int ft_step_grid(int n) { return std::max(1, std::min(n, device_sm_count() * STEP_CTAS)); }
 
-void ft_rounds_setup(const FtRounds& a, int copies) {
-    SGR_CUDA(cudaFuncSetAttribute(ft_step_kernel<STEP_NW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)step_smem(a)));
-    SGR_CUDA(cudaFuncSetAttribute(ft_step_kernel<STEP_NW_FEW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)step_smem(a)));
-    if (copies == 8) scan_attr<8>(a.Wt);
-    else if (copies == 4) scan_attr<4>(a.Wt);
-    else if (copies == 2) scan_attr<2>(a.Wt);
-    else scan_attr<1>(a.Wt);
+void ft_rounds_setup(int copies) {
+    allow_smem(ft_step_kernel<STEP_NW>, kStepSmem);
+    allow_smem(ft_step_kernel<STEP_NW_FEW>, kStepSmem);
+    if (copies == 8) scan_attr<8>();
+    else if (copies == 4) scan_attr<4>();
+    else if (copies == 2) scan_attr<2>();
+    else scan_attr<1>();
 }
 
 // Step k, the cells that go on put in order, and the quads of round k.  n: no more cells than this.
@@ -1398,14 +1397,14 @@ void launch_ft_step(const FtRounds& a, int k, int n, bool quads, int32_t* scan_s
 
 int ft_scan32_warps(int Wt) {
     for (int w = 8; w >= 1; --w)
-        if (scan32_smem(Wt, w) <= 200 * 1024) return w;
+        if (scan32_smem(Wt, w) <= kScan32Smem) return w;
     return 0;
 }
 
 void launch_ft_scan32(const FtRounds& a, int k, int n, cudaStream_t s) {
     const int warps = ft_scan32_warps(a.Wt);
     const size_t smem = scan32_smem(a.Wt, warps);
-    SGR_CUDA(cudaFuncSetAttribute(ft_scan32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_smem(ft_scan32_kernel, kScan32Smem);
     int per_sm = 0;
     SGR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ft_scan32_kernel, 32 * warps, smem));
     const int grid = device_sm_count() * std::max(1, per_sm);

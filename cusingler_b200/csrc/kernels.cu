@@ -867,7 +867,7 @@ void launch_rank_tier(const RankLaunch& a, long max_blocks, cudaStream_t s) {
     }
     if (wpb < 1) fail(SGR_ERR_UNSUPPORTED, "gene subset too wide for the rank kernel's shared memory");
     const int smem = map_bytes + wpb * warp_bytes;
-    SGR_CUDA(cudaFuncSetAttribute(rank_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    allow_smem(rank_kernel, 200 * 1024);
     const int per_sm = std::max(1, std::min(8, (228 * 1024) / (smem + 1024)));
     long blocks = (long)sm_count() * per_sm;
     if (max_blocks > 0) blocks = std::min(blocks * 4, (max_blocks + wpb - 1) / wpb);
@@ -1076,7 +1076,7 @@ void launch_corr_few(const int8_t* A, const int8_t* B, int nq, int R, int Kp, co
     const int n = nq <= 1 ? 1 : nq <= 2 ? 2 : nq <= 4 ? 4 : 8;
     auto kern = n == 1 ? corr_few_kernel<1> : n == 2 ? corr_few_kernel<2> : n == 4 ? corr_few_kernel<4> : corr_few_kernel<8>;
     const size_t smem = (size_t)n * 3 * Kp;
-    SGR_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_smem(kern, 96 * 1024);
     const int blocks = std::min((R + 7) / 8, sm_count() * 4);
     kern<<<blocks, 256, smem, s>>>(A, B, nq, R, Kp, ra, rb, scores, ld, ext, k1, cbase);
     SGR_LAUNCH_CHECK();
@@ -1141,7 +1141,7 @@ void launch_select_first(const float* scores, int64_t ld, int nq, int L, const L
     } else if (lorder && stage_bytes <= 200 * 1024) {
         auto kern = warps == 8 ? select_first_kernel<true, 8> : select_first_kernel<true, 16>;
         const int threads = 32 * (warps == 8 ? 8 : 16);
-        SGR_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)stage_bytes));
+        allow_smem(kern, 200 * 1024);
         int per_sm = 0;
         SGR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, stage_bytes));
         per_sm = std::max(1, std::min(per_sm, 2));  // at most 32 warps per SM use scratch

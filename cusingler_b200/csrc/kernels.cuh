@@ -387,7 +387,7 @@ void launch_ft_rows(const int32_t* cells, int n, const float* data, const int32_
                     uint16_t* s_hi, int32_t* row_len, int* longest, cudaStream_t s);
 int ft_step_grid(int n);
 // Function attributes of the step and scan kernels; call before the launches of a batch.
-void ft_rounds_setup(const FtRounds& a, int copies);
+void ft_rounds_setup(int copies);
 // Step k over at most n cells and (quads) the quads of round k.  scan_scratch: launch_exclusive_scan's, 2^20 values.
 void launch_ft_step(const FtRounds& a, int k, int n, bool quads, int32_t* scan_scratch, cudaStream_t s);
 // Round k's correlations in the reference's FP32 order.  ft_scan32_warps: 0 for a pool too wide for it.
