@@ -189,8 +189,8 @@ struct sgr_ctx {
     int max_row = 0;               // longest thre-pool row of the reference
     DevBuf<uint4> fr_groups;
     DevBuf<int32_t> fr_blk_voff;
-    DevBuf<uint32_t> fr_perm, fr_pair_mask;
-    bool fr_masks = false;
+    DevBuf<uint32_t> fr_perm, fr_pair_mask, fr_cut_mask;
+    bool fr_masks = false, fr_cut_masks = false;
     // its per-call and per-batch buffers
     DevBuf<int32_t> fr_cells;
     DevBuf<int64_t> fr_blk_off;
@@ -765,12 +765,6 @@ void train(sgr_ctx* ctx, const sgr_csr* ref, const int32_t* celltypes, const cha
     }
     ctx->d_ft_genes.upload(mk.ft_genes.empty() ? std::vector<uint32_t>{0} : mk.ft_genes, s);
     ctx->d_ft_idx.upload(mk.ft_idx, s);
-    // each pair's whole fine-tune list as bits over the pool (unless that takes over 256 MiB)
-    const size_t nwords = (std::max<size_t>(ctx->Wt, 1) + 31) / 32, mask_words = (size_t)mk.n_labels * mk.n_labels * nwords;
-    ctx->fr_masks = ctx->ft_copies && mask_words <= ((size_t)64 << 20);
-    if (ctx->fr_masks)
-        launch_pair_masks(ctx->d_ft_genes.p, ctx->d_ft_idx.p, (int)mk.n_labels, (int)nwords,
-                          ctx->fr_pair_mask.ensure(mask_words), s);
     {
         std::vector<int32_t> lorder(mk.n_labels);
         for (uint32_t l = 0; l < mk.n_labels; ++l) lorder[l] = (int32_t)l;
@@ -782,6 +776,15 @@ void train(sgr_ctx* ctx, const sgr_csr* ref, const int32_t* celltypes, const cha
     std::vector<int32_t> gt(mk.n_labels + 1, 0);
     for (uint32_t n = 1; n <= mk.n_labels; ++n) gt[n] = marker_count(n);
     ctx->d_gene_thre.upload(gt, s);
+    // the pairs' fine-tune lists as bits over the pool, whole and as each candidate count cuts them (unless
+    // that takes over 256 MiB each)
+    const size_t nwords = (std::max<size_t>(ctx->Wt, 1) + 31) / 32, nl = mk.n_labels, rows_words = nl * nl * nwords;
+    ctx->fr_masks = ctx->ft_copies && rows_words <= ((size_t)64 << 20);
+    ctx->fr_cut_masks = ctx->fr_masks && nl >= 2 && rows_words * (nl - 1) <= ((size_t)64 << 20);
+    if (ctx->fr_masks)
+        launch_pair_masks(ctx->d_ft_genes.p, ctx->d_ft_idx.p, (int)nl, (int)nwords, ctx->d_gene_thre.p,
+                          ctx->fr_pair_mask.ensure(rows_words),
+                          ctx->fr_cut_masks ? ctx->fr_cut_mask.ensure(rows_words * (nl - 1)) : nullptr, s);
     check_status(ctx);
     ctx->trained = true;
 }
@@ -1379,6 +1382,7 @@ void finetune_rounds(sgr_ctx* ctx, const DevCsr& q, const uint8_t* flags_dev, fl
     a.ft_genes = ctx->d_ft_genes.p;
     a.ft_idx = ctx->d_ft_idx.p;
     a.pair_mask = ctx->fr_masks ? ctx->fr_pair_mask.p : nullptr;
+    a.cut_mask = ctx->fr_cut_masks ? ctx->fr_cut_mask.p : nullptr;
     a.gene_thre = ctx->d_gene_thre.p;
     a.lq = ctx->d_lq_label.p;
     a.L = (int)L;
@@ -1398,7 +1402,7 @@ void finetune_rounds(sgr_ctx* ctx, const DevCsr& q, const uint8_t* flags_dev, fl
     a.row_stride = row_stride;
     a.flags = flags_dev;
     a.top = ctx->fr_top.ensure((size_t)nb * L);
-    int* ints = ctx->fr_ints.ensure((size_t)nb * 4);
+    int* ints = ctx->fr_ints.ensure((size_t)nb * 5);
     a.ntop = ints;
     a.used = ints + nb;
     a.par = ctx->fr_par.ensure(nb);
@@ -1409,13 +1413,13 @@ void finetune_rounds(sgr_ctx* ctx, const DevCsr& q, const uint8_t* flags_dev, fl
     a.un = ctx->fr_un.ensure(nb);
     a.key_count = ctx->fr_keys.ensure(((size_t)2 << 20) + 1);
     int32_t* scan_scratch = ctx->scan_part.ensure(2 * (((size_t)1 << 20) / 4096) + 1);
-    const size_t n_quads = ((size_t)nb + 3) / 4;
+    const size_t n_quads = std::max<size_t>(((size_t)nb + 3) / 4, std::min<size_t>(nb, kFtDirectCells));
     a.list = ctx->fr_list.ensure((size_t)nb * L + n_quads * L * 4);
     a.q_entry = a.list + (size_t)nb * L;
     a.quads = ctx->fr_quads.ensure(n_quads);
     a.q_label = ctx->fr_q_label.ensure(n_quads * L);
     a.act = ints + 2 * nb;
-    a.row_len = ints + 3 * nb;
+    a.row_len = ints + 4 * nb;
     a.n_list = d->n_list;
     a.queue = d->queue;
     a.n_act = d->n_act;
@@ -1442,7 +1446,7 @@ void finetune_rounds(sgr_ctx* ctx, const DevCsr& q, const uint8_t* flags_dev, fl
         if (b > 0) SGR_CUDA(cudaMemsetAsync(d, 0, sizeof(FtCtl), s));
         SGR_CUDA(cudaMemsetAsync(a.used, 0, a.n_cells * sizeof(int), s));
         launch_ft_rows(a.cells, a.n_cells, q.data, q.indices, q.indptr, q.n_cols, ctx->qry_map_thre.p, (int)Wt, row_stride,
-                       sorted, sorted + (size_t)nb * row_stride, sorted + 2 * (size_t)nb * row_stride, ints + 3 * nb,
+                       sorted, sorted + (size_t)nb * row_stride, sorted + 2 * (size_t)nb * row_stride, ints + 4 * nb,
                        &d->longest, s);
         bool x64 = ctx->pack_scan != 2 || !narrow(Wt);
         // each round drops at least one candidate, so L rounds finish every cell
@@ -1457,7 +1461,7 @@ void finetune_rounds(sgr_ctx* ctx, const DevCsr& q, const uint8_t* flags_dev, fl
                 x64 = !narrow(host_ctl(0)->longest);
             }
             if (fp32) launch_ft_scan32(a, r, most, s);
-            else launch_ft_scan(a, r, ctx->ft_copies, x64, s);
+            else launch_ft_scan(a, r, most, ctx->ft_copies, x64, s);
             if (r == 0) continue;
             SGR_CUDA(cudaEventSynchronize(ctx->ev_ft[(r - 1) & 1]));
             const FtCtl* c = host_ctl((r - 1) & 1);

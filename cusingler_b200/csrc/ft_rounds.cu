@@ -123,6 +123,35 @@ __global__ void pair_mask_kernel(const uint32_t* ft_genes, const uint32_t* ft_id
     }
 }
 
+// The same for the first gene_thre(n) genes of the lists that n candidates cut, n = 2 .. L: row (n - 2) *
+// n_pairs + pair.  One warp per pair; gene_thre falls with n.  dynamic shared memory: nwords per warp.
+__global__ void cut_mask_kernel(const uint32_t* ft_genes, const uint32_t* ft_idx, int n_pairs, int L, int nwords,
+                                const int32_t* gene_thre, uint32_t* mask) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpb = blockDim.x >> 5;
+    uint32_t* m = reinterpret_cast<uint32_t*>(smem) + (size_t)warp * nwords;
+    for (int p = blockIdx.x * wpb + warp; p < n_pairs; p += gridDim.x * wpb) {
+        const uint32_t pos = ft_idx[2 * p];
+        const int len = (int)ft_idx[2 * p + 1];
+        for (int w = lane; w < nwords; w += 32) m[w] = 0u;
+        __syncwarp();
+        int done = 0;
+        for (int n = L; n >= 2; --n) {
+            const int t = gene_thre[n];
+            if (t >= len) break;  // not cut, nor by fewer candidates
+            for (int i = done + lane; i < t; i += 32) {
+                const uint32_t g = ft_genes[pos + i];
+                atomicOr(&m[g >> 5], 1u << (g & 31));
+            }
+            done = max(done, t);
+            __syncwarp();
+            uint32_t* out = mask + ((size_t)(n - 2) * n_pairs + p) * nwords;
+            for (int w = lane; w < nwords; w += 32) out[w] = m[w];
+            __syncwarp();
+        }
+    }
+}
+
 // ---- per call: the cells to fine-tune ----------------------------------------------------------
 
 // Cells with fewer than two candidates are decided here; the others are appended to `cells` with the
@@ -430,11 +459,16 @@ struct StepSmem {
 };
 
 // Step k of the batch's cells.  k = 0: candidates from the flags, the first round's setup; k > 0: the
-// decisions of round k - 1, then the setup of round k.  A cell that goes on is appended to `un` with its
-// sort key; bits > 0: and counted under the key's leading bits.  dynamic shared memory: eq (eq_stride
+// decisions of round k - 1, then the setup of round k.  A cell that goes on is appended, by `mode`:
+//   STEP_ORDER  to `un` with its sort key (bits_key > 0: and counted under the key's leading bits);
+//   STEP_QUAD   to `act` with a quad of its own, so that nothing has to be ordered and planned;
+//   STEP_LIST   to `act` alone.  dynamic shared memory: eq (eq_stride
 // words), bits (nwords), in / before (Wt / 32 + 2 words each).
+enum StepMode { STEP_ORDER = 0, STEP_QUAD = 1, STEP_LIST = 2 };
+
 template <int NW>
-__global__ void __launch_bounds__(NW * 32, NW == STEP_NW ? 4 : 1) ft_step_kernel(FtRounds a, int k, int bits_key) {
+__global__ void __launch_bounds__(NW * 32, NW == STEP_NW ? 4 : 1) ft_step_kernel(FtRounds a, int k, int mode,
+                                                                                int bits_key) {
     extern __shared__ __align__(16) unsigned char dyn[];
     __shared__ StepSmem<NW> sh;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -447,7 +481,7 @@ __global__ void __launch_bounds__(NW * 32, NW == STEP_NW ? 4 : 1) ft_step_kernel
     const int n = k == 0 ? a.n_cells : a.n_act[cur];
     unsigned long long my_rounds = 0, my_rows = 0;
     for (int it = blockIdx.x; it < n; it += gridDim.x) {
-        const int c = k == 0 ? it : a.act[it];
+        const int c = k == 0 ? it : a.act[(size_t)cur * a.n_cells + it];
         const int cell = a.cells[c];
         uint8_t* gtop = a.top + (size_t)c * a.L;
         const uint32_t blk0 = (uint32_t)(a.blk_off[c] - a.blk_base0);
@@ -526,13 +560,13 @@ __global__ void __launch_bounds__(NW * 32, NW == STEP_NW ? 4 : 1) ft_step_kernel
             continue;
         }
         // gene set: union over ordered candidate pairs of the first min(len, gene_thre(n)) genes of the
-        // pair's list (src/cusingler.cu:1141-1156); a list that is not cut is one precomputed mask
+        // pair's list (src/cusingler.cu:1141-1156), precomputed masks where they fit (launch_pair_masks)
         const int gthre = a.gene_thre[ntop], np = ntop * ntop, nw = a.nwords;
         for (int w = tid; w < nw; w += NT) bits[w] = 0u;
         __syncthreads();
         // A warp takes up to 32 pairs at a time, few enough that every warp gets some.  Each lane fetches
         // one pair's list range; then the warp walks the pairs together, lanes over the mask's words (or
-        // over a cut list's genes), so that the loads of several pairs are in flight at once.
+        // over a list's genes), so that the loads of several pairs are in flight at once.
         const int ppw = min(32, (np + NW - 1) / NW);
         for (int base = warp * ppw; base < np; base += NW * ppw) {
             const int pr = base + lane;
@@ -547,18 +581,20 @@ __global__ void __launch_bounds__(NW * 32, NW == STEP_NW ? 4 : 1) ft_step_kernel
                     len = (int)r.y;
                 }
             }
-            const bool whole = a.pair_mask && len <= gthre;
-            const unsigned by_mask = __ballot_sync(FULL, whole && len > 0);
+            const bool cut = len > gthre, masked = cut ? a.cut_mask != nullptr : a.pair_mask != nullptr;
+            const unsigned by_mask = __ballot_sync(FULL, masked && len > 0), is_cut = __ballot_sync(FULL, cut);
+            const uint32_t* cut_rows = a.cut_mask + (size_t)(ntop - 2) * a.L * a.L * nw;
             for (int w0 = 0; by_mask && w0 < nw; w0 += 32) {
                 uint32_t m = 0;
 #pragma unroll 16
                 for (int t = 0; t < ppw; ++t) {
                     const size_t p = __shfl_sync(FULL, pi, t);
-                    if (((by_mask >> t) & 1u) && w0 + lane < nw) m |= __ldg(a.pair_mask + p * nw + w0 + lane);
+                    if (((by_mask >> t) & 1u) && w0 + lane < nw)
+                        m |= __ldg(((is_cut >> t) & 1u ? cut_rows : a.pair_mask) + p * nw + w0 + lane);
                 }
                 if (m) atomicOr(&bits[w0 + lane], m);
             }
-            if (whole) len = 0;
+            if (masked) len = 0;
             len = min(len, gthre);
             const int maxn = __reduce_max_sync(FULL, len);
             for (int e0 = 0; e0 < maxn; e0 += 32) {
@@ -644,7 +680,8 @@ __global__ void __launch_bounds__(NW * 32, NW == STEP_NW ? 4 : 1) ft_step_kernel
             a.ntop[c] = ntop;
             a.used[c] = done + 1;
         }
-        if (warp == 0) {
+        if (mode == STEP_LIST && tid == 0) a.act[(size_t)nxt * a.n_cells + atomicAdd(a.n_act + nxt, 1)] = c;
+        if (mode == STEP_ORDER && warp == 0) {
             // sort key: the candidates among the 32 longest labels as a reflected Gray code, so that cells
             // whose candidates differ little are close
             const unsigned m = __ballot_sync(FULL, lane < a.L && sh.is_cand[a.lorder[min(lane, a.L - 1)]]);
@@ -656,6 +693,11 @@ __global__ void __launch_bounds__(NW * 32, NW == STEP_NW ? 4 : 1) ft_step_kernel
         }
         if (warp == NW - 1) {  // the candidates' score blocks
             uint32_t acc = 0;
+            int quad = 0;
+            if (mode == STEP_QUAD) {
+                if (lane == 0) quad = atomicAdd(a.n_act + nxt, 1);
+                quad = __shfl_sync(FULL, quad, 0);
+            }
             for (int base = 0; base < ntop; base += 32) {
                 const int i = base + lane;
                 const int l = i < ntop ? sh.top[i] : 0;
@@ -664,9 +706,21 @@ __global__ void __launch_bounds__(NW * 32, NW == STEP_NW ? 4 : 1) ft_step_kernel
                 if (i < ntop) {
                     a.ext_min[(size_t)c * a.L + i] = 0xffffffffu;
                     a.ext_max[(size_t)c * a.L + i] = 0u;
-                    a.blk_of[(size_t)c * a.L + i] = blk0 + acc + (uint32_t)(incl - nb);
+                    const uint32_t blk = blk0 + acc + (uint32_t)(incl - nb);
+                    a.blk_of[(size_t)c * a.L + i] = blk;
+                    if (mode == STEP_QUAD) {
+                        const size_t at = (size_t)quad * a.L + i;
+                        a.q_label[at] = make_int2(l, (int)acc + incl - nb);
+                        a.q_entry[4 * at] = FtEntry{(uint32_t)(c * a.L + i), blk};
+#pragma unroll
+                        for (int t = 1; t < 4; ++t) a.q_entry[4 * at + t] = FtEntry{~0u, 0u};
+                    }
                 }
                 acc += (uint32_t)__shfl_sync(FULL, incl, 31);
+            }
+            if (mode == STEP_QUAD && lane == 0) {
+                a.act[(size_t)nxt * a.n_cells + quad] = c;
+                a.quads[quad] = FtQuad{{c, c, c, c}, 1, ntop, (int)acc};
             }
             if (lane == 0) my_rows += (unsigned long long)acc * 32;
         }
@@ -726,21 +780,23 @@ constexpr int SPLIT_QUADS = 64;    // from this many quads on, a label that one 
 // keys), or by the keys' leading bits (start: exclusive scan of their counts, advanced here).
 __global__ void __launch_bounds__(256) ft_rank_kernel(FtRounds a, int k) {
     const int n = a.n_act[(k & 1) ^ 1], lane = threadIdx.x & 31;
+    int* act = a.act + (size_t)((k & 1) ^ 1) * a.n_cells;
     for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n; i += (gridDim.x * blockDim.x) >> 5) {
         const unsigned long long mine = a.un[i];
         int less = 0;
 #pragma unroll 4
         for (int j = lane; j < n; j += 32) less += a.un[j] < mine;
         less = __reduce_add_sync(FULL, less);
-        if (lane == 0) a.act[less] = (int)(uint32_t)mine;
+        if (lane == 0) act[less] = (int)(uint32_t)mine;
     }
 }
 
 __global__ void __launch_bounds__(256) ft_place_kernel(FtRounds a, int k, int bits_key, int32_t* start) {
     const int n = a.n_act[(k & 1) ^ 1];
+    int* act = a.act + (size_t)((k & 1) ^ 1) * a.n_cells;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const unsigned long long u = a.un[i];
-        a.act[atomicAdd(start + (uint32_t)(u >> (64 - bits_key)), 1)] = (int)(uint32_t)u;
+        act[atomicAdd(start + (uint32_t)(u >> (64 - bits_key)), 1)] = (int)(uint32_t)u;
     }
 }
 
@@ -752,7 +808,7 @@ __global__ void __launch_bounds__(PLAN_NW * 32) ft_plan_kernel(FtRounds a, int k
     const int n_quads = (n + 3) / 4, least = n_quads >= SPLIT_QUADS ? 2 : 1;
     for (int q = blockIdx.x * PLAN_NW + warp; q < n_quads; q += gridDim.x * PLAN_NW) {
         const int nq = min(4, n - 4 * q);
-        const int c = lane < nq ? a.act[4 * q + lane] : 0;
+        const int c = lane < nq ? a.act[(size_t)(cur ^ 1) * a.n_cells + 4 * q + lane] : 0;
         for (int i = lane; i < 4 * 256; i += 32) (&pos[warp][0][0])[i] = 0xffffu;
         __syncwarp();
         const int m_c = lane < nq ? a.ntop[c] : 0, most = __reduce_max_sync(FULL, m_c);
@@ -830,7 +886,7 @@ constexpr int SCAN_PF = 4;  // genes of the next table that a thread holds in re
 // loads its share of the next table into registers before it waits for the others, so that between two
 // items only the table's stores are left.
 template <int C, bool X64>
-__global__ void __launch_bounds__(SCAN_NW * 32, 1) ft_scan_kernel(FtRounds a, int k) {
+__global__ void __launch_bounds__(SCAN_NW * 32, 1) ft_scan_kernel(FtRounds a, int k, int per_quad) {
     extern __shared__ __align__(16) unsigned char dyn[];
     __shared__ int pre[257];      // work-list items before each label (in lorder)
     __shared__ int2 labs[256];    // the current item's labels and the units before each
@@ -847,7 +903,7 @@ __global__ void __launch_bounds__(SCAN_NW * 32, 1) ft_scan_kernel(FtRounds a, in
             a.n_act[cur] = 0;
         }
     }
-    const int n_quads = (a.n_act[nxt] + 3) / 4;
+    const int n_quads = (a.n_act[nxt] + per_quad - 1) / per_quad;  // one cell per quad in rounds of a few cells
     if (n_quads == 0) return;
     // Many quads: the same number of parts for each.  Few: parts of `upp` units so that every CTA gets some.
     // Filling a table costs about as much as scanning one unit at full rate, and four warps (one per
@@ -1120,7 +1176,7 @@ __global__ void __launch_bounds__(256) ft_scan32_kernel(FtRounds a, int k, int d
         __syncthreads();
         const int item = s_item;
         if (item >= n * parts) return;
-        const int c = a.act[item / parts], part = item % parts, ntop = a.ntop[c];
+        const int c = a.act[(size_t)nxt * a.n_cells + item / parts], part = item % parts, ntop = a.ntop[c];
         for (int i = tid; i < ntop; i += NT) top[i] = a.top[(size_t)c * a.L + i];
         __syncthreads();
         if (warp == 0) {
@@ -1262,10 +1318,10 @@ constexpr size_t kScan32Smem = 200 * 1024;
 constexpr size_t kScanSmem = 221 * 1024;  // with the kernel's static shared memory (6 KB), under 227 KB
 
 template <int C>
-void launch_scan_c(const FtRounds& a, int k, bool x64, cudaStream_t s) {
+void launch_scan_c(const FtRounds& a, int k, int per_quad, bool x64, cudaStream_t s) {
     const size_t smem = scan_smem(a.Wt, C);
     auto kern = x64 ? ft_scan_kernel<C, true> : ft_scan_kernel<C, false>;
-    kern<<<device_sm_count(), SCAN_NW * 32, smem, s>>>(a, k);
+    kern<<<device_sm_count(), SCAN_NW * 32, smem, s>>>(a, k, per_quad);
 }
 
 template <int C>
@@ -1304,11 +1360,16 @@ void launch_row_groups(const uint16_t* sorted, const int32_t* ptr, const int32_t
     count_launch();
 }
 
-void launch_pair_masks(const uint32_t* ft_genes, const uint32_t* ft_idx, int L, int nwords, uint32_t* mask,
-                       cudaStream_t s) {
+void launch_pair_masks(const uint32_t* ft_genes, const uint32_t* ft_idx, int L, int nwords, const int32_t* gene_thre,
+                       uint32_t* mask, uint32_t* cut_mask, cudaStream_t s) {
     SGR_CUDA(cudaMemsetAsync(mask, 0, (size_t)L * L * nwords * sizeof(uint32_t), s));
-    pair_mask_kernel<<<std::max(1, std::min((L * L + 7) / 8, device_sm_count() * 8)), 256, 0, s>>>(ft_genes, ft_idx,
-                                                                                              L * L, nwords, mask);
+    const int blocks = std::max(1, std::min((L * L + 7) / 8, device_sm_count() * 8));
+    pair_mask_kernel<<<blocks, 256, 0, s>>>(ft_genes, ft_idx, L * L, nwords, mask);
+    SGR_LAUNCH_CHECK();
+    count_launch();
+    if (!cut_mask) return;
+    cut_mask_kernel<<<blocks, 256, sizeof(uint32_t) * 8 * nwords, s>>>(ft_genes, ft_idx, L * L, L, nwords, gene_thre,
+                                                                     cut_mask);
     SGR_LAUNCH_CHECK();
     count_launch();
 }
@@ -1360,12 +1421,13 @@ void ft_rounds_setup(int copies) {
     else scan_attr<1>();
 }
 
-// Step k, the cells that go on put in order, and the quads of round k.  n: no more cells than this.
+// Step k, and the quads of round k (quads; the FP32-order scan needs none).  n: no more cells than this.
 void launch_ft_step(const FtRounds& a, int k, int n, bool quads, int32_t* scan_scratch, cudaStream_t s) {
+    const int mode = !quads ? STEP_LIST : n <= kFtDirectCells ? STEP_QUAD : STEP_ORDER;
     // Few cells are ordered by counting the smaller keys (4,096 cells: 4,096 warps of 128 steps); more by a
     // counting sort on a few more key bits than the cells are many, at most 20.
     int bits = 0;
-    if (n > 4096) {
+    if (mode == STEP_ORDER && n > 4096) {
         bits = 8;
         while (bits < 20 && (1 << bits) < 16 * n) ++bits;
         SGR_CUDA(cudaMemsetAsync(a.key_count, 0, sizeof(int32_t) << bits, s));
@@ -1375,10 +1437,12 @@ void launch_ft_step(const FtRounds& a, int k, int n, bool quads, int32_t* scan_s
     // others, so there the line lies higher.
     if (n <= (a.L > 64 ? 16 : 2) * device_sm_count())
         ft_step_kernel<STEP_NW_FEW><<<std::max(std::min(n, 2 * device_sm_count()), 1), STEP_NW_FEW * 32, step_smem(a),
-                                      s>>>(a, k, bits);
+                                      s>>>(a, k, mode, bits);
     else
-        ft_step_kernel<STEP_NW><<<ft_step_grid(n), STEP_NW * 32, step_smem(a), s>>>(a, k, bits);
+        ft_step_kernel<STEP_NW><<<ft_step_grid(n), STEP_NW * 32, step_smem(a), s>>>(a, k, mode, bits);
     SGR_LAUNCH_CHECK();
+    count_launch();
+    if (mode != STEP_ORDER) return;
     if (bits) {
         int32_t* start = a.key_count + ((size_t)1 << bits);
         launch_exclusive_scan(a.key_count, start, 1u << bits, scan_scratch, s);
@@ -1387,12 +1451,10 @@ void launch_ft_step(const FtRounds& a, int k, int n, bool quads, int32_t* scan_s
         ft_rank_kernel<<<std::max(1, std::min((n + 7) / 8, device_sm_count() * 8)), 256, 0, s>>>(a, k);
     }
     SGR_LAUNCH_CHECK();
-    count_launch(2);
-    if (!quads) return;
     const int blocks = std::max(1, std::min((n + 4 * PLAN_NW - 1) / (4 * PLAN_NW), device_sm_count() * 4));
     ft_plan_kernel<<<blocks, PLAN_NW * 32, 0, s>>>(a, k);
     SGR_LAUNCH_CHECK();
-    count_launch();
+    count_launch(2);
 }
 
 int ft_scan32_warps(int Wt) {
@@ -1415,11 +1477,12 @@ void launch_ft_scan32(const FtRounds& a, int k, int n, cudaStream_t s) {
     count_launch();
 }
 
-void launch_ft_scan(const FtRounds& a, int k, int copies, bool x64, cudaStream_t s) {
-    if (copies == 8) launch_scan_c<8>(a, k, x64, s);
-    else if (copies == 4) launch_scan_c<4>(a, k, x64, s);
-    else if (copies == 2) launch_scan_c<2>(a, k, x64, s);
-    else launch_scan_c<1>(a, k, x64, s);
+void launch_ft_scan(const FtRounds& a, int k, int n, int copies, bool x64, cudaStream_t s) {
+    const int per_quad = n <= kFtDirectCells ? 1 : 4;
+    if (copies == 8) launch_scan_c<8>(a, k, per_quad, x64, s);
+    else if (copies == 4) launch_scan_c<4>(a, k, per_quad, x64, s);
+    else if (copies == 2) launch_scan_c<2>(a, k, per_quad, x64, s);
+    else launch_scan_c<1>(a, k, per_quad, x64, s);
     SGR_LAUNCH_CHECK();
     count_launch();
 }

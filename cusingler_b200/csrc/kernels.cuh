@@ -306,6 +306,11 @@ struct FtCell {        // a cell's query side in the current round
     int32_t nS, kq;    // genes of the set, the query's stored entries among them
 };
 
+// Up to this many cells of a round each is a quad of its own (and the quads' arrays hold that many).  Its
+// lookups then serve one cell instead of four, but a scan of so few cells is bound by latency, and the
+// ordering and planning launches (7 us) are saved.
+constexpr int kFtDirectCells = 8;
+
 struct FtQuad {        // four active cells of a round and the labels scanned for them together
     int cell[4];       // the last repeated where there are fewer
     int nq, n_lab, units;  // cells, labels, 32-row blocks of the labels
@@ -324,6 +329,7 @@ struct FtRounds {
     const uint32_t* ft_genes;   // fine-tune pair lists (pool ids)
     const uint32_t* ft_idx;     // (start, len) per ordered pair
     const uint32_t* pair_mask;  // bits of each pair's whole list (nwords each), or nullptr
+    const uint32_t* cut_mask;   // bits of the lists as n candidates cut them (launch_pair_masks), or nullptr
     const int32_t* gene_thre;   // marker count per candidate count
     const LabelQ* lq;           // quantile grid per label (start 0)
     int L, Wt, nwords, eq_stride, shift;
@@ -347,12 +353,12 @@ struct FtRounds {
     uint32_t *ext_min, *ext_max;  // n_cells x L score extremes (order keys)
     uint32_t* blk_of;           // n_cells x L: first score block of each candidate
     FtEntry* list;              // L x n_cells work lists (labels that one cell of its quad needs)
-    FtQuad* quads;              // ceil(n_cells / 4)
+    FtQuad* quads;              // ceil(n_cells / 4), at least min(n_cells, kFtDirectCells)
     int2* q_label;              // per quad L: label, blocks of the quad's labels before it
     FtEntry* q_entry;           // per quad L x 4: the cells' entries (cellp = ~0: label not needed)
     unsigned long long* un;     // n_cells: the cells that go on, unordered (sort key << 32 | cell)
     int* key_count;             // counts of the keys' leading bits and their scan (2 << 20 ints + 1)
-    int* act;                   // n_cells: the active cells in order
+    int* act;                   // 2 x n_cells: the active cells in order (by the parity of the round)
     int* n_act;                 // 2: their number
     int* n_list;                // 2 x 256 work-list lengths
     int* queue;                 // 2 work-item counters
@@ -370,8 +376,10 @@ void launch_row_runs(const float* data, const int32_t* idx, const int32_t* ptr, 
                      uint16_t* sorted, int32_t* n_groups, cudaStream_t s);
 void launch_row_groups(const uint16_t* sorted, const int32_t* ptr, const int32_t* slot_row, const int32_t* blk_voff,
                        uint32_t n_slots, uint32_t pad, uint4* groups, cudaStream_t s);
-void launch_pair_masks(const uint32_t* ft_genes, const uint32_t* ft_idx, int L, int nwords, uint32_t* mask,
-                       cudaStream_t s);
+// Bits of each ordered pair's whole fine-tune list, and (cut_mask, may be null: (L - 1) L L rows) of its first
+// gene_thre(n) genes for the n = 2 .. L candidates that cut it.
+void launch_pair_masks(const uint32_t* ft_genes, const uint32_t* ft_idx, int L, int nwords, const int32_t* gene_thre,
+                       uint32_t* mask, uint32_t* cut_mask, cudaStream_t s);
 // n cells (or the first *n_dev of `list`): those with fewer than two candidates get their final label,
 // the others go to `cells` / `blk_off` (counter: cells << 36 | 32-row score blocks).
 void launch_ft_cells(int n, const int32_t* list, const int* n_dev, int L, const uint8_t* flags,
@@ -394,6 +402,6 @@ void launch_ft_step(const FtRounds& a, int k, int n, bool quads, int32_t* scan_s
 int ft_scan32_warps(int Wt);
 void launch_ft_scan32(const FtRounds& a, int k, int n, cudaStream_t s);
 // x64: the run sums in 64 bits (when 32 could overflow)
-void launch_ft_scan(const FtRounds& a, int k, int copies, bool x64, cudaStream_t s);
+void launch_ft_scan(const FtRounds& a, int k, int n, int copies, bool x64, cudaStream_t s);
 
 }  // namespace sgr
