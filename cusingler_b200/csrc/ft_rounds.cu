@@ -729,34 +729,41 @@ __global__ void __launch_bounds__(NW * 32, NW == STEP_NW ? 4 : 1) ft_step_kernel
     if (warp == NW - 1 && lane == 0 && my_rows) atomicAdd(a.stats + 1, my_rows);
 }
 
-__device__ __forceinline__ uint4 lds128(uint32_t addr) {
-    uint4 v;
-    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
-    return v;
-}
-
-// State of one row's pass for the four cells.
-template <bool X64>
+// State of one row's pass for NC cells.
+template <int NC, bool X64>
 struct RowSums {
     using T = typename std::conditional<X64, uint64_t, uint32_t>::type;
-    uint32_t P[4], tot[4], ka[4], B3[4];
-    T X[4];
+    uint32_t P[NC], tot[NC], ka[NC], B3[NC];
+    T X[NC];
 };
+
+// The table's words of one gene for NC cells.
+template <int NC>
+__device__ __forceinline__ void lookup(uint32_t addr, uint32_t (&v)[NC]) {
+    if (NC == 1) {
+        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v[0]) : "r"(addr));
+    } else {
+        asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                     : "=r"(v[0]), "=r"(v[1 % NC]), "=r"(v[2 % NC]), "=r"(v[3 % NC])
+                     : "r"(addr));
+    }
+}
 
 // One group of four entries: w0 = entries 0 | 1 << 16 (bit 15: the group ends a run), w1 = 2 | 3 << 16.
 // m = {16 C, 2, -1} as run-time values: with them the addresses, z and acc are multiply-adds, which
 // leaves the integer ALU (half rate, as the multiplier is) and the multiplier with about the same number
 // of instructions.
-template <int C, bool X64>
-__device__ __forceinline__ void scan_group(RowSums<X64>& s, uint32_t w0, uint32_t w1, uint32_t tab, int sh,
+template <int NC, bool X64>
+__device__ __forceinline__ void scan_group(RowSums<NC, X64>& s, uint32_t w0, uint32_t w1, uint32_t tab, int sh,
                                            uint32_t low, int3 m) {
-    const uint4 a = lds128((w0 & 0x7fffu) * (uint32_t)m.x + tab), b = lds128((w0 >> 16) * (uint32_t)m.x + tab);
-    const uint4 c = lds128((w1 & 0xffffu) * (uint32_t)m.x + tab), d = lds128((w1 >> 16) * (uint32_t)m.x + tab);
+    uint32_t va[NC], vb[NC], vc[NC], vd[NC];
+    lookup<NC>((w0 & 0x7fffu) * (uint32_t)m.x + tab, va);
+    lookup<NC>((w0 >> 16) * (uint32_t)m.x + tab, vb);
+    lookup<NC>((w1 & 0xffffu) * (uint32_t)m.x + tab, vc);
+    lookup<NC>((w1 >> 16) * (uint32_t)m.x + tab, vd);
     const bool end = (w0 & 0x8000u) != 0;
-    const uint32_t va[4] = {a.x, a.y, a.z, a.w}, vb[4] = {b.x, b.y, b.z, b.w};
-    const uint32_t vc[4] = {c.x, c.y, c.z, c.w}, vd[4] = {d.x, d.y, d.z, d.w};
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < NC; ++i) {
         s.P[i] += va[i] + vb[i];
         s.P[i] += vc[i] + vd[i];
         const uint32_t t = end ? s.P[i] : s.tot[i];
@@ -885,8 +892,10 @@ constexpr int SCAN_PF = 4;  // genes of the next table that a thread holds in re
 // Items are fetched two ahead while the current one is scanned, and a warp that has finished its blocks
 // loads its share of the next table into registers before it waits for the others, so that between two
 // items only the table's stores are left.
-template <int C, bool X64>
-__global__ void __launch_bounds__(SCAN_NW * 32, 1) ft_scan_kernel(FtRounds a, int k, int per_quad) {
+// NC = 1: every quad is one cell (rounds of a few cells).  Its table is the same memory with the cell's word
+// in all four places, 4 C copies of 4 bytes, and a row's pass takes half the instructions.
+template <int C, int NC, bool X64>
+__global__ void __launch_bounds__(SCAN_NW * 32, 1) ft_scan_kernel(FtRounds a, int k) {
     extern __shared__ __align__(16) unsigned char dyn[];
     __shared__ int pre[257];      // work-list items before each label (in lorder)
     __shared__ int2 labs[256];    // the current item's labels and the units before each
@@ -903,7 +912,7 @@ __global__ void __launch_bounds__(SCAN_NW * 32, 1) ft_scan_kernel(FtRounds a, in
             a.n_act[cur] = 0;
         }
     }
-    const int n_quads = (a.n_act[nxt] + per_quad - 1) / per_quad;  // one cell per quad in rounds of a few cells
+    const int n_quads = (a.n_act[nxt] + NC - 1) / NC;
     if (n_quads == 0) return;
     // Many quads: the same number of parts for each.  Few: parts of `upp` units so that every CTA gets some.
     // Filling a table costs about as much as scanning one unit at full rate, and four warps (one per
@@ -1030,7 +1039,8 @@ __global__ void __launch_bounds__(SCAN_NW * 32, 1) ft_scan_kernel(FtRounds a, in
         fetch(items[1]);
     }
     __syncthreads();
-    const uint32_t tab = (uint32_t)__cvta_generic_to_shared(dyn) + (lane & (C - 1)) * 16;
+    const uint32_t tab = (uint32_t)__cvta_generic_to_shared(dyn) +
+                         (NC == 1 ? (lane & (4 * C - 1)) * 4 : (lane & (C - 1)) * 16);
     const uint32_t low = (1u << a.shift) - 1u;
     const int3 mul = a.mul;
     // the table's words of gene g for an item's four cells
@@ -1087,11 +1097,11 @@ __global__ void __launch_bounds__(SCAN_NW * 32, 1) ft_scan_kernel(FtRounds a, in
             FtEntry my = {~0u, 0u};
             if (lane < 4) my = quad >= 0 ? a.q_entry[((size_t)quad * a.L + uj) * 4 + lane] : it.entry[lane];
             const uint4* p = a.groups + v0 + lane;
-            RowSums<X64> s = {};
+            RowSums<NC, X64> s = {};
             for (int v = 0; v < nv; ++v) {
                 const uint4 wn = v + 2 < nv ? __ldg(p + 32 * (v + 2)) : w;  // two vectors ahead
-                scan_group<C, X64>(s, w.x, w.y, tab, a.shift, low, mul);
-                scan_group<C, X64>(s, w.z, w.w, tab, a.shift, low, mul);
+                scan_group<NC, X64>(s, w.x, w.y, tab, a.shift, low, mul);
+                scan_group<NC, X64>(s, w.z, w.w, tab, a.shift, low, mul);
                 w = w2;
                 w2 = wn;
             }
@@ -1099,7 +1109,7 @@ __global__ void __launch_bounds__(SCAN_NW * 32, 1) ft_scan_kernel(FtRounds a, in
             const bool valid = ub * 32 + lane < (int)a.ctidx[2 * labs[uj].x + 1];
             if (u < u1) open(u);  // the next unit's first vectors, on their way during the last steps
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
+            for (int i = 0; i < NC; ++i) {
                 const uint32_t cellp = __shfl_sync(FULL, my.cellp, i), sblk = __shfl_sync(FULL, my.blk, i);
                 if (cellp == ~0u) continue;  // the cell does not need this label
                 const FtCell c = it.par[i];
@@ -1318,16 +1328,19 @@ constexpr size_t kScan32Smem = 200 * 1024;
 constexpr size_t kScanSmem = 221 * 1024;  // with the kernel's static shared memory (6 KB), under 227 KB
 
 template <int C>
-void launch_scan_c(const FtRounds& a, int k, int per_quad, bool x64, cudaStream_t s) {
+void launch_scan_c(const FtRounds& a, int k, bool one, bool x64, cudaStream_t s) {
     const size_t smem = scan_smem(a.Wt, C);
-    auto kern = x64 ? ft_scan_kernel<C, true> : ft_scan_kernel<C, false>;
-    kern<<<device_sm_count(), SCAN_NW * 32, smem, s>>>(a, k, per_quad);
+    auto kern = one ? (x64 ? ft_scan_kernel<C, 1, true> : ft_scan_kernel<C, 1, false>)
+                    : (x64 ? ft_scan_kernel<C, 4, true> : ft_scan_kernel<C, 4, false>);
+    kern<<<device_sm_count(), SCAN_NW * 32, smem, s>>>(a, k);
 }
 
 template <int C>
 void scan_attr() {
-    allow_smem(ft_scan_kernel<C, true>, kScanSmem);
-    allow_smem(ft_scan_kernel<C, false>, kScanSmem);
+    allow_smem(ft_scan_kernel<C, 4, true>, kScanSmem);
+    allow_smem(ft_scan_kernel<C, 4, false>, kScanSmem);
+    allow_smem(ft_scan_kernel<C, 1, true>, kScanSmem);
+    allow_smem(ft_scan_kernel<C, 1, false>, kScanSmem);
 }
 
 }  // namespace
@@ -1478,11 +1491,11 @@ void launch_ft_scan32(const FtRounds& a, int k, int n, cudaStream_t s) {
 }
 
 void launch_ft_scan(const FtRounds& a, int k, int n, int copies, bool x64, cudaStream_t s) {
-    const int per_quad = n <= kFtDirectCells ? 1 : 4;
-    if (copies == 8) launch_scan_c<8>(a, k, per_quad, x64, s);
-    else if (copies == 4) launch_scan_c<4>(a, k, per_quad, x64, s);
-    else if (copies == 2) launch_scan_c<2>(a, k, per_quad, x64, s);
-    else launch_scan_c<1>(a, k, per_quad, x64, s);
+    const bool one = n <= kFtDirectCells;
+    if (copies == 8) launch_scan_c<8>(a, k, one, x64, s);
+    else if (copies == 4) launch_scan_c<4>(a, k, one, x64, s);
+    else if (copies == 2) launch_scan_c<2>(a, k, one, x64, s);
+    else launch_scan_c<1>(a, k, one, x64, s);
     SGR_LAUNCH_CHECK();
     count_launch();
 }

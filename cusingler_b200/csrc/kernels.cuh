@@ -307,9 +307,11 @@ struct FtCell {        // a cell's query side in the current round
 };
 
 // Up to this many cells of a round each is a quad of its own (and the quads' arrays hold that many).  Its
-// lookups then serve one cell instead of four, but a scan of so few cells is bound by latency, and the
-// ordering and planning launches (7 us) are saved.
-constexpr int kFtDirectCells = 8;
+// lookups then serve one cell instead of four, but a round of so few cells is bound by latency: a pass for
+// one cell takes half the instructions, and the ordering and planning launches (7 us) are saved.  Whole
+// calls, with 8 / 24 / 64 / 148 cells: 856 / 815 / 780 / 779 us for 100 queries x 1,900 cells, 191.9 /
+// 191.7 / 191.2 / 201.1 ms for 3 x 16,384 x 40,000 in 120 labels.
+constexpr int kFtDirectCells = 64;
 
 struct FtQuad {        // four active cells of a round and the labels scanned for them together
     int cell[4];       // the last repeated where there are fewer
