@@ -148,7 +148,7 @@ struct sgr_ctx {
     int corr_f16 = 0;              // tuning: score-step correlation on FP16 operands (not exact)
     int corr_pair = 0;             // tuning: exact correlation on SM pairs (cta_group::2, 256-row tiles)
     int corr_gm = 16;              // tuning: row bands per group of the correlation's tile order
-    int select_warps = -1;         // tuning: score-step selection, 8 or 16 warps per row-staging CTA, 0 / 1 a warp per row, -1 by size
+    int select_warps = -1;         // tuning: score-step selection, 8 / 16 a CTA per row, 0 / 1 a warp per row and label, -1 by size
     int host_training = 0;         // tuning: marker medians and pair lists on the host instead of the device
     int pipeline = 0;              // tuning: fine-tune each score block on its own stream while the next is scored
     cudaStream_t ft_s = nullptr;   // the pipelined fine-tune's stream

@@ -164,58 +164,54 @@ __device__ __forceinline__ uint32_t warp_max_u32(uint32_t x) { return __reduce_m
 
 // Keys of order statistics j and j+1 (0-based) of v[0..n) (no NaN, kmin < kmax) by one warp: a
 // 256-bin histogram over a monotone linear map of [min, max] locates the bin holding statistic j;
-// that bin's keys (at most 256) are compacted into `buf` (the histogram's memory) and sorted.
+// that bin's keys (at most 256) are compacted into `buf` (the histogram's memory, 16-byte aligned) and sorted.
 // Returns false (nothing decided) when the bin is larger than 256 or the range is degenerate.
 __device__ bool bucket_select(const float* v, int n, int j, int* hist, int lane, uint32_t kmin, uint32_t kmax,
                               uint32_t* ka, uint32_t* kb) {
     const float fmin = key_float(kmin), fmax = key_float(kmax);
     const float span = fmax - fmin;
     if (!(span > 1e-30f) || !(span < 1e30f)) return false;
-    const float scale = __fdividef(256.0f, span);  // any positive scale keeps the map monotone
-    // The bin of x is round-to-nearest((x - min) * scale), read from the bits of one FMA whose result
-    // lies in [2^23, 2^24), where floats are the integers: bits(y) = 0x4B000000 + y - 2^23.  The map
-    // from x to those bits is monotone non-decreasing, which is all the selection needs (both passes
-    // use the same map).  Clamped both ways on the bits, so that a value outside [min, max] (extremes
-    // that do not match the list) still lands in a bin rather than outside the histogram.
+    // The bin of x is round-to-nearest(255 * y) with y = (x - min) / span saturated to [0, 1], so that a value
+    // outside [min, max] (extremes that do not match the list) still lands in a bin.  The second FMA's result
+    // lies in [2^23, 2^23 + 255], where floats are the integers: bits = 0x4B000000 + bin.  The map from x to
+    // those bits is monotone non-decreasing for any positive scale, which is all the selection needs (both
+    // passes use the same map).
     constexpr int B0 = 0x4B000000;
-    const float shift = fmaf(-fmin, scale, 8388608.0f);
-    auto bin_bits = [&](float x) { return __float_as_int(fmaf(x, scale, shift)); };
-    auto bin_of = [&](float x) { return min(max(bin_bits(x), B0), B0 + 255) - B0; };
-    for (int b = lane; b < 256; b += 32) hist[b] = 0;
+    const float scale = __fdividef(1.0f, span);
+    const float shift = -fmin * scale;
+    auto bin_bits = [&](float x) {
+        return __float_as_int(fmaf(__saturatef(fmaf(x, scale, shift)), 255.0f, 8388608.0f));
+    };
+    int4* h4 = reinterpret_cast<int4*>(hist);
+    h4[lane] = make_int4(0, 0, 0, 0);
+    h4[32 + lane] = make_int4(0, 0, 0, 0);
     __syncwarp();
     int i = lane;
     for (; i + 96 < n; i += 128) {  // four independent loads in flight per lane
         const float x0 = v[i], x1 = v[i + 32], x2 = v[i + 64], x3 = v[i + 96];
-        atomicAdd(&hist[bin_of(x0)], 1);
-        atomicAdd(&hist[bin_of(x1)], 1);
-        atomicAdd(&hist[bin_of(x2)], 1);
-        atomicAdd(&hist[bin_of(x3)], 1);
+        atomicAdd(&hist[bin_bits(x0) - B0], 1);
+        atomicAdd(&hist[bin_bits(x1) - B0], 1);
+        atomicAdd(&hist[bin_bits(x2) - B0], 1);
+        atomicAdd(&hist[bin_bits(x3) - B0], 1);
     }
-    for (; i < n; i += 32) atomicAdd(&hist[bin_of(v[i])], 1);
+    for (; i < n; i += 32) atomicAdd(&hist[bin_bits(v[i]) - B0], 1);
     __syncwarp();
-    int c[8], s = 0;
-#pragma unroll
-    for (int t = 0; t < 8; ++t) {
-        c[t] = hist[8 * lane + t];
-        s += c[t];
-    }
-    const int incl = warp_incl_scan(s, lane), excl = incl - s;
+    // Lane l holds bins 4 l .. 4 l + 3 of each half of the histogram (conflict-free 16-byte loads).  The half
+    // with statistic j is known from the first half's total, and only that half's counts are scanned.
+    const int4 ch[2] = {h4[lane], h4[32 + lane]};
+    const int s0 = ch[0].x + ch[0].y + ch[0].z + ch[0].w, s1 = ch[1].x + ch[1].y + ch[1].z + ch[1].w;
+    const int tot0 = __reduce_add_sync(FULL, s0);
+    const bool upper = j >= tot0;
+    const int4 c = upper ? ch[1] : ch[0];
+    const int s = upper ? s1 : s0;
+    const int incl = warp_incl_scan(s, lane) + (upper ? tot0 : 0), excl = incl - s;
     const unsigned own = __ballot_sync(FULL, excl <= j && j < incl);
     const int src = __ffs(own) - 1;
-    int bin = 0, before = 0, cnt = 0;
-    if (lane == src) {
-        int acc = excl;
-#pragma unroll
-        for (int t = 0; t < 8; ++t) {
-            if (j < acc + c[t]) {
-                bin = 8 * lane + t;
-                before = acc;
-                cnt = c[t];
-                break;
-            }
-            acc += c[t];
-        }
-    }
+    const int e1 = excl + c.x, e2 = e1 + c.y, e3 = e2 + c.z;
+    const bool p1 = j >= e1, p2 = j >= e2, p3 = j >= e3;
+    int bin = (upper ? 128 : 0) + 4 * lane + (p1 ? 1 : 0) + (p2 ? 1 : 0) + (p3 ? 1 : 0);
+    int before = p3 ? e3 : p2 ? e2 : p1 ? e1 : excl;
+    int cnt = p3 ? c.w : p2 ? c.z : p1 ? c.y : c.x;
     bin = __shfl_sync(FULL, bin, src);
     before = __shfl_sync(FULL, before, src);
     cnt = __shfl_sync(FULL, cnt, src);
@@ -225,41 +221,49 @@ __device__ bool bucket_select(const float* v, int n, int j, int* hist, int lane,
     int nb = -1, total = cnt;
     if (j + 1 >= before + cnt && j + 1 < n) {
         int cand = 256, ccand = 0;
-#pragma unroll
-        for (int t = 0; t < 8; ++t)
-            if (cand == 256 && 8 * lane + t > bin && c[t] > 0) {
-                cand = 8 * lane + t;
-                ccand = c[t];
+        auto look = [&](int b, int count) {
+            if (cand == 256 && b > bin && count > 0) {
+                cand = b;
+                ccand = count;
             }
+        };
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            look(128 * h + 4 * lane, ch[h].x);
+            look(128 * h + 4 * lane + 1, ch[h].y);
+            look(128 * h + 4 * lane + 2, ch[h].z);
+            look(128 * h + 4 * lane + 3, ch[h].w);
+        }
         nb = __reduce_min_sync(FULL, cand);
         const int cnb = __reduce_add_sync(FULL, cand == nb ? ccand : 0);
         if (cnt + cnb <= 256) total = cnt + cnb;
         else nb = -1;
     }
     __syncwarp();
-    // Collect the values of bins bin..last (the bins between bin and nb are empty), compared on the
-    // map's bits: bin(x) >= bin holds for every x when bin is 0, else exactly when bits >= B0 + bin;
-    // bin(x) <= last likewise.  Raw float bits are stored and turned into order keys afterwards.
+    // Collect the values of bins bin..last (the bins between bin and nb are empty), compared on the map's
+    // bits.  Raw float bits are stored and turned into order keys afterwards.
     const int last = nb >= 0 ? nb : bin;
-    const int lo = bin == 0 ? INT_MIN : B0 + bin, hi = last == 255 ? INT_MAX : B0 + last;
+    const unsigned lo = (unsigned)(B0 + bin), width = (unsigned)(last - bin);
     uint32_t* buf = reinterpret_cast<uint32_t*>(hist);
     int w = 0;
     const unsigned lt = (1u << lane) - 1u;
     int base = 0;
-    for (; base + 64 <= n; base += 64) {  // two 32-value chunks per step
-        const float x0 = v[base + lane], x1 = v[base + 32 + lane];
-        const int y0 = bin_bits(x0), y1 = bin_bits(x1);
-        const bool in0 = y0 >= lo && y0 <= hi, in1 = y1 >= lo && y1 <= hi;
-        const unsigned m0 = __ballot_sync(FULL, in0), m1 = __ballot_sync(FULL, in1);
-        if (in0) buf[w + __popc(m0 & lt)] = __float_as_uint(x0);
-        if (in1) buf[w + __popc(m0) + __popc(m1 & lt)] = __float_as_uint(x1);
-        w += __popc(m0) + __popc(m1);
+    for (; base + 128 <= n; base += 128) {  // four 32-value chunks per step
+        float x[4];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) x[t] = v[base + 32 * t + lane];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+            const bool in = (unsigned)bin_bits(x[t]) - lo <= width;
+            const unsigned m = __ballot_sync(FULL, in);
+            if (in) buf[w + __popc(m & lt)] = __float_as_uint(x[t]);
+            w += __popc(m);
+        }
     }
     for (; base < n; base += 32) {
         const int i0 = base + lane;
         const float x0 = i0 < n ? v[i0] : 0.f;
-        const int y0 = bin_bits(x0);
-        const bool in0 = i0 < n && y0 >= lo && y0 <= hi;
+        const bool in0 = i0 < n && (unsigned)bin_bits(x0) - lo <= width;
         const unsigned m0 = __ballot_sync(FULL, in0);
         if (in0) buf[w + __popc(m0 & lt)] = __float_as_uint(x0);
         w += __popc(m0);
@@ -268,16 +272,13 @@ __device__ bool bucket_select(const float* v, int n, int j, int* hist, int lane,
     const int r = j - before;  // statistic j is the r-th smallest collected key (r < cnt <= total)
     bool have_b = r + 1 < total;
     if (total <= 32) {
-        // one key per lane; its rank among the collected keys (ties by position) picks r and r + 1
+        // one key per lane; with le = the number of collected keys not above it, statistic r is the smallest
+        // key with le > r, and r + 1 the smallest with le > r + 1
         const uint32_t key = lane < total ? ord_key(__uint_as_float(buf[lane])) : 0xffffffffu;
-        int rank = 0;
-        for (int t = 0; t < total; ++t) {
-            const uint32_t kt = __shfl_sync(FULL, key, t);
-            rank += (kt < key) | ((kt == key) & (t < lane));
-        }
-        *ka = __shfl_sync(FULL, key, __ffs(__ballot_sync(FULL, lane < total && rank == r)) - 1);
-        const unsigned mb = __ballot_sync(FULL, lane < total && rank == r + 1);
-        if (have_b) *kb = __shfl_sync(FULL, key, __ffs(mb) - 1);
+        int le = 0;
+        for (int t = 0; t < total; ++t) le += __shfl_sync(FULL, key, t) <= key;
+        *ka = __reduce_min_sync(FULL, lane < total && le > r ? key : 0xffffffffu);
+        if (have_b) *kb = __reduce_min_sync(FULL, lane < total && le > r + 1 ? key : 0xffffffffu);
     } else {
         for (int i = lane; i < total; i += 32) buf[i] = ord_key(__uint_as_float(buf[i]));
         int np = 1;

@@ -720,7 +720,7 @@ __global__ void __launch_bounds__(256) split_scan_kernel(FtPersistentArgs a, FtS
 __global__ void __launch_bounds__(SPLIT_NW * 32) split_decide_kernel(FtPersistentArgs a, FtSplit sp, int q) {
     extern __shared__ __align__(16) unsigned char smem[];
     constexpr int NW = SPLIT_NW;
-    __shared__ int hist[NW * 256];
+    __shared__ __align__(16) int hist[NW * 256];
     __shared__ float lsc[256];
     __shared__ int off[257];
     __shared__ uint8_t top[256], tmp[256];

@@ -448,7 +448,7 @@ __device__ int keep_candidates(const float* lsc, int ntop, uint8_t* top, uint8_t
 
 template <int NW>
 struct StepSmem {
-    int hist[NW][256];
+    alignas(16) int hist[NW][256];
     float lsc[256];
     uint32_t off[256];  // first 32-row block of each candidate's scores
     uint8_t top[256], tmp[256];

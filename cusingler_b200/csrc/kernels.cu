@@ -11,7 +11,7 @@
 //   spearman (918-945)        -> corr_simt_kernel (fp32ref: fma chain over genes in order).
 //   spearman_reduce (803-856) -> ft_corr_kernel (fp32ref: 128 contiguous chunks + pairwise tree).
 //   percentile + get_label's argmax and flags (947-978, 1080-1133)
-//       -> select_first_kernel (radix selection of the two order statistics per label, libstdc++
+//       -> select_items_kernel / select_row_kernel (selection of the two order statistics per label, libstdc++
 //          std::sort restated for NaN-bearing lists, std::minmax_element order for the argmax).
 
 #include <algorithm>
@@ -603,70 +603,52 @@ __global__ void __launch_bounds__(256) corr_few_kernel(const int8_t* A, const in
 
 // ---- per-label quantile ------------------------------------------------------------------------
 
-// STAGE: the block first copies the query's score row (row_len floats) into shared memory with
-// 16-byte loads, and warps take labels from `lorder` (longest first) through a shared counter; every
-// selection pass then reads shared memory instead of global memory.
-template <bool STAGE, int NW = STAGE ? 16 : 8>
-__global__ void __launch_bounds__(NW * 32) select_first_kernel(const float* scores, int64_t ld, int nq, int L,
-                                                           const LabelQ* lq, float p, float thre, const int64_t* qn2,
-                                                           float* label_scores, int32_t* first, uint8_t* flags,
-                                                           float* scratch, int64_t spw, int* status, int row_len,
-                                                           const int32_t* lorder, const uint32_t* ext_min,
-                                                           const uint32_t* ext_max) {
+// Row form: the block copies the query's score row (row_len floats) into shared memory with 16-byte loads,
+// and its warps take labels from `lorder` (longest first) through a shared counter; every selection pass then
+// reads shared memory.
+template <int NW>
+__global__ void __launch_bounds__(NW * 32) select_row_kernel(const float* scores, int64_t ld, int nq, int L,
+                                                            const LabelQ* lq, float p, float thre,
+                                                            const int64_t* qn2, float* label_scores, int32_t* first,
+                                                            uint8_t* flags, float* scratch, int64_t spw, int* status,
+                                                            int row_len, const int32_t* lorder,
+                                                            const uint32_t* ext_min, const uint32_t* ext_max) {
     extern __shared__ __align__(16) float srow[];
     __shared__ float ls[256];
-    __shared__ int hist[NW][256];
+    __shared__ __align__(16) int hist[NW][256];
     __shared__ int s_mx, s_next;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     float* my_scratch = scratch ? scratch + (size_t)(blockIdx.x * NW + warp) * spw : nullptr;
-    const bool vec = STAGE && (ld % 4) == 0 && (reinterpret_cast<uintptr_t>(scores) & 15) == 0;
+    const bool vec = (ld % 4) == 0 && (reinterpret_cast<uintptr_t>(scores) & 15) == 0;
     for (int q = blockIdx.x; q < nq; q += gridDim.x) {
         const float* row = scores + (size_t)q * ld;
         const bool qnan = qn2[q] == 0;
-        if (STAGE) {
-            if (!qnan) {
-                if (vec) {
-                    const float4* src = reinterpret_cast<const float4*>(row);
-                    float4* dst = reinterpret_cast<float4*>(srow);
-                    for (int i = threadIdx.x; i < row_len / 4; i += NW * 32) dst[i] = __ldcs(src + i);
-                    for (int i = (row_len & ~3) + threadIdx.x; i < row_len; i += NW * 32) srow[i] = __ldcs(row + i);
-                } else {
-                    for (int i = threadIdx.x; i < row_len; i += NW * 32) srow[i] = __ldcs(row + i);
-                }
+        if (!qnan) {
+            if (vec) {
+                const float4* src = reinterpret_cast<const float4*>(row);
+                float4* dst = reinterpret_cast<float4*>(srow);
+                for (int i = threadIdx.x; i < row_len / 4; i += NW * 32) dst[i] = __ldcs(src + i);
+                for (int i = (row_len & ~3) + threadIdx.x; i < row_len; i += NW * 32) srow[i] = __ldcs(row + i);
+            } else {
+                for (int i = threadIdx.x; i < row_len; i += NW * 32) srow[i] = __ldcs(row + i);
             }
-            // the block's next row is brought into L2 while this one is selected, so that its staging
-            // loads hit L2 (16-byte aligned rows, ld % 4 == 0: the rounded-up size stays in the row)
-            if (vec && threadIdx.x == 0 && q + (int)gridDim.x < nq && qn2[q + gridDim.x] != 0) {
-                const float* nxt = scores + (size_t)(q + gridDim.x) * ld;
-                const uint32_t bytes = (uint32_t)(row_len * 4 + 15) & ~15u;
-                asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(nxt), "r"(bytes) : "memory");
-            }
-            if (threadIdx.x == 0) s_next = 0;
-            __syncthreads();
-            row = srow;
-            for (;;) {
-                int i = 0;
-                if (lane == 0) i = atomicAdd(&s_next, 1);
-                i = __shfl_sync(FULL, i, 0);
-                if (i >= L) break;
-                const int l = lorder[i];
-                const LabelQ d = lq[l];
-                float r;
-                if (qnan) r = __int_as_float(0x7fffffff);
-                else if (ext_min && !d.has_nan && d.kind != 0)  // extremes from the correlation epilogue
-                    r = quantile_warp_core(row + d.start, d, p, hist[warp], my_scratch, lane, status,
-                                           ext_min[(size_t)q * L + l], ext_max[(size_t)q * L + l], false);
-                else r = quantile_warp(row + d.start, d, p, hist[warp], my_scratch, lane, status);
-                if (lane == 0) ls[l] = r;
-            }
-        } else {
-            for (int l = warp; l < L; l += NW) {
-                const LabelQ d = lq[l];
-                float r;
-                if (qnan) r = __int_as_float(0x7fffffff);
-                else r = quantile_warp(row + d.start, d, p, hist[warp], my_scratch, lane, status);
-                if (lane == 0) ls[l] = r;
-            }
+        }
+        if (threadIdx.x == 0) s_next = 0;
+        __syncthreads();
+        for (;;) {
+            int i = 0;
+            if (lane == 0) i = atomicAdd(&s_next, 1);
+            i = __shfl_sync(FULL, i, 0);
+            if (i >= L) break;
+            const int l = lorder[i];
+            const LabelQ d = lq[l];
+            float r;
+            if (qnan) r = __int_as_float(0x7fffffff);
+            else if (ext_min && !d.has_nan && d.kind != 0)  // extremes from the correlation epilogue
+                r = quantile_warp_core(srow + d.start, d, p, hist[warp], my_scratch, lane, status,
+                                       ext_min[(size_t)q * L + l], ext_max[(size_t)q * L + l], false);
+            else r = quantile_warp(srow + d.start, d, p, hist[warp], my_scratch, lane, status);
+            if (lane == 0) ls[l] = r;
         }
         __syncthreads();
         if (threadIdx.x == 0) {
@@ -685,72 +667,66 @@ __global__ void __launch_bounds__(NW * 32) select_first_kernel(const float* scor
     }
 }
 
-// Warp-per-row form: each warp selects every label of its query rows straight from the score rows
-// (global memory; a label's second pass hits L1 / L2), so no block barrier waits for a row's longest
-// label, and a CTA needs only a histogram per warp (up to 64 warps per SM).  Every row has the same
-// labels, so the warps' work is balanced by construction.  Each warp prefetches into L2 the list of the
-// label two ahead in its row.
-// MINB: CTAs per SM the register allocation is sized for (2: 64 registers and 32 warps per SM,
-// 3: 40 registers and 48 warps per SM).
+// Item form: one warp per (label, query row), straight from the score rows in global memory (a list's second
+// pass hits L1 / L2).  Items run label by label, longest label first, rows inside: the warps of a turn have
+// lists of the same length, no barrier waits for a row's longest label, and the last turn is one of the
+// shortest lists.  (Whole rows per warp left the last turn of rows nearly empty: 562 us at 12,345 x 20,000
+// scores and 1,288 us at 8,192 x 40,000, against 453 and 886 here; the bound, one read of the scores, is 151 and
+// 200 us.)  It is bound by instruction issue and load latency together: 48 registers, 40 warps per SM and two
+// passes of four loads in flight are faster than 64 registers and 32 warps (480) or 40 and 48 (500 us, spills);
+// an L2 prefetch of the warp's next list does not help (462).  first_rows_kernel then takes each row's maximum
+// and flags.
 template <int NW, int MINB>
-__global__ void __launch_bounds__(NW * 32, MINB) select_rows_kernel(const float* scores, int64_t ld, int nq, int L,
-                                                           const LabelQ* lq, float p, float thre,
-                                                           const int64_t* qn2, float* label_scores, int32_t* first,
-                                                           uint8_t* flags, float* scratch, int64_t spw, int* status,
-                                                           int row_len, const int32_t* lorder,
-                                                           const uint32_t* ext_min, const uint32_t* ext_max) {
-    __shared__ int hist[NW][256];
-    __shared__ float ls_all[NW][256];
+__global__ void __launch_bounds__(NW * 32, MINB) select_items_kernel(const float* scores, int64_t ld, int nq, int L,
+                                                            const LabelQ* lq, float p, const int64_t* qn2,
+                                                            float* label_scores, float* scratch, int64_t spw,
+                                                            int* status, const int32_t* lorder,
+                                                            const uint32_t* ext_min, const uint32_t* ext_max) {
+    __shared__ __align__(16) int hist[NW][256];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int gw = blockIdx.x * NW + warp, n_warps = gridDim.x * NW;
     float* my_scratch = scratch ? scratch + (size_t)gw * spw : nullptr;
-    float* ls = ls_all[warp];
-    // rows start on 16 bytes when ld is a multiple of 4, so a label's list widened to 16-byte bounds
-    // stays inside its row
-    const bool pf = (ld % 4) == 0 && (reinterpret_cast<uintptr_t>(scores) & 15) == 0;
-    for (int q = gw; q < nq; q += n_warps) {
-        const float* row = scores + (size_t)q * ld;
-        const bool qnan = qn2[q] == 0;
-        // L2 prefetch of the list of the label two ahead (a whole row fetched a row ahead is evicted
-        // before use: every warp of the GPU streams its own rows meanwhile)
-        auto prefetch_label = [&](int idx) {
-            if (pf && !qnan && lane == 0 && idx < L) {
-                const LabelQ dn = lq[lorder[idx]];
-                const uintptr_t a0 = reinterpret_cast<uintptr_t>(row + dn.start) & ~uintptr_t(15);
-                const uintptr_t a1 = (reinterpret_cast<uintptr_t>(row + dn.start + dn.len) + 15) & ~uintptr_t(15);
-                if (a1 > a0)
-                    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a0), "r"((uint32_t)(a1 - a0))
-                                 : "memory");
-            }
-        };
-        prefetch_label(0);
-        prefetch_label(1);
-        for (int i = 0; i < L; ++i) {
-            prefetch_label(i + 2);
-            const int l = lorder[i];
-            const LabelQ d = lq[l];
-            float r;
-            if (qnan) r = __int_as_float(0x7fffffff);
-            else if (ext_min && !d.has_nan && d.kind != 0)  // extremes from the correlation epilogue
-                r = quantile_warp_core(row + d.start, d, p, hist[warp], my_scratch, lane, status,
-                                       ext_min[(size_t)q * L + l], ext_max[(size_t)q * L + l], false);
-            else r = quantile_warp(row + d.start, d, p, hist[warp], my_scratch, lane, status);
-            if (lane == 0) ls[l] = r;
+    int i = gw / nq, q = gw % nq, l = 0, held = -1;
+    LabelQ d{};
+    while (i < L) {
+        if (i != held) {
+            l = lorder[i];
+            d = lq[l];
+            held = i;
         }
+        const float* v = scores + (size_t)q * ld + d.start;
+        float r;
+        if (qn2[q] == 0) r = __int_as_float(0x7fffffff);
+        else if (ext_min && !d.has_nan && d.kind != 0)  // extremes from the correlation epilogue
+            r = quantile_warp_core(v, d, p, hist[warp], my_scratch, lane, status, ext_min[(size_t)q * L + l],
+                                   ext_max[(size_t)q * L + l], false);
+        else r = quantile_warp(v, d, p, hist[warp], my_scratch, lane, status);
+        if (lane == 0) label_scores[(size_t)q * L + l] = r;
         __syncwarp();
-        int mn = 0, mx = 0;
-        if (lane == 0) {
-            stl::minmax(ls, L, &mn, &mx);
-            first[q] = mx;
-        }
-        mx = __shfl_sync(FULL, mx, 0);
-        const float t = __fsub_rn(ls[mx], thre);
-        for (int l = lane; l < L; l += 32) {
-            label_scores[(size_t)q * L + l] = ls[l];
-            if (flags) flags[(size_t)q * L + l] = ls[l] >= t ? 1 : 0;
-        }
-        __syncwarp();
+        for (q += n_warps; q >= nq; q -= nq) ++i;
     }
+}
+
+// Per query row, one warp: the label of the largest score as std::minmax_element picks it, and the flags of
+// the labels within thre of it.
+__global__ void __launch_bounds__(256) first_rows_kernel(const float* label_scores, int nq, int L, float thre,
+                                                         int32_t* first, uint8_t* flags) {
+    __shared__ float ls_all[8][256];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int q = blockIdx.x * 8 + warp;
+    if (q >= nq) return;
+    float* ls = ls_all[warp];
+    for (int l = lane; l < L; l += 32) ls[l] = label_scores[(size_t)q * L + l];
+    __syncwarp();
+    int mn = 0, mx = 0;
+    if (lane == 0) {
+        stl::minmax(ls, L, &mn, &mx);
+        first[q] = mx;
+    }
+    mx = __shfl_sync(FULL, mx, 0);
+    if (!flags) return;
+    const float t = __fsub_rn(ls[mx], thre);
+    for (int l = lane; l < L; l += 32) flags[(size_t)q * L + l] = ls[l] >= t ? 1 : 0;
 }
 
 // ---- fine-tune correlation and selection ------------------------------------------------------
@@ -806,7 +782,7 @@ __global__ void __launch_bounds__(256) ft_select_kernel(const FtGroup* groups, c
                                                         const LabelQ* lq, float p, const float* scores,
                                                         float* label_scores, float* scratch, int64_t spw,
                                                         int* status) {
-    __shared__ int hist[8][256];
+    __shared__ __align__(16) int hist[8][256];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     float* my_scratch = scratch ? scratch + (size_t)(blockIdx.x * 8 + warp) * spw : nullptr;
     for (uint32_t w = blockIdx.x * 8 + warp; w < n_items; w += gridDim.x * 8) {
@@ -1120,40 +1096,31 @@ void launch_select_first(const float* scores, int64_t ld, int nq, int L, const L
                          const uint32_t* ext_min, const uint32_t* ext_max, int warps) {
     if (nq <= 0) return;
     const size_t stage_bytes = (((size_t)std::max(row_len, 1) * 4 + 15) & ~size_t(15));
-    if (warps < 0) {
-        // By size.  A staging CTA takes a row's labels 16 at a time, a warp one by one, so few rows go to CTAs;
-        // with many rows the warp form has more rows in flight and no barriers.  They meet at about 40 rows per
-        // SM where two staging CTAs fit an SM (us, CTA / warp form: 261 / 291 for 5,000 x 20,000 scores, 624 / 562
-        // for 12,345 x 20,000), and at 16 where only one does (527 / 546 for 2,400 x 40,000, 1,746 / 1,288 for
-        // 8,192 x 40,000).  Up to two turns of the 64-register form's 32 warps per SM, the 48 warps of the
-        // 40-register form finish earlier (1,288 against 1,492 at the last size), beyond they do not.
-        const long per_sm = stage_bytes <= 100 * 1024 ? 40 : 16;
-        warps = nq < per_sm * sm_count() ? 16 : nq < 64L * sm_count() ? 1 : 0;
-    }
-    if (lorder && (warps == 0 || warps == 1)) {  // one warp per row, 16 warps per CTA
-        auto kern = warps == 1 ? select_rows_kernel<16, 3> : select_rows_kernel<16, 2>;
-        int per_sm = 0;
-        SGR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 512, 0));
-        per_sm = std::max(1, std::min(per_sm, 4));  // scratch is sized for 64 warps per SM
-        const unsigned blocks = (unsigned)std::min<long>((nq + 15) / 16, (long)sm_count() * per_sm);
-        kern<<<blocks, 512, 0, s>>>(scores, ld, nq, L, lq, p, thre, qn2, label_scores, first, flags, scratch, spw,
-                                    status, row_len, lorder, ext_min, ext_max);
-    } else if (lorder && stage_bytes <= 200 * 1024) {
-        auto kern = warps == 8 ? select_first_kernel<true, 8> : select_first_kernel<true, 16>;
-        const int threads = 32 * (warps == 8 ? 8 : 16);
+    // By size.  Up to one row per SM, a CTA that stages its row is the shorter way (10.7 against 14.5 us for up to
+    // 148 rows of 1,900 scores, 18.9 / 20.9 for 148 of 20,001), and one launch less; with more rows the items are
+    // spread better (us, items / rows: 14.9 / 16.8 for 400 x 1,900, 204 / 249 for 5,000 x 20,000, 453 / 589 for
+    // 12,345 x 20,000, 886 / 1,632 for 8,192 x 40,000).  Rows over 200 KB can not be staged.
+    if (warps < 0) warps = nq <= sm_count() ? 16 : 0;
+    if (warps >= 8 && stage_bytes <= 200 * 1024) {
+        auto kern = select_row_kernel<16>;
         allow_smem(kern, 200 * 1024);
         int per_sm = 0;
-        SGR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, stage_bytes));
+        SGR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 512, stage_bytes));
         per_sm = std::max(1, std::min(per_sm, 2));  // at most 32 warps per SM use scratch
         const unsigned blocks = (unsigned)std::min<long>(nq, (long)sm_count() * per_sm);
-        kern<<<blocks, threads, stage_bytes, s>>>(scores, ld, nq, L, lq, p, thre, qn2, label_scores, first, flags,
-                                                  scratch, spw, status, row_len, lorder, ext_min, ext_max);
+        kern<<<blocks, 512, stage_bytes, s>>>(scores, ld, nq, L, lq, p, thre, qn2, label_scores, first, flags, scratch,
+                                              spw, status, row_len, lorder, ext_min, ext_max);
     } else {
-        const unsigned blocks = scratch ? (unsigned)std::min<long>(nq, sm_count() * 2)
-                                        : (unsigned)std::min<long>(nq, sm_count() * 8);
-        select_first_kernel<false><<<blocks, 256, 0, s>>>(scores, ld, nq, L, lq, p, thre, qn2, label_scores, first,
-                                                          flags, scratch, spw, status, row_len, lorder, nullptr,
-                                                          nullptr);
+        auto kern = select_items_kernel<8, 5>;
+        int per_sm = 0;
+        SGR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 256, 0));
+        per_sm = std::max(1, std::min(per_sm, 8));  // scratch is sized for 64 warps per SM
+        const unsigned blocks = (unsigned)std::min<long>(((long)nq * L + 7) / 8, (long)sm_count() * per_sm);
+        kern<<<blocks, 256, 0, s>>>(scores, ld, nq, L, lq, p, qn2, label_scores, scratch, spw, status, lorder, ext_min,
+                                    ext_max);
+        SGR_LAUNCH_CHECK();
+        count_launch();
+        first_rows_kernel<<<(nq + 7) / 8, 256, 0, s>>>(label_scores, nq, L, thre, first, flags);
     }
     SGR_LAUNCH_CHECK();
     count_launch();

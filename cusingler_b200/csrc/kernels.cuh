@@ -135,12 +135,10 @@ struct LabelQ {
 // grid i * step with step = 1/(len-1), lower_bound of p (src/cusingler.cu:947-978).  Host function.
 LabelQ make_lq(int start, int len, float p);
 
-// row_len: floats of a score row that the labels cover.  With `lorder` (label ids, longest first)
-// and rows of at most 200 KB, each block stages its row in shared memory before selecting.
-// ext_min / ext_max (optional, staged path): per (row, label) extreme order keys from the
-// correlation epilogue, used instead of a min / max pass for lists that cannot hold NaN.  warps: 8 or 16
-// warps per CTA of the staged form (a block per row), 0 the warp-per-row form (with `lorder`), 1 the
-// warp-per-row form with 40 registers per thread (48 warps per SM), -1 chosen by the sizes.
+// row_len: floats of a score row that the labels cover; lorder: label ids, longest first.
+// ext_min / ext_max (optional): per (row, label) extreme order keys from the correlation epilogue, used instead
+// of a min / max pass for lists that cannot hold NaN.  warps: 8 or 16 a CTA per row that stages it in shared
+// memory (rows of at most 200 KB), 0 or 1 a warp per (row, label), -1 chosen by the sizes.
 void launch_select_first(const float* scores, int64_t ld, int nq, int L, const LabelQ* lq, float p,
                          float thre, const int64_t* qn2, float* label_scores, int32_t* first, uint8_t* flags,
                          float* scratch, int64_t scratch_per_warp, int* status, int row_len, const int32_t* lorder,

@@ -43,7 +43,7 @@ __global__ void __launch_bounds__(ROWS_NW * 32, 3) select_noalloc_rows_kernel(co
                                                                              int L, const __grid_constant__ LabelTable lt,
                                                                              float p, float thre, float* label_scores,
                                                                              int32_t* first, uint8_t* flags) {
-    __shared__ int hist[ROWS_NW][256];
+    __shared__ __align__(16) int hist[ROWS_NW][256];
     __shared__ float ls_all[ROWS_NW][256];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     float* ls = ls_all[warp];
@@ -123,7 +123,7 @@ __global__ void __launch_bounds__(256) select_noalloc_kernel(const float* scores
                                                              float thre, float* label_scores, int32_t* first,
                                                              uint8_t* flags, float* scratch, int spw, bool marked) {
     __shared__ float ls[256];
-    __shared__ int hist[8][256];
+    __shared__ __align__(16) int hist[8][256];
     __shared__ int s_mx;
     // Status bits of the selection are not reported by this entry point: it only enqueues work and
     // has no context to return them through.  Bit 8 (no sort scratch) cannot arise, the scratch is

@@ -147,9 +147,9 @@ sgr_status sgr_set_profiling(sgr_ctx* ctx, int on);
  * 1 runs the exact correlation on SM pairs (clusters of two CTAs, tcgen05 cta_group::2, 256-row
  * tiles), 0 one CTA per 128-row tile; what 6: row bands per group of the correlation's tile order
  * (1 to 4096, default 16; the bands of a group sweep the reference together so that the CTAs at work share
- * operand tiles in L2); what 7: the score-step selection's form: 8 or 16 warps per CTA that stages
- * a query row in shared memory, 0 for one warp per query row reading the scores directly, 1 the
- * same with 40 registers per thread (half again the warps per SM); until it is set, chosen by the sizes;
+ * operand tiles in L2); what 7: the score-step selection's form: 8 or 16 for a CTA of 16 warps that
+ * stages a query row in shared memory (rows of at most 200 KB), 0 or 1 for one warp per query row and
+ * label reading the scores directly; until it is set, chosen by the number of rows;
  * what 8: 1 trains the markers on the host instead of the device; what 9 (exact mode): 1 fine-tunes
  * each score block on a second stream while the next block is scored; what 10: the exact
  * correlation's tile: 8 or 16 for 128 x 256 tiles with two accumulators (when the trained marker

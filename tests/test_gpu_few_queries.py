@@ -1,8 +1,9 @@
 """Scores of a few queries (the CUDA-core correlation, up to 8 rows) and of one row more (the tensor cores)
-equal the oracle's exact scores bit for bit, for either limb split."""
+equal the oracle's exact scores bit for bit, for either limb split; the selection by number of rows."""
 
 import numpy as np
 import pytest
+import torch
 
 from cusingler_b200 import abi
 from tests import helpers as H
@@ -26,3 +27,22 @@ def test_few_queries(kind, base128):
             assert H.ulp_diff(scores, res["scores"][at:at + n]).max() == 0
             assert np.array_equal(first, res["first"][at:at + n])
             assert np.array_equal(flags, res["flags"][at:at + n].astype(np.uint8))
+
+
+@pytest.mark.parametrize("rows", ["one", "sms", "sms + 1", "all"])
+def test_selection_by_size(rows):
+    """A row per SM is selected by row CTAs, more rows by warps per row and label: the same label scores, first
+    labels and flags as the oracle's, chosen by size or set."""
+    prob = H.problem("small")
+    res = H.oracle_run("small", 1)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    n = min({"one": 1, "sms": sms, "sms + 1": sms + 1, "all": prob.qry.n_rows}[rows], prob.qry.n_rows)
+    a = abi.Annotator(gpuid=0)
+    a.train(prob.ref, prob.celltypes, prob.label_names, prob.ref_genes, prob.qry_genes)
+    for form in (None, 0, 16):
+        if form is not None:
+            a.set_tuning(7, form)
+        first, scores, flags = a.score_first(prob.qry.rows(0, n))
+        assert H.ulp_diff(scores, res["scores"][:n]).max() == 0
+        assert np.array_equal(first, res["first"][:n])
+        assert np.array_equal(flags, res["flags"][:n].astype(np.uint8))
