@@ -1158,9 +1158,11 @@ __device__ __forceinline__ float tree128(const float (&c)[4], int lane) {
 // (an entry's z is the kept entries before its run's end plus those before its start), so no row is sorted
 // or bucketed again.  They are scattered into a dense row in shared memory laid out [gene in chunk][chunk],
 // so that a lane reads its four chunks' next genes with one conflict-free 16-byte load.
-// Bound: issue (the row's passes over its entries and chunks).  1,000 queries x 20,000 reference cells,
-// 1,215 cell rounds of 13 candidates: 1,014 ms with the host's lists of (candidate set, row) rankings, 19 ms
-// for the 13.4e6 rows here (1.4 ns a row).
+// Bound: the shared-memory pipe (73 % of its wavefronts in the first round: dense rows, scatters, shuffles), with
+// 68 % of the issue slots.  1,000 queries x 20,000 reference cells, 1,215 cell rounds of 13 candidates, 13.4e6
+// rows: 1,014 ms with the host's lists of (candidate set, row) rankings; 21.8 ms with rows dealt to the warps one
+// by one, each after the loads of its place, genes and runs in turn; 18.5 ms (1.4 ns a row) with consecutive
+// rows, 32 places and a row's genes and runs read at once.
 // dense_len: floats of a dense row (128 x the longest chunk).  dynamic shared memory: the query's dense
 // row, one per warp, the slot of each pool gene (halfwords).
 __global__ void __launch_bounds__(256) ft_scan32_kernel(FtRounds a, int k, int dense_len, int parts) {
@@ -1243,20 +1245,64 @@ __global__ void __launch_bounds__(256) ft_scan32_kernel(FtRounds a, int k, int d
             qn[3] = fmaf(v.w, v.w, qn[3]);
         }
         const float qf = tree128(qn, lane);
-        for (int r = r0 + warp; r < r1; r += nwarp) {
-            int lo = 0, hi = ntop - 1;  // off[lo] <= r < off[lo + 1]
-            while (lo < hi) {
-                const int mid = (lo + hi + 1) >> 1;
-                if (off[mid] <= r) lo = mid;
-                else hi = mid - 1;
+        // a warp takes consecutive rows: the place of 32 of them is read at once, one per lane, and a label's
+        // extremes are written once
+        const int each = (r1 - r0 + nwarp - 1) / nwarp, w0 = r0 + warp * each, w1 = min(r1, w0 + each);
+        int lab = 0, lab_end = 0, my_beg = 0, my_len = 0;
+        size_t out = 0;
+        uint32_t kmin = 0xffffffffu, kmax = 0u;
+        auto flush = [&](int l) {
+            if (lane == 0) {
+                atomicMin(a.ext_min + (size_t)c * a.L + l, kmin);
+                atomicMax(a.ext_max + (size_t)c * a.L + l, kmax);
             }
-            const uint32_t start = a.ctidx[2 * top[lo]];
-            const int j = r - off[lo];
-            const uint32_t row = start + a.perm[start + j];
-            const int beg = a.ref_ptr[row], len = a.ref_ptr[row + 1] - beg, nwd = (len + 31) / 32;
-            // the row's entries inside S as bits: lane w holds entries 32 w ..
-            uint32_t in = 0;
-            for (int w = 0; w < nwd; ++w) {
+            kmin = 0xffffffffu;
+            kmax = 0u;
+        };
+        for (int r = w0; r < w1; ++r) {
+            if (((r - w0) & 31) == 0) {
+                const int ri = min(r + lane, w1 - 1);
+                int lo = 0, hi = ntop - 1;  // off[lo] <= ri < off[lo + 1]
+                while (lo < hi) {
+                    const int mid = (lo + hi + 1) >> 1;
+                    if (off[mid] <= ri) lo = mid;
+                    else hi = mid - 1;
+                }
+                const uint32_t start = a.ctidx[2 * top[lo]];
+                const uint32_t row = start + a.perm[start + ri - off[lo]];
+                my_beg = a.ref_ptr[row];
+                my_len = a.ref_ptr[row + 1] - my_beg;
+                if (r == w0) {
+                    lab = __shfl_sync(FULL, lo, 0);
+                    lab_end = off[lab + 1];
+                    out = (size_t)a.blk_of[(size_t)c * a.L + lab] * 32;
+                }
+            }
+            if (r >= lab_end) {
+                flush(lab);
+                while (off[lab + 1] <= r) ++lab;
+                lab_end = off[lab + 1];
+                out = (size_t)a.blk_of[(size_t)c * a.L + lab] * 32;
+            }
+            const int beg = __shfl_sync(FULL, my_beg, (r - w0) & 31), len = __shfl_sync(FULL, my_len, (r - w0) & 31);
+            const int nwd = (len + 31) / 32;
+            // the row's entries inside S as bits: lane w holds entries 32 w .. ; the first HELD words' slots and
+            // run bounds stay in registers, all their loads in flight together
+            constexpr int HELD = 4;
+            uint32_t in = 0, sl[HELD], lh[HELD];
+#pragma unroll
+            for (int w = 0; w < HELD; ++w) {
+                const int e = 32 * w + lane;
+                sl[w] = e < len ? a.ref_gene[beg + e] : 0xffffffffu;
+                lh[w] = e < len ? a.ref_lo[beg + e] | (uint32_t)a.ref_hi[beg + e] << 16 : 0u;
+            }
+#pragma unroll
+            for (int w = 0; w < HELD; ++w) {
+                sl[w] = sl[w] != 0xffffffffu ? slot[sl[w]] : 0xffffu;
+                const unsigned m = __ballot_sync(FULL, sl[w] != 0xffffu);
+                if (lane == w) in = m;
+            }
+            for (int w = HELD; w < nwd; ++w) {
                 const int e = 32 * w + lane;
                 const bool hit = e < len && slot[a.ref_gene[beg + e]] != 0xffffu;
                 const unsigned m = __ballot_sync(FULL, hit);
@@ -1272,16 +1318,21 @@ __global__ void __launch_bounds__(256) ft_scan32_kernel(FtRounds a, int k, int d
                                                 i + 2 * step < nS ? d0 : 0.f, i + 3 * step < nS ? d0 : 0.f);
             }
             __syncwarp();
-            for (int w = 0; w < nwd; ++w) {
-                const int e = 32 * w + lane;
-                const uint32_t bits = __shfl_sync(FULL, in, w);
-                const bool hit = (bits >> lane) & 1u;
-                const int l0 = hit ? a.ref_lo[beg + e] : 0, h0 = hit ? a.ref_hi[beg + e] : 0;
+            auto place = [&](uint32_t at, int l0, int h0) {
                 const int z = __shfl_sync(FULL, before, l0 >> 5) +
                               __popc(__shfl_sync(FULL, in, l0 >> 5) & ((1u << (l0 & 31)) - 1u)) +
                               __shfl_sync(FULL, before, h0 >> 5) +
                               __popc(__shfl_sync(FULL, in, h0 >> 5) & ((1u << (h0 & 31)) - 1u));
-                if (hit) y[slot[a.ref_gene[beg + e]]] = (float)(nS - 2 * kr + z) * 0.5f;
+                if (at != 0xffffu) y[at] = (float)(nS - 2 * kr + z) * 0.5f;
+            };
+#pragma unroll
+            for (int w = 0; w < HELD; ++w)
+                if (w < nwd) place(sl[w], (int)(lh[w] & 0xffffu), (int)(lh[w] >> 16));
+            for (int w = HELD; w < nwd; ++w) {
+                const int e = 32 * w + lane;
+                const bool hit = e < len;
+                place(hit ? slot[a.ref_gene[beg + e]] : 0xffffu, hit ? a.ref_lo[beg + e] : 0,
+                      hit ? a.ref_hi[beg + e] : 0);
             }
             __syncwarp();
             float d[4] = {0.f, 0.f, 0.f, 0.f}, rn[4] = {0.f, 0.f, 0.f, 0.f};
@@ -1297,17 +1348,15 @@ __global__ void __launch_bounds__(256) ft_scan32_kernel(FtRounds a, int k, int d
                 rn[3] = fmaf(v.w, v.w, rn[3]);
             }
             const float s = tree128(d, lane), rf = tree128(rn, lane);
-            if (lane == 0) {
-                const float div = sqrtf(qf * rf);
-                const float v = div != 0.f ? s / div : __int_as_float(0x7fffffff);
-                const size_t cp = (size_t)c * a.L + lo;
-                a.scores[(size_t)a.blk_of[cp] * 32 + j] = v;
-                const uint32_t key = ord_key(v);
-                atomicMin(a.ext_min + cp, key);
-                atomicMax(a.ext_max + cp, key);
-            }
+            const float div = sqrtf(qf * rf);
+            const float v = div != 0.f ? s / div : __int_as_float(0x7fffffff);  // lane 0's counts
+            if (lane == 0) a.scores[out + (r - off[lab])] = v;
+            const uint32_t key = ord_key(v);
+            kmin = min(kmin, key);
+            kmax = max(kmax, key);
             __syncwarp();
         }
+        if (w0 < w1) flush(lab);
     }
 }
 
