@@ -252,13 +252,19 @@ __device__ bool bucket_select(const float* v, int n, int j, int* hist, int lane,
         float x[4];
 #pragma unroll
         for (int t = 0; t < 4; ++t) x[t] = v[base + 32 * t + lane];
+        bool in[4];
+        unsigned m[4];
 #pragma unroll
         for (int t = 0; t < 4; ++t) {
-            const bool in = (unsigned)bin_bits(x[t]) - lo <= width;
-            const unsigned m = __ballot_sync(FULL, in);
-            if (in) buf[w + __popc(m & lt)] = __float_as_uint(x[t]);
-            w += __popc(m);
+            in[t] = (unsigned)bin_bits(x[t]) - lo <= width;
+            m[t] = __ballot_sync(FULL, in[t]);
         }
+        const int w1 = w + __popc(m[0]), w2 = w1 + __popc(m[1]), w3 = w2 + __popc(m[2]);
+        if (in[0]) buf[w + __popc(m[0] & lt)] = __float_as_uint(x[0]);
+        if (in[1]) buf[w1 + __popc(m[1] & lt)] = __float_as_uint(x[1]);
+        if (in[2]) buf[w2 + __popc(m[2] & lt)] = __float_as_uint(x[2]);
+        if (in[3]) buf[w3 + __popc(m[3] & lt)] = __float_as_uint(x[3]);
+        w = w3 + __popc(m[3]);
     }
     for (; base < n; base += 32) {
         const int i0 = base + lane;

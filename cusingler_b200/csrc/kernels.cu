@@ -671,7 +671,7 @@ __global__ void __launch_bounds__(NW * 32) select_row_kernel(const float* scores
 // pass hits L1 / L2).  Items run label by label, longest label first, rows inside: the warps of a turn have
 // lists of the same length, no barrier waits for a row's longest label, and the last turn is one of the
 // shortest lists.  (Whole rows per warp left the last turn of rows nearly empty: 562 us at 12,345 x 20,000
-// scores and 1,288 us at 8,192 x 40,000, against 453 and 886 here; the bound, one read of the scores, is 151 and
+// scores and 1,288 us at 8,192 x 40,000, against 455 and 888 here; the bound, one read of the scores, is 151 and
 // 200 us.)  It is bound by instruction issue and load latency together: 48 registers, 40 warps per SM and two
 // passes of four loads in flight are faster than 64 registers and 32 warps (480) or 40 and 48 (500 us, spills);
 // an L2 prefetch of the warp's next list does not help (462).  first_rows_kernel then takes each row's maximum
@@ -1096,10 +1096,10 @@ void launch_select_first(const float* scores, int64_t ld, int nq, int L, const L
                          const uint32_t* ext_min, const uint32_t* ext_max, int warps) {
     if (nq <= 0) return;
     const size_t stage_bytes = (((size_t)std::max(row_len, 1) * 4 + 15) & ~size_t(15));
-    // By size.  Up to one row per SM, a CTA that stages its row is the shorter way (10.7 against 14.5 us for up to
-    // 148 rows of 1,900 scores, 18.9 / 20.9 for 148 of 20,001), and one launch less; with more rows the items are
-    // spread better (us, items / rows: 14.9 / 16.8 for 400 x 1,900, 204 / 249 for 5,000 x 20,000, 453 / 589 for
-    // 12,345 x 20,000, 886 / 1,632 for 8,192 x 40,000).  Rows over 200 KB can not be staged.
+    // By size.  Up to one row per SM, a CTA that stages its row is the shorter way (10.6 against 14.0 us for up to
+    // 148 rows of 1,900 scores, 18.8 / 21.6 for 148 of 20,001), and one launch less; with more rows the items are
+    // spread better (us, items / rows: 15.4 / 15.9 for 400 x 1,900, 198 / 251 for 5,000 x 20,000, 455 / 603 for
+    // 12,345 x 20,000, 888 / 1,633 for 8,192 x 40,000).  Rows over 200 KB can not be staged.
     if (warps < 0) warps = nq <= sm_count() ? 16 : 0;
     if (warps >= 8 && stage_bytes <= 200 * 1024) {
         auto kern = select_row_kernel<16>;

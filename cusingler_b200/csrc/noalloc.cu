@@ -31,93 +31,92 @@ static __device__ __align__(256) float g_noalloc_scratch[kNoallocScratchFloats];
 
 struct LabelTable {
     LabelQ q[256];
+    uint8_t order[256];  // longest label first
 };
 
-constexpr int ROWS_NW = 16;  // warps of a CTA of the warp-per-row kernel
+constexpr int ITEMS_NW = 8;                   // warps of a CTA of the item kernel
+constexpr uint32_t kSortMark = 0x7fa5a5a5u;  // a NaN that no arithmetic gives: a list to be sorted
 
-// One warp per score row: every list without NaN (the fixed scratch is not used, so the grid is sized to
-// the GPU: three CTAs per SM, 48 warps).  A row with a list that the reference would sort with NaN in it is
-// left to select_noalloc_kernel, marked by first = -1.  8,000 rows x 20,000 scores in 30 labels: 1.56 ms
-// with the scratch-bound grid of select_noalloc_kernel alone (65 CTAs of 8 warps), 0.42 ms so.
-__global__ void __launch_bounds__(ROWS_NW * 32, 3) select_noalloc_rows_kernel(const float* scores, int64_t ld, int nq,
-                                                                             int L, const __grid_constant__ LabelTable lt,
-                                                                             float p, float thre, float* label_scores,
-                                                                             int32_t* first, uint8_t* flags) {
-    __shared__ __align__(16) int hist[ROWS_NW][256];
-    __shared__ float ls_all[ROWS_NW][256];
+// One warp per (label, score row), label by label, longest first (as the score step's select_items_kernel, with
+// the extremes in a pass of their own): every list without NaN.  The fixed scratch is not used, so the grid is
+// sized to the GPU.  A list that the reference would sort with NaN in it is marked.  8,000 rows x 20,000 scores in
+// 30 labels: 1.56 ms with the scratch-bound grid of select_noalloc_kernel alone (65 CTAs of 8 warps), 0.50 with a
+// warp per row, 0.46 so (uneven labels); 300 rows: 160 us with the CTAs, 40 so.
+__global__ void __launch_bounds__(ITEMS_NW * 32, 5) select_noalloc_items_kernel(const float* scores, int64_t ld, int nq,
+                                                                               int L,
+                                                                               const __grid_constant__ LabelTable lt,
+                                                                               float p, float* label_scores) {
+    __shared__ __align__(16) int hist[ITEMS_NW][256];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    float* ls = ls_all[warp];
-    // a label's list widened to 16-byte bounds stays inside its row when rows start on 16 bytes
-    const bool pf = (ld % 4) == 0 && (reinterpret_cast<uintptr_t>(scores) & 15) == 0;
-    for (int q = blockIdx.x * ROWS_NW + warp; q < nq; q += gridDim.x * ROWS_NW) {
-        const float* row = scores + (size_t)q * ld;
-        auto prefetch_label = [&](int l) {  // into L2, two labels ahead (as in the score step's selection)
-            if (pf && lane == 0 && l < L) {
-                const LabelQ& d = lt.q[l];
-                const uintptr_t a0 = reinterpret_cast<uintptr_t>(row + d.start) & ~uintptr_t(15);
-                const uintptr_t a1 = (reinterpret_cast<uintptr_t>(row + d.start + d.len) + 15) & ~uintptr_t(15);
-                asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a0), "r"((uint32_t)(a1 - a0))
-                             : "memory");
+    const int gw = blockIdx.x * ITEMS_NW + warp, n_warps = gridDim.x * ITEMS_NW;
+    int i = gw / nq, q = gw % nq;
+    while (i < L) {
+        const int l = lt.order[i];
+        const LabelQ d = lt.q[l];
+        const float* v = scores + (size_t)q * ld + d.start;
+        float r = v[0] == v[0] ? v[0] : __int_as_float(0x7fffffff);
+        if (d.kind != 0) {
+            bool nan = false, num = false;
+            uint32_t kmin = 0xffffffffu, kmax = 0u;
+            int t = lane;
+            for (; t + 96 < d.len; t += 128) {  // four independent loads in flight per lane
+                const float x0 = v[t], x1 = v[t + 32], x2 = v[t + 64], x3 = v[t + 96];
+                nan |= (x0 != x0) | (x1 != x1) | (x2 != x2) | (x3 != x3);
+                num |= (x0 == x0) | (x1 == x1) | (x2 == x2) | (x3 == x3);
+                const uint32_t u0 = ord_key(x0), u1 = ord_key(x1), u2 = ord_key(x2), u3 = ord_key(x3);
+                kmin = min(min(kmin, min(u0, u1)), min(u2, u3));
+                kmax = max(max(kmax, max(u0, u1)), max(u2, u3));
             }
-        };
-        prefetch_label(0);
-        prefetch_label(1);
-        bool sort = false;
-        for (int l = 0; l < L && !sort; ++l) {
-            prefetch_label(l + 2);
-            const LabelQ d = lt.q[l];
-            const float* v = row + d.start;
-            float r = v[0] == v[0] ? v[0] : __int_as_float(0x7fffffff);
-            if (d.kind != 0) {
-                bool nan = false, num = false;
-                uint32_t kmin = 0xffffffffu, kmax = 0u;
-                int i = lane;
-                for (; i + 96 < d.len; i += 128) {  // four independent loads in flight per lane
-                    const float x0 = v[i], x1 = v[i + 32], x2 = v[i + 64], x3 = v[i + 96];
-                    nan |= (x0 != x0) | (x1 != x1) | (x2 != x2) | (x3 != x3);
-                    num |= (x0 == x0) | (x1 == x1) | (x2 == x2) | (x3 == x3);
-                    const uint32_t u0 = ord_key(x0), u1 = ord_key(x1), u2 = ord_key(x2), u3 = ord_key(x3);
-                    kmin = min(min(kmin, min(u0, u1)), min(u2, u3));
-                    kmax = max(max(kmax, max(u0, u1)), max(u2, u3));
-                }
-                for (; i < d.len; i += 32) {
-                    const float x = v[i];
-                    nan |= x != x;
-                    num |= x == x;
-                    kmin = min(kmin, ord_key(x));
-                    kmax = max(kmax, ord_key(x));
-                }
-                nan = __any_sync(FULL, nan);
-                num = __any_sync(FULL, num);
-                kmin = __reduce_min_sync(FULL, kmin);
-                kmax = __reduce_max_sync(FULL, kmax);
-                if (nan && !num) r = __int_as_float(0x7fffffff);  // a constant query row: NaN at every grid position
-                else if (nan) sort = true;
-                else r = quantile_warp_core(v, d, p, hist[warp], nullptr, lane, nullptr, kmin, kmax, false);
+            for (; t < d.len; t += 32) {
+                const float x = v[t];
+                nan |= x != x;
+                num |= x == x;
+                kmin = min(kmin, ord_key(x));
+                kmax = max(kmax, ord_key(x));
             }
-            if (lane == 0) ls[l] = r;
+            nan = __any_sync(FULL, nan);
+            num = __any_sync(FULL, num);
+            kmin = __reduce_min_sync(FULL, kmin);
+            kmax = __reduce_max_sync(FULL, kmax);
+            if (nan) r = __uint_as_float(num ? kSortMark : 0x7fffffffu);  // (all NaN: NaN at every grid position)
+            else r = quantile_warp_core(v, d, p, hist[warp], nullptr, lane, nullptr, kmin, kmax, false);
         }
+        if (lane == 0) label_scores[(size_t)q * L + l] = r;
         __syncwarp();
-        if (sort) {
-            if (lane == 0) first[q] = -1;
-            continue;
-        }
-        int mn = 0, mx = 0;
-        if (lane == 0) {
-            stl::minmax(ls, L, &mn, &mx);
-            first[q] = mx;
-        }
-        mx = __shfl_sync(FULL, mx, 0);
-        const float t = __fsub_rn(ls[mx], thre);
-        for (int l = lane; l < L; l += 32) {
-            label_scores[(size_t)q * L + l] = ls[l];
-            if (flags) flags[(size_t)q * L + l] = ls[l] >= t ? 1 : 0;
-        }
-        __syncwarp();
+        for (q += n_warps; q >= nq; q -= nq) ++i;
     }
 }
 
-// A CTA per row, with the fixed scratch.  marked: only the rows that select_noalloc_rows_kernel left.
+// Per row, one warp: first label and flags; a row with a marked list is left to select_noalloc_kernel (first = -1).
+__global__ void __launch_bounds__(256) noalloc_first_kernel(const float* label_scores, int nq, int L, float thre,
+                                                            int32_t* first, uint8_t* flags) {
+    __shared__ float ls_all[8][256];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int q = blockIdx.x * 8 + warp;
+    if (q >= nq) return;
+    float* ls = ls_all[warp];
+    bool sort = false;
+    for (int l = lane; l < L; l += 32) {
+        ls[l] = label_scores[(size_t)q * L + l];
+        sort |= __float_as_uint(ls[l]) == kSortMark;
+    }
+    if (__any_sync(FULL, sort)) {
+        if (lane == 0) first[q] = -1;
+        return;
+    }
+    __syncwarp();
+    int mn = 0, mx = 0;
+    if (lane == 0) {
+        stl::minmax(ls, L, &mn, &mx);
+        first[q] = mx;
+    }
+    mx = __shfl_sync(FULL, mx, 0);
+    if (!flags) return;
+    const float t = __fsub_rn(ls[mx], thre);
+    for (int l = lane; l < L; l += 32) flags[(size_t)q * L + l] = ls[l] >= t ? 1 : 0;
+}
+
+// A CTA per row, with the fixed scratch.  marked: only the rows that noalloc_first_kernel left.
 __global__ void __launch_bounds__(256) select_noalloc_kernel(const float* scores, int64_t ld, int nq, int L,
                                                              const __grid_constant__ LabelTable lt, float p,
                                                              float thre, float* label_scores, int32_t* first,
@@ -200,11 +199,13 @@ extern "C" sgr_status sgr_select_labels_noalloc(const float* d_scores, int64_t l
     if (n_labels == 0 || n_labels > 256) return SGR_ERR_UNSUPPORTED;
     LabelTable lt{};
     uint32_t max_len = 1;
+    uint64_t total = 0;
     for (uint32_t l = 0; l < n_labels; ++l) {
         const uint32_t start = label_ranges[2 * l], len = label_ranges[2 * l + 1];
         if (len == 0) return SGR_ERR_EMPTY_LABEL;
         if ((uint64_t)start + len > (uint64_t)ld) return SGR_ERR_INVALID_ARGUMENT;
         max_len = std::max(max_len, len);
+        total += len;
         // the reference's float index grid (src/cusingler.cu:947-978 of STOmics/cusingler)
         lt.q[l] = make_lq((int)start, (int)len, quantile);
     }
@@ -218,21 +219,30 @@ extern "C" sgr_status sgr_select_labels_noalloc(const float* d_scores, int64_t l
         float* scratch = scratch_address(dev);
         const unsigned blocks =
             (unsigned)std::min<long>({(long)n_rows, fit_blocks, (long)device_sm_count() * 2});
-        // A CTA takes its row's labels eight at a time; a warp takes a row's labels one by one, but the grid
-        // runs 48 warps per SM.  So rows go to warps from the eighth turn of the CTAs on.
-        const bool by_warp = (long)n_rows > 8L * blocks;
-        if (by_warp) {
-            const unsigned row_blocks =
-                (unsigned)std::min<long>(((long)n_rows + ROWS_NW - 1) / ROWS_NW, (long)device_sm_count() * 3);
-            select_noalloc_rows_kernel<<<row_blocks, ROWS_NW * 32, 0, (cudaStream_t)stream>>>(
-                d_scores, ld, (int)n_rows, (int)n_labels, lt, quantile, finetune_thre, d_label_scores, d_first_labels,
-                d_flags);
+        // A CTA takes its row's labels eight at a time, and the scratch allows `blocks` of them.  More rows than
+        // that are spread better as items on all SMs, unless they are so short that the CTAs' few turns cost less
+        // than the two launches more (us, CTAs / items: 12.4 / 16.6 for 300 x 1,000 scores in 5 labels, 28.5 / 16.6
+        // for 1,000 x 1,000; 22.7 / 18.6 for 300 x 3,000 in 20; 97.9 / 30.5 for 100 x 20,000 in 30, 24.9 / 28.9 for 30
+        // of them, which fit one turn).
+        const bool by_item = n_rows > blocks && (n_rows * (double)total > 5e5 || n_rows > 8L * blocks);
+        if (by_item) {
+            for (uint32_t l = 0; l < n_labels; ++l) lt.order[l] = (uint8_t)l;
+            std::sort(lt.order, lt.order + n_labels,
+                      [&](uint8_t x, uint8_t y) { return lt.q[x].len != lt.q[y].len ? lt.q[x].len > lt.q[y].len : x < y; });
+            const unsigned item_blocks = (unsigned)std::min<long>(
+                ((long)n_rows * n_labels + ITEMS_NW - 1) / ITEMS_NW, (long)device_sm_count() * 5);
+            select_noalloc_items_kernel<<<item_blocks, ITEMS_NW * 32, 0, (cudaStream_t)stream>>>(
+                d_scores, ld, (int)n_rows, (int)n_labels, lt, quantile, d_label_scores);
+            SGR_CUDA(cudaGetLastError());
+            count_launch();
+            noalloc_first_kernel<<<(n_rows + 7) / 8, 256, 0, (cudaStream_t)stream>>>(
+                d_label_scores, (int)n_rows, (int)n_labels, finetune_thre, d_first_labels, d_flags);
             SGR_CUDA(cudaGetLastError());
             count_launch();
         }
         select_noalloc_kernel<<<blocks, 256, 0, (cudaStream_t)stream>>>(
             d_scores, ld, (int)n_rows, (int)n_labels, lt, quantile, finetune_thre, d_label_scores, d_first_labels,
-            d_flags, scratch, (int)max_len, by_warp);
+            d_flags, scratch, (int)max_len, by_item);
         SGR_CUDA(cudaGetLastError());
         count_launch();
     } catch (const Error& e) {

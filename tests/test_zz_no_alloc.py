@@ -116,3 +116,36 @@ def test_noalloc_many_rows_with_nan_lists(n_rows, L, pad):
         assert first[q] == top
         with np.errstate(invalid="ignore"):
             assert np.array_equal(flags[q], (want >= np.float32(want[top] - np.float32(0.05))).astype(np.uint8)), q
+
+
+@pytest.mark.parametrize("n_rows,L,longest", [(296, 9, 800), (297, 9, 800), (40, 3, 30000), (300, 256, 40)])
+def test_noalloc_rows_around_the_turn_of_the_ctas(n_rows, L, longest):
+    """As many rows as CTAs fit, and more of them (a warp per label and row): lists with and without NaN, ties and
+    a row that is all NaN, against the oracle's percentile."""
+    import torch
+
+    rng = np.random.default_rng(n_rows + L)
+    lens = rng.integers(1, longest, L)
+    lens[L // 2] = longest
+    starts = np.concatenate([[0], np.cumsum(lens)[:-1]])
+    ld = int(lens.sum())
+    raw = rng.normal(0.4, 0.1, (n_rows, ld)).astype(np.float32)
+    raw[3] = np.nan
+    raw[5, starts[L // 2] + longest // 2] = np.nan
+    raw[7, starts[L // 2]:starts[L // 2] + longest // 2] = raw[7, starts[L // 2]]
+    ranges = np.stack([starts, lens], 1).astype(np.uint32).reshape(-1)
+    dev = torch.device("cuda", 0)
+    d = torch.from_numpy(raw).to(dev)
+    ls = torch.empty((n_rows, L), device=dev)
+    first = torch.empty(n_rows, dtype=torch.int32, device=dev)
+    flags = torch.empty((n_rows, L), dtype=torch.uint8, device=dev)
+    assert abi.select_labels_noalloc(d.data_ptr(), ld, n_rows, ranges, 0.8, 0.05, ls.data_ptr(), first.data_ptr(),
+                                     flags.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
+    ls, first, flags = ls.cpu().numpy(), first.cpu().numpy(), flags.cpu().numpy()
+    for q in (0, 3, 5, 7, n_rows // 2, n_rows - 1):
+        want = np.array([O.percentile(raw[q, s:s + n], 0.8) for s, n in zip(starts, lens)], np.float32)
+        assert H.ulp_diff(ls[q], want).max() == 0, q
+        top = O.minmax(want)[1]
+        assert first[q] == top
+        with np.errstate(invalid="ignore"):
+            assert np.array_equal(flags[q], (want >= np.float32(want[top] - np.float32(0.05))).astype(np.uint8)), q
