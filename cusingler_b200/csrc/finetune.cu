@@ -1,5 +1,10 @@
 // Persistent fine-tune kernel (exact arithmetic) and the reference pre-sort it reads.
 //
+// The fine-tune runs by rounds over all cells (ft_rounds.cu) wherever its packed 32-bit words can hold the
+// trained reference.  The kernels here remain for what it cannot take: gene pools too wide for one table of
+// e-values in shared memory (above about 14,000 genes), rows too long for the packed words, and the two-register
+// scan asked for by sgr_set_tuning (what 3, 0).
+//
 // Restates the reference's per-cell fine-tune loop (src/cusingler.cu:1138-1333 of
 // STOmics/cusingler: finetune_round + cufinetune) as one persistent kernel.  Each CTA takes the
 // next query cell from a device work queue and runs all of that cell's rounds on the device:

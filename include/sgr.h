@@ -128,22 +128,24 @@ typedef struct sgr_timings {
     uint64_t select_launches;
     uint64_t select_bytes;  /* algorithmic bytes 4*Q*R read by the score-step selection          */
     uint64_t ft_queue_cells;/* fine-tune cells run whole by one CTA of the work-queue kernel      */
-    uint64_t ft_split_cells;/* fine-tune cells whose rounds were spread over the GPU             */
-    uint64_t ft_split_rounds;/* rounds of the spread path (each: prepare, scan, decide launches)  */
-    uint64_t ft_split_rows; /* reference rows scored by the spread path, summed over its rounds   */
+    uint64_t ft_split_cells;/* fine-tune cells whose rounds were batched over the GPU            */
+    uint64_t ft_split_rounds;/* batched rounds (each a few launches over all cells in work)       */
+    uint64_t ft_split_rows; /* reference rows scored by the batched rounds, summed                */
     uint64_t ft_cells;      /* cells that ran at least one fine-tune round                      */
     uint64_t ft_candidates; /* first-round candidate labels of those cells, summed               */
 } sgr_timings;
 
 sgr_status sgr_set_profiling(sgr_ctx* ctx, int on);
 
-/* Launch-shape choices.  what 0: warps per CTA of the persistent fine-tune kernel (8 or 32);
- * what 1: candidate count from which a cell's fine-tune rounds are spread over the whole GPU
- * instead of one CTA (>= 2; large values disable the split path); what 2: MiB of score-step
+/* Launch-shape choices.  The fine-tune runs by rounds over all cells where the trained reference allows
+ * it; what 0 and 1 then have no effect.  Otherwise what 0: warps per CTA of the persistent fine-tune
+ * kernel (8 or 32); what 1: candidate count from which a cell's fine-tune rounds are spread over the whole
+ * GPU instead of one CTA (>= 2; large values disable the split path); what 2: MiB of score-step
  * correlations per block of queries (small blocks are read back from L2 by the selection); what 3:
  * 1 lets the fine-tune row scan keep each value run's count and e-sum in one packed 32-bit word when
  * the trained reference allows it, 2 (default) also keeps the run sums in 32 bits and applies run
- * ends with masks when the row lengths allow it, 0 always uses the two-register scan; what 5:
+ * ends with masks when the row lengths allow it, 0 always uses the two-register scan of the persistent
+ * kernel; what 5:
  * 1 runs the exact correlation on SM pairs (clusters of two CTAs, tcgen05 cta_group::2, 256-row
  * tiles), 0 one CTA per 128-row tile; what 6: row bands per group of the correlation's tile order
  * (1 to 4096, default 16; the bands of a group sweep the reference together so that the CTAs at work share
