@@ -11,7 +11,6 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cmath>
-#include <cstddef>
 #include <map>
 #include <random>
 #include <set>
@@ -88,6 +87,14 @@ struct Profiler {
         for (auto e : pool) cudaEventDestroy(e);
         if (h_rounds) cudaFreeHost(h_rounds);
     }
+};
+
+// Counters of the fine-tune by rounds that the host reads back.
+struct FtRead {
+    unsigned long long counter, cand;  // cells to fine-tune << 36 | their score blocks; their candidates
+    int32_t longest, pad;              // longest of their compacted rows (this batch's)
+    int32_t n_act[2];                  // cells that go on (by the parity of the round)
+    unsigned long long stats[2];       // cell rounds, reference rows scored
 };
 
 }  // namespace
@@ -209,7 +216,7 @@ struct sgr_ctx {
     DevBuf<uint16_t> fr_ref_runs;  // FP32 order: the reference's entries by value, with their runs
     size_t fr_ref_runs_stride = 0;
     bool fr_ref_runs_ready = false;
-    unsigned long long* h_ft = nullptr;  // pinned: counters read back
+    FtRead* h_ft = nullptr;        // pinned, two: counters read back, by the parity of the round
     cudaEvent_t ev_ft[2] = {nullptr, nullptr};
 
     // learned proposal
@@ -1285,12 +1292,9 @@ cudaStream_t side_stream(sgr_ctx* ctx) {
     return ctx->side;
 }
 
-// Counters of the fine-tune by rounds on the device.
+// Counters of the fine-tune by rounds on the device, the part that the host reads first.
 struct FtCtl {
-    unsigned long long counter, cand;  // cells to fine-tune << 36 | their score blocks; their candidates
-    int32_t longest, pad;              // longest of their compacted rows (this batch's)
-    int32_t n_act[2];                  // cells that go on (by the parity of the round)
-    unsigned long long stats[2];       // cell rounds, reference rows scored
+    FtRead read;
     int32_t queue[2];
     int32_t n_list[2 * 256];
 };
@@ -1315,22 +1319,20 @@ void finetune_rounds(sgr_ctx* ctx, const DevCsr& q, const uint8_t* flags_dev, fl
     const uint32_t Q = q.n_rows, L = mk.n_labels, Wt = std::max<uint32_t>(ctx->Wt, 1);
     const bool fp32 = ctx->mode == SGR_MODE_FP32REF;
     if (!ctx->h_ft) {
-        SGR_CUDA(cudaMallocHost(reinterpret_cast<void**>(&ctx->h_ft), 2 * offsetof(FtCtl, queue)));
+        SGR_CUDA(cudaMallocHost(reinterpret_cast<void**>(&ctx->h_ft), 2 * sizeof(FtRead)));
         for (auto& e : ctx->ev_ft) SGR_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     }
-    constexpr size_t kRead = offsetof(FtCtl, queue);  // the part of the counters that the host reads
     FtCtl* d = reinterpret_cast<FtCtl*>(ctx->fr_ctl.ensure((sizeof(FtCtl) + 7) / 8));
-    auto host_ctl = [&](int i) { return reinterpret_cast<FtCtl*>(reinterpret_cast<char*>(ctx->h_ft) + i * kRead); };
     SGR_CUDA(cudaMemsetAsync(d, 0, sizeof(FtCtl), s));
     ctx->d_final.ensure((size_t)out_row0 + Q);
     ctx->d_rounds.ensure((size_t)out_row0 + Q);
     ctx->fr_cells.ensure(Q);
     ctx->fr_blk_off.ensure(Q);
     launch_ft_cells((int)Q, cell_list, n_list, (int)L, flags_dev, ctx->d_ctidx.p, ctx->fr_cells.p, ctx->fr_blk_off.p,
-                    ctx->d_final.p + out_row0, ctx->d_rounds.p + out_row0, &d->counter, &d->cand, s);
-    SGR_CUDA(cudaMemcpyAsync(ctx->h_ft, d, kRead, cudaMemcpyDeviceToHost, s));
+                    ctx->d_final.p + out_row0, ctx->d_rounds.p + out_row0, &d->read.counter, &d->read.cand, s);
+    SGR_CUDA(cudaMemcpyAsync(ctx->h_ft, &d->read, sizeof(FtRead), cudaMemcpyDeviceToHost, s));
     SGR_CUDA(cudaStreamSynchronize(s));
-    const FtCtl h = *host_ctl(0);
+    const FtRead h = ctx->h_ft[0];
     const int64_t n_cells = (int64_t)(h.counter >> 36), n_blocks = (int64_t)(h.counter & ((1ull << 36) - 1));
     ctx->prof.acc.ft_cells += (uint64_t)n_cells;
     ctx->prof.acc.ft_candidates += h.cand;
@@ -1422,8 +1424,8 @@ void finetune_rounds(sgr_ctx* ctx, const DevCsr& q, const uint8_t* flags_dev, fl
     a.row_len = ints + 4 * nb;
     a.n_list = d->n_list;
     a.queue = d->queue;
-    a.n_act = d->n_act;
-    a.stats = d->stats;
+    a.n_act = d->read.n_act;
+    a.stats = d->read.stats;
     a.scores = ctx->fr_scores.ensure((size_t)nblk * 32);
     const int grid = ft_step_grid((int)nb);
     a.nan_scratch = ctx->fr_nan.ensure((size_t)grid * max_label);
@@ -1447,24 +1449,24 @@ void finetune_rounds(sgr_ctx* ctx, const DevCsr& q, const uint8_t* flags_dev, fl
         SGR_CUDA(cudaMemsetAsync(a.used, 0, a.n_cells * sizeof(int), s));
         launch_ft_rows(a.cells, a.n_cells, q.data, q.indices, q.indptr, q.n_cols, ctx->qry_map_thre.p, (int)Wt, row_stride,
                        sorted, sorted + (size_t)nb * row_stride, sorted + 2 * (size_t)nb * row_stride, ints + 4 * nb,
-                       &d->longest, s);
+                       &d->read.longest, s);
         bool x64 = ctx->pack_scan != 2 || !narrow(Wt);
         // each round drops at least one candidate, so L rounds finish every cell
         int most = a.n_cells;  // no more cells than this are active
         for (int r = 0;; ++r) {
             if (r > (int)L + 2) fail(SGR_ERR_STATE, "fine-tune rounds did not converge");
             launch_ft_step(a, r, most, !fp32, scan_scratch, s);
-            SGR_CUDA(cudaMemcpyAsync(host_ctl(r & 1), d, kRead, cudaMemcpyDeviceToHost, s));
+            SGR_CUDA(cudaMemcpyAsync(&ctx->h_ft[r & 1], &d->read, sizeof(FtRead), cudaMemcpyDeviceToHost, s));
             SGR_CUDA(cudaEventRecord(ctx->ev_ft[r & 1], s));
             if (r == 0 && ask_longest) {
                 SGR_CUDA(cudaEventSynchronize(ctx->ev_ft[0]));
-                x64 = !narrow(host_ctl(0)->longest);
+                x64 = !narrow(ctx->h_ft[0].longest);
             }
             if (fp32) launch_ft_scan32(a, r, most, s);
             else launch_ft_scan(a, r, most, ctx->ft_copies, x64, s);
             if (r == 0) continue;
             SGR_CUDA(cudaEventSynchronize(ctx->ev_ft[(r - 1) & 1]));
-            const FtCtl* c = host_ctl((r - 1) & 1);
+            const FtRead* c = &ctx->h_ft[(r - 1) & 1];
             most = c->n_act[r & 1];  // cells that go on after step r - 1
             if (most != 0) continue;
             ctx->prof.acc.ft_cell_rounds += c->stats[0];
@@ -2121,7 +2123,7 @@ sgr_status sgr_destroy(sgr_ctx* ctx) {
     cudaStream_t s = ctx->own_stream, side = ctx->side;
     cudaEvent_t e1 = ctx->ev_fork, e2 = ctx->ev_join, e3 = ctx->ev_state[0], e4 = ctx->ev_state[1];
     int32_t* hs = ctx->h_state;
-    unsigned long long* hft = ctx->h_ft;
+    FtRead* hft = ctx->h_ft;
     cudaStream_t cp = ctx->copy;
     if (cp) cudaStreamSynchronize(cp);
     std::vector<cudaEvent_t> up = ctx->up_ev;
