@@ -214,6 +214,7 @@ struct sgr_ctx {
     DevBuf<unsigned long long> fr_ctl;  // counters (FtCtl)
     DevBuf<float> fr_scores, fr_nan;
     DevBuf<uint16_t> fr_ref_runs;  // FP32 order: the reference's entries by value, with their runs
+    DevBuf<int> fr_ref_nan;        // whether some of them are NaN
     size_t fr_ref_runs_stride = 0;
     bool fr_ref_runs_ready = false;
     FtRead* h_ft = nullptr;        // pinned, two: counters read back, by the parity of the round
@@ -1304,8 +1305,9 @@ void ensure_ref_runs(sgr_ctx* ctx) {
     if (ctx->fr_ref_runs_ready) return;
     const size_t n = ctx->fr_ref_runs_stride = std::max<size_t>(ctx->reff_indices.n, 1);
     uint16_t* r = ctx->fr_ref_runs.ensure(3 * n);
+    SGR_CUDA(cudaMemsetAsync(ctx->fr_ref_nan.ensure(1), 0, sizeof(int), ctx->stream));
     launch_ft_sort_rows((int)ctx->R, ctx->reff_data.p, ctx->reff_indices.p, ctx->reff_indptr.p, ctx->max_row, r,
-                        r + n, r + 2 * n, ctx->stream);
+                        r + n, r + 2 * n, ctx->fr_ref_nan.p, ctx->stream);
     ctx->fr_ref_runs_ready = true;
 }
 
@@ -1380,6 +1382,7 @@ void finetune_rounds(sgr_ctx* ctx, const DevCsr& q, const uint8_t* flags_dev, fl
         a.ref_lo = a.ref_gene + n;
         a.ref_hi = a.ref_lo + n;
         a.ref_ptr = ctx->reff_indptr.p;
+        a.ref_nan = ctx->fr_ref_nan.p;
     }
     a.ft_genes = ctx->d_ft_genes.p;
     a.ft_idx = ctx->d_ft_idx.p;
@@ -1449,7 +1452,7 @@ void finetune_rounds(sgr_ctx* ctx, const DevCsr& q, const uint8_t* flags_dev, fl
         SGR_CUDA(cudaMemsetAsync(a.used, 0, a.n_cells * sizeof(int), s));
         launch_ft_rows(a.cells, a.n_cells, q.data, q.indices, q.indptr, q.n_cols, ctx->qry_map_thre.p, (int)Wt, row_stride,
                        sorted, sorted + (size_t)nb * row_stride, sorted + 2 * (size_t)nb * row_stride, ints + 4 * nb,
-                       &d->read.longest, s);
+                       &d->read.longest, fp32, s);
         bool x64 = ctx->pack_scan != 2 || !narrow(Wt);
         // each round drops at least one candidate, so L rounds finish every cell
         int most = a.n_cells;  // no more cells than this are active

@@ -209,10 +209,19 @@ __global__ void __launch_bounds__(256) ft_cells_kernel(int n, const int32_t* lis
     }
 }
 
-// One warp per row: its pool entries by value, with each entry's run as positions [lo, hi).
+// The FP32 order refuses a NaN that it ranks.  Which entries it ranks is known per round only, so the sorted
+// rows carry the mark: bit 15 of the gene (pools are narrower than 2^15).
+constexpr uint32_t NAN_GENE = 0x8000u, GENE = 0x7fffu;
+
+__device__ __forceinline__ bool key_is_nan(uint32_t u) {
+    return u > 0xff800000u || u < 0x007fffffu;  // beyond ord_key of the infinities
+}
+
+// One warp per row: its pool entries by value (NaN marked), with each entry's run as positions [lo, hi).
+// any_nan: set where a row holds a NaN.
 __global__ void __launch_bounds__(256) ft_sort_rows_kernel(int n, const float* data, const int32_t* idx,
                                                            const int32_t* ptr, int cap, uint16_t* s_gene,
-                                                           uint16_t* s_lo, uint16_t* s_hi) {
+                                                           uint16_t* s_lo, uint16_t* s_hi, int* any_nan) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpb = blockDim.x >> 5;
     uint64_t* keys = reinterpret_cast<uint64_t*>(smem) + (size_t)warp * cap;
@@ -227,7 +236,9 @@ __global__ void __launch_bounds__(256) ft_sort_rows_kernel(int n, const float* d
         for (int j = lane; j < k; j += 32) {
             const uint64_t key = keys[j];
             const uint32_t hv = (uint32_t)(key >> 32);
-            s_gene[beg + j] = (uint16_t)(uint32_t)key;
+            const bool nan = key_is_nan(hv);
+            if (nan) *any_nan = 1;
+            s_gene[beg + j] = (uint16_t)((uint32_t)key | (nan ? NAN_GENE : 0u));
             s_lo[beg + j] = (uint16_t)lower_hi(keys, k, hv);
             s_hi[beg + j] = (uint16_t)upper_hi(keys, k, hv);
         }
@@ -242,13 +253,14 @@ __global__ void __launch_bounds__(256) ft_sort_rows_kernel(int n, const float* d
 // Values are counted into 256 buckets of a linear map; an entry's place in its bucket is the smaller values
 // plus the equal ones in earlier slots.  A bucket above 128 entries (few distinct values) is sorted instead.
 // dynamic shared memory: 2 x cap keys (cap: the pool's genes; a row's columns are distinct).
+// mark_nan (FP32 order): NaN entries' genes are marked.
 constexpr int ROWS_NT = 256;
 
 __global__ void __launch_bounds__(ROWS_NT) ft_rows_kernel(const int32_t* cells, int n, const float* data,
                                                          const int32_t* indices, const int32_t* indptr,
                                                          uint32_t n_cols, const int32_t* map, int cap, int row_stride,
                                                          uint16_t* s_gene, uint16_t* s_lo, uint16_t* s_hi,
-                                                         int32_t* row_len, int* longest) {
+                                                         int32_t* row_len, int* longest, bool mark_nan) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int start[257], w_tot[ROWS_NT / 32];
     __shared__ uint32_t s_min, s_max;
@@ -316,6 +328,9 @@ __global__ void __launch_bounds__(ROWS_NT) ft_rows_kernel(const int32_t* cells, 
         __syncthreads();
         int before = incl - mine;
         for (int w = 0; w < warp; ++w) before += w_tot[w];
+        auto marked = [&](uint64_t key) {
+            return (uint16_t)((uint32_t)key | (mark_nan && key_is_nan((uint32_t)(key >> 32)) ? NAN_GENE : 0u));
+        };
         uint16_t* gene = s_gene + (size_t)c * row_stride;
         uint16_t* lo_out = s_lo + (size_t)c * row_stride;
         uint16_t* hi_out = s_hi + (size_t)c * row_stride;
@@ -339,7 +354,7 @@ __global__ void __launch_bounds__(ROWS_NT) ft_rows_kernel(const int32_t* cells, 
                     eq_before += v == u && t < j;
                 }
                 const int lo = s0 + less, at = lo + eq_before;
-                gene[at] = (uint16_t)(uint32_t)key;
+                gene[at] = marked(key);
                 lo_out[at] = (uint16_t)lo;
                 hi_out[at] = (uint16_t)(lo + eq);
             }
@@ -363,7 +378,7 @@ __global__ void __launch_bounds__(ROWS_NT) ft_rows_kernel(const int32_t* cells, 
             for (int j = tid; j < k; j += ROWS_NT) {
                 const uint64_t key = keys[j];
                 const uint32_t u = (uint32_t)(key >> 32);
-                gene[j] = (uint16_t)(uint32_t)key;
+                gene[j] = marked(key);
                 lo_out[j] = (uint16_t)lower_hi(keys, k, u);
                 hi_out[j] = (uint16_t)upper_hi(keys, k, u);
             }
@@ -633,7 +648,7 @@ __global__ void __launch_bounds__(NW * 32, NW == STEP_NW ? 4 : 1) ft_step_kernel
 #pragma unroll 4
         for (int w = warp; w < nwd; w += NW) {
             const int j = 32 * w + lane;
-            const uint32_t g = j < len ? a.s_gene[beg + j] : 0u;
+            const uint32_t g = j < len ? a.s_gene[beg + j] & GENE : 0u;
             const unsigned b = __ballot_sync(FULL, j < len && ((bits[g >> 5] >> (g & 31)) & 1u));
             if (lane == 0) in[w] = b;
         }
@@ -664,7 +679,9 @@ __global__ void __launch_bounds__(NW * 32, NW == STEP_NW ? 4 : 1) ft_step_kernel
         for (int j = tid; j < len; j += NT) {
             if (!((in[j >> 5] >> (j & 31)) & 1u)) continue;
             const int e = nS - kq + kept(a.s_lo[beg + j]) + kept(a.s_hi[beg + j]);
-            eq[a.s_gene[beg + j]] = one + (uint32_t)e;
+            const uint32_t g = a.s_gene[beg + j];
+            if (g & NAN_GENE) atomicOr(a.status, 2);  // a NaN inside the gene set
+            eq[g & GENE] = one + (uint32_t)e;
             sq += (long long)(e - kq) * (e - kq);
         }
         sq = warp_sum_i64(sq);
@@ -1182,6 +1199,7 @@ __global__ void __launch_bounds__(256) ft_scan32_kernel(FtRounds a, int k, int d
     }
     const int n = a.n_act[nxt];
     const uint32_t low = (1u << a.shift) - 1u;
+    const bool nan_rows = *a.ref_nan != 0;
     for (;;) {
         __syncthreads();
         if (tid == 0) s_item = atomicAdd(a.queue + cur, 1);
@@ -1286,6 +1304,14 @@ __global__ void __launch_bounds__(256) ft_scan32_kernel(FtRounds a, int k, int d
             }
             const int beg = __shfl_sync(FULL, my_beg, (r - w0) & 31), len = __shfl_sync(FULL, my_len, (r - w0) & 31);
             const int nwd = (len + 31) / 32;
+            if (nan_rows) {  // somewhere in the reference: a NaN inside the gene set is refused
+                bool bad = false;
+                for (int e = lane; e < len; e += 32) {
+                    const uint32_t g = a.ref_gene[beg + e];
+                    bad |= (g & NAN_GENE) && slot[g & GENE] != 0xffffu;
+                }
+                if (bad) atomicOr(a.status, 2);
+            }
             // the row's entries inside S as bits: lane w holds entries 32 w .. ; the first HELD words' slots and
             // run bounds stay in registers, all their loads in flight together
             constexpr int HELD = 4;
@@ -1298,13 +1324,13 @@ __global__ void __launch_bounds__(256) ft_scan32_kernel(FtRounds a, int k, int d
             }
 #pragma unroll
             for (int w = 0; w < HELD; ++w) {
-                sl[w] = sl[w] != 0xffffffffu ? slot[sl[w]] : 0xffffu;
+                sl[w] = sl[w] != 0xffffffffu ? slot[sl[w] & GENE] : 0xffffu;
                 const unsigned m = __ballot_sync(FULL, sl[w] != 0xffffu);
                 if (lane == w) in = m;
             }
             for (int w = HELD; w < nwd; ++w) {
                 const int e = 32 * w + lane;
-                const bool hit = e < len && slot[a.ref_gene[beg + e]] != 0xffffu;
+                const bool hit = e < len && slot[a.ref_gene[beg + e] & GENE] != 0xffffu;
                 const unsigned m = __ballot_sync(FULL, hit);
                 if (lane == w) in = m;
             }
@@ -1331,7 +1357,7 @@ __global__ void __launch_bounds__(256) ft_scan32_kernel(FtRounds a, int k, int d
             for (int w = HELD; w < nwd; ++w) {
                 const int e = 32 * w + lane;
                 const bool hit = e < len;
-                place(hit ? slot[a.ref_gene[beg + e]] : 0xffffu, hit ? a.ref_lo[beg + e] : 0,
+                place(hit ? slot[a.ref_gene[beg + e] & GENE] : 0xffffu, hit ? a.ref_lo[beg + e] : 0,
                       hit ? a.ref_hi[beg + e] : 0);
             }
             __syncwarp();
@@ -1447,7 +1473,7 @@ void launch_ft_cells(int n, const int32_t* list, const int* n_dev, int L, const 
 }
 
 void launch_ft_sort_rows(int n, const float* data, const int32_t* idx, const int32_t* ptr, int longest,
-                         uint16_t* s_gene, uint16_t* s_lo, uint16_t* s_hi, cudaStream_t s) {
+                         uint16_t* s_gene, uint16_t* s_lo, uint16_t* s_hi, int* any_nan, cudaStream_t s) {
     if (n <= 0) return;
     int cap = 32;
     while (cap < longest) cap <<= 1;
@@ -1455,19 +1481,20 @@ void launch_ft_sort_rows(int n, const float* data, const int32_t* idx, const int
     const size_t smem = (size_t)wpb * cap * 8;
     allow_smem(ft_sort_rows_kernel, 96 * 1024);
     const int blocks = std::min((n + wpb - 1) / wpb, device_sm_count() * 16);
-    ft_sort_rows_kernel<<<blocks, 32 * wpb, smem, s>>>(n, data, idx, ptr, cap, s_gene, s_lo, s_hi);
+    ft_sort_rows_kernel<<<blocks, 32 * wpb, smem, s>>>(n, data, idx, ptr, cap, s_gene, s_lo, s_hi, any_nan);
     SGR_LAUNCH_CHECK();
     count_launch();
 }
 
 void launch_ft_rows(const int32_t* cells, int n, const float* data, const int32_t* indices, const int32_t* indptr,
                     uint32_t n_cols, const int32_t* map, int Wt, int row_stride, uint16_t* s_gene, uint16_t* s_lo,
-                    uint16_t* s_hi, int32_t* row_len, int* longest, cudaStream_t s) {
+                    uint16_t* s_hi, int32_t* row_len, int* longest, bool mark_nan, cudaStream_t s) {
     if (n <= 0) return;
     const size_t smem = (size_t)Wt * 16;
     allow_smem(ft_rows_kernel, kScanSmem);
     ft_rows_kernel<<<std::min(n, device_sm_count() * 16), ROWS_NT, smem, s>>>(
-        cells, n, data, indices, indptr, n_cols, map, Wt, row_stride, s_gene, s_lo, s_hi, row_len, longest);
+        cells, n, data, indices, indptr, n_cols, map, Wt, row_stride, s_gene, s_lo, s_hi, row_len, longest,
+        mark_nan);
     SGR_LAUNCH_CHECK();
     count_launch();
 }

@@ -326,6 +326,7 @@ struct FtRounds {
     const int32_t* lorder;      // labels, longest first
     const uint16_t *ref_gene, *ref_lo, *ref_hi;  // FP32 order: entries by value, with their runs (CSR order)
     const int32_t* ref_ptr;
+    const int* ref_nan;         // FP32 order: not 0 where some reference row holds a NaN (marked in ref_gene)
     const uint32_t* ft_genes;   // fine-tune pair lists (pool ids)
     const uint32_t* ft_idx;     // (start, len) per ordered pair
     const uint32_t* pair_mask;  // bits of each pair's whole list (nwords each), or nullptr
@@ -385,14 +386,15 @@ void launch_pair_masks(const uint32_t* ft_genes, const uint32_t* ft_idx, int L, 
 void launch_ft_cells(int n, const int32_t* list, const int* n_dev, int L, const uint8_t* flags,
                      const uint32_t* ctidx, int32_t* cells, int64_t* blk_off, int32_t* final_labels, int32_t* rounds,
                      unsigned long long* counter, unsigned long long* cand, cudaStream_t s);
-// Rows 0 .. n - 1 of a compacted CSR by value, with their runs (at the CSR's positions).
+// Rows 0 .. n - 1 of a compacted CSR by value, with their runs (at the CSR's positions); bit 15 of the gene marks a
+// NaN, and any_nan is set where there is one.
 void launch_ft_sort_rows(int n, const float* data, const int32_t* idx, const int32_t* ptr, int longest,
-                         uint16_t* s_gene, uint16_t* s_lo, uint16_t* s_hi, cudaStream_t s);
+                         uint16_t* s_gene, uint16_t* s_lo, uint16_t* s_hi, int* any_nan, cudaStream_t s);
 // The cells' query rows compacted to the pool (map) and by value, with their runs, row_stride apart.
-// longest: atomic maximum of the rows' lengths.
+// longest: atomic maximum of the rows' lengths.  mark_nan: as launch_ft_sort_rows marks them.
 void launch_ft_rows(const int32_t* cells, int n, const float* data, const int32_t* indices, const int32_t* indptr,
                     uint32_t n_cols, const int32_t* map, int Wt, int row_stride, uint16_t* s_gene, uint16_t* s_lo,
-                    uint16_t* s_hi, int32_t* row_len, int* longest, cudaStream_t s);
+                    uint16_t* s_hi, int32_t* row_len, int* longest, bool mark_nan, cudaStream_t s);
 int ft_step_grid(int n);
 // Function attributes of the step and scan kernels; call before the launches of a batch.
 void ft_rounds_setup(int copies);
