@@ -1685,7 +1685,7 @@ void finetune_persistent(sgr_ctx* ctx, const DevCsr& q, const uint8_t* flags_dev
                    ctx->sp_state.p, ctx->sp_nS.p, ctx->sp_kq.p, ctx->sp_nq.p, ctx->sp_rq.p, ctx->sp_total.p,
                    ctx->sp_off.p, ctx->sp_eqv.p, ctx->sp_scores.p, ctx->sp_nan.p, (int)ctx->R32, ctx->sp_rows.p,
                    ctx->sp_items.p, ctx->sp_nitems.p, H * max_chunks, max_chunks};
-        split_round_setup(a);
+        split_round_setup();
         launch_split_first(a, sp, H, s);
         // Rounds run kRoundsPerGraph at a time from one CUDA graph (rounds of finished cells do
         // nothing), with one host check of the cells' states per graph launch; a stream that

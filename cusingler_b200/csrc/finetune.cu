@@ -768,13 +768,10 @@ size_t split_decide_smem(int Wt, int capq) {
 size_t split_scan_smem(int Wt) { return sizeof(int) * (((Wt + 4) & ~3) + 260) + 256; }
 }  // namespace
 
-void split_round_setup(const FtPersistentArgs& a) {
-    SGR_CUDA(cudaFuncSetAttribute(split_first_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)split_prepare_smem(a.Wt, a.capq)));
-    SGR_CUDA(cudaFuncSetAttribute(split_scan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)split_scan_smem(a.Wt)));
-    SGR_CUDA(cudaFuncSetAttribute(split_decide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)split_decide_smem(a.Wt, a.capq)));
+void split_round_setup() {
+    allow_most_smem(split_first_kernel);
+    allow_most_smem(split_scan_kernel);
+    allow_most_smem(split_decide_kernel);
 }
 
 void launch_split_first(const FtPersistentArgs& a, const FtSplit& sp, int H, cudaStream_t s) {
@@ -825,7 +822,7 @@ void launch_ref_presort(const float* data, const int32_t* idx, const int32_t* pt
 namespace {
 template <int NW>
 int ft_grid_t(size_t smem) {
-    SGR_CUDA(cudaFuncSetAttribute(ft_persistent_kernel<NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_most_smem(ft_persistent_kernel<NW>);
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ft_persistent_kernel<NW>, NW * 32, smem);
     if (per_sm < 1) per_sm = 1;
@@ -836,13 +833,8 @@ int ft_grid_t(size_t smem) {
 int ft_persistent_grid(size_t smem, int nw) { return nw == 32 ? ft_grid_t<32>(smem) : ft_grid_t<8>(smem); }
 
 void launch_ft_persistent(const FtPersistentArgs& a, int grid, size_t smem, int nw, cudaStream_t s) {
-    if (nw == 32) {
-        SGR_CUDA(cudaFuncSetAttribute(ft_persistent_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        ft_persistent_kernel<32><<<grid, 1024, smem, s>>>(a);
-    } else {
-        SGR_CUDA(cudaFuncSetAttribute(ft_persistent_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        ft_persistent_kernel<8><<<grid, 256, smem, s>>>(a);
-    }
+    if (nw == 32) ft_persistent_kernel<32><<<grid, 1024, smem, s>>>(a);
+    else ft_persistent_kernel<8><<<grid, 256, smem, s>>>(a);
     SGR_LAUNCH_CHECK();
     count_launch();
 }

@@ -273,7 +273,7 @@ struct FtSplit {
 
 // Function attributes of the split-round kernels; call once before launch_split_first (and before
 // capturing rounds into a CUDA graph).
-void split_round_setup(const FtPersistentArgs& a);
+void split_round_setup();
 // First round's setup of the H cells (chunk list 0; n_items must be zero).
 void launch_split_first(const FtPersistentArgs& a, const FtSplit& sp, int H, cudaStream_t s);
 // One round: scan of chunk list q, then the decisions and the next round's setup (list q ^ 1).
@@ -282,7 +282,7 @@ void launch_split_round(const FtPersistentArgs& a, const FtSplit& sp, int H, int
 size_t ft_persistent_smem(int Wt, int capq, int nw);
 void launch_ft_keys(int n, const int32_t* list, int L, const uint8_t* flags, const uint32_t* ctidx, int64_t* keys,
                     int32_t* ncand, cudaStream_t s);
-// nw: warps per CTA (8 or 32)
+// nw: warps per CTA (8 or 32).  Sets the function attributes that launch_ft_persistent needs.
 int ft_persistent_grid(size_t smem, int nw);
 void launch_ft_persistent(const FtPersistentArgs& a, int grid, size_t smem, int nw, cudaStream_t s);
 // Value-sorted, run-flagged fine-tune lists of the reference rows in 32-row blocks: entry j of row r

@@ -44,6 +44,16 @@ inline void allow_smem(K kern, size_t most) {
     SGR_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
 }
 
+// The same for kernels whose launches take what the trained reference needs: all that a CTA can have next to the
+// kernel's own shared arrays.
+template <class K>
+inline void allow_most_smem(K kern) {
+    constexpr size_t kBlock = 227 * 1024;
+    cudaFuncAttributes at;
+    SGR_CUDA(cudaFuncGetAttributes(&at, kern));
+    allow_smem(kern, kBlock - at.sharedSizeBytes);
+}
+
 // Device memory of one context in slabs: buffers up to 16 MiB are carved from 64 MiB slabs instead of a
 // cudaMalloc and a cudaFree each (0.33 ms a call here, about 100 buffers per context: 10 of 22 ms of a whole
 // drop-in run on 1,900 x 800 cells).  A context's arena is used by the thread that is in a call on the

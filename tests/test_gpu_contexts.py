@@ -59,3 +59,38 @@ def test_contexts_in_threads():
     for t in threads:
         t.join()
     assert not wrong
+
+
+@pytest.mark.parametrize("heavy", [2, 1 << 30])
+def test_per_cell_kernels_in_threads(heavy):
+    """The per-cell fine-tune kernels take shared memory by the gene pool's size: contexts of several sizes in
+    several threads do not lower the limit under one another's launches."""
+    wrong = []
+    start = threading.Barrier(4)
+
+    def work(kind):
+        try:
+            a, prob = _trained(kind)
+            a.set_tuning(3, 0)
+            a.set_tuning(1, heavy)
+            res = H.oracle_run(kind, 1)
+            q, flags = prob.qry.rows(0, 8), res["flags"][:8].astype(np.uint8)
+            start.wait()
+            for _ in range(150):
+                final, rounds = a.finetune(q, flags)
+                if not (np.array_equal(final, res["final"][:8]) and np.array_equal(rounds, res["rounds"][:8])):
+                    wrong.append(kind)
+            a.close()
+        except Exception as e:  # noqa: BLE001
+            wrong.append((kind, e))
+            start.abort()
+
+    kinds = ("tiny", "small", "families", "small")
+    for kind in kinds:
+        H.oracle_run(kind, 1)
+    threads = [threading.Thread(target=work, args=(k,)) for k in kinds]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
