@@ -217,6 +217,22 @@ struct sgr_ctx {
     DevBuf<int> fr_ref_nan;        // whether some of them are NaN
     size_t fr_ref_runs_stride = 0;
     bool fr_ref_runs_ready = false;
+    // gives the buffers sized by a batch back
+    void release_round_buffers() {
+        fr_sorted.release();
+        fr_top.release();
+        fr_ints.release();
+        fr_par.release();
+        fr_eq.release();
+        fr_ext.release();
+        fr_list.release();
+        fr_quads.release();
+        fr_q_label.release();
+        fr_un.release();
+        fr_keys.release();
+        fr_scores.release();
+        fr_nan.release();
+    }
     FtRead* h_ft = nullptr;        // pinned, two: counters read back, by the parity of the round
     cudaEvent_t ev_ft[2] = {nullptr, nullptr};
 
@@ -311,10 +327,14 @@ struct PhaseClock {
     }
 };
 
-// After a failed call: nothing queued may read caller memory or a released buffer any more.
-void drain(sgr_ctx* ctx) {
+void finish_streams(sgr_ctx* ctx) {
     for (cudaStream_t s : {ctx->stream, ctx->side, ctx->copy, ctx->ft_s})
         if (s) cudaStreamSynchronize(s);
+}
+
+// After a failed call: nothing queued may read caller memory or a released buffer any more.
+void drain(sgr_ctx* ctx) {
+    finish_streams(ctx);
     cudaGetLastError();
     ctx->prof.spans.clear();
     ctx->prof.used = 0;
@@ -1311,10 +1331,53 @@ void ensure_ref_runs(sgr_ctx* ctx) {
     ctx->fr_ref_runs_ready = true;
 }
 
+// Runs f, which allocates device memory; false where there was not enough.
+template <class F>
+bool fits_memory(F&& f) {
+    try {
+        f();
+        return true;
+    } catch (const Error& e) {
+        if (e.code != SGR_ERR_OUT_OF_MEMORY) throw;
+        return false;
+    }
+}
+
+// The buffers of a batch of nb cells with nblk score blocks, set in `a`; returns the ordering's scan scratch.
+int32_t* round_buffers(sgr_ctx* ctx, FtRounds& a, int64_t nb, int64_t nblk) {
+    const size_t n = (size_t)nb, L = (size_t)a.L, row_words = n * a.row_stride;
+    uint16_t* sorted = ctx->fr_sorted.ensure(3 * row_words);
+    a.s_gene = sorted;
+    a.s_lo = sorted + row_words;
+    a.s_hi = sorted + 2 * row_words;
+    a.top = ctx->fr_top.ensure(n * L);
+    int* ints = ctx->fr_ints.ensure(n * 5);
+    a.ntop = ints;
+    a.used = ints + n;
+    a.act = ints + 2 * n;
+    a.row_len = ints + 4 * n;
+    a.par = ctx->fr_par.ensure(n);
+    a.eq = ctx->fr_eq.ensure(n * a.eq_stride);
+    a.ext_min = ctx->fr_ext.ensure(n * L * 3);
+    a.ext_max = a.ext_min + n * L;
+    a.blk_of = a.ext_max + n * L;
+    a.un = ctx->fr_un.ensure(n);
+    a.key_count = ctx->fr_keys.ensure(((size_t)2 << 20) + 1);
+    const size_t n_quads = std::max<size_t>((n + 3) / 4, std::min<size_t>(n, kFtDirectCells));
+    a.list = ctx->fr_list.ensure(n * L + n_quads * L * 4);
+    a.q_entry = a.list + n * L;
+    a.quads = ctx->fr_quads.ensure(n_quads);
+    a.q_label = ctx->fr_q_label.ensure(n_quads * L);
+    a.scores = ctx->fr_scores.ensure((size_t)nblk * 32);
+    a.nan_scratch = ctx->fr_nan.ensure((size_t)ft_step_grid((int)nb) * a.max_label);
+    return ctx->scan_part.ensure(2 * (((size_t)1 << 20) / 4096) + 1);
+}
+
 // Fine-tune by rounds over all cells (ft_rounds.cu), in the context's arithmetic; arguments as
-// finetune_persistent.  A batch's rounds are queued one ahead of the
-// host: the count of active cells after step k is read while the scan of round k runs.
-void finetune_rounds(sgr_ctx* ctx, const DevCsr& q, const uint8_t* flags_dev, float p, float thre, int times,
+// finetune_persistent.  A batch's rounds are queued one ahead of the host: the count of active cells after
+// step k is read while the scan of round k runs.  False, with nothing done, where device memory does not
+// hold the buffers of even one cell.
+bool finetune_rounds(sgr_ctx* ctx, const DevCsr& q, const uint8_t* flags_dev, float p, float thre, int times,
                      const int32_t* cell_list, const int* n_list, uint32_t out_row0) {
     cudaStream_t s = ctx->stream;
     const Markers& mk = ctx->mk;
@@ -1328,18 +1391,21 @@ void finetune_rounds(sgr_ctx* ctx, const DevCsr& q, const uint8_t* flags_dev, fl
     SGR_CUDA(cudaMemsetAsync(d, 0, sizeof(FtCtl), s));
     ctx->d_final.ensure((size_t)out_row0 + Q);
     ctx->d_rounds.ensure((size_t)out_row0 + Q);
-    ctx->fr_cells.ensure(Q);
-    ctx->fr_blk_off.ensure(Q);
+    if (!fits_memory([&] {
+            ctx->fr_cells.ensure(Q);
+            ctx->fr_blk_off.ensure(Q);
+            if (fp32) ensure_ref_runs(ctx);
+        })) {
+        ctx->release_round_buffers();
+        return false;
+    }
     launch_ft_cells((int)Q, cell_list, n_list, (int)L, flags_dev, ctx->d_ctidx.p, ctx->fr_cells.p, ctx->fr_blk_off.p,
                     ctx->d_final.p + out_row0, ctx->d_rounds.p + out_row0, &d->read.counter, &d->read.cand, s);
     SGR_CUDA(cudaMemcpyAsync(ctx->h_ft, &d->read, sizeof(FtRead), cudaMemcpyDeviceToHost, s));
     SGR_CUDA(cudaStreamSynchronize(s));
     const FtRead h = ctx->h_ft[0];
     const int64_t n_cells = (int64_t)(h.counter >> 36), n_blocks = (int64_t)(h.counter & ((1ull << 36) - 1));
-    ctx->prof.acc.ft_cells += (uint64_t)n_cells;
-    ctx->prof.acc.ft_candidates += h.cand;
-    ctx->prof.acc.ft_split_cells += (uint64_t)n_cells;
-    if (n_cells == 0) return;
+    if (n_cells == 0) return true;
     uint32_t max_label = 1;
     std::vector<LabelQ> lq(L);
     for (uint32_t l = 0; l < L; ++l) {
@@ -1347,27 +1413,6 @@ void finetune_rounds(sgr_ctx* ctx, const DevCsr& q, const uint8_t* flags_dev, fl
         lq[l] = make_lq(0, (int)mk.ctidx[2 * l + 1], p);
     }
     ctx->d_lq_label.upload(lq, s);
-    // batches: score blocks (4 GiB), cells (their e-value rows 1 GiB)
-    const int eq_stride = round_up((int)Wt + 1, 4);
-    const int64_t max_blocks = std::max<int64_t>((int64_t)1 << 25, ctx->R32 / 32);
-    const int64_t max_cells = std::max<int64_t>(1, std::min<int64_t>(131072, ((int64_t)1 << 28) / eq_stride));
-    std::vector<int64_t> cuts{0}, off;
-    if (n_blocks > max_blocks || n_cells > max_cells) {
-        off.resize(n_cells);
-        SGR_CUDA(cudaMemcpyAsync(off.data(), ctx->fr_blk_off.p, n_cells * sizeof(int64_t), cudaMemcpyDeviceToHost, s));
-        SGR_CUDA(cudaStreamSynchronize(s));
-        for (int64_t i = 1; i < n_cells; ++i) {
-            const int64_t end = i + 1 < n_cells ? off[i + 1] : n_blocks;
-            if (end - off[cuts.back()] > max_blocks || i - cuts.back() >= max_cells) cuts.push_back(i);
-        }
-    }
-    cuts.push_back(n_cells);
-    int64_t nb = 0, nblk = 0;
-    for (size_t b = 0; b + 1 < cuts.size(); ++b) {
-        nb = std::max(nb, cuts[b + 1] - cuts[b]);
-        nblk = std::max(nblk, off.empty() ? n_blocks
-                                          : (cuts[b + 1] < n_cells ? off[cuts[b + 1]] : n_blocks) - off[cuts[b]]);
-    }
     FtRounds a{};
     a.groups = ctx->fr_groups.p;
     a.blk_base = ctx->d_blk_base.p;
@@ -1376,7 +1421,6 @@ void finetune_rounds(sgr_ctx* ctx, const DevCsr& q, const uint8_t* flags_dev, fl
     a.ctidx = ctx->d_ctidx.p;
     a.lorder = ctx->d_lorder.p;
     if (fp32) {
-        ensure_ref_runs(ctx);
         const size_t n = ctx->fr_ref_runs_stride;
         a.ref_gene = ctx->fr_ref_runs.p;
         a.ref_lo = a.ref_gene + n;
@@ -1393,49 +1437,60 @@ void finetune_rounds(sgr_ctx* ctx, const DevCsr& q, const uint8_t* flags_dev, fl
     a.L = (int)L;
     a.Wt = (int)Wt;
     a.nwords = ((int)Wt + 31) / 32;
-    a.eq_stride = eq_stride;
+    a.eq_stride = round_up((int)Wt + 1, 4);
     a.shift = ctx->pack_shift;
     a.mul = make_int3(16 * ctx->ft_copies, 2, -1);
     a.p = p;
     a.thre = thre;
     a.times = times;
-    const int row_stride = round_up((int)Wt, 8);
-    uint16_t* sorted = ctx->fr_sorted.ensure(3 * (size_t)nb * row_stride);
-    a.s_gene = sorted;
-    a.s_lo = sorted + (size_t)nb * row_stride;
-    a.s_hi = sorted + 2 * (size_t)nb * row_stride;
-    a.row_stride = row_stride;
+    a.row_stride = round_up((int)Wt, 8);
     a.flags = flags_dev;
-    a.top = ctx->fr_top.ensure((size_t)nb * L);
-    int* ints = ctx->fr_ints.ensure((size_t)nb * 5);
-    a.ntop = ints;
-    a.used = ints + nb;
-    a.par = ctx->fr_par.ensure(nb);
-    a.eq = ctx->fr_eq.ensure((size_t)nb * eq_stride);
-    a.ext_min = ctx->fr_ext.ensure((size_t)nb * L * 3);
-    a.ext_max = a.ext_min + (size_t)nb * L;
-    a.blk_of = a.ext_max + (size_t)nb * L;
-    a.un = ctx->fr_un.ensure(nb);
-    a.key_count = ctx->fr_keys.ensure(((size_t)2 << 20) + 1);
-    int32_t* scan_scratch = ctx->scan_part.ensure(2 * (((size_t)1 << 20) / 4096) + 1);
-    const size_t n_quads = std::max<size_t>(((size_t)nb + 3) / 4, std::min<size_t>(nb, kFtDirectCells));
-    a.list = ctx->fr_list.ensure((size_t)nb * L + n_quads * L * 4);
-    a.q_entry = a.list + (size_t)nb * L;
-    a.quads = ctx->fr_quads.ensure(n_quads);
-    a.q_label = ctx->fr_q_label.ensure(n_quads * L);
-    a.act = ints + 2 * nb;
-    a.row_len = ints + 4 * nb;
     a.n_list = d->n_list;
     a.queue = d->queue;
     a.n_act = d->read.n_act;
     a.stats = d->read.stats;
-    a.scores = ctx->fr_scores.ensure((size_t)nblk * 32);
-    const int grid = ft_step_grid((int)nb);
-    a.nan_scratch = ctx->fr_nan.ensure((size_t)grid * max_label);
     a.max_label = (int)max_label;
     a.final_labels = ctx->d_final.p + out_row0;
     a.rounds = ctx->d_rounds.p + out_row0;
     a.status = ctx->status.p;
+    // Batches: score blocks of 4 GiB, cells whose e-value rows take 1 GiB; smaller ones where device memory does
+    // not hold the buffers of those (another context or framework may have most of it).
+    int64_t max_blocks = std::max<int64_t>((int64_t)1 << 25, ctx->R32 / 32);
+    int64_t max_cells = std::max<int64_t>(1, std::min<int64_t>(131072, ((int64_t)1 << 28) / a.eq_stride));
+    std::vector<int64_t> cuts, off;
+    int32_t* scan_scratch = nullptr;
+    for (;;) {
+        if (off.empty() && (n_blocks > max_blocks || n_cells > max_cells)) {
+            off.resize(n_cells);
+            SGR_CUDA(cudaMemcpyAsync(off.data(), ctx->fr_blk_off.p, n_cells * sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+            SGR_CUDA(cudaStreamSynchronize(s));
+        }
+        auto end_of = [&](int64_t i) { return i < n_cells ? off[i] : n_blocks; };  // blocks before cell i
+        cuts.assign(1, 0);
+        int64_t nb = n_cells, nblk = n_blocks;
+        if (!off.empty()) {
+            nb = nblk = 0;
+            for (int64_t i = 1; i <= n_cells; ++i) {
+                const int64_t b = cuts.back();
+                if (i < n_cells && end_of(i + 1) - off[b] <= max_blocks && i - b < max_cells) continue;
+                nb = std::max(nb, i - b);
+                nblk = std::max(nblk, end_of(i) - off[b]);
+                cuts.push_back(i);
+            }
+        } else {
+            cuts.push_back(n_cells);
+        }
+        if (fits_memory([&] { scan_scratch = round_buffers(ctx, a, nb, nblk); })) break;
+        ctx->release_round_buffers();
+        if (nb <= 1) return false;
+        finish_streams(ctx);
+        ctx->arena.settle();  // the small ones may be cut from the same slabs again
+        max_cells = (nb + 1) / 2;
+        max_blocks = std::max<int64_t>(nblk / 2, ctx->R32 / 32);
+    }
+    ctx->prof.acc.ft_cells += (uint64_t)n_cells;
+    ctx->prof.acc.ft_candidates += h.cand;
+    ctx->prof.acc.ft_split_cells += (uint64_t)n_cells;
     // 32-bit run sums: X = sum z s <= 2 k (e-sum of the kept entries), each e below 2 Wt and all of the
     // query's e together k_q |S|, k_q at most the longest query row.  That row is read back only where the
     // pool's width alone does not decide.
@@ -1450,9 +1505,8 @@ void finetune_rounds(sgr_ctx* ctx, const DevCsr& q, const uint8_t* flags_dev, fl
         a.n_cells = (int)(cuts[b + 1] - cuts[b]);
         if (b > 0) SGR_CUDA(cudaMemsetAsync(d, 0, sizeof(FtCtl), s));
         SGR_CUDA(cudaMemsetAsync(a.used, 0, a.n_cells * sizeof(int), s));
-        launch_ft_rows(a.cells, a.n_cells, q.data, q.indices, q.indptr, q.n_cols, ctx->qry_map_thre.p, (int)Wt, row_stride,
-                       sorted, sorted + (size_t)nb * row_stride, sorted + 2 * (size_t)nb * row_stride, ints + 4 * nb,
-                       &d->read.longest, fp32, s);
+        launch_ft_rows(a.cells, a.n_cells, q.data, q.indices, q.indptr, q.n_cols, ctx->qry_map_thre.p, (int)Wt, a.row_stride,
+                       a.s_gene, a.s_lo, a.s_hi, a.row_len, &d->read.longest, fp32, s);
         bool x64 = ctx->pack_scan != 2 || !narrow(Wt);
         // each round drops at least one candidate, so L rounds finish every cell
         int most = a.n_cells;  // no more cells than this are active
@@ -1478,6 +1532,7 @@ void finetune_rounds(sgr_ctx* ctx, const DevCsr& q, const uint8_t* flags_dev, fl
             break;
         }
     }
+    return true;
 }
 
 // The fine-tune by rounds where the trained reference allows it, and its results on the host
@@ -1489,7 +1544,7 @@ bool finetune_by_rounds(sgr_ctx* ctx, const DevCsr& q, const uint8_t* flags_dev,
     const uint32_t Q = q.n_rows;
     if (!ctx->ft_copies || Q == 0) return false;
     if (ctx->mode == SGR_MODE_FP32REF && !ft_scan32_warps((int)std::max<uint32_t>(ctx->Wt, 1))) return false;
-    finetune_rounds(ctx, q, flags_dev, p, thre, times, cell_list, n_list, out_row0);
+    if (!finetune_rounds(ctx, q, flags_dev, p, thre, times, cell_list, n_list, out_row0)) return false;
     if (!final_labels) return true;
     SGR_CUDA(cudaMemcpyAsync(final_labels, ctx->d_final.p + out_row0, Q * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
     if (rounds_out)

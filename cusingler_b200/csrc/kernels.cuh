@@ -338,8 +338,8 @@ struct FtRounds {
     float p, thre;
     int times;
     // query rows of the cells, compacted to the pool and sorted by value
-    const uint16_t *s_gene, *s_lo, *s_hi;
-    const int32_t* row_len;     // per cell; its entries start at cell * row_stride
+    uint16_t *s_gene, *s_lo, *s_hi;
+    int32_t* row_len;           // per cell; its entries start at cell * row_stride
     int row_stride;
     const uint8_t* flags;
     // batch of n_cells cells

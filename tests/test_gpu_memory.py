@@ -1,0 +1,75 @@
+"""A GPU that another framework has nearly filled: calls take less workspace instead of failing, and give the
+same results.  Device memory is filled by ordinary allocations and given back after each test."""
+
+import contextlib
+
+import numpy as np
+import pytest
+
+from cusingler_b200 import abi, synth
+from tests import helpers as H
+
+pytestmark = pytest.mark.gpu
+
+
+@contextlib.contextmanager
+def _free_mib(mib):
+    """Only this much device memory free inside."""
+    import torch
+
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    held = []
+    try:
+        for step in (1 << 30, 1 << 26, 1 << 21):
+            while torch.cuda.mem_get_info(0)[0] - (mib << 20) >= step:
+                spare = (torch.cuda.mem_get_info(0)[0] - (mib << 20)) // step * step
+                held.append(torch.empty(spare, dtype=torch.uint8, device="cuda"))
+        yield
+    finally:
+        held.clear()
+        torch.cuda.empty_cache()
+
+
+def _trained(prob, mode=abi.MODE_EXACT):
+    a = abi.Annotator(gpuid=0, mode=mode)
+    return a.train(prob.ref, prob.celltypes, prob.label_names, prob.ref_genes, prob.qry_genes)
+
+
+def _tiled_query(m, times):
+    """The rows, `times` times over, on the device."""
+    import torch
+
+    nnz = int(m.indptr[-1])
+    indptr = np.concatenate([[0]] + [m.indptr[1:].astype(np.int64) + nnz * t for t in range(times)])
+    keep = [torch.from_numpy(x).cuda() for x in (m.data, m.indices.astype(np.int32))]
+    keep = [t.repeat(times) for t in keep] + [torch.from_numpy(indptr.astype(np.int32)).cuda()]
+    return abi.device_csr(m.n_rows * times, m.n_cols, *(t.data_ptr() for t in keep)), keep
+
+
+@pytest.mark.parametrize("mode", [abi.MODE_EXACT, abi.MODE_FP32REF])
+def test_finetune_in_several_batches(mode):
+    """100,000 cells' round buffers take several times the free memory: the call runs them in batches."""
+    prob = H.problem("families")
+    res = H.oracle_run("families", 0 if mode == abi.MODE_FP32REF else 1)
+    times = 500
+    a = _trained(prob, mode)
+    flags = res["flags"].astype(np.uint8)
+    a.finetune(prob.qry, flags)
+    q, keep = _tiled_query(prob.qry, times)
+    many = np.tile(flags, (times, 1))
+    batched = []
+    with _free_mib(250):
+        for _ in range(2):
+            a.reset_timings()
+            final, rounds = a.finetune(q, many)
+            batched.append(a.timings()["ft_split_rounds"])
+            assert np.array_equal(final, np.tile(res["final"], times))
+            assert np.array_equal(rounds, np.tile(res["rounds"], times))
+    a.reset_timings()
+    final, rounds = a.finetune(q, many)  # and again in one
+    assert min(batched) >= 2 * a.timings()["ft_split_rounds"] > 0
+    assert np.array_equal(final, np.tile(res["final"], times))
+    assert np.array_equal(rounds, np.tile(res["rounds"], times))
+    a.close()
+    del q, keep
