@@ -58,7 +58,8 @@ inline void allow_most_smem(K kern) {
 // cudaMalloc and a cudaFree each (0.33 ms a call here, about 100 buffers per context: 10 of 22 ms of a whole
 // drop-in run on 1,900 x 800 cells).  A context's arena is used by the thread that is in a call on the
 // context.  A released block is handed out again only after settle(), which the context calls when its
-// streams have finished, so no queued work can still use it; the slabs are freed with the context.
+// streams have finished, so no queued work can still use it; the slabs are freed with the context.  Where there
+// is no room for another slab, buffers are cudaMalloc'ed at their own size.
 class DevArena {
 public:
     static constexpr size_t kSlab = (size_t)64 << 20, kLargest = (size_t)16 << 20;
@@ -68,24 +69,30 @@ public:
     ~DevArena() {
         for (char* s : slabs_) cudaFree(s);
     }
-    // bytes is rounded up to what the block holds
+    // bytes is rounded up to what the block holds; null (bytes as given) where there is no room for a slab
     void* alloc(size_t& bytes) {
         const int c = size_class(bytes);
-        bytes = class_bytes(c);
         if (!free_[c].empty()) {
             char* p = free_[c].back();
             free_[c].pop_back();
+            bytes = class_bytes(c);
             return p;
         }
         const size_t n = class_bytes(c);
         if (slabs_.empty() || used_ + n > kSlab) {
             char* s = nullptr;
-            SGR_CUDA(cudaMalloc(reinterpret_cast<void**>(&s), kSlab));
+            const cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&s), kSlab);
+            if (e == cudaErrorMemoryAllocation) {
+                cudaGetLastError();
+                return nullptr;
+            }
+            SGR_CUDA(e);
             slabs_.push_back(s);
             used_ = 0;
         }
         char* p = slabs_.back() + used_;
         used_ += n;
+        bytes = n;
         return p;
     }
     void release(void* p, size_t bytes) { pending_.push_back({size_class(bytes), static_cast<char*>(p)}); }
@@ -138,12 +145,9 @@ struct DevBuf {
             release();
             size_t bytes = count * sizeof(T);
             DevArena* a = DevArena::current();
-            if (a && bytes <= DevArena::kLargest) {
-                p = static_cast<T*>(a->alloc(bytes));
-                home = a;
-            } else {
-                SGR_CUDA(cudaMalloc(reinterpret_cast<void**>(&p), bytes));
-            }
+            if (a && bytes <= DevArena::kLargest) p = static_cast<T*>(a->alloc(bytes));
+            if (p) home = a;
+            else SGR_CUDA(cudaMalloc(reinterpret_cast<void**>(&p), bytes));
             n = bytes / sizeof(T);
         }
         return p;

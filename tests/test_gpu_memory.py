@@ -73,3 +73,15 @@ def test_finetune_in_several_batches(mode):
     assert np.array_equal(rounds, np.tile(res["rounds"], times))
     a.close()
     del q, keep
+
+
+def test_small_context():
+    """A small training and call where less than one slab of buffers is free."""
+    prob = H.problem("tiny")
+    res = H.oracle_run("tiny", 1)
+    _trained(prob).annotate(prob.qry)  # the kernels are loaded
+    with _free_mib(60):
+        a = _trained(prob)
+        first, final = a.annotate(prob.qry)
+        assert np.array_equal(first, res["first"]) and np.array_equal(final, res["final"])
+        a.close()
