@@ -58,18 +58,19 @@ inline void allow_most_smem(K kern) {
 // cudaMalloc and a cudaFree each (0.33 ms a call here, about 100 buffers per context: 10 of 22 ms of a whole
 // drop-in run on 1,900 x 800 cells).  A context's arena is used by the thread that is in a call on the
 // context.  A released block is handed out again only after settle(), which the context calls when its
-// streams have finished, so no queued work can still use it; the slabs are freed with the context.  Where there
-// is no room for another slab, buffers are cudaMalloc'ed at their own size.
+// streams have finished, so no queued work can still use it; the slabs are freed with the context.  Where less
+// than kSpare of the device's memory is free, a slab's unused part would be missed, and buffers are cudaMalloc'ed
+// at their own size.
 class DevArena {
 public:
-    static constexpr size_t kSlab = (size_t)64 << 20, kLargest = (size_t)16 << 20;
+    static constexpr size_t kSlab = (size_t)64 << 20, kLargest = (size_t)16 << 20, kSpare = (size_t)1 << 30;
     DevArena() = default;
     DevArena(const DevArena&) = delete;
     DevArena& operator=(const DevArena&) = delete;
     ~DevArena() {
         for (char* s : slabs_) cudaFree(s);
     }
-    // bytes is rounded up to what the block holds; null (bytes as given) where there is no room for a slab
+    // bytes is rounded up to what the block holds; null (bytes as given) where memory is short
     void* alloc(size_t& bytes) {
         const int c = size_class(bytes);
         if (!free_[c].empty()) {
@@ -80,13 +81,11 @@ public:
         }
         const size_t n = class_bytes(c);
         if (slabs_.empty() || used_ + n > kSlab) {
+            size_t left = 0, total = 0;
+            SGR_CUDA(cudaMemGetInfo(&left, &total));
+            if (left < kSpare) return nullptr;
             char* s = nullptr;
-            const cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&s), kSlab);
-            if (e == cudaErrorMemoryAllocation) {
-                cudaGetLastError();
-                return nullptr;
-            }
-            SGR_CUDA(e);
+            SGR_CUDA(cudaMalloc(reinterpret_cast<void**>(&s), kSlab));
             slabs_.push_back(s);
             used_ = 0;
         }
