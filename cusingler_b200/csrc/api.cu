@@ -378,6 +378,18 @@ sgr_status guarded(sgr_ctx* ctx, F&& f) {
     }
 }
 
+// Runs f, which allocates device memory; false where there was not enough.
+template <class F>
+bool fits_memory(F&& f) {
+    try {
+        f();
+        return true;
+    } catch (const Error& e) {
+        if (e.code != SGR_ERR_OUT_OF_MEMORY) throw;
+        return false;
+    }
+}
+
 void check_csr_shape(const sgr_csr* m, const char* what) {
     if (!m) fail(SGR_ERR_INVALID_ARGUMENT, std::string(what) + ": null matrix");
     if (m->n_rows && (!m->indptr)) fail(SGR_ERR_INVALID_ARGUMENT, std::string(what) + ": null indptr");
@@ -593,7 +605,10 @@ void build_row_groups(sgr_ctx* ctx, const std::vector<int32_t>& fptr, const std:
             if (j % 32 == 0) {  // the block's first row is its longest
                 voff[blk_base[l] + j / 32] = (int32_t)at;
                 at += 32ll * ((ng[start + order[j]] + 1) / 2);
-                if (at > INT32_MAX) fail(SGR_ERR_UNSUPPORTED, "fine-tune reference lists exceed 2^31 vectors");
+                if (at > INT32_MAX) {  // too long for the blocks' offsets
+                    ctx->ft_copies = 0;
+                    return;
+                }
             }
         }
     }
@@ -773,7 +788,6 @@ void train(sgr_ctx* ctx, const sgr_csr* ref, const int32_t* celltypes, const cha
         ctx->pack_narrow = ctx->pack_shift > 0 && 4 * max_row * max_row * wt < (int64_t(1) << 32) &&
                            max_row * max_row * max_row < (int64_t(1) << 32);
     }
-    build_row_groups(ctx, fptr, blk_base);
     ctx->d_row_perm.upload(row_perm, s);
     ctx->d_blk_base.upload(blk_base, s);
     ctx->d_ell_off.upload(ell_off, s);
@@ -804,15 +818,21 @@ void train(sgr_ctx* ctx, const sgr_csr* ref, const int32_t* celltypes, const cha
     std::vector<int32_t> gt(mk.n_labels + 1, 0);
     for (uint32_t n = 1; n <= mk.n_labels; ++n) gt[n] = marker_count(n);
     ctx->d_gene_thre.upload(gt, s);
+    // What only the rounds over all cells read, last: where device memory does not hold it, the fine-tune does without.
+    if (!fits_memory([&] { build_row_groups(ctx, fptr, blk_base); })) {
+        ctx->ft_copies = 0;
+        ctx->fr_groups.release();
+    }
     // the pairs' fine-tune lists as bits over the pool, whole and as each candidate count cuts them (unless
     // that takes over 256 MiB each)
     const size_t nwords = (std::max<size_t>(ctx->Wt, 1) + 31) / 32, nl = mk.n_labels, rows_words = nl * nl * nwords;
-    ctx->fr_masks = ctx->ft_copies && rows_words <= ((size_t)64 << 20);
-    ctx->fr_cut_masks = ctx->fr_masks && nl >= 2 && rows_words * (nl - 1) <= ((size_t)64 << 20);
+    ctx->fr_masks = ctx->ft_copies && rows_words <= ((size_t)64 << 20) &&
+                    fits_memory([&] { ctx->fr_pair_mask.ensure(rows_words); });
+    ctx->fr_cut_masks = ctx->fr_masks && nl >= 2 && rows_words * (nl - 1) <= ((size_t)64 << 20) &&
+                        fits_memory([&] { ctx->fr_cut_mask.ensure(rows_words * (nl - 1)); });
     if (ctx->fr_masks)
-        launch_pair_masks(ctx->d_ft_genes.p, ctx->d_ft_idx.p, (int)nl, (int)nwords, ctx->d_gene_thre.p,
-                          ctx->fr_pair_mask.ensure(rows_words),
-                          ctx->fr_cut_masks ? ctx->fr_cut_mask.ensure(rows_words * (nl - 1)) : nullptr, s);
+        launch_pair_masks(ctx->d_ft_genes.p, ctx->d_ft_idx.p, (int)nl, (int)nwords, ctx->d_gene_thre.p, ctx->fr_pair_mask.p,
+                          ctx->fr_cut_masks ? ctx->fr_cut_mask.p : nullptr, s);
     check_status(ctx);
     ctx->trained = true;
 }
@@ -1329,18 +1349,6 @@ void ensure_ref_runs(sgr_ctx* ctx) {
     launch_ft_sort_rows((int)ctx->R, ctx->reff_data.p, ctx->reff_indices.p, ctx->reff_indptr.p, ctx->max_row, r,
                         r + n, r + 2 * n, ctx->fr_ref_nan.p, ctx->stream);
     ctx->fr_ref_runs_ready = true;
-}
-
-// Runs f, which allocates device memory; false where there was not enough.
-template <class F>
-bool fits_memory(F&& f) {
-    try {
-        f();
-        return true;
-    } catch (const Error& e) {
-        if (e.code != SGR_ERR_OUT_OF_MEMORY) throw;
-        return false;
-    }
 }
 
 // The buffers of a batch of nb cells with nblk score blocks, set in `a`; returns the ordering's scan scratch.

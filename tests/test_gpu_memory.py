@@ -85,3 +85,17 @@ def test_small_context():
         first, final = a.annotate(prob.qry)
         assert np.array_equal(first, res["first"]) and np.array_equal(final, res["final"])
         a.close()
+
+
+def test_training_without_room_for_the_optional_tables():
+    """The pairs' masks per candidate count (147 MiB here) do not fit: the rounds use the lists."""
+    from tests import test_gpu_wide_pool as T
+
+    sizes = dict(L=60, block=100)
+    prob, (flags, final, rounds) = T._problem(**sizes), T._solved(1, **sizes)
+    _trained(prob).finetune(prob.qry, flags, thre=T.THRE)
+    with _free_mib(100):
+        a = _trained(prob)
+        got, got_rounds = a.finetune(prob.qry, flags, thre=T.THRE)
+        assert np.array_equal(got, final) and np.array_equal(got_rounds, rounds)
+        a.close()

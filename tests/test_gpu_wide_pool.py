@@ -14,21 +14,20 @@ from tests import helpers as H
 pytestmark = pytest.mark.gpu
 
 THRE = 0.15
-L, BLOCK = 50, 300  # labels, genes that only one label has
 
 
 @functools.lru_cache(maxsize=None)
-def _problem():
-    """Labels of six cells with 300 genes of their own each; queries that mix the genes of four labels."""
+def _problem(L=50, block=300):
+    """Labels of six cells with genes (block) of their own each; queries that mix the genes of four labels."""
     rng = np.random.default_rng(11)
-    n_genes = L * BLOCK
+    n_genes = L * block
 
     def cells(labels, others):
         ptr, idx, val = [0], [], []
         for lab in labels:
             p = np.full(n_genes, 0.002)
             for m in [lab, *rng.choice(L, others, replace=False)]:
-                p[m * BLOCK:(m + 1) * BLOCK] = 0.5 if others else 0.75
+                p[m * block:(m + 1) * block] = 0.5 if others else 0.75
             c = np.flatnonzero(rng.random(n_genes) < p)
             idx.append(c)
             val.append(np.log2(1 + rng.integers(1, 40, len(c))))
@@ -43,8 +42,8 @@ def _problem():
 
 
 @functools.lru_cache(maxsize=None)
-def _solved(mode):
-    orc = O.Oracle(_problem())
+def _solved(mode, **sizes):
+    orc = O.Oracle(_problem(**sizes))
     orc.train()
     flags = orc.score(mode=mode, thre=THRE)[2].astype(np.uint8)
     final, rounds = orc.finetune(mode=mode, thre=THRE)
