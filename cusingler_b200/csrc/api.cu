@@ -630,11 +630,17 @@ void train(sgr_ctx* ctx, const sgr_csr* ref, const int32_t* celltypes, const cha
     cudaStream_t s = ctx->stream;
     // The rows as given, copied to the device once; their column ids are checked there, and the label-grouped
     // reference is gathered from them below.  (On the host the check took 16 ms and the regrouping 115 ms of
-    // a 195 ms training on 20,000 cells, 30e6 entries; the copy itself takes 22 ms from pageable memory.)
+    // a 195 ms training on 20,000 cells, 30e6 entries; the copy itself takes 22 ms from pageable memory.)  Where
+    // device memory does not hold the rows twice, the host does both.
     const size_t nnz = (size_t)ref->indptr[ref->n_rows];
     DevBuf<float> raw_data;
     DevBuf<int32_t> raw_indices, raw_indptr;
-    if (ctx->device >= 0) {
+    bool raw_rows = ctx->device >= 0 && fits_memory([&] {
+                        raw_indices.ensure(nnz);
+                        raw_data.ensure(nnz);
+                        raw_indptr.ensure((size_t)ref->n_rows + 1);
+                    });
+    if (raw_rows) {
         raw_indices.upload(ref->indices, nnz, s);
         raw_data.upload(ref->data, nnz, s);
         raw_indptr.upload(ref->indptr, (size_t)ref->n_rows + 1, s);
@@ -645,6 +651,8 @@ void train(sgr_ctx* ctx, const sgr_csr* ref, const int32_t* celltypes, const cha
         SGR_CUDA(cudaStreamSynchronize(s));
         if (st & 1) fail(SGR_ERR_INVALID_ARGUMENT, "reference column index out of range");
     } else {
+        raw_indices.release();
+        raw_data.release();
         for (size_t i = 0; i < nnz; ++i)
             if ((uint32_t)ref->indices[i] >= ref->n_cols)
                 fail(SGR_ERR_INVALID_ARGUMENT, "reference column index out of range");
@@ -676,9 +684,26 @@ void train(sgr_ctx* ctx, const sgr_csr* ref, const int32_t* celltypes, const cha
         indptr[j + 1] = indptr[j] + (ref->indptr[r + 1] - ref->indptr[r]);
     }
     ctx->ref_indptr.upload(indptr, s);
-    ctx->ref_data.ensure(nnz);
-    ctx->ref_indices.ensure(nnz);
-    {
+    if (raw_rows && !fits_memory([&] {
+            ctx->ref_data.ensure(nnz);
+            ctx->ref_indices.ensure(nnz);
+        })) {
+        raw_rows = false;
+        raw_data.release();
+        raw_indices.release();
+    }
+    if (!raw_rows) {
+        std::vector<float> data(nnz);
+        std::vector<int32_t> indices(nnz);
+        for (uint32_t j = 0; j < ctx->R; ++j) {
+            const uint32_t r = mk.ref_order[j];
+            std::copy(ref->data + ref->indptr[r], ref->data + ref->indptr[r + 1], data.begin() + indptr[j]);
+            std::copy(ref->indices + ref->indptr[r], ref->indices + ref->indptr[r + 1], indices.begin() + indptr[j]);
+        }
+        ctx->ref_data.upload(data, s);
+        ctx->ref_indices.upload(indices, s);
+        SGR_CUDA(cudaStreamSynchronize(s));
+    } else {
         DevBuf<uint32_t> order;
         order.upload(mk.ref_order, s);
         launch_gather_rows(raw_data.p, raw_indices.p, raw_indptr.p, order.p, ctx->R, ctx->ref_indptr.p, ctx->ref_data.p,

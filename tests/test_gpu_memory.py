@@ -99,3 +99,33 @@ def test_training_without_room_for_the_optional_tables():
         got, got_rounds = a.finetune(prob.qry, flags, thre=T.THRE)
         assert np.array_equal(got, final) and np.array_equal(got_rounds, rounds)
         a.close()
+
+
+def test_training_without_room_for_a_second_copy():
+    """The reference as given and regrouped (120 MB each) do not fit together."""
+    rng = np.random.default_rng(3)
+    R, W, k, L = 10000, 4000, 1500, 4
+    keys = rng.random((R, W), np.float32)
+    labels = rng.integers(0, L, R).astype(np.int32)
+    for lab in range(L):  # genes that a label's cells store more often
+        keys[labels == lab, 100 * lab:100 * (lab + 1)] *= 0.5
+    indices = np.sort(keys.argpartition(k, axis=1)[:, :k], axis=1).astype(np.int32)
+    data = rng.integers(1, 60, (R, k)).astype(np.float32)
+    ref = synth.CSR(R, W, data.reshape(-1), indices.reshape(-1), (np.arange(R + 1) * k).astype(np.int32), labels)
+    names, genes = synth.names("CT", L), synth.names("G", W)
+    q = ref.rows(0, 50)
+    a = abi.Annotator(gpuid=0).train(ref, labels, names, genes, genes)
+    tables, labels_of = [a.u32(what) for what in range(8)], a.annotate(q)
+    a.close()
+    bad = indices.reshape(-1).copy()
+    bad[-1] = W
+    with _free_mib(245):
+        a = abi.Annotator(gpuid=0)
+        for _ in range(2):  # the second training finds the first one's buffers
+            a.train(ref, labels, names, genes, genes)
+            assert all(np.array_equal(a.u32(what), tables[what]) for what in range(8))
+        with pytest.raises(abi.SgrError) as e:
+            a.train(synth.CSR(R, W, ref.data, bad, ref.indptr, labels), labels, names, genes, genes)
+        assert e.value.status == 1
+    assert all(np.array_equal(x, y) for x, y in zip(a.annotate(q), labels_of))
+    a.close()
