@@ -217,8 +217,9 @@ struct sgr_ctx {
     DevBuf<int> fr_ref_nan;        // whether some of them are NaN
     size_t fr_ref_runs_stride = 0;
     bool fr_ref_runs_ready = false;
-    // gives the buffers sized by a batch back
-    void release_round_buffers() {
+    // gives the buffers sized by a batch back; whether there were any
+    bool release_round_buffers() {
+        const bool held = fr_sorted.p != nullptr;
         fr_sorted.release();
         fr_top.release();
         fr_ints.release();
@@ -232,6 +233,15 @@ struct sgr_ctx {
         fr_keys.release();
         fr_scores.release();
         fr_nan.release();
+        return held;
+    }
+    // the same for the masks that a training left: the rounds take the lists
+    bool release_masks() {
+        const bool held = fr_masks;
+        fr_masks = fr_cut_masks = false;
+        fr_pair_mask.release();
+        fr_cut_mask.release();
+        return held;
     }
     FtRead* h_ft = nullptr;        // pinned, two: counters read back, by the parity of the round
     cudaEvent_t ev_ft[2] = {nullptr, nullptr};
@@ -353,28 +363,37 @@ sgr_status guarded(sgr_ctx* ctx, F&& f) {
         }
         ~UseArena() { DevArena::current() = before; }
     } use_arena(ctx->arena);
-    try {
-        if (ctx->device >= 0) SGR_CUDA(cudaSetDevice(ctx->device));
-        const uint64_t l0 = launch_count();
-        f();
-        if (ctx->stream) {
-            SGR_CUDA(cudaStreamSynchronize(ctx->stream));
-            ctx->prof.collect();
+    for (int attempt = 0;; ++attempt) {
+        const sgr_timings before = ctx->prof.acc;
+        try {
+            if (ctx->device >= 0) SGR_CUDA(cudaSetDevice(ctx->device));
+            const uint64_t l0 = launch_count();
+            f();
+            if (ctx->stream) {
+                SGR_CUDA(cudaStreamSynchronize(ctx->stream));
+                ctx->prof.collect();
+            }
+            ctx->prof.acc.launches += launch_count() - l0;
+            return SGR_OK;
+        } catch (const Error& e) {
+            ctx->err = e.what();
+            drain(ctx);
+            // what only the rounds of an earlier fine-tune used may be what is missing: given back, and the call anew
+            if (e.code != SGR_ERR_OUT_OF_MEMORY || attempt == 3 ||
+                !(ctx->release_round_buffers() || ctx->release_masks()))
+                return e.code;
+            ctx->arena.settle();
+            ctx->prof.acc = before;
+            ctx->err.clear();
+        } catch (const std::bad_alloc&) {
+            ctx->err = "host allocation failed";
+            drain(ctx);
+            return SGR_ERR_OUT_OF_MEMORY;
+        } catch (const std::exception& e) {
+            ctx->err = e.what();
+            drain(ctx);
+            return SGR_ERR_INVALID_ARGUMENT;
         }
-        ctx->prof.acc.launches += launch_count() - l0;
-        return SGR_OK;
-    } catch (const Error& e) {
-        ctx->err = e.what();
-        drain(ctx);
-        return e.code;
-    } catch (const std::bad_alloc&) {
-        ctx->err = "host allocation failed";
-        drain(ctx);
-        return SGR_ERR_OUT_OF_MEMORY;
-    } catch (const std::exception& e) {
-        ctx->err = e.what();
-        drain(ctx);
-        return SGR_ERR_INVALID_ARGUMENT;
     }
 }
 

@@ -129,3 +129,24 @@ def test_training_without_room_for_a_second_copy():
         assert e.value.status == 1
     assert all(np.array_equal(x, y) for x, y in zip(a.annotate(q), labels_of))
     a.close()
+
+
+def test_held_round_buffers_are_given_back():
+    """The score step needs more than what the fine-tune of an earlier call left free."""
+    prob = H.problem("families")
+    res = H.oracle_run("families", 1)
+    times = 500
+    a = _trained(prob)
+    a.set_tuning(2, 16)
+    a.annotate(prob.qry)
+    q, keep = _tiled_query(prob.qry, times)
+    flags = np.tile(res["flags"].astype(np.uint8), (times, 1))
+    with _free_mib(500):
+        for _ in range(2):
+            final, rounds = a.finetune(q, flags)
+            assert np.array_equal(final, np.tile(res["final"], times))
+            first, final = a.annotate(q)
+            assert np.array_equal(first, np.tile(res["first"], times))
+            assert np.array_equal(final, np.tile(res["final"], times))
+    a.close()
+    del q, keep
