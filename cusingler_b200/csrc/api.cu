@@ -2370,7 +2370,9 @@ sgr_status sgr_autotune(sgr_ctx* ctx, const sgr_csr* sample, float quantile, flo
     ctx->corr_wide = best.corr_wide;
     ctx->corr_gm = best.corr_gm;
     ctx->score_chunk_bytes = (size_t)best.score_chunk_mb << 20;
-    ctx->select_warps = best.select_warps;
+    // where the fastest form is the one that the number of rows picks, it stays so: smaller calls have their own
+    const int rows = (int)std::max<size_t>(1, std::min<size_t>(Q, ctx->score_chunk_bytes / (4 * std::max<size_t>(ctx->R, 1))));
+    ctx->select_warps = (best.select_warps >= 8) == (select_form(rows) >= 8) ? -1 : best.select_warps;
     best.score_best_ms = score_best;
 
     // phase 2: fine-tune shapes with the chosen score step, timed on the whole annotation; first and
@@ -2450,7 +2452,7 @@ sgr_status sgr_set_tuning(sgr_ctx* ctx, int what, int value) {
         return SGR_OK;
     }
     if (what == 7) {
-        if (value != 0 && value != 1 && value != 8 && value != 16) return SGR_ERR_INVALID_ARGUMENT;
+        if (value != -1 && value != 0 && value != 1 && value != 8 && value != 16) return SGR_ERR_INVALID_ARGUMENT;
         ctx->select_warps = value;
         return SGR_OK;
     }

@@ -1090,17 +1090,19 @@ LabelQ make_lq(int start, int len, float p) {
     return q;
 }
 
+// By size.  Up to one row per SM, a CTA that stages its row is the shorter way (10.6 against 14.0 us for up to
+// 148 rows of 1,900 scores, 18.8 / 21.6 for 148 of 20,001), and one launch less; with more rows the items are
+// spread better (us, items / rows: 15.4 / 15.9 for 400 x 1,900, 198 / 251 for 5,000 x 20,000, 455 / 603 for
+// 12,345 x 20,000, 888 / 1,633 for 8,192 x 40,000).  Rows over 200 KB can not be staged.
+int select_form(int nq) { return nq <= sm_count() ? 16 : 0; }
+
 void launch_select_first(const float* scores, int64_t ld, int nq, int L, const LabelQ* lq, float p, float thre,
                          const int64_t* qn2, float* label_scores, int32_t* first, uint8_t* flags, float* scratch,
                          int64_t spw, int* status, int row_len, const int32_t* lorder, cudaStream_t s,
                          const uint32_t* ext_min, const uint32_t* ext_max, int warps) {
     if (nq <= 0) return;
     const size_t stage_bytes = (((size_t)std::max(row_len, 1) * 4 + 15) & ~size_t(15));
-    // By size.  Up to one row per SM, a CTA that stages its row is the shorter way (10.6 against 14.0 us for up to
-    // 148 rows of 1,900 scores, 18.8 / 21.6 for 148 of 20,001), and one launch less; with more rows the items are
-    // spread better (us, items / rows: 15.4 / 15.9 for 400 x 1,900, 198 / 251 for 5,000 x 20,000, 455 / 603 for
-    // 12,345 x 20,000, 888 / 1,633 for 8,192 x 40,000).  Rows over 200 KB can not be staged.
-    if (warps < 0) warps = nq <= sm_count() ? 16 : 0;
+    if (warps < 0) warps = select_form(nq);
     if (warps >= 8 && stage_bytes <= 200 * 1024) {
         auto kern = select_row_kernel<16>;
         allow_smem(kern, 200 * 1024);

@@ -139,6 +139,8 @@ LabelQ make_lq(int start, int len, float p);
 // ext_min / ext_max (optional): per (row, label) extreme order keys from the correlation epilogue, used instead
 // of a min / max pass for lists that cannot hold NaN.  warps: 8 or 16 a CTA per row that stages it in shared
 // memory (rows of at most 200 KB), 0 or 1 a warp per (row, label), -1 chosen by the sizes.
+// The form (16: a CTA per row, 0: a warp per row and label) that launch_select_first takes for nq rows by itself.
+int select_form(int nq);
 void launch_select_first(const float* scores, int64_t ld, int nq, int L, const LabelQ* lq, float p,
                          float thre, const int64_t* qn2, float* label_scores, int32_t* first, uint8_t* flags,
                          float* scratch, int64_t scratch_per_warp, int* status, int row_len, const int32_t* lorder,

@@ -151,7 +151,7 @@ sgr_status sgr_set_profiling(sgr_ctx* ctx, int on);
  * (1 to 4096, default 16; the bands of a group sweep the reference together so that the CTAs at work share
  * operand tiles in L2); what 7: the score-step selection's form: 8 or 16 for a CTA of 16 warps that
  * stages a query row in shared memory (rows of at most 200 KB), 0 or 1 for one warp per query row and
- * label reading the scores directly; until it is set, chosen by the number of rows;
+ * label reading the scores directly, -1 (default) chosen by the number of rows;
  * what 8: 1 trains the markers on the host instead of the device; what 9 (exact mode): 1 fine-tunes
  * each score block on a second stream while the next block is scored; what 10: the exact
  * correlation's tile: 8 or 16 for 128 x 256 tiles with two accumulators (when the trained marker
@@ -169,9 +169,10 @@ sgr_status sgr_reset_timings(sgr_ctx* ctx);
 /* Autotuner (no counterpart in the reference).  A host `sample` is first copied to the device once
  * (the trials then time the kernels, not the copy).  Phase 1 times the score step of `sample` for
  * every score-step shape -- correlation on one CTA or an SM pair per tile x tile
- * order of 1 or 16 bands per group x score block {256, 1024} MiB x selection form {warp per row at
- * 64 or 32 registers, 16-warp row-staging CTA}
- * (exact mode; fp32ref mode tunes the last two) -- and keeps the fastest; phase 2 then times the
+ * order of 1 or 16 bands per group x score block {256, 1024} MiB x selection form {0, 1: the same, a warp per
+ * row and label; 16: 16-warp row-staging CTA}
+ * (exact mode; fp32ref mode tunes the last two) -- and keeps the fastest; a selection form that the sample's
+ * size would pick by itself stays chosen by size; phase 2 then times the
  * whole annotation for every fine-tune shape -- pipelined or not (exact mode) x warps per CTA
  * {8, 32} x split-path threshold {4, 6, 9, 16, off} -- and keeps the fastest by wall time.  All choices stay set in the context.
  * learned = 1 tunes the learned form (sgr_annotate_learned with min_confidence / check_fraction), 0

@@ -46,3 +46,27 @@ def test_selection_by_size(rows):
         assert H.ulp_diff(scores, res["scores"][:n]).max() == 0
         assert np.array_equal(first, res["first"][:n])
         assert np.array_equal(flags, res["flags"][:n].astype(np.uint8))
+
+
+def _launches_of_one_row(a, prob):
+    a.reset_timings()
+    a.score_first(prob.qry.rows(0, 1))
+    return a.timings()["launches"]
+
+
+def test_selection_by_size_can_be_set_again():
+    """A set form holds for every size (one row: the items take one launch more); -1 chooses by size again, and
+    tuning on a large sample leaves a one-row call its own form."""
+    prob = H.problem("small")
+    a = abi.Annotator(gpuid=0)
+    a.train(prob.ref, prob.celltypes, prob.label_names, prob.ref_genes, prob.qry_genes)
+    by_size = _launches_of_one_row(a, prob)
+    a.set_tuning(7, 0)
+    assert _launches_of_one_row(a, prob) == by_size + 1
+    a.set_tuning(7, -1)
+    assert _launches_of_one_row(a, prob) == by_size
+    for bad in (-2, 2, 32):
+        with pytest.raises(abi.SgrError):
+            a.set_tuning(7, bad)
+    a.autotune(prob.qry)
+    assert _launches_of_one_row(a, prob) == by_size
