@@ -14,9 +14,12 @@ namespace {
 
 constexpr unsigned FULL = 0xffffffffu;
 
+// Unsigned keys in the order of the floats, the NaNs beyond the infinities on their sign's side.  The mask is computed:
+// setting the sign bit of a float in so many words (u | 0x80000000) may be compiled to -|f|, which gives the NaN
+// 0x7fffffff back as it is, a key near that of +0.
 __device__ __forceinline__ uint32_t ord_key(float f) {
-    uint32_t u = __float_as_uint(f);
-    return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+    const uint32_t u = __float_as_uint(f);
+    return u ^ ((uint32_t)((int32_t)u >> 31) | 0x80000000u);
 }
 
 __device__ __forceinline__ float key_float(uint32_t k) {

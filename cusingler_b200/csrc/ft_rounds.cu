@@ -50,7 +50,7 @@ constexpr int STEP_NW = 8;             // warps of a step CTA, and of one where 
 constexpr int STEP_NW_FEW = 32;
 constexpr int STEP_CTAS = 8;           // step CTAs per SM
 constexpr int SCAN_NW = 16;            // warps of a scan CTA (one CTA per SM: the table fills it)
-constexpr uint32_t NAN_KEY = 0xffffffffu;  // ord_key of the NaN that the scan writes
+constexpr uint32_t NAN_KEY = 0xffffffffu;  // extreme of a list with a NaN: above every number's key
 
 // ---- at training: the reference rows in groups --------------------------------------------------
 
@@ -1143,7 +1143,7 @@ __global__ void __launch_bounds__(SCAN_NW * 32, 1) ft_scan_kernel(FtRounds a, in
                 const float v = nan ? __int_as_float(0x7fffffff)
                                     : (float)(((double)N * c.rq) * (1.0 / sqrt((double)nr)));
                 if (valid) a.scores[(size_t)(sblk + ub) * 32 + lane] = v;
-                const uint32_t key = ord_key(v);
+                const uint32_t key = nan ? NAN_KEY : ord_key(v);
                 const uint32_t mn = __reduce_min_sync(FULL, valid ? key : 0xffffffffu);
                 const uint32_t mx = __reduce_max_sync(FULL, valid ? key : 0u);
                 if (lane == 0) {
@@ -1377,7 +1377,7 @@ __global__ void __launch_bounds__(256) ft_scan32_kernel(FtRounds a, int k, int d
             const float div = sqrtf(qf * rf);
             const float v = div != 0.f ? s / div : __int_as_float(0x7fffffff);  // lane 0's counts
             if (lane == 0) a.scores[out + (r - off[lab])] = v;
-            const uint32_t key = ord_key(v);
+            const uint32_t key = div != 0.f ? ord_key(v) : NAN_KEY;
             kmin = min(kmin, key);
             kmax = max(kmax, key);
             __syncwarp();

@@ -94,3 +94,25 @@ def test_label_sizes_around_blocks(mode):
     flags, final, rounds = _solve(prob, mode=0 if mode == abi.MODE_FP32REF else 1)
     got, got_rounds = _annotator(prob, mode).finetune(qry, flags)
     assert np.array_equal(got, final) and np.array_equal(got_rounds, rounds)
+
+
+@pytest.mark.parametrize("mode", [abi.MODE_EXACT, abi.MODE_FP32REF])
+@pytest.mark.parametrize("n", [40, 120, 400])
+def test_score_lists_with_nan(n, mode):
+    """Empty reference rows make NaN-bearing lists in every round, constant and empty query rows lists of NaN alone:
+    cells scanned one by one, in quads, and with work lists."""
+    ref, qry, L = H.dataset("tiny")
+    keep = np.ones(len(ref.indices), bool)
+    for i in (0, 1, 50, 51, 52, 300):
+        keep[ref.indptr[i]:ref.indptr[i + 1]] = False
+    ptr = np.concatenate([[0], np.cumsum(keep)])[ref.indptr].astype(np.int32)
+    r = synth.CSR(ref.n_rows, ref.n_cols, ref.data[keep], ref.indices[keep], ptr, ref.labels)
+    q = qry.take(np.arange(40))
+    q.data[q.indptr[5]:q.indptr[6]] = 1.0
+    genes = synth.names("G", ref.n_cols)
+    prob = O.Problem(r, q, synth.names("CT", L), ref.labels, genes, genes)
+    flags, final, rounds = _solve(prob, WIDE, mode=0 if mode == abi.MODE_FP32REF else 1)
+    assert (flags.sum(1) >= 2).sum() >= 30
+    at = np.random.default_rng(n).permutation(n) * 3 % 40
+    got, got_rounds = _annotator(prob, mode).finetune(q.take(at), flags[at], thre=WIDE)
+    assert np.array_equal(got, final[at]) and np.array_equal(got_rounds, rounds[at])
