@@ -96,6 +96,34 @@ def test_label_sizes_around_blocks(mode):
     assert np.array_equal(got, final) and np.array_equal(got_rounds, rounds)
 
 
+@pytest.mark.parametrize("kind", list(POOLS))
+@pytest.mark.parametrize("scan", [1, 2])
+@pytest.mark.parametrize("times", [2, 7])
+def test_table_copies_in_quads(kind, scan, times):
+    """Each table width with four cells to a pass: 80 cells (more than are scanned one by one), and 280, from which
+    on a label that one cell of a quad needs goes to the label's work list."""
+    prob, (flags, final, rounds) = _pool(kind)
+    a = _annotator(prob)
+    a.set_tuning(3, scan)
+    got, got_rounds = a.finetune(prob.qry.take(np.tile(np.arange(40), times)), np.tile(flags, (times, 1)), thre=WIDE)
+    assert (flags.sum(1) >= 2).sum() * times > 64
+    assert np.array_equal(got, np.tile(final, times)) and np.array_equal(got_rounds, np.tile(rounds, times))
+
+
+@pytest.mark.parametrize("mode", [abi.MODE_EXACT, abi.MODE_FP32REF])
+@pytest.mark.parametrize("n", [63, 64, 65, 66, 67, 68, 69, 255, 256, 257, 300, 2047, 4097])
+def test_cell_counts_past_the_direct_form(n, mode):
+    """Around the most cells that are scanned one by one (64), quads that are not full, 64 quads (work lists from there
+    on), 512 quads (items sized by the round) and 4,096 cells (ordered by counting from there on); the cells in an
+    order of their own."""
+    prob = H.problem("families")
+    res = H.oracle_run("families", 0 if mode == abi.MODE_FP32REF else 1)
+    assert (res["flags"].sum(1) >= 2).all()
+    at = np.random.default_rng(n).permutation(n) * 7 % prob.qry.n_rows
+    got, rounds = _annotator(prob, mode).finetune(prob.qry.take(at), res["flags"][at].astype(np.uint8))
+    assert np.array_equal(got, res["final"][at]) and np.array_equal(rounds, res["rounds"][at])
+
+
 @pytest.mark.parametrize("mode", [abi.MODE_EXACT, abi.MODE_FP32REF])
 @pytest.mark.parametrize("n", [40, 120, 400])
 def test_score_lists_with_nan(n, mode):
