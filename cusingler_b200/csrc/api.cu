@@ -1395,6 +1395,11 @@ void ensure_ref_runs(sgr_ctx* ctx) {
     ctx->fr_ref_runs_ready = true;
 }
 
+// No cell runs more rounds than this.  A round whose first candidate has a number as its score drops one at least
+// (the smallest score).  One with a NaN there may drop none, but then puts a candidate with a number first, and the
+// next round has the same candidates, the same genes and the same scores.
+int most_rounds(uint32_t L) { return 2 * (int)L; }
+
 // The buffers of a batch of nb cells with nblk score blocks, set in `a`; returns the ordering's scan scratch.
 int32_t* round_buffers(sgr_ctx* ctx, FtRounds& a, int64_t nb, int64_t nblk) {
     const size_t n = (size_t)nb, L = (size_t)a.L, row_words = n * a.row_stride;
@@ -1560,10 +1565,9 @@ bool finetune_rounds(sgr_ctx* ctx, const DevCsr& q, const uint8_t* flags_dev, fl
         launch_ft_rows(a.cells, a.n_cells, q.data, q.indices, q.indptr, q.n_cols, ctx->qry_map_thre.p, (int)Wt, a.row_stride,
                        a.s_gene, a.s_lo, a.s_hi, a.row_len, &d->read.longest, fp32, s);
         bool x64 = ctx->pack_scan != 2 || !narrow(Wt);
-        // each round drops at least one candidate, so L rounds finish every cell
         int most = a.n_cells;  // no more cells than this are active
         for (int r = 0;; ++r) {
-            if (r > (int)L + 2) fail(SGR_ERR_STATE, "fine-tune rounds did not converge");
+            if (r > most_rounds(L) + 1) fail(SGR_ERR_STATE, "fine-tune rounds did not converge");
             launch_ft_step(a, r, most, !fp32, scan_scratch, s);
             SGR_CUDA(cudaMemcpyAsync(&ctx->h_ft[r & 1], &d->read, sizeof(FtRead), cudaMemcpyDeviceToHost, s));
             SGR_CUDA(cudaEventRecord(ctx->ev_ft[r & 1], s));
@@ -1820,8 +1824,7 @@ void finetune_persistent(sgr_ctx* ctx, const DevCsr& q, const uint8_t* flags_dev
         cudaGetLastError();
         // Launches are pipelined: launch k + 1 is queued before the cells' states after launch k are
         // read (copied asynchronously into pinned memory), so the device never waits for the host;
-        // the launch queued after the last cell finished runs rounds that do nothing.  Each round
-        // drops at least one candidate, so L + 2 rounds finish every cell.
+        // the launch queued after the last cell finished runs rounds that do nothing.
         uint32_t rounds_run = 0, rounds_at[2] = {0, 0};
         for (int launched = 0;; ++launched) {
             if (exec) {
@@ -1848,7 +1851,7 @@ void finetune_persistent(sgr_ctx* ctx, const DevCsr& q, const uint8_t* flags_dev
             bool all = true;
             for (int i = 0; i < H; ++i) all &= state[i] == 2;
             if (all) break;
-            if (rounds_at[prev] > L + 3) {
+            if (rounds_at[prev] > (uint32_t)most_rounds(L) + 1) {
                 if (exec) cudaGraphExecDestroy(exec);
                 fail(SGR_ERR_STATE, "fine-tune split path did not converge");
             }

@@ -30,7 +30,7 @@
 //
 // Measured (B200, 20,000 reference cells in 30 labels, 100,000 queries of which 48,412 take 117,724 rounds,
 // 1.3e9 row correlations of 304 entries): fine-tune 319 -> 98 ms against the per-cell kernels of
-// finetune.cu, of it the scan 89 ms (68 ps a correlation; shared-memory pipe 77 % busy, issue 71 %).
+// finetune.cu, of it the scan 89 ms (68 ps a correlation; shared-memory pipe 77 % busy, issue 69 %).
 // Scanning per label instead of per quad left a third of the warps waiting at the table's barriers
 // (82 ps); 12, 24 and 32 warps per CTA were 2 % slower, no different and 9 % slower than 16.
 

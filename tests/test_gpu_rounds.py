@@ -144,3 +144,25 @@ def test_score_lists_with_nan(n, mode):
     at = np.random.default_rng(n).permutation(n) * 3 % 40
     got, got_rounds = _annotator(prob, mode).finetune(q.take(at), flags[at], thre=WIDE)
     assert np.array_equal(got, final[at]) and np.array_equal(got_rounds, rounds[at])
+
+
+@pytest.mark.parametrize("mode", [abi.MODE_EXACT, abi.MODE_FP32REF])
+@pytest.mark.parametrize("scan", [0, 2])
+def test_rounds_that_drop_no_candidate(scan, mode):
+    """A NaN score of the first candidate lets a round drop none, so a cell can take more rounds than it has labels."""
+    ref, qry, L = H.dataset("families")
+    keep = np.ones(len(ref.indices), bool)
+    for i in np.flatnonzero(np.random.default_rng(2).random(ref.n_rows) < 0.03):
+        keep[ref.indptr[i]:ref.indptr[i + 1]] = False
+    ptr = np.concatenate([[0], np.cumsum(keep)])[ref.indptr].astype(np.int32)
+    r = synth.CSR(ref.n_rows, ref.n_cols, ref.data[keep], ref.indices[keep], ptr, ref.labels)
+    genes = synth.names("G", ref.n_cols)
+    prob = O.Problem(r, qry.rows(0, 150), synth.names("CT", L), ref.labels, genes, genes)
+    flags, final, rounds = _solve(prob, 1e9, mode=0 if mode == abi.MODE_FP32REF else 1)
+    assert rounds.max() >= L + 2
+    a = _annotator(prob, mode)
+    a.set_tuning(3, scan)
+    for heavy in (2, 1 << 30):
+        a.set_tuning(1, heavy)
+        got, got_rounds = a.finetune(prob.qry, flags, thre=1e9)
+        assert np.array_equal(got, final) and np.array_equal(got_rounds, rounds)
