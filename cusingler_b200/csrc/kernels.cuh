@@ -328,7 +328,6 @@ struct FtRounds {
     const int32_t* lorder;      // labels, longest first
     const uint16_t *ref_gene, *ref_lo, *ref_hi;  // FP32 order: entries by value, with their runs (CSR order)
     const int32_t* ref_ptr;
-    const int* ref_nan;         // FP32 order: not 0 where some reference row holds a NaN (marked in ref_gene)
     const uint32_t* ft_genes;   // fine-tune pair lists (pool ids)
     const uint32_t* ft_idx;     // (start, len) per ordered pair
     const uint32_t* pair_mask;  // bits of each pair's whole list (nwords each), or nullptr
@@ -371,6 +370,7 @@ struct FtRounds {
     int max_label;
     int32_t *final_labels, *rounds;
     int* status;
+    const int* ref_nan;         // FP32 order: not 0 where some reference row holds a NaN (marked in ref_gene)
 };
 
 // Copies of the scan's lookup table that fit shared memory for a pool of Wt genes (8, 4, 2, 1; 0: none).
