@@ -214,7 +214,7 @@ struct sgr_ctx {
     DevBuf<unsigned long long> fr_ctl;  // counters (FtCtl)
     DevBuf<float> fr_scores, fr_nan;
     DevBuf<uint16_t> fr_ref_runs;  // FP32 order: the reference's entries by value, with their runs
-    DevBuf<int> fr_ref_nan;        // whether some of them are NaN
+    bool fr_ref_nan = false;       // whether some of them are NaN
     size_t fr_ref_runs_stride = 0;
     bool fr_ref_runs_ready = false;
     // gives the buffers sized by a batch back; whether there were any
@@ -1389,9 +1389,14 @@ void ensure_ref_runs(sgr_ctx* ctx) {
     if (ctx->fr_ref_runs_ready) return;
     const size_t n = ctx->fr_ref_runs_stride = std::max<size_t>(ctx->reff_indices.n, 1);
     uint16_t* r = ctx->fr_ref_runs.ensure(3 * n);
-    SGR_CUDA(cudaMemsetAsync(ctx->fr_ref_nan.ensure(1), 0, sizeof(int), ctx->stream));
+    DevBuf<int> any;
+    int nan = 0;
+    SGR_CUDA(cudaMemsetAsync(any.ensure(1), 0, sizeof(int), ctx->stream));
     launch_ft_sort_rows((int)ctx->R, ctx->reff_data.p, ctx->reff_indices.p, ctx->reff_indptr.p, ctx->max_row, r,
-                        r + n, r + 2 * n, ctx->fr_ref_nan.p, ctx->stream);
+                        r + n, r + 2 * n, any.p, ctx->stream);
+    SGR_CUDA(cudaMemcpyAsync(&nan, any.p, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+    SGR_CUDA(cudaStreamSynchronize(ctx->stream));
+    ctx->fr_ref_nan = nan != 0;
     ctx->fr_ref_runs_ready = true;
 }
 
@@ -1483,7 +1488,6 @@ bool finetune_rounds(sgr_ctx* ctx, const DevCsr& q, const uint8_t* flags_dev, fl
         a.ref_lo = a.ref_gene + n;
         a.ref_hi = a.ref_lo + n;
         a.ref_ptr = ctx->reff_indptr.p;
-        a.ref_nan = ctx->fr_ref_nan.p;
     }
     a.ft_genes = ctx->d_ft_genes.p;
     a.ft_idx = ctx->d_ft_idx.p;
@@ -1575,7 +1579,7 @@ bool finetune_rounds(sgr_ctx* ctx, const DevCsr& q, const uint8_t* flags_dev, fl
                 SGR_CUDA(cudaEventSynchronize(ctx->ev_ft[0]));
                 x64 = !narrow(ctx->h_ft[0].longest);
             }
-            if (fp32) launch_ft_scan32(a, r, most, s);
+            if (fp32) launch_ft_scan32(a, r, most, ctx->fr_ref_nan, s);
             else launch_ft_scan(a, r, most, ctx->ft_copies, x64, s);
             if (r == 0) continue;
             SGR_CUDA(cudaEventSynchronize(ctx->ev_ft[(r - 1) & 1]));

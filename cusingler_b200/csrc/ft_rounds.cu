@@ -1182,6 +1182,8 @@ __device__ __forceinline__ float tree128(const float (&c)[4], int lane) {
 // rows, 32 places and a row's genes and runs read at once.
 // dense_len: floats of a dense row (128 x the longest chunk).  dynamic shared memory: the query's dense
 // row, one per warp, the slot of each pool gene (halfwords).
+// NANS: some reference row holds a NaN, and the rows' genes may be marked.
+template <bool NANS>
 __global__ void __launch_bounds__(256) ft_scan32_kernel(FtRounds a, int k, int dense_len, int parts) {
     extern __shared__ __align__(16) unsigned char dyn[];
     __shared__ int off[257];  // candidate rows before each label of the cell's list
@@ -1199,7 +1201,6 @@ __global__ void __launch_bounds__(256) ft_scan32_kernel(FtRounds a, int k, int d
     }
     const int n = a.n_act[nxt];
     const uint32_t low = (1u << a.shift) - 1u;
-    const bool nan_rows = *a.ref_nan != 0;
     for (;;) {
         __syncthreads();
         if (tid == 0) s_item = atomicAdd(a.queue + cur, 1);
@@ -1304,7 +1305,8 @@ __global__ void __launch_bounds__(256) ft_scan32_kernel(FtRounds a, int k, int d
             }
             const int beg = __shfl_sync(FULL, my_beg, (r - w0) & 31), len = __shfl_sync(FULL, my_len, (r - w0) & 31);
             const int nwd = (len + 31) / 32;
-            if (nan_rows) {  // somewhere in the reference: a NaN inside the gene set is refused
+            constexpr uint32_t ref_gene = NANS ? GENE : 0xffffu;
+            if (NANS) {  // a NaN inside the gene set is refused
                 bool bad = false;
                 for (int e = lane; e < len; e += 32) {
                     const uint32_t g = a.ref_gene[beg + e];
@@ -1324,13 +1326,13 @@ __global__ void __launch_bounds__(256) ft_scan32_kernel(FtRounds a, int k, int d
             }
 #pragma unroll
             for (int w = 0; w < HELD; ++w) {
-                sl[w] = sl[w] != 0xffffffffu ? slot[sl[w] & GENE] : 0xffffu;
+                sl[w] = sl[w] != 0xffffffffu ? slot[sl[w] & ref_gene] : 0xffffu;
                 const unsigned m = __ballot_sync(FULL, sl[w] != 0xffffu);
                 if (lane == w) in = m;
             }
             for (int w = HELD; w < nwd; ++w) {
                 const int e = 32 * w + lane;
-                const bool hit = e < len && slot[a.ref_gene[beg + e] & GENE] != 0xffffu;
+                const bool hit = e < len && slot[a.ref_gene[beg + e] & ref_gene] != 0xffffu;
                 const unsigned m = __ballot_sync(FULL, hit);
                 if (lane == w) in = m;
             }
@@ -1357,7 +1359,7 @@ __global__ void __launch_bounds__(256) ft_scan32_kernel(FtRounds a, int k, int d
             for (int w = HELD; w < nwd; ++w) {
                 const int e = 32 * w + lane;
                 const bool hit = e < len;
-                place(hit ? slot[a.ref_gene[beg + e] & GENE] : 0xffffu, hit ? a.ref_lo[beg + e] : 0,
+                place(hit ? slot[a.ref_gene[beg + e] & ref_gene] : 0xffffu, hit ? a.ref_lo[beg + e] : 0,
                       hit ? a.ref_hi[beg + e] : 0);
             }
             __syncwarp();
@@ -1554,16 +1556,17 @@ int ft_scan32_warps(int Wt) {
     return 0;
 }
 
-void launch_ft_scan32(const FtRounds& a, int k, int n, cudaStream_t s) {
+void launch_ft_scan32(const FtRounds& a, int k, int n, bool nans, cudaStream_t s) {
     const int warps = ft_scan32_warps(a.Wt);
     const size_t smem = scan32_smem(a.Wt, warps);
-    allow_smem(ft_scan32_kernel, kScan32Smem);
+    auto kern = nans ? ft_scan32_kernel<true> : ft_scan32_kernel<false>;
+    allow_smem(kern, kScan32Smem);
     int per_sm = 0;
-    SGR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, ft_scan32_kernel, 32 * warps, smem));
+    SGR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * warps, smem));
     const int grid = device_sm_count() * std::max(1, per_sm);
     // about eight items per CTA, so that the last ones do not leave the GPU idle
     const int parts = std::max(1, (8 * grid + n - 1) / std::max(n, 1));
-    ft_scan32_kernel<<<grid, 32 * warps, smem, s>>>(a, k, dense_len_of(a.Wt), parts);
+    kern<<<grid, 32 * warps, smem, s>>>(a, k, dense_len_of(a.Wt), parts);
     SGR_LAUNCH_CHECK();
     count_launch();
 }

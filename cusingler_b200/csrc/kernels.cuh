@@ -370,7 +370,6 @@ struct FtRounds {
     int max_label;
     int32_t *final_labels, *rounds;
     int* status;
-    const int* ref_nan;         // FP32 order: not 0 where some reference row holds a NaN (marked in ref_gene)
 };
 
 // Copies of the scan's lookup table that fit shared memory for a pool of Wt genes (8, 4, 2, 1; 0: none).
@@ -403,8 +402,9 @@ void ft_rounds_setup(int copies);
 // Step k over at most n cells and (quads) the quads of round k.  scan_scratch: launch_exclusive_scan's, 2^20 values.
 void launch_ft_step(const FtRounds& a, int k, int n, bool quads, int32_t* scan_scratch, cudaStream_t s);
 // Round k's correlations in the reference's FP32 order.  ft_scan32_warps: 0 for a pool too wide for it.
+// nans: some reference row holds a NaN (launch_ft_sort_rows).
 int ft_scan32_warps(int Wt);
-void launch_ft_scan32(const FtRounds& a, int k, int n, cudaStream_t s);
+void launch_ft_scan32(const FtRounds& a, int k, int n, bool nans, cudaStream_t s);
 // x64: the run sums in 64 bits (when 32 could overflow)
 void launch_ft_scan(const FtRounds& a, int k, int n, int copies, bool x64, cudaStream_t s);
 
