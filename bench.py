@@ -54,13 +54,12 @@ FALLBACK_BF16_TFLOPS = 1590.0
 NEAR_TIE = 1e-5
 
 # DRAM bytes per query row of each score-step kernel, from one ncu capture of the 8,192-query case
-# of the mid workload (profiles/corr_tc_mid_8192q.md, select_first_mid_8192q.md,
-# rank_kernel_mid_8192q.md: read + write); a launch's traffic is this times its query rows (each
-# row's traffic is the same).
+# of the mid workload (profiles/score_step_traffic_mid_8192q.md: read + write); a launch's traffic is
+# this times its query rows (each row's traffic is the same).
 TRAFFIC_PER_QUERY = {
-    "corr": (1.170260e9 + 0.632710e9) / 8192,
-    "select": (0.657572e9 + 4.554752e6) / 8192,
-    "rank": (0.098440e9 + 6.304e6) / 8192,
+    "corr": (0.309528e9 + 0.617947e9) / 8192,
+    "select": (0.697411e9 + 1.121e6 + 0.992e6) / 8192,
+    "rank": (0.098465e9 + 3.346e6) / 8192,
 }
 
 
